@@ -20,12 +20,156 @@ namespace {
 using namespace beam_detail;
 constexpr int kBeamThreads = 256;
 
-__global__ void __launch_bounds__(kBeamThreads) beam_deposit_kernel(const BeamArgs B, double* __restrict__ bsrc) {
+// ---------------------------------------------------------------- warp-wide deposits
+// A particle adds 2 (xi) rows of 2 neighbouring nodes: 2 NC contiguous doubles per row. Added by the
+// particle's own lane, each value is an L2 transaction of its own; here the warp's values go through
+// shared memory and consecutive lanes add consecutive addresses, so that a transaction carries up to four
+// of them: FP64 reductions at random nodes 196 -> 554 G values/s (10 per row), 76 -> 277 G (42 per row).
+// Lanes with the same (row, node) are summed first (in lane order): one addition per cell of the warp,
+// which bounds the serialisation on the few cells of a pinched beam.
+template <int NC>
+struct WarpDep {
+    double val[32][2 * NC + 1];        // odd row length: no bank conflicts between lanes
+    long off[32];                      // offset of the row's first value in bsrc
+    unsigned mask[32];                 // lanes that share it
+    unsigned char lead[32];            // lanes that add, compacted
+    int node[32];
+};
+
+// the values of one particle (src/Beam.cpp:725-785): f[c] times the corner's weight
+template <int NC>
+struct DepOne {
+    int k, j;
+    double d0, tk, t, f[NC];
+};
+
+template <int NC>
+__device__ __forceinline__ bool dep_one(const BeamArgs& B, double X, double Y, double PX, double PY, double PZ,
+                                        double XI, double wi, int jguess, DepOne<NC>& D) {
+    const double r = sqrt(X * X + Y * Y);
+    if (r > B.R) return false;
+    double c = 1.0, s = 0.0;
+    if (r > 0.0) {
+        const Recip ir(r);
+        c = ir(X);
+        s = ir(Y);
+    }
+    const double sx = (XI - B.xi_min) * B.idxi;
+    D.k = B.ngp ? (int)floor(sx + 0.5) : (int)floor(sx);
+    if (D.k < -1 || D.k >= B.K) return false;
+    D.tk = B.ngp ? 0.0 : sx - D.k;
+    const double p2 = PX * PX + PY * PY;
+    const double gam = sqrt(1.0 + p2 + PZ * PZ);
+    const double omvz = (1.0 + p2) / (gam * (gam + PZ));
+    const Recip ig(gam);
+    const double vz = ig(PZ), vx = ig(PX), vy = ig(PY);
+    const double vr = c * vx + s * vy, vt = c * vy - s * vx;
+    D.j = locate_near(B.r, B.N, B.R, r, jguess);
+    const double t = (r - B.r[D.j]) * B.inv_h[D.j];
+    D.t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
+    D.d0 = wi * B.q;
+    D.f[B_RT0] = omvz; D.f[B_JZ0] = vz; D.f[B_JP1R] = vr; D.f[B_JP1I] = vt; D.f[B_RHO0] = 1.0;
+    if constexpr (NC == B_NC1) {
+        const double c2 = c * c - s * s, s2 = 2.0 * c * s;
+        D.f[B_RT1R] = omvz * c; D.f[B_RT1I] = -omvz * s;
+        D.f[B_JZ1R] = vz * c; D.f[B_JZ1I] = -vz * s;
+        D.f[B_RHO1R] = c; D.f[B_RHO1I] = -s;
+        D.f[B_JP0R] = vx; D.f[B_JP0I] = vy;
+        D.f[B_JP2R] = vx * c2 + vy * s2; D.f[B_JP2I] = vy * c2 - vx * s2;
+    }
+    return true;
+}
+
+// every lane of the warp calls it; act: the lane has a particle to deposit
+template <int NC>
+__device__ __forceinline__ void warp_deposit(const BeamArgs& B, double* __restrict__ bsrc, bool act,
+                                             const DepOne<NC>& D, WarpDep<NC>& W) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int a = 0; a < (B.ngp ? 1 : 2); ++a) {
+        const int kk = D.k + a;
+        const bool row = act && kk >= 0 && kk < B.K;
+        const long off = row ? ((long)kk * B.M + D.j) * NC : -1 - lane;
+        const unsigned same = __match_any_sync(FULL, (unsigned long long)off);
+        const bool lead = row && lane == __ffs(same) - 1;
+        const unsigned leads = __ballot_sync(FULL, lead);
+        if (row) {
+            const double Wk = a ? D.tk : 1.0 - D.tk;
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const double d = D.d0 * Wk * (b ? D.t : 1.0 - D.t) * B.inv_V[D.j + b] * B.idxi;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) W.val[lane][b * NC + c] = d * D.f[c];
+            }
+        }
+        if (lead) {
+            W.off[lane] = off;
+            W.mask[lane] = same;
+            W.node[lane] = D.j;
+            W.lead[__popc(leads & ((1u << lane) - 1u))] = (unsigned char)lane;
+        }
+        __syncwarp();
+        const int total = __popc(leads) * 2 * NC;
+        for (int q = lane; q < total; q += 32) {
+            const int sl = q / (2 * NC), w = q - sl * 2 * NC, src = W.lead[sl];
+            double* const o = bsrc + W.off[src] + w;
+            unsigned m = W.mask[src];
+            if (B.fx_scale) {          // exact (m = 0 runs of qz_sim): the limbs are integers, and so are their sums
+                const double sc = B.fx_scale[W.node[src] + (w >= NC ? 1 : 0)];
+                double hi = 0.0, lo = 0.0;
+                for (; m; m &= m - 1) beam_fx_split(W.val[__ffs(m) - 1][w], sc, B.fx_inv2s, B.fx_2s, hi, lo);
+                if (hi != 0.0) atomicAdd(o, hi);
+                if (lo != 0.0) atomicAdd(o + B.fx_lo, lo);
+            } else {
+                double v = 0.0;
+                for (; m; m &= m - 1) v += W.val[__ffs(m) - 1][w];
+                atomicAdd(o, v);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// particles per CTA of the depositing kernels: 8 warps with 5 components, 4 with 15 (their shared scratch)
+template <int NC>
+constexpr int kDepThreads = NC == B_NC0 ? 256 : 128;
+constexpr int kDepNodes = 1024;        // radial nodes kept in shared memory (8 KB); longer grids are searched in L1
+
+template <int NC>
+struct DepSmem {
+    WarpDep<NC> w[kDepThreads<NC> / 32];
+    double r[kDepNodes];
+};
+
+// the CTA's copy of the radial nodes, for the cell searches
+template <int NC>
+__device__ __forceinline__ void dep_nodes(BeamArgs& B, DepSmem<NC>& S) {
+    if (B.M > kDepNodes) return;
+    for (int j = threadIdx.x; j < B.M; j += blockDim.x) S.r[j] = B.r[j];
+    __syncthreads();
+    B.r = S.r;
+}
+
+// Bound by the L2 reductions (2 rows x 2 nodes x NC values per particle). 1e6 particles on 512 x 2400
+// nodes: see warp_deposit for the two ways of adding.
+template <int NC>
+__global__ void __launch_bounds__(kDepThreads<NC>) beam_deposit_kernel(const BeamArgs Bg, double* __restrict__ bsrc) {
+    __shared__ DepSmem<NC> S;
+    BeamArgs B = Bg;
+    dep_nodes(B, S);
+    const int lane = threadIdx.x & 31;
     const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += stride) {
-        const double wi = B.w[i];
-        if (wi == 0.0) continue;
-        deposit_one(B, bsrc, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi);
+    for (long base = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < B.n; base += stride) {
+        const long i = base + lane;
+        DepOne<NC> D;
+        D.k = D.j = 0;
+        bool act = false;
+        if (i < B.n) {
+            const double wi = B.w[i];
+            if (wi != 0.0) act = dep_one<NC>(B, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi, -1, D);
+        }
+        warp_deposit<NC>(B, bsrc, act, D, S.w[threadIdx.x >> 5]);
     }
 }
 
@@ -140,24 +284,51 @@ __global__ void __launch_bounds__(kBeamThreads) slice_sums_kernel(const BeamArgs
     }
 }
 
-template <bool kDeposit>
-__global__ void __launch_bounds__(kBeamThreads) beam_push_kernel(const BeamArgs B, const double* __restrict__ fld,
-                                                                 double dt_kick, double dt, int move,
-                                                                 double* __restrict__ bsrc_next) {
-    const double qm = B.q / B.m;
+// the particle columns after one step of Beam::advance; false when the particle was removed
+struct Moved {
+    double x, y, px, py, pz, xi;
+    int j;                             // radial cell before the move
+    bool live;
+};
+template <bool kVec>
+__device__ __forceinline__ Moved move_one(const BeamArgs& B, const double* __restrict__ fld, long i, double h,
+                                          double dt) {
+    const double X = B.x[i], Y = B.y[i], XI = B.xi[i];
+    double c, sn;
+    V3 E, Bf;
+    Moved m;
+    gather<false, kVec>(B, fld, X, Y, XI, c, sn, E, Bf, &m.j);
+    V3 u = {B.px[i], B.py[i], B.pz[i]};
+    u = B.pusher ? push_u(B.pusher, u, E, Bf, h) : vay(u, E, Bf, h);
+    const double p2 = u.x * u.x + u.y * u.y;
+    const double gam = sqrt(1.0 + p2 + u.z * u.z);
+    const double omvz = (1.0 + p2) / (gam * (gam + u.z));
+    const Recip ig(gam);
+    m.x = X + ig(u.x) * dt;
+    m.y = Y + ig(u.y) * dt;
+    m.xi = XI + omvz * dt;
+    m.px = u.x; m.py = u.y; m.pz = u.z;
+    B.x[i] = m.x; B.y[i] = m.y;
+    B.px[i] = u.x; B.py[i] = u.y; B.pz[i] = u.z;
+    B.xi[i] = m.xi;
     const double xmin = B.xi_min, xmax = B.xi_min + (B.K - 1) * B.dxi;
-    const double R = B.R;
+    m.live = !(m.x * m.x + m.y * m.y >= B.R * B.R || m.xi < xmin || m.xi > xmax);
+    if (!m.live) B.w[i] = 0.0;
+    return m;
+}
+
+template <bool kVec>
+__global__ void __launch_bounds__(kBeamThreads) beam_push_kernel(const BeamArgs B, const double* __restrict__ fld,
+                                                                 double dt_kick, double dt, int move) {
+    const double h = 0.5 * (B.q / B.m) * dt_kick;
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += stride) {
-        const double wi = B.w[i];
-        if (wi == 0.0) continue;
-        const double X = B.x[i], Y = B.y[i], XI = B.xi[i];
-        double c, sn;
-        V3 E, Bf;
-        gather<false>(B, fld, X, Y, XI, c, sn, E, Bf);
-        V3 u = {B.px[i], B.py[i], B.pz[i]};
-        const double h = 0.5 * qm * dt_kick;
+        if (B.w[i] == 0.0) continue;
         if (!move) {                 // leapfrog start-up: explicit kick (src/Beam.cpp:1038-1044)
+            double c, sn;
+            V3 E, Bf;
+            gather<false, kVec>(B, fld, B.x[i], B.y[i], B.xi[i], c, sn, E, Bf);
+            V3 u = {B.px[i], B.py[i], B.pz[i]};
             const double g0 = sqrt(1.0 + dot3(u, u));
             const double ig = 1.0 / g0;
             const V3 v = {ig * u.x, ig * u.y, ig * u.z};
@@ -167,18 +338,35 @@ __global__ void __launch_bounds__(kBeamThreads) beam_push_kernel(const BeamArgs 
             B.px[i] = u.x; B.py[i] = u.y; B.pz[i] = u.z;
             continue;
         }
-        u = B.pusher ? push_u(B.pusher, u, E, Bf, h) : vay(u, E, Bf, h);
-        const double p2 = u.x * u.x + u.y * u.y;
-        const double gam = sqrt(1.0 + p2 + u.z * u.z);
-        const double omvz = (1.0 + p2) / (gam * (gam + u.z));
-        const double xn = X + u.x / gam * dt, yn = Y + u.y / gam * dt;
-        const double xin = XI + omvz * dt;
-        B.x[i] = xn; B.y[i] = yn;
-        B.px[i] = u.x; B.py[i] = u.y; B.pz[i] = u.z;
-        B.xi[i] = xin;
-        double wn = wi;
-        if (xn * xn + yn * yn >= R * R || xin < xmin || xin > xmax) { wn = 0.0; B.w[i] = 0.0; }
-        if (kDeposit && wn != 0.0) deposit_one(B, bsrc_next, xn, yn, u.x, u.y, u.z, xin, wn);
+        move_one<kVec>(B, fld, i, h, dt);
+    }
+}
+
+// the push and the deposit of the moved particles (one pass over the particles)
+template <int NC, bool kVec>
+__global__ void __launch_bounds__(kDepThreads<NC>) beam_push_deposit_kernel(const BeamArgs Bg,
+                                                                            const double* __restrict__ fld,
+                                                                            double dt_kick, double dt,
+                                                                            double* __restrict__ bsrc_next) {
+    __shared__ DepSmem<NC> S;
+    BeamArgs B = Bg;
+    dep_nodes(B, S);
+    const int lane = threadIdx.x & 31;
+    const double h = 0.5 * (B.q / B.m) * dt_kick;
+    const long stride = (long)gridDim.x * blockDim.x;
+    for (long base = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < B.n; base += stride) {
+        const long i = base + lane;
+        DepOne<NC> D;
+        D.k = D.j = 0;
+        bool act = false;
+        if (i < B.n) {
+            const double wi = B.w[i];
+            if (wi != 0.0) {
+                const Moved m = move_one<kVec>(B, fld, i, h, dt);
+                act = m.live && dep_one<NC>(B, m.x, m.y, m.px, m.py, m.pz, m.xi, wi, m.j, D);
+            }
+        }
+        warp_deposit<NC>(B, bsrc_next, act, D, S.w[threadIdx.x >> 5]);
     }
 }
 
@@ -237,6 +425,15 @@ int grid_for(long n) {
     return (int)b;
 }
 
+// CTAs of a depositing kernel: as many as fit (at most 8 of 256 threads per SM)
+template <int NC>
+int grid_dep(long n) {
+    const long b = (n + kDepThreads<NC> - 1) / kDepThreads<NC>, cap = 148L * 8 * 256 / kDepThreads<NC>;
+    return (int)(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 }  // namespace
 
 int beam_sums_blocks(long n) {
@@ -248,7 +445,8 @@ int beam_sums_blocks(long n) {
 
 cudaError_t launch_beam_deposit(const BeamArgs& B, double* bsrc, cudaStream_t s) {
     if (B.n <= 0) return cudaSuccess;
-    beam_deposit_kernel<<<grid_for(B.n), kBeamThreads, 0, s>>>(B, bsrc);
+    if (B.modes) beam_deposit_kernel<B_NC1><<<grid_dep<B_NC1>(B.n), kDepThreads<B_NC1>, 0, s>>>(B, bsrc);
+    else beam_deposit_kernel<B_NC0><<<grid_dep<B_NC0>(B.n), kDepThreads<B_NC0>, 0, s>>>(B, bsrc);
     return cudaGetLastError();
 }
 
@@ -274,15 +472,30 @@ cudaError_t launch_deposit_analytic(const AnalyticArgs& P, double* bsrc, cudaStr
 cudaError_t launch_beam_push(const BeamArgs& B, const double* fld, double dt_kick, double dt_drift, int move,
                              cudaStream_t s) {
     if (B.n <= 0) return cudaSuccess;
-    beam_push_kernel<false><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, fld, dt_kick, dt_drift, move, nullptr);
+    // two components per load when the caller's field store starts on a 16-byte boundary
+    if (aligned16(fld)) beam_push_kernel<true><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, fld, dt_kick, dt_drift, move);
+    else beam_push_kernel<false><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, fld, dt_kick, dt_drift, move);
     return cudaGetLastError();
 }
+
+namespace {
+template <int NC>
+cudaError_t push_deposit(const BeamArgs& B, const double* fld, double dt_kick, double dt_drift, double* bsrc_next,
+                         cudaStream_t s) {
+    const int grid = grid_dep<NC>(B.n);
+    if (aligned16(fld))
+        beam_push_deposit_kernel<NC, true><<<grid, kDepThreads<NC>, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
+    else
+        beam_push_deposit_kernel<NC, false><<<grid, kDepThreads<NC>, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
+    return cudaGetLastError();
+}
+}  // namespace
 
 cudaError_t launch_beam_push_deposit(const BeamArgs& B, const double* fld, double dt_kick, double dt_drift,
                                      double* bsrc_next, cudaStream_t s) {
     if (B.n <= 0) return cudaSuccess;
-    beam_push_kernel<true><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, fld, dt_kick, dt_drift, 1, bsrc_next);
-    return cudaGetLastError();
+    return B.modes ? push_deposit<B_NC1>(B, fld, dt_kick, dt_drift, bsrc_next, s)
+                   : push_deposit<B_NC0>(B, fld, dt_kick, dt_drift, bsrc_next, s);
 }
 
 cudaError_t launch_beam_sums(const BeamArgs& B, double gref, double xiref, double* partial, int nblocks,

@@ -13,6 +13,16 @@ namespace beam_detail {
 // kL2: the data was written by other SMs during the same launch, so it is read from L2 (ld.global.cg)
 template <bool kL2>
 __device__ __forceinline__ double fload(const double* p) { return kL2 ? __ldcg(p) : *p; }
+// two neighbouring doubles: one 16-byte load when the address allows it (kVec)
+template <bool kL2, bool kVec>
+__device__ __forceinline__ double2 fload2(const double* p) {
+    if constexpr (kVec) {
+        const double2* q = reinterpret_cast<const double2*>(p);
+        return kL2 ? __ldcg(q) : *q;
+    } else {
+        return make_double2(fload<kL2>(p), fload<kL2>(p + 1));
+    }
+}
 
 __device__ __forceinline__ void deposit_one(const BeamArgs& B, double* __restrict__ bsrc, double X, double Y,
                                             double PX, double PY, double PZ, double XI, double wi) {
@@ -204,13 +214,19 @@ __device__ __forceinline__ void deposit_add1(const BeamArgs& B, double* __restri
     for (int c = 0; c < kDep1; ++c) atomicAdd(o + comp[c], v[c]);
 }
 
-// bilinear (xi, r) gather and mode sums at the particle (src/Beam.cpp:972-1008)
-template <bool kL2>
+// bilinear (xi, r) gather and mode sums at the particle (src/Beam.cpp:972-1008). kVec: fld starts on a
+// 16-byte boundary (its rows of 6 or 18 doubles then do too), so the components are read two at a time
+template <bool kL2, bool kVec = false>
 __device__ __forceinline__ void gather(const BeamArgs& B, const double* __restrict__ fld, double X, double Y,
                                        double XI, double& c, double& sn, V3& E, V3& Bf, int* jcell = nullptr) {
     const double r = sqrt(X * X + Y * Y);
-    c = r > 0.0 ? X / r : 1.0;
-    sn = r > 0.0 ? Y / r : 0.0;
+    c = 1.0;
+    sn = 0.0;
+    if (r > 0.0) {
+        const Recip ir(r);
+        c = ir(X);
+        sn = ir(Y);
+    }
     double s = (XI - B.xi_min) * B.idxi;
     const int nloc = B.K;
     int k;
@@ -235,39 +251,39 @@ __device__ __forceinline__ void gather(const BeamArgs& B, const double* __restri
     const double* f01 = f00 + nc;
     const double* f10 = fld + ((size_t)k1 * B.M + j) * nc;
     const double* f11 = f10 + nc;
-    auto bil = [&](int comp) {
-        return (1.0 - tk) * ((1.0 - t) * fload<kL2>(f00 + comp) + t * fload<kL2>(f01 + comp)) +
-               tk * ((1.0 - t) * fload<kL2>(f10 + comp) + t * fload<kL2>(f11 + comp));
+    // components comp and comp + 1 (comp even): a complex field component, or E_z and B_z
+    auto bil = [&](int comp, double& u, double& v) {
+        const double2 a = fload2<kL2, kVec>(f00 + comp), b = fload2<kL2, kVec>(f01 + comp);
+        const double2 d = fload2<kL2, kVec>(f10 + comp), e = fload2<kL2, kVec>(f11 + comp);
+        u = (1.0 - tk) * ((1.0 - t) * a.x + t * b.x) + tk * ((1.0 - t) * d.x + t * e.x);
+        v = (1.0 - tk) * ((1.0 - t) * a.y + t * b.y) + tk * ((1.0 - t) * d.y + t * e.y);
     };
+    double er, ei, br, bi, ez, bz;
+    bil(F_EP1R, er, ei);
+    bil(F_BP1R, br, bi);
+    bil(F_EZ0, ez, bz);
+    E.x = er * c - ei * sn;
+    E.y = er * sn + ei * c;
+    Bf.x = br * c - bi * sn;
+    Bf.y = br * sn + bi * c;
+    E.z = ez;
+    Bf.z = bz;
     if (B.modes) {
         // eval_vector / eval_scalar with m = 1 (src/SliceData.hpp:70-83)
         const double c2 = c * c - sn * sn, s2 = 2.0 * c * sn;
-        {
-            const double r0 = bil(F_EP0R), i0 = bil(F_EP0I), r1 = bil(F_EP1R), i1 = bil(F_EP1I);
-            const double r2 = bil(F_EP2R), i2 = bil(F_EP2I);
-            E.x = r1 * c - i1 * sn;
-            E.y = r1 * sn + i1 * c;
-            E.x += r0 + r2 * c2 - i2 * s2;
-            E.y += i0 + r2 * s2 + i2 * c2;
-        }
-        {
-            const double r0 = bil(F_BP0R), i0 = bil(F_BP0I), r1 = bil(F_BP1R), i1 = bil(F_BP1I);
-            const double r2 = bil(F_BP2R), i2 = bil(F_BP2I);
-            Bf.x = r1 * c - i1 * sn;
-            Bf.y = r1 * sn + i1 * c;
-            Bf.x += r0 + r2 * c2 - i2 * s2;
-            Bf.y += i0 + r2 * s2 + i2 * c2;
-        }
-        E.z = bil(F_EZ0) + 2.0 * (bil(F_EZ1R) * c - bil(F_EZ1I) * sn);
-        Bf.z = bil(F_BZ0) + 2.0 * (bil(F_BZ1R) * c - bil(F_BZ1I) * sn);
-    } else {
-        const double er = bil(F_EP1R), ei = bil(F_EP1I), br = bil(F_BP1R), bi = bil(F_BP1I);
-        E.x = er * c - ei * sn;
-        E.y = er * sn + ei * c;
-        Bf.x = br * c - bi * sn;
-        Bf.y = br * sn + bi * c;
-        E.z = bil(F_EZ0);
-        Bf.z = bil(F_BZ0);
+        double r0, i0, r2, i2;
+        bil(F_EP0R, r0, i0);
+        bil(F_EP2R, r2, i2);
+        E.x += r0 + r2 * c2 - i2 * s2;
+        E.y += i0 + r2 * s2 + i2 * c2;
+        bil(F_BP0R, r0, i0);
+        bil(F_BP2R, r2, i2);
+        Bf.x += r0 + r2 * c2 - i2 * s2;
+        Bf.y += i0 + r2 * s2 + i2 * c2;
+        bil(F_EZ1R, r0, i0);
+        E.z += 2.0 * (r0 * c - i0 * sn);
+        bil(F_BZ1R, r0, i0);
+        Bf.z += 2.0 * (r0 * c - i0 * sn);
     }
 }
 
