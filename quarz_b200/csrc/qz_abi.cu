@@ -56,10 +56,11 @@ struct qz_grid {
     std::vector<double> gm, g0, gp, ir;
     std::vector<double> consts;  // per-node constants of the sweep (13 x M)
     std::vector<double> consts1; // and of the modes = 1 sweep (9 x M)
+    std::vector<double> consts0; // the arrays the modes = 0 sweep reads (9 x M)
     // device
-    double *d_r = nullptr, *d_inv_h = nullptr, *d_inv_V = nullptr, *d_consts = nullptr, *d_consts1 = nullptr;
+    double *d_r = nullptr, *d_inv_h = nullptr, *d_inv_V = nullptr, *d_consts = nullptr, *d_consts1 = nullptr, *d_consts0 = nullptr;
     ~qz_grid() {
-        for (double* p : {d_r, d_inv_h, d_inv_V, d_consts, d_consts1})
+        for (double* p : {d_r, d_inv_h, d_inv_V, d_consts, d_consts1, d_consts0})
             if (p) cudaFree(p);
     }
 };
@@ -182,6 +183,14 @@ extern "C" qz_status qz_grid_create(const double* nodes, int M, qz_grid** out) {
         put(7, g->opa[1]); put(8, g->opb[1]); put(9, g->opc[1]);
         put(10, g->opa[2]); put(11, g->opb[2]); put(12, g->opc[2]);
         g->consts = cs;
+        std::vector<double> cz((size_t)qzb::kConsts0 * M, 0.0);
+        for (int k = 0; k < 4; ++k) std::copy(cs.begin() + (size_t)k * M, cs.begin() + (size_t)(k + 1) * M, cz.begin() + (size_t)k * M);
+        for (int i = 0; i < M; ++i) {
+            cz[(size_t)4 * M + i] = g->V[i] / (2 * PI);
+            cz[(size_t)5 * M + i] = i < N ? g->h[i] / g->rmid[i] : 0.0;
+        }
+        for (int k = 0; k < 3; ++k) std::copy(cs.begin() + (size_t)(7 + k) * M, cs.begin() + (size_t)(8 + k) * M, cz.begin() + (size_t)(6 + k) * M);
+        g->consts0 = cz;
         // modes = 1: Thomas factors of L1D (its Dirichlet rows 0 and N are rows b = 1), L0 and L2D rows
         std::vector<double> c1((size_t)9 * M, 0.0);
         const std::vector<double>&a1 = g->opa[1], &b1 = g->opb[1], &cc1 = g->opc[1];
@@ -204,7 +213,7 @@ extern "C" qz_status qz_grid_create(const double* nodes, int M, qz_grid** out) {
     qz_status st;
     if ((st = dev_upload(&g->d_r, g->r)) || (st = dev_upload(&g->d_inv_h, g->inv_h)) ||
         (st = dev_upload(&g->d_inv_V, g->inv_V)) || (st = dev_upload(&g->d_consts, g->consts)) ||
-        (st = dev_upload(&g->d_consts1, g->consts1))) {
+        (st = dev_upload(&g->d_consts1, g->consts1)) || (st = dev_upload(&g->d_consts0, g->consts0))) {
         delete g;
         return st;
     }
@@ -445,6 +454,9 @@ extern "C" qz_status qz_sweep_create(const qz_grid* g, const qz_sweep_params* p,
     A.idxi = 1.0 / p->dxi;
     A.r = g->d_r; A.inv_h = g->d_inv_h; A.inv_V = g->d_inv_V;
     A.consts = g->d_consts;
+    A.consts0 = g->d_consts0;
+    A.lfa_N = g->opa[2][g->N];
+    A.lfb_N = g->opb[2][g->N];
     A.flux_coef = g->flux_coef;
     A.np = s->np;
     A.npad = s->npad;

@@ -14,6 +14,8 @@ namespace qzb {
 constexpr int kSweepThreads = QZ_SWEEP_THREADS;
 constexpr int kMaxSpecies = 4;
 
+constexpr int kConsts0 = 9;          // arrays of SweepArgs::consts0
+
 // Everything the m = 0 sweep kernel reads or writes. Pointers are device pointers.
 struct SweepArgs {
     int M, N, K;                    // nodes, cells, slices
@@ -25,6 +27,10 @@ struct SweepArgs {
     // per-node constants, 13 arrays of M: gradient stencils gm g0 gp, 1/r (src/FieldSolver.cpp:157-176);
     // L0 Thomas factors 1/u, -a/u, -c/u; rows a b c of L1D and of L1F (src/FieldSolver.cpp:117-156)
     const double* consts;
+    // the arrays the m = 0 sweep reads, 9 x M: gm g0 gp, 1/r; L0 in flux form V / 2 pi, h / r_mid; rows a b c of
+    // L1D; and row N of L1F (its other rows are L1D's)
+    const double* consts0;
+    double lfa_N, lfb_N;
     double flux_coef;               // coefficient of g in the flux row of L1F
     // mobile plasma species: particles [sp_off[s], sp_off[s+1])
     int nsp;

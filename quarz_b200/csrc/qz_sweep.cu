@@ -13,8 +13,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_m0_kernel(const SweepA
 }
 
 size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter, int pcache) {
-    size_t d = (size_t)(3 + 2 + 6 + (dbuf ? 18 : 9)) * M + 2 * 8 * (kSweepThreads / 32);
-    if (const_smem) d += 13 * (size_t)M;
+    size_t d = (size_t)(3 + 2 + 6 + (dbuf ? 18 : 9)) * M + sweep_detail::kTot;
+    if (const_smem) d += (size_t)kConsts0 * M;
     if (filter) d += 4 * (size_t)M + 2 * 14 * (kSweepThreads / 32);
     // + lost, flag, 14 exponent maxima and counters, the cells-crossed word (128 B with the particle copy
     // behind them: 6 doubles and a cell index per particle)

@@ -11,17 +11,17 @@
 // weight and the Adams-Bashforth history -- in registers for the whole sweep; larger plasmas keep
 // the state in a global scratch buffer.
 //
-// Tridiagonal solves. Every system is solved by all 512 threads at once: thread t owns rows
-// [t*R, t*R + R), and the three Thomas recurrences -- pivots u_i = b_i - a_i c_{i-1} / u_{i-1},
-// forward y_i = (d_i - a_i y_{i-1}) / u_i, backward x_i = y_i - (c_i / u_i) x_{i+1} -- are evaluated
-// as block-wide scans: pivots as normalised prefix products of 2x2 matrices, the substitutions as
-// scans of affine maps. Each scan costs five warp-shuffle levels and one block barrier. The psi,
-// E_z and B_z systems share the constant operator L0, whose pivots are computed once on the host.
+// Tridiagonal solves. Each system is solved by a group of warps of its own, a thread owning a few
+// consecutive rows (l0_solve, bplus_solve): the three Thomas recurrences -- pivots u_i = b_i - a_i c_{i-1} /
+// u_{i-1}, forward y_i = (d_i - a_i y_{i-1}) / u_i, backward x_i = y_i - (c_i / u_i) x_{i+1} -- run along a
+// thread's rows and as scans over the group's threads: pivots as normalised prefix products of 2x2
+// matrices, the substitutions as scans of affine maps. The psi, E_z and B_z systems share the constant
+// operator L0, whose substitutions are plain sums.
 //
-// Slice schedule (4 phase barriers + 5 scan barriers per slice):
-//   P2  psi, E_z, B_z (two scans, three right-hand sides); sources of slice k+1 = beam + background
+// Slice schedule (barriers of the CTA between the phases, of a system's group inside the solves):
+//   P2  psi, E_z, B_z and W+; sources of slice k+1 = beam + background
 //   P3  S+ deposit by the particles
-//   P4  B_r, B_theta (pivot scan + forward and backward scans of the two systems)
+//   P4  B_r, B_theta
 //   P5  store slice k; push k -> k+1 and deposit into the sources of slice k+1
 #pragma once
 #include "qz_device.cuh"
@@ -53,7 +53,8 @@ struct NoGate {
 };
 
 // ---------------------------------------------------------------- block scans
-// Shared scratch for the warp totals of one scan: 8 x kW doubles; two of them alternate.
+// Block-wide scans of one row per thread (the smoothing filter and the adjoint's reverse sweep). Shared
+// scratch for the warp totals of one scan: 8 x kW doubles; two of them alternate.
 
 // exact power-of-two rescaling of a 2x2 matrix (its largest entry into [1, 2))
 __device__ __forceinline__ void renorm(double& m00, double& m01, double& m10, double& m11) {
@@ -408,6 +409,125 @@ __device__ __forceinline__ void fx_max(const int (&e)[NC], int* E) {
 // headroom bits for n contributions per node: 2^bits > 2 n
 __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1); }
 
+// ---------------------------------------------------------------- solves by groups of warps
+// A slice has three systems with L0 (psi, E_z, B_z) and two with the shifted L1D and L1F (B_r, B_theta). A
+// block-wide scan of one row per thread needs 10 (L0) to 16 (pivots) 64-bit shuffles per level and lane for
+// all of them, and an SM executes one shuffle per cycle: the five scans took 1,800 to 3,600 cycles each. Here
+// every system has its own warps and a thread owns several of its rows: the recurrences run along
+// a thread's rows in registers (9 cycles per step), and the shuffles per system drop by the number of rows.
+// psi, E_z, B_z together went from 9,800 to 2,900 cycles per slice and B+ from 10,800 to 4,400 (512 nodes).
+// The row count is odd, so that the lanes' rows lie in different shared-memory banks.
+constexpr int kG2 = 5, kG4 = 8;                           // warps per system: 3 x 5 and 2 x 8
+constexpr int kTot = 256;                                 // S.tot: 24 + 24 (L0), 64 + 32 + 32 (B+)
+__device__ __forceinline__ int group_rows(int M, int warps) { return ((M + 32 * warps - 1) / (32 * warps)) | 1; }
+__device__ __forceinline__ void group_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// exclusive sum over a group's threads in thread order (up) or reverse order (!up); tot: one double per warp
+template <bool kUp, int kWarps>
+__device__ __forceinline__ double group_sum(double v, int wl, double* tot, int id) {
+    const int lane = threadIdx.x & 31;
+    double s = v;
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+        const double t = kUp ? __shfl_up_sync(FULL, s, st) : __shfl_down_sync(FULL, s, st);
+        if (kUp ? lane >= st : lane + st < 32) s += t;
+    }
+    if (lane == (kUp ? 31 : 0)) tot[wl] = s;
+    double e = kUp ? __shfl_up_sync(FULL, s, 1) : __shfl_down_sync(FULL, s, 1);
+    if (lane == (kUp ? 0 : 31)) e = 0.0;
+    group_sync(id, 32 * kWarps);
+    double c = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        const int o = kUp ? w : kWarps - 1 - w;
+        if (kUp ? o < wl : o > wl) c += tot[o];
+    }
+    return c + e;
+}
+
+// exclusive scan of the affine maps y -> a y + b in thread order (up) or reverse order: y before this
+// thread's rows (0 at the start); tot: 2 doubles per warp
+template <bool kUp, int kWarps>
+__device__ __forceinline__ double group_affine(double a, double b, int wl, double* tot, int id) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+        const double ap = kUp ? __shfl_up_sync(FULL, a, st) : __shfl_down_sync(FULL, a, st);
+        const double bp = kUp ? __shfl_up_sync(FULL, b, st) : __shfl_down_sync(FULL, b, st);
+        if (kUp ? lane >= st : lane + st < 32) { b = fma(a, bp, b); a *= ap; }
+    }
+    if (lane == (kUp ? 31 : 0)) { tot[2 * wl] = a; tot[2 * wl + 1] = b; }
+    double ea = kUp ? __shfl_up_sync(FULL, a, 1) : __shfl_down_sync(FULL, a, 1);
+    double eb = kUp ? __shfl_up_sync(FULL, b, 1) : __shfl_down_sync(FULL, b, 1);
+    if (lane == (kUp ? 0 : 31)) { ea = 1.0; eb = 0.0; }
+    group_sync(id, 32 * kWarps);
+    double c = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        const int o = kUp ? w : kWarps - 1 - w;
+        if (kUp ? o < wl : o > wl) c = fma(tot[2 * o], c, tot[2 * o + 1]);
+    }
+    return fma(ea, c, eb);
+}
+
+// exclusive product (later rows on the left) of the threads' 2x2 matrices, its first column (p, q) up to a
+// power of two. The matrices come renormalised (largest entry in [1, 2)): a product of 32 of them stays
+// below 2^63, and the column of kWarps renormalised totals below 2^(2 kWarps). tot: 4 doubles per warp
+template <int kWarps>
+__device__ __forceinline__ void group_pivots(double (&m)[4], double& p, double& q, int wl, double* tot, int id) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+        const double p00 = __shfl_up_sync(FULL, m[0], st), p01 = __shfl_up_sync(FULL, m[1], st);
+        const double p10 = __shfl_up_sync(FULL, m[2], st), p11 = __shfl_up_sync(FULL, m[3], st);
+        if (lane >= st) {
+            const double n00 = m[0] * p00 + m[1] * p10, n01 = m[0] * p01 + m[1] * p11;
+            const double n10 = m[2] * p00 + m[3] * p10, n11 = m[2] * p01 + m[3] * p11;
+            m[0] = n00; m[1] = n01; m[2] = n10; m[3] = n11;
+        }
+    }
+    renorm(m[0], m[1], m[2], m[3]);
+    if (lane == 31)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tot[4 * wl + e] = m[e];
+    double ex[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ex[e] = __shfl_up_sync(FULL, m[e], 1);
+    if (lane == 0) { ex[0] = 1.0; ex[1] = 0.0; ex[2] = 0.0; ex[3] = 1.0; }
+    group_sync(id, 32 * kWarps);
+    double c0 = 1.0, c1 = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps - 1; ++w)
+        if (w < wl) {
+            const double n0 = tot[4 * w] * c0 + tot[4 * w + 1] * c1;
+            c1 = tot[4 * w + 2] * c0 + tot[4 * w + 3] * c1;
+            c0 = n0;
+        }
+    p = ex[0] * c0 + ex[1] * c1;
+    q = ex[2] * c0 + ex[3] * c1;
+}
+
+// (p, q) scaled by the power of two that brings |p| into [1, 2); exact
+__device__ __forceinline__ void pivot_scale(double& p, double& q) {
+    const int e = (__double2hiint(p) >> 20) & 0x7ff;
+    const double s = __hiloint2double((e > 2045 ? 1 : 2046 - e) << 20, 0);
+    p *= s;
+    q *= s;
+}
+
+// q / p for |p| in [1, 2): Newton's iteration for 1/p from a single-precision reciprocal (22 bits, doubled
+// twice), then the quotient with one residual correction (Markstein, as Recip). No branch, so the quotients
+// of a thread's rows overlap.
+__device__ __forceinline__ double pivot_quot(double q, double p) {
+    double y = (double)__fdividef(1.0f, (float)p);
+    y = fma(y, fma(-p, y, 1.0), y);
+    y = fma(y, fma(-p, y, 1.0), y);
+    const double r = q * y;
+    return fma(fma(-p, r, q), y, r);
+}
+
 // ---------------------------------------------------------------- shared-memory layout
 struct Src {                                              // plasma + beam sources of one slice
     double *rhot, *drho, *jz, *chi, *ne, *ni, *jpi1, *S1r, *S1i;
@@ -416,12 +536,13 @@ struct Src {                                              // plasma + beam sourc
 struct Smem {
     double *r, *iv, *ih;                                  // grid
     const double *gm, *g0, *gp, *ir;                      // gradient stencils, 1/r
-    const double *l0r, *l0f, *l0b;                        // L0 Thomas: 1/u, -a/u, -c/u
-    const double *l1a, *l1b, *l1c, *lfa, *lfb, *lfc;      // L1D and L1F rows
+    const double *vw, *gw;                                // L0 in flux form: V / 2 pi, h / r_mid (l0_solve)
+    const double *l1a, *l1b, *l1c;                        // L1D rows; L1F's differ in row N only (lfa, lfb, c = 0)
+    double lfa, lfb;
     double* src0;                                         // sources: 9 arrays, twice when A.dbuf
     double *bgt, *bgr;                                    // neutralising background
     double *psi, *ez, *bz, *wr1, *bpr, *bpi;              // fields of the slice (wr1 = -psi')
-    double* tot;                                          // scan scratch, 2 x 8 x kW
+    double* tot;                                          // scan scratch of the solves, kTot doubles
     double* stage;                                        // A.filter: beam + background part of the next slice (4 x M)
     double* ftot;                                         // A.filter: scan scratch of the filter, 2 x 14 x kW
     int* lost;
@@ -443,17 +564,18 @@ __device__ __forceinline__ Smem carve(double* base, const SweepArgs& A) {
     Smem S;
     double* p = base;
     S.r = p; p += M; S.iv = p; p += M; S.ih = p; p += M;
-    const double* q = A.const_smem ? p : A.consts;
+    // the 9 arrays the sweep reads, behind one another as in A.consts0
+    const double* q = A.const_smem ? p : A.consts0;
     S.gm = q; S.g0 = q + M; S.gp = q + 2 * M; S.ir = q + 3 * M;
-    S.l0r = q + 4 * M; S.l0f = q + 5 * M; S.l0b = q + 6 * M;
-    S.l1a = q + 7 * M; S.l1b = q + 8 * M; S.l1c = q + 9 * M;
-    S.lfa = q + 10 * M; S.lfb = q + 11 * M; S.lfc = q + 12 * M;
-    if (A.const_smem) p += 13 * (size_t)M;
+    S.vw = q + 4 * M; S.gw = q + 5 * M;
+    S.l1a = q + 6 * M; S.l1b = q + 7 * M; S.l1c = q + 8 * M;
+    S.lfa = A.lfa_N; S.lfb = A.lfb_N;
+    if (A.const_smem) p += (size_t)kConsts0 * M;
     S.src0 = p;
     p += (A.dbuf ? 18 : 9) * (size_t)M;
     S.bgt = p; p += M; S.bgr = p; p += M;
     S.psi = p; p += M; S.ez = p; p += M; S.bz = p; p += M; S.wr1 = p; p += M; S.bpr = p; p += M; S.bpi = p; p += M;
-    S.tot = p; p += 2 * 8 * kW;
+    S.tot = p; p += kTot;
     S.stage = S.ftot = nullptr;
     if (A.filter) { S.stage = p; p += 4 * (size_t)M; S.ftot = p; p += 2 * 14 * kW; }
     S.lost = reinterpret_cast<int*>(p);
@@ -530,6 +652,38 @@ __device__ __forceinline__ BeamRow beam_row(const SweepArgs& A, const double* bs
     } else {
         r.drt = 0.5 * (ld(bk + st + B_RT0) - ld(bk + B_RT0 - (ptrdiff_t)st)) * A.idxi;
     }
+    return r;
+}
+
+// the values beam_row needs, loaded and not yet used: rho - J_z, J_z, J_theta of row k and rho - J_z of the
+// rows ahead of and behind it (w: their low limbs in the exact format)
+struct BeamRaw { double v[5], w[5]; };
+template <bool kL2>
+__device__ __forceinline__ void raw_load(const SweepArgs& A, const double* bsrc, int k, int j, BeamRaw& b) {
+    const size_t st = (size_t)A.M * B_NC0;
+    const double* const bk = bsrc + (size_t)k * st + (size_t)j * B_NC0;
+    const double* const p[5] = {bk + B_RT0, bk + B_JZ0, bk + B_JP1I, k > 0 ? bk + B_RT0 - (ptrdiff_t)st : bk + B_RT0,
+                                k + 1 < A.K ? bk + st + B_RT0 : bk + B_RT0};
+#pragma unroll
+    for (int c = 0; c < 5; ++c) b.v[c] = ldb<kL2>(p[c]);
+    if (A.bq)
+#pragma unroll
+        for (int c = 0; c < 5; ++c) b.w[c] = ldb<kL2>(p[c] + A.bfx_lo);
+}
+// beam_row of slice k > 0 from its loaded values; with static sources (which raw_load leaves out) beam_row itself
+template <bool kL2, bool kStat>
+__device__ __forceinline__ BeamRow raw_row(const SweepArgs& A, const double* bsrc, int k, int j, const BeamRaw& b) {
+    if constexpr (kStat)
+        if (A.bstat) return beam_row<kL2, kStat>(A, bsrc, k, j);
+    double v[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) v[c] = A.bq ? beam_fx_value(b.v[c], b.w[c], A.bq[j], A.bfx_2s) : b.v[c];
+    BeamRow r;
+    r.rt = v[0];
+    r.jz = v[1];
+    r.jt = v[2];
+    if (A.ngp || k == A.K - 1) r.drt = (v[0] - v[3]) * A.idxi;
+    else r.drt = 0.5 * (v[4] - v[3]) * A.idxi;
     return r;
 }
 
@@ -1081,35 +1235,163 @@ __device__ __forceinline__ BeamRow beam_row_at(const SweepArgs& A, const double*
     return r;
 }
 
-// right-hand sides of the psi, E_z, B_z systems at row i (src/Simulation.cpp:798-799, :517-527)
-__device__ __forceinline__ void rhs_l0(const Smem& S, const Src& s, int N, int i, double& d0, double& d1,
-                                       double& d2) {
-    d0 = d1 = d2 = 0.0;
-    if (i < N) {
-        d0 = -1.0 * s.rhot[i];
-        d1 = -1.0 * s.drho[i];
-        const double t1 = grad_at(S, N, s.jpi1, i, true);
-        const double t2 = (i == 0 ? s.jpi1[1] : s.jpi1[i]) * S.ir[i];
-        d2 = 1.0 * (-(t1 + t2));
+// right-hand side of system e (psi, E_z, B_z) at row i < N (src/Simulation.cpp:798-799, :517-527)
+__device__ __forceinline__ double rhs_l0(const Smem& S, const Src& s, int N, int e, int i) {
+    if (e == 0) return -1.0 * s.rhot[i];
+    if (e == 1) return -1.0 * s.drho[i];
+    const double t1 = grad_at(S, N, s.jpi1, i, true);
+    const double t2 = (i == 0 ? s.jpi1[1] : s.jpi1[i]) * S.ir[i];
+    return 1.0 * (-(t1 + t2));
+}
+
+// row i of (L1D - chi) (sys 0) or (L1F - chi) (sys 1) with its right-hand side; cm = c_{i-1}
+// (src/FieldSolver.cpp:172-191, src/Simulation.cpp:535-591)
+__device__ __forceinline__ void row_b(const Smem& S, const Src& s, int N, double fc, int sys, int i, double sv,
+                                      double& a, double& b, double& cm, double& d) {
+    a = S.l1a[i]; b = S.l1b[i]; cm = i > 0 ? S.l1c[i - 1] : 0.0;
+    d = 0.0;
+    if (sys == 0) {
+        if (i >= 1 && i < N) { b = b - s.chi[i]; d = 1.0 * (-sv); }
+    } else if (i >= 1) {
+        if (i == N) { a = S.lfa; b = S.lfb; }
+        b = b - s.chi[i];
+        d = 1.0 * (grad_at(S, N, s.jz, i, false) + sv);
+        if (i == N) d -= fc * s.jz[N];
     }
 }
 
-// row i of (L1D - chi) (sys 0) and (L1F - chi) (sys 1) with its right-hand side
-// (src/FieldSolver.cpp:172-191, src/Simulation.cpp:535-591)
-__device__ __forceinline__ void row_b(const Smem& S, const Src& s, int N, double fc, int sys, int i, double& a,
-                                      double& b, double& cm, double& d) {
-    if (sys == 0) {
-        a = S.l1a[i]; b = S.l1b[i]; cm = i > 0 ? S.l1c[i - 1] : 0.0;
-        if (i >= 1 && i < N) { b = b - s.chi[i]; d = 1.0 * (-s.S1i[i]); } else { d = 0.0; }
-    } else {
-        a = S.lfa[i]; b = S.lfb[i]; cm = i > 0 ? S.lfc[i - 1] : 0.0;
-        if (i >= 1) {
-            b = b - s.chi[i];
-            d = 1.0 * (grad_at(S, N, s.jz, i, false) + s.S1r[i]);
-            if (i == N) d -= fc * s.jz[N];
-        } else {
-            d = 0.0;
+// psi, E_z, B_z and W+ (src/Simulation.cpp:797-807, :501-532, :477-498). L0 is D^-1 times a Laplacian: with
+// w_i = V_i / 2 pi and g_i = r_mid,i / h_i its rows say that the flux g_i (x_{i+1} - x_i) is the sum of w d up
+// to node i. The Thomas pivots of that matrix are -g_i / w_i exactly, so the two substitutions are plain
+// sums: z_i = z_{i-1} + w_i d_i and x_i = x_{i+1} - z_i / g_i.
+template <int kR>
+__device__ __forceinline__ void l0_solve(const Smem& S, const Src& s, int M, int N) {
+    const int warp = threadIdx.x >> 5, e = warp / kG2, wl = warp - e * kG2;
+    if (e >= 3) return;
+    const int R = group_rows(M, kG2), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
+    double* const tz = S.tot + 8 * e;
+    double* const tx = S.tot + 24 + 8 * e;
+    double v[kR], sum = 0.0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        v[u] = 0.0;
+        if (u < R && i < N) v[u] = S.vw[i] * rhs_l0(S, s, N, e, i);
+        sum += v[u];
+    }
+    double z = group_sum<true, kG2>(sum, wl, tz, 1 + e);
+    const double z0 = z;
+    sum = 0.0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        z += v[u];
+        v[u] = (u < R && i < N) ? -(z * S.gw[i]) : 0.0;
+    }
+#pragma unroll
+    for (int u = kR - 1; u >= 0; --u) sum += v[u];
+    double x = group_sum<false, kG2>(sum, wl, tx, 1 + e);
+    double* const out = e == 0 ? S.psi : (e == 1 ? S.ez : S.bz);
+    const double xn = x;                                  // x just after this thread's rows
+#pragma unroll
+    for (int u = kR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        x += v[u];
+        v[u] = x;
+        if (u < R && i < M) out[i] = x;
+    }
+    if (e != 0) return;
+    // W+ = -psi' on the thread's rows; psi just before them from the flux that enters them
+    double xm = (row0 >= 1 && row0 < M) ? v[0] - z0 * S.gw[row0 - 1] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        if (u >= R || i >= M) break;
+        const double xc = v[u], xp = (u + 1 < kR && u + 1 < R) ? v[u + 1 < kR ? u + 1 : u] : xn;
+        if (i == 0) S.wr1[0] = -0.0;
+        else if (i < N) S.wr1[i] = -(S.gm[i] * xm + S.g0[i] * xc + S.gp[i] * xp);
+        if (i == N - 1) S.wr1[N] = -(S.g0[N] * xp + S.gm[N] * xc + S.gp[N] * xm);   // one-sided: psi_N, N-1, N-2
+        xm = xc;
+    }
+}
+
+// B_r and B_theta (src/Simulation.cpp:535-591, m = 0: one pass): (L1D - chi) B_r0 = -S_i (rows 0, N Dirichlet)
+// and (L1F - chi) B_theta0 = J_z' + S_r with flux wall J_z(R). 1/u_i = p_{i-1} / p_i, where (p_i, p_{i-1}) is the
+// first column of the product of T_i = [[b_i, -a_i c_{i-1}], [1, 0]] up to row i. Sv: the S+ values of a row
+// (kFinish: turned from the exact accumulators here, each by its only reader)
+template <int kR, bool kFinish>
+__device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, int N, double fc, int bits) {
+    const int warp = threadIdx.x >> 5, sy = warp / kG4, wl = warp - sy * kG4;
+    const int R = group_rows(M, kG4), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
+    double* const tp = S.tot + 64 + 32 * sy;
+    double* const tf = S.tot + 128 + 16 * sy;
+    double* const tb = S.tot + 160 + 16 * sy;
+    double* const sa = sy ? s.S1r : s.S1i;
+    const double qs = kFinish ? fx_quantum(S.fx[sy ? 7 : 8], bits) : 0.0;
+    const int es = kFinish ? S.fx[sy ? 7 : 8] : 0;
+    double ra[kR], rb[kR], rc[kR], rd[kR];
+    double m[4] = {1.0, 0.0, 0.0, 1.0};
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        ra[u] = 0.0; rb[u] = 1.0; rc[u] = 0.0; rd[u] = 0.0;
+        if (u < R && i < M) {
+            const double sv = kFinish ? fx_value(sa + i, es, qs) : sa[i];
+            row_b(S, s, N, fc, sy, i, sv, ra[u], rb[u], rc[u], rd[u]);
+            const double t01 = -ra[u] * rc[u];
+            const double n00 = rb[u] * m[0] + t01 * m[2], n01 = rb[u] * m[1] + t01 * m[3];
+            m[2] = m[0]; m[3] = m[1];
+            m[0] = n00; m[1] = n01;
+            if ((u & 3) == 3) renorm(m[0], m[1], m[2], m[3]);
         }
+    }
+    renorm(m[0], m[1], m[2], m[3]);
+    double p, q;
+    group_pivots<kG4>(m, p, q, wl, tp, 4 + sy);
+    // 1/u of the rows (into rc), the composite of the forward substitution
+    double fA = 1.0, fB = 0.0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const double pn = rb[u] * p - ra[u] * rc[u] * q;
+        q = p;
+        p = pn;
+        pivot_scale(p, q);
+        rc[u] = pivot_quot(q, p);
+    }
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        if (u >= R || i >= M) { rc[u] = 0.0; continue; }
+        ra[u] = -rc[u] * ra[u];
+        rd[u] = rc[u] * rd[u];
+        fB = fma(ra[u], fB, rd[u]);
+        fA *= ra[u];
+    }
+    double y = group_affine<true, kG4>(fA, fB, wl, tf, 4 + sy);
+    double bA = 1.0, bB = 0.0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int i = row0 + u;
+        if (u >= R || i >= M) continue;
+        y = fma(ra[u], y, rd[u]);
+        rd[u] = y;
+        rc[u] = -((sy && i == N ? 0.0 : S.l1c[i]) * rc[u]);      // x_i = -(c_i / u_i) x_{i+1} + y_i
+    }
+#pragma unroll
+    for (int u = kR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= R || i >= M) continue;
+        bB = fma(rc[u], bB, rd[u]);
+        bA *= rc[u];
+    }
+    double x = group_affine<false, kG4>(bA, bB, wl, tb, 4 + sy);
+    double* const out = sy ? S.bpi : S.bpr;
+#pragma unroll
+    for (int u = kR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= R || i >= M) continue;
+        x = fma(rc[u], x, rd[u]);
+        out[i] = x;
     }
 }
 
@@ -1141,6 +1423,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             t_prev = tn;                                                      \
         }                                                                     \
     } while (0)
+// parts of the solve phase, by thread 0 (a warp of the psi system): [5] the solves, [6] the next slice's start values
 #define SUB_MARK(slot)                                                        \
     do {                                                                      \
         if (tim && tid == 0) {                                                \
@@ -1162,7 +1445,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         src_of(S, M, 0).ne[j] = 0.0;
     }
     if (A.const_smem)
-        for (int t = tid; t < 13 * M; t += kThreads) const_cast<double*>(S.gm)[t] = A.consts[t];
+        for (int t = tid; t < kConsts0 * M; t += kThreads) const_cast<double*>(S.gm)[t] = A.consts0[t];
     if (tid == 0) *S.lost = 0;
     if (tid < 14) S.fx[tid] = 0;
     const int bits_p = fx_bits(np), bits_bg = fx_bits(A.nbg);
@@ -1351,7 +1634,6 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     __syncthreads();
     PHASE_MARK(0);
 
-    int scan_par = 0;                                            // alternates the scan scratch
     const double fc = A.flux_coef;
     // The xi positions of the last ORD pushes (tn[0] the newest; the same in every thread) give the
     // Adams-Bashforth coefficients of the next push: the classical ones for uniform steps, the
@@ -1411,102 +1693,24 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         if constexpr (EXT)
             if (A.filter) filter_sources<kMaxR>(s, S, A, Rw);
         if (tim && tid == 0) t_sub = clock64();
-        // beam rows of slice k+1 for this thread's nodes (consumed below, latency overlaps the solves)
-        BeamRow pre[kMaxR];
+        // beam rows of slice k+1 for this thread's nodes: loaded here without a use, so that the latency
+        // (L2 or DRAM) overlaps the solves
+        BeamRaw pre[kMaxR];
         if (A.dbuf && k + 1 < K && ss == 0)
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u)
-                if (u < Rw && row0 + u < M) pre[u] = beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, row0 + u);
+                raw_load<Gate::kActive>(A, gate.bsrc(A), k + 1, min(tid + u * kThreads, N), pre[u]);
 
-        // ---------------- P2: psi, E_z, B_z with L0 (src/Simulation.cpp:797-807, :501-532)
-        {
-            // forward: y_i = (-a_i/u_i) y_{i-1} + d_i/u_i
-            double cA = 1.0, cB[3] = {0.0, 0.0, 0.0};
-            double dv[kMaxR][3];
+        // ---------------- P2: psi, E_z, B_z with L0, W+
+        l0_solve<kMaxR == 1 ? 5 : 11>(S, s, M, N);
+        SUB_MARK(5);
+        if (A.dbuf && k + 1 < K && ss == 0)
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-                dv[u][0] = dv[u][1] = dv[u][2] = 0.0;
-                if (u >= Rw || i >= M) continue;
-                rhs_l0(S, s, N, i, dv[u][0], dv[u][1], dv[u][2]);
-                const double rr = S.l0r[i], af = S.l0f[i];
-#pragma unroll
-                for (int e = 0; e < 3; ++e) cB[e] = fma(af, cB[e], rr * dv[u][e]);
-                cA *= af;
+                const int j = tid + u * kThreads;
+                if (j < M) init_sources<EXT>(sn, S, j, raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j, pre[u]), M);
             }
-            SUB_MARK(5);
-            double yb[3];
-            scan_fwd<3>(cA, cB, yb, S.tot + (scan_par++ & 1) * 8 * kW);
-            SUB_MARK(6);
-            const double ypsi_prev = yb[0];                         // y of psi just before this thread's rows
-            double y[kMaxR][3];
-#pragma unroll
-            for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-                y[u][0] = y[u][1] = y[u][2] = 0.0;
-                if (u >= Rw || i >= M) continue;
-                const double rr = S.l0r[i], af = S.l0f[i];
-#pragma unroll
-                for (int e = 0; e < 3; ++e) { yb[e] = fma(af, yb[e], rr * dv[u][e]); y[u][e] = yb[e]; }
-            }
-            // backward: x_i = (-c_i/u_i) x_{i+1} + y_i
-            double bA = 1.0, bB[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-            for (int u = kMaxR - 1; u >= 0; --u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
-                const double ab = S.l0b[i];
-#pragma unroll
-                for (int e = 0; e < 3; ++e) bB[e] = fma(ab, bB[e], y[u][e]);
-                bA *= ab;
-            }
-            double xa[3];
-            scan_bwd<3>(bA, bB, xa, S.tot + (scan_par++ & 1) * 8 * kW);
-            SUB_MARK(7);
-            // psi on the window [row0 - 1, row0 + Rw]: the rows of this thread, x after them (the
-            // backward carry) and x before them, x_{row0-1} = y_{row0-1} - (c/u)_{row0-1} x_{row0}
-            // with y_{row0-1} the forward carry -- so W+ = -psi' needs no further exchange
-            double pw[kMaxR + 2];
-            pw[kMaxR + 1] = 0.0;
-            {
-                double xr = xa[0];
-#pragma unroll
-                for (int u = kMaxR; u >= 1; --u) pw[u] = 0.0;
-                const int last = (row0 + Rw <= M ? Rw : M - row0);
-                if (last >= 0) pw[last + 1 > kMaxR + 1 ? kMaxR + 1 : last + 1] = xr;
-            }
-#pragma unroll
-            for (int u = kMaxR - 1; u >= 0; --u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
-                const double ab = S.l0b[i];
-#pragma unroll
-                for (int e = 0; e < 3; ++e) xa[e] = fma(ab, xa[e], y[u][e]);
-                S.psi[i] = xa[0];
-                S.ez[i] = xa[1];
-                S.bz[i] = xa[2];
-                pw[u + 1] = xa[0];
-            }
-            pw[0] = (row0 >= 1 && row0 < M) ? fma(S.l0b[row0 - 1], pw[1], ypsi_prev) : 0.0;
-#pragma unroll
-            for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
-                if (i == 0) {
-                    S.wr1[0] = -0.0;
-                } else if (i < N) {
-                    S.wr1[i] = -(S.gm[i] * pw[u] + S.g0[i] * pw[u + 1] + S.gp[i] * pw[u + 2]);
-                }
-                if (i == N - 1) {                                  // the one-sided wall stencil needs psi_{N-2..N}
-                    S.wr1[N] = -(S.g0[N] * pw[u + 2] + S.gm[N] * pw[u + 1] + S.gp[N] * pw[u]);
-                }
-            }
-            if (A.dbuf && k + 1 < K && ss == 0)
-#pragma unroll
-                for (int u = 0; u < kMaxR; ++u)
-                    if (u < Rw && row0 + u < M) init_sources<EXT>(sn, S, row0 + u, pre[u], M);
-            SUB_MARK(8);
-        }
+        SUB_MARK(6);
         __syncthreads();
         PHASE_MARK(1);
 
@@ -1550,108 +1754,20 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         }
         __syncthreads();
         PHASE_MARK(2);
-        // this thread's rows of S+ into values: the only rows its B+ rows (and the filter) read
         if (tid == 0) S.fx[13] += (S.fx[7] == 2047) + (S.fx[8] == 2047);
-#pragma unroll
-        for (int u = 0; u < kMaxR; ++u)
-            if (u < Rw && row0 + u < M) depositS_finish(s, row0 + u, S.fx + 7, bits_p);
 
-        // ---------------- P4: B+ (src/Simulation.cpp:535-591, m = 0: one pass)
-        //   (L1D - chi) B_r0 = -S_i (rows 0, N Dirichlet); (L1F - chi) B_theta0 = J_z' + S_r, flux wall J_z(R)
-        if (EXT && A.filter) {              // S+ smoothed with F1 (src/Simulation.cpp:810-812): the rows of
-            FilterSet<2> fsS;               // this thread, which are the only ones its B+ rows read
+        // ---------------- P4: B+
+        if (EXT && A.filter) {              // S+ smoothed with F1 (src/Simulation.cpp:810-812)
+#pragma unroll
+            for (int u = 0; u < kMaxR; ++u)
+                if (u < Rw && row0 + u < M) depositS_finish(s, row0 + u, S.fx + 7, bits_p);
+            FilterSet<2> fsS;
             fsS.f[0] = s.S1r; fsS.f[1] = s.S1i; fsS.op[0] = fsS.op[1] = 1;
             filter_rows<2, kMaxR>(fsS, A.fconsts, M, Rw, S.ftot);
-        }
-        {
-            // pivots: product of T_i = [[b_i, -a_i c_{i-1}], [1, 0]] over the thread's rows
-            double m[2][4];
-#pragma unroll
-            for (int sy = 0; sy < 2; ++sy) { m[sy][0] = 1.0; m[sy][1] = 0.0; m[sy][2] = 0.0; m[sy][3] = 1.0; }
-            double ra[kMaxR][2], rb[kMaxR][2], rc[kMaxR][2], rd[kMaxR][2];
-#pragma unroll
-            for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    ra[u][sy] = 0.0; rb[u][sy] = 1.0; rc[u][sy] = 0.0; rd[u][sy] = 0.0;
-                    if (u >= Rw || i >= M) continue;
-                    row_b(S, s, N, fc, sy, i, ra[u][sy], rb[u][sy], rc[u][sy], rd[u][sy]);
-                    const double t01 = -ra[u][sy] * rc[u][sy];
-                    const double n00 = rb[u][sy] * m[sy][0] + t01 * m[sy][2];
-                    const double n01 = rb[u][sy] * m[sy][1] + t01 * m[sy][3];
-                    m[sy][2] = m[sy][0]; m[sy][3] = m[sy][1];
-                    m[sy][0] = n00; m[sy][1] = n01;
-                    renorm(m[sy][0], m[sy][1], m[sy][2], m[sy][3]);
-                }
-            }
-            double pp[2], qq[2];
-            scan_pivots<2>(m, pp, qq, S.tot + (scan_par++ & 1) * 8 * kW);
-            // this thread's pivots (rc holds c_{i-1}; rinv = 1/u_i = p_{i-1}/p_i), forward composites
-            double rinv[kMaxR][2];
-            double fA[2] = {1.0, 1.0}, fB[2] = {0.0, 0.0};
-#pragma unroll
-            for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    rinv[u][sy] = 0.0;
-                    if (u >= Rw || i >= M) continue;
-                    const double pn = rb[u][sy] * pp[sy] - ra[u][sy] * rc[u][sy] * qq[sy];
-                    qq[sy] = pp[sy];
-                    pp[sy] = pn;
-                    const double rr = qq[sy] / pp[sy];
-                    const double sc = fabs(pp[sy]);
-                    if (sc > 1e100 || sc < 1e-100) { pp[sy] /= sc; qq[sy] /= sc; }
-                    rinv[u][sy] = rr;
-                    const double af = -rr * ra[u][sy];
-                    fB[sy] = fma(af, fB[sy], rr * rd[u][sy]);
-                    fA[sy] *= af;
-                }
-            }
-            // forward substitution of both systems
-            double yy[2];
-            scan_fwd_n<2>(fA, fB, yy, S.tot + (scan_par++ & 1) * 8 * kW);
-            double y[kMaxR][2];
-#pragma unroll
-            for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    y[u][sy] = 0.0;
-                    if (u >= Rw || i >= M) continue;
-                    yy[sy] = fma(-rinv[u][sy] * ra[u][sy], yy[sy], rinv[u][sy] * rd[u][sy]);
-                    y[u][sy] = yy[sy];
-                }
-            }
-            // backward substitution: x_i = -(c_i / u_i) x_{i+1} + y_i
-            double bA[2] = {1.0, 1.0}, bB[2] = {0.0, 0.0};
-#pragma unroll
-            for (int u = kMaxR - 1; u >= 0; --u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    const double c = sy ? S.lfc[i] : S.l1c[i];
-                    const double ab = -(c * rinv[u][sy]);
-                    bB[sy] = fma(ab, bB[sy], y[u][sy]);
-                    bA[sy] *= ab;
-                }
-            }
-            double xx[2];
-            scan_bwd_n<2>(bA, bB, xx, S.tot + (scan_par++ & 1) * 8 * kW);
-#pragma unroll
-            for (int u = kMaxR - 1; u >= 0; --u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    const double c = sy ? S.lfc[i] : S.l1c[i];
-                    xx[sy] = fma(-(c * rinv[u][sy]), xx[sy], y[u][sy]);
-                }
-                S.bpr[i] = xx[0];
-                S.bpi[i] = xx[1];
-            }
+            __syncthreads();
+            bplus_solve<kMaxR == 1 ? 3 : 7, false>(S, s, M, N, fc, bits_p);
+        } else {
+            bplus_solve<kMaxR == 1 ? 3 : 7, true>(S, s, M, N, fc, bits_p);
         }
         __syncthreads();
         PHASE_MARK(3);
@@ -1721,11 +1837,12 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             BeamRow nxt[kMaxR];
             if (!to_next || !A.dbuf)
 #pragma unroll
-                for (int u = 0; u < kMaxR; ++u)
-                    if (u < Rw && row0 + u < M)
-                        nxt[u] = to_next ? beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, row0 + u)
-                                         : beam_row_at<Gate::kActive, EXT>(A, gate.bsrc(A), k, row0 + u,
-                                                                            (ss + 1) * hstep);
+                for (int u = 0; u < kMaxR; ++u) {
+                    const int j = tid + u * kThreads;
+                    if (j < M)
+                        nxt[u] = to_next ? beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j)
+                                         : beam_row_at<Gate::kActive, EXT>(A, gate.bsrc(A), k, j, (ss + 1) * hstep);
+                }
             const bool first = (k == 0) && (ss == 0) && !A.pin_pushed;
             coeffs(hstep, first);
             if (REG) {
@@ -1806,8 +1923,8 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 for (int c = 0; c < 7; ++c) S.fx[13] += S.fx[c] == 2047;
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u) {
-                const int i = row0 + u;
-                if (u >= Rw || i >= M) continue;
+                const int i = tid + u * kThreads;
+                if (i >= M) continue;
                 double b0[7];
                 if (to_next && A.dbuf) {
 #pragma unroll
