@@ -796,9 +796,11 @@ __device__ void recompute_segment(const SweepArgs& A, const AdjSm& S, const doub
         }
         __syncthreads();
         if (has_p) {
-            if (P.w != 0.0)
-                (void)sweep_detail::push_particle<ORD>(P, geometry(S.r, S.ih, N, A.R, P.x, P.y), F, A, k == 0, ab,
+            if (P.w != 0.0) {
+                sweep_detail::PKin kin = sweep_detail::kin_of(P.px, P.py, P.dl);
+                (void)sweep_detail::push_particle<ORD>(P, geometry(S.r, S.ih, N, A.R, P.x, P.y), kin, F, A, k == 0, ab,
                                                        A.dxi);
+            }
             put(k + 1 - k0);
         }
     }

@@ -384,12 +384,30 @@ __device__ __forceinline__ bool warp_runs_sum(int key, double (&v)[NV]) {
 __device__ __forceinline__ int fx_bexp(double v) {         // biased exponent: 0 for 0, 2047 for Inf / NaN
     return (int)((__double_as_longlong(v) >> 52) & 0x7ff);
 }
-__device__ __forceinline__ int fx_qexp(int e, int bits) { return e - 1085 + bits; }   // (e - 1022) + bits - 63
-// 1 / quantum (0 when every contribution is zero) and the quantum of a block maximum e
-__device__ __forceinline__ double fx_scale(int e, int bits) { return e == 0 ? 0.0 : scalbn(1.0, -fx_qexp(e, bits)); }
-__device__ __forceinline__ double fx_quantum(int e, int bits) { return scalbn(1.0, fx_qexp(e, bits)); }
-__device__ __forceinline__ void fx_add(double* p, double v, double scale) {
-    if (v != 0.0) atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__double2ll_rn(v * scale));
+// 1 / quantum and the quantum of a block maximum e, as powers of two by their exponent fields: quantum
+// 2^(e - 1085 + bits) (the largest contribution below 2^(e - 1022), |sum| < 2^63 quanta), not below 2^-1022
+__device__ __forceinline__ double fx_scale(int e, int bits) {
+    return __hiloint2double(min(2108 - bits - e, 2045) << 20, 0);
+}
+__device__ __forceinline__ double fx_quantum(int e, int bits) { return __hiloint2double(max(e - 62 + bits, 1) << 20, 0); }
+// p[i] += round(v[i] scale[i]) for NA accumulators in shared memory. A 64-bit shared-memory add is a
+// compare-and-swap loop the thread waits for (104 cycles each, one after the other); two 32-bit adds, the
+// low words first and then the high words with the carries, are native and overlap (12 values of a full warp:
+// 1,254 cycles as 64-bit adds). Sums of integers modulo 2^64: the order of the adds does not matter.
+template <int NA>
+__device__ __forceinline__ void fx_add(double* const (&p)[NA], const double (&v)[NA], const double (&scale)[NA]) {
+    unsigned lo[NA], hi[NA], old[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        const unsigned long long q = (unsigned long long)__double2ll_rn(v[i] * scale[i]);
+        lo[i] = (unsigned)q;
+        hi[i] = (unsigned)(q >> 32);
+    }
+#pragma unroll
+    for (int i = 0; i < NA; ++i) old[i] = atomicAdd(reinterpret_cast<unsigned*>(p[i]), lo[i]);
+#pragma unroll
+    for (int i = 0; i < NA; ++i)
+        atomicAdd(reinterpret_cast<unsigned*>(p[i]) + 1, hi[i] + (old[i] + lo[i] < lo[i] ? 1u : 0u));
 }
 // the value of an accumulator (its 64 bits as stored in the double slot p); e == 2047: a non-finite
 // contribution was seen
@@ -397,14 +415,18 @@ __device__ __forceinline__ double fx_value(const double* p, int e, double quantu
     if (e == 2047) return __longlong_as_double(0x7ff8000000000000LL);
     return (double)__double_as_longlong(*p) * quantum;
 }
-// warp-wide: E[c] = max(E[c], the largest e[c] of the warp's lanes) (shared-memory block maxima)
+// warp-wide: E[c] = max(E[c], the largest e[c] of the warp's lanes) (shared-memory block maxima); lane c
+// holds the maximum of e[c], so one atomic instruction updates all of them
 template <int NC>
 __device__ __forceinline__ void fx_max(const int (&e)[NC], int* E) {
+    const int lane = threadIdx.x & 31;
+    unsigned mine = 0;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const unsigned m = __reduce_max_sync(FULL, (unsigned)e[c]);
-        if ((threadIdx.x & 31) == 0 && m) atomicMax(E + c, (int)m);
+        if (lane == c) mine = m;
     }
+    if (lane < NC && mine) atomicMax(E + lane, (int)mine);
 }
 // headroom bits for n contributions per node: 2^bits > 2 n
 __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1); }
@@ -854,6 +876,16 @@ __device__ __forceinline__ int locate_from(const double* __restrict__ r, int N, 
     return locate(r, N, R, x);
 }
 
+// two neighbouring doubles: one 16-byte store when v16 (p on a 16-byte boundary)
+__device__ __forceinline__ void put2(double* p, double a, double b, bool v16) {
+    if (v16) {
+        *reinterpret_cast<double2*>(p) = make_double2(a, b);
+    } else {
+        p[0] = a;
+        p[1] = b;
+    }
+}
+
 // ---------------------------------------------------------------- one plasma particle
 // history h[m] holds the force m pushes ago (h[0] newest): the reference's ring buffer
 // (src/PlasmaSpecies.cpp:621-632) with the slot rotation done by moving values.
@@ -926,6 +958,25 @@ __device__ __forceinline__ void species_params(const SweepArgs& A, int p, double
     qm = A.sp_qm[s];
 }
 
+// gamma = (1 + p_perp^2 + Delta^2) / 2 Delta and 1 / Delta of a particle
+struct PKin { double gam, invd; };
+__device__ __forceinline__ PKin kin_of(double px, double py, double d) {
+    const Recip q(d);
+    PKin k;
+    k.invd = q.y;
+    k.gam = 0.5 * q(1.0 + px * px + py * py + d * d);
+    return k;
+}
+// What the phases of a slice need of a particle whose state is kept in registers, computed once per push: its
+// polar position and kinematics (a square root and two reciprocals)
+struct PKeep {
+    double rp, ir, c, s;
+    PKin k;
+};
+__device__ __forceinline__ PGeo keep_geo(const Smem& S, const PKeep& K, int j) {
+    return geometry_at(S.r, S.ih, j, K.rp, K.ir, K.c, K.s);
+}
+
 // W+ mode 1 at the particle: lin(w1), w1 = -psi' (src/Simulation.cpp:477-498)
 __device__ __forceinline__ double w1_at(const Smem& S, int N, const PGeo& g) { return lin(S.wr1, g); }
 
@@ -933,10 +984,10 @@ __device__ __forceinline__ double w1_at(const Smem& S, int N, const PGeo& g) { r
 // Contributions of one particle to nodes j (v[0..5]) and j+1 (v[6..11]): rho - J_z, d/dxi, J_z, chi,
 // density, J_theta.
 template <int ORD>
-__device__ __forceinline__ void deposit_values(const PState<ORD>& P, const PGeo& g, const Smem& S, double (&v)[12]) {
+__device__ __forceinline__ void deposit_values(const PState<ORD>& P, const PGeo& g, const PKin& kin, const Smem& S,
+                                               double (&v)[12]) {
     const double PX = P.px, PY = P.py, D = P.dl, w = P.w;
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const double gam = kin.gam, invd = kin.invd;
     const double pz = gam - D;
     const double ux = PX * invd, uy = PY * invd;
     const double ur = g.c * ux + g.s * uy, uth = g.c * uy - g.s * ux;
@@ -1010,16 +1061,12 @@ __device__ __forceinline__ void deposit_add(bool tail, int j, bool neg, const do
     if (!tail) return;
     const double s0 = fx_scale(E[0], bits), s1 = fx_scale(E[1], bits), s2 = fx_scale(E[2], bits);
     const double s3 = fx_scale(E[3], bits), s4 = fx_scale(E[neg ? 4 : 5], bits), s6 = fx_scale(E[6], bits);
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-        const int jj = j + cc;
-        fx_add(acc.rhot + jj, v[6 * cc + 0], s0);
-        fx_add(acc.drho + jj, v[6 * cc + 1], s1);
-        fx_add(acc.jz + jj, v[6 * cc + 2], s2);
-        fx_add(acc.chi + jj, v[6 * cc + 3], s3);
-        fx_add((neg ? acc.ne : acc.ni) + jj, v[6 * cc + 4], s4);
-        fx_add(acc.jpi1 + jj, v[6 * cc + 5], s6);
-    }
+    double* const dens = neg ? acc.ne : acc.ni;
+    double* const adr[12] = {acc.rhot + j, acc.drho + j, acc.jz + j, acc.chi + j, dens + j, acc.jpi1 + j,
+                             acc.rhot + j + 1, acc.drho + j + 1, acc.jz + j + 1, acc.chi + j + 1, dens + j + 1,
+                             acc.jpi1 + j + 1};
+    const double sc[12] = {s0, s1, s2, s3, s4, s6, s0, s1, s2, s3, s4, s6};
+    fx_add<12>(adr, v, sc);
 }
 
 // the values of node j: dst = base + accumulated deposit (acc and dst may be the same arrays)
@@ -1032,15 +1079,14 @@ __device__ __forceinline__ void deposit_finish(const Src& dst, const Src& acc, i
 
 // src/PlasmaSpecies.cpp:508-559, m = 0: S+ contributions to nodes j (v[0..1]) and j+1 (v[2..3])
 template <int ORD>
-__device__ __forceinline__ void depositS_values(const PState<ORD>& P, const PGeo& g, const Smem& S, int N,
-                                                double (&v)[4]) {
+__device__ __forceinline__ void depositS_values(const PState<ORD>& P, const PGeo& g, const PKin& kin, const Smem& S,
+                                                int N, double (&v)[4]) {
     const double qm = P.qm;
-    const double PX = P.px, PY = P.py, D = P.dl;
+    const double PX = P.px, PY = P.py;
     const double r1 = w1_at(S, N, g);
     const double Wx = r1 * g.c - 0.0 * g.s, Wy = r1 * g.s + 0.0 * g.c;
     const double Ez = lin(S.ez, g), Bz = lin(S.bz, g);
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const double gam = kin.gam, invd = kin.invd;
     const double ux = PX * invd, uy = PY * invd;
     const double ur = g.c * ux + g.s * uy, uth = g.c * uy - g.s * ux;
     const double dD = qm * ((PX * Wx + PY * Wy) * invd - Ez);
@@ -1090,10 +1136,9 @@ __device__ __forceinline__ void depositS_add(bool tail, int j, const double (&v)
                                              int bits) {
     if (!tail) return;
     const double sr = fx_scale(E[0], bits), si = fx_scale(E[1], bits);
-    fx_add(s.S1r + j, v[0], sr);
-    fx_add(s.S1i + j, v[1], si);
-    fx_add(s.S1r + j + 1, v[2], sr);
-    fx_add(s.S1i + j + 1, v[3], si);
+    double* const adr[4] = {s.S1r + j, s.S1i + j, s.S1r + j + 1, s.S1i + j + 1};
+    const double sc[4] = {sr, si, sr, si};
+    fx_add<4>(adr, v, sc);
 }
 
 __device__ __forceinline__ void depositS_finish(const Src& s, int i, const int* E, int bits) {
@@ -1103,10 +1148,11 @@ __device__ __forceinline__ void depositS_finish(const Src& s, int i, const int* 
 
 // src/PlasmaSpecies.cpp:561-668 with uniform steps (the classical AB coefficients); returns 1 when the
 // particle moved, 0 when it was removed beyond the wall, -1 when removed as trapped (Delta <= delta_min
-// or gamma > max_qsa Delta: no longer quasi-static, src/PlasmaSpecies.cpp:636-650)
+// or gamma > max_qsa Delta: no longer quasi-static, src/PlasmaSpecies.cpp:636-650). kin: the particle's
+// kinematics before the push, on return those after it
 template <int ORD>
-__device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, const Smem& S, const SweepArgs& A,
-                                              bool first, const double (&ab)[5], double h) {
+__device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin& kin, const Smem& S,
+                                             const SweepArgs& A, bool first, const double (&ab)[5], double h) {
     const double qm = P.qm;
     const double X = P.x, Y = P.y, PX = P.px, PY = P.py, D = P.dl;
     const double r1 = w1_at(S, A.N, g);
@@ -1114,8 +1160,7 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, cons
     const double Ez = lin(S.ez, g), Bz = lin(S.bz, g);
     const double br = lin(S.bpr, g), bi = lin(S.bpi, g);
     const double Bx = br * g.c - bi * g.s, By = br * g.s + bi * g.c;
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const double gam = kin.gam, invd = kin.invd;
     double fv[5];
     fv[0] = PX * invd;
     fv[1] = PY * invd;
@@ -1146,8 +1191,8 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, cons
     double xn = X + dxi * sum[0], yn = Y + dxi * sum[1];
     double pxn = PX + dxi * sum[2], pyn = PY + dxi * sum[3];
     const double dn = D + dxi * sum[4];
-    const double gn = (1.0 + pxn * pxn + pyn * pyn + dn * dn) / (2.0 * dn);
-    if (!(dn > A.delta_min) || gn > A.max_qsa * dn) {
+    kin = kin_of(pxn, pyn, dn);
+    if (!(dn > A.delta_min) || kin.gam > A.max_qsa * dn) {
         P.w = 0.0;
         return -1;
     }
@@ -1160,6 +1205,7 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, cons
         xn = nx * rr; yn = ny * rr;
         const double pn = pxn * nx + pyn * ny;
         pxn -= 2.0 * pn * nx; pyn -= 2.0 * pn * ny;
+        kin = kin_of(pxn, pyn, dn);
 #pragma unroll
         for (int m = 0; m < ORD; ++m) {
             const double a = P.h[m][0] * nx + P.h[m][1] * ny;
@@ -1451,6 +1497,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     const int bits_p = fx_bits(np), bits_bg = fx_bits(A.nbg);
     PState<ORD> P;
     int J = 0;                                             // cell of the thread's particle
+    PKeep kp{0.0, 0.0, 1.0, 0.0, {1.0, 1.0}};              // and its polar position and kinematics
     if (REG) {
         if (tid < np) {
             if (A.pin) {                                  // a later slab: the plasma handed on, with its history
@@ -1505,11 +1552,9 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             if (pass == 0) {
                 ebg = max(ebg, max(fx_bexp(a0), fx_bexp(a1)));
             } else {
-                const double sc = fx_scale(S.fx[9], bits_bg);
-                fx_add(S.bgt + g.j, a0, sc);
-                fx_add(S.bgr + g.j, a0, sc);
-                fx_add(S.bgt + g.j + 1, a1, sc);
-                fx_add(S.bgr + g.j + 1, a1, sc);
+                const double sc = fx_scale(S.fx[9], bits_bg), v[4] = {a0, a0, a1, a1}, s4[4] = {sc, sc, sc, sc};
+                double* const adr[4] = {S.bgt + g.j, S.bgr + g.j, S.bgt + g.j + 1, S.bgr + g.j + 1};
+                fx_add<4>(adr, v, s4);
             }
         }
         if (A.neutralize)
@@ -1523,9 +1568,9 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 if (pass == 0) {
                     ene = max(ene, max(fx_bexp(a0), fx_bexp(a1)));
                 } else {
-                    const double sc = fx_scale(S.fx[10], bits_p);
-                    fx_add(ne0 + g.j, a0, sc);
-                    fx_add(ne0 + g.j + 1, a1, sc);
+                    const double sc = fx_scale(S.fx[10], bits_p), v[2] = {a0, a1}, s2[2] = {sc, sc};
+                    double* const adr[2] = {ne0 + g.j, ne0 + g.j + 1};
+                    fx_add<2>(adr, v, s2);
                 }
             }
         if (pass == 0) {
@@ -1583,9 +1628,10 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             const bool act = tid < np && P.w != 0.0;
             double v[12];
             if (act) {
-                const PGeo G = geometry(S.r, S.ih, N, R, P.x, P.y);
-                J = G.j;
-                deposit_values(P, G, S, v);
+                polar(P.x, P.y, kp.rp, kp.ir, kp.c, kp.s);
+                kp.k = kin_of(P.px, P.py, P.dl);
+                J = locate(S.r, N, R, kp.rp);
+                deposit_values(P, keep_geo(S, kp, J), kp.k, S, v);
             }
             const bool tail = deposit_runs<true>(act, J, P.q < 0.0, v, S.fx);
             __syncthreads();
@@ -1609,7 +1655,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                                      : pgeo(S, A, N, R, p, Q.x, Q.y);
                             if (pass == 0 && A.pcache) S.pj[p] = g.j;
                             j = g.j;
-                            deposit_values(Q, g, S, v);
+                            deposit_values(Q, g, kin_of(Q.px, Q.py, Q.dl), S, v);
                         }
                     }
                     const bool neg = act && Q.q < 0.0;
@@ -1720,7 +1766,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         if (REG) {
             const bool act = tid < np && P.w != 0.0;
             double v[4];
-            if (act) depositS_values(P, geometry_in(S.r, S.ih, P.x, P.y, J), S, N, v);
+            if (act) depositS_values(P, keep_geo(S, kp, J), kp.k, S, N, v);
             const bool tail = depositS_runs<true>(act, J, v, S.fx + 7);
             __syncthreads();
             depositS_add(tail, J, v, s, S.fx + 7, bits_p);
@@ -1740,7 +1786,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                         if (act) {
                             const PGeo g = pgeo(S, A, N, R, p, Q.x, Q.y);
                             j = g.j;
-                            depositS_values(Q, g, S, N, v);
+                            depositS_values(Q, g, kin_of(Q.px, Q.py, Q.dl), S, N, v);
                         }
                     }
                     if (pass == 0) {
@@ -1808,20 +1854,20 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         const Src dst = to_next ? sn : s;
         {
             const size_t fb = (size_t)k * M;
+            // a node's 6 field components start on 16 bytes when the field store does
+            const bool f16 = (reinterpret_cast<uintptr_t>(gate.fld(A)) & 15) == 0;
             for (int j = tid; j < M; j += kThreads) {
                 if (ss == 0) {
                     double* F = gate.fld(A) + (fb + j) * F_NC0;
-                    F[F_EP1R] = S.wr1[j] + S.bpi[j];
-                    F[F_EP1I] = 0.0 - S.bpr[j];
-                    F[F_BP1R] = S.bpr[j];
-                    F[F_BP1I] = S.bpi[j];
-                    F[F_EZ0] = S.ez[j];
-                    F[F_BZ0] = S.bz[j];
+                    const double br = S.bpr[j], bi = S.bpi[j], w1 = S.wr1[j];
+                    put2(F + F_EP1R, w1 + bi, 0.0 - br, f16);
+                    put2(F + F_BP1R, br, bi, f16);
+                    put2(F + F_EZ0, S.ez[j], S.bz[j], f16);
                     double* D = gate.diag(A) + (fb + j) * D_NC0;
                     D[D_PSI0] = S.psi[j];
                     D[D_NE0] = s.ne[j];
                     D[D_NI0] = s.ni[j];
-                    if (double* const W = gate.wrec(A)) W[fb + j] = S.wr1[j];
+                    if (double* const W = gate.wrec(A)) W[fb + j] = w1;
                 }
                 if (k + 1 < K) {
 #pragma unroll
@@ -1849,11 +1895,11 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 bool act = tid < np && P.w != 0.0;
                 double v[12];
                 if (act) {
-                    const int pr = push_particle(P, geometry_in(S.r, S.ih, P.x, P.y, J), S, A, first, abc, hstep);
+                    const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, hstep);
                     if (pr > 0) {
-                        const double rn = sqrt(P.x * P.x + P.y * P.y);
-                        J = locate_from(S.r, N, R, rn, J);
-                        deposit_values(P, geometry_in(S.r, S.ih, P.x, P.y, J), S, v);
+                        polar(P.x, P.y, kp.rp, kp.ir, kp.c, kp.s);
+                        J = locate_from(S.r, N, R, kp.rp, J);
+                        deposit_values(P, keep_geo(S, kp, J), kp.k, S, v);
                     } else {
                         act = false;
                         atomicAdd(S.lost, 1);
@@ -1881,18 +1927,15 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                 if (pass == 0) {
                                     phist(Q, gate.ps(A), npad, p);
                                     const PGeo g = pgeo(S, A, N, R, p, Q.x, Q.y);
-                                    const int pr = push_particle(Q, g, S, A, first, abc, hstep);
+                                    PKin kin = kin_of(Q.px, Q.py, Q.dl);
+                                    const int pr = push_particle(Q, g, kin, S, A, first, abc, hstep);
                                     if (pr > 0) {
-                                        PGeo g2;
-                                        if (A.pcache) {        // the new cell by a short walk from the old one
-                                            const int jn = locate_from(S.r, N, R, sqrt(Q.x * Q.x + Q.y * Q.y), g.j);
-                                            g2 = geometry_in(S.r, S.ih, Q.x, Q.y, jn);
-                                            S.pj[p] = jn;
-                                        } else {
-                                            g2 = geometry(S.r, S.ih, N, R, Q.x, Q.y);
-                                        }
-                                        j = g2.j;
-                                        deposit_values(Q, g2, S, v);
+                                        // the new cell by a short walk from the old one
+                                        PKeep q;
+                                        polar(Q.x, Q.y, q.rp, q.ir, q.c, q.s);
+                                        j = locate_from(S.r, N, R, q.rp, g.j);
+                                        if (A.pcache) S.pj[p] = j;
+                                        deposit_values(Q, keep_geo(S, q, j), kin, S, v);
                                         act = true;
                                     } else {
                                         atomicAdd(S.lost, 1);
@@ -1903,7 +1946,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                 } else {
                                     const PGeo g2 = pgeo(S, A, N, R, p, Q.x, Q.y);
                                     j = g2.j;
-                                    deposit_values(Q, g2, S, v);
+                                    deposit_values(Q, g2, kin_of(Q.px, Q.py, Q.dl), S, v);
                                     act = true;
                                 }
                             }
@@ -1958,7 +2001,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         coeffs(A.dxi, first);
         if (REG) {
             if (tid < np && P.w != 0.0) {
-                const int pr = push_particle(P, geometry_in(S.r, S.ih, P.x, P.y, J), S, A, first, abc, A.dxi);
+                const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, A.dxi);
                 if (pr <= 0) { atomicAdd(S.lost, 1); if (pr < 0) atomicAdd(S.fx + 12, 1); }
             }
             if (tid < np) pstore(P, A.pout, npad, tid);
@@ -1968,7 +2011,8 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 pload(Q, gate.ps(A), npad, p);
                 species_params(A, p, Q.q, Q.qm);
                 if (Q.w != 0.0) {
-                    const int pr = push_particle(Q, geometry(S.r, S.ih, N, R, Q.x, Q.y), S, A, first, abc, A.dxi);
+                    PKin kin = kin_of(Q.px, Q.py, Q.dl);
+                    const int pr = push_particle(Q, geometry(S.r, S.ih, N, R, Q.x, Q.y), kin, S, A, first, abc, A.dxi);
                     if (pr <= 0) { atomicAdd(S.lost, 1); if (pr < 0) atomicAdd(S.fx + 12, 1); }
                 }
                 pstore(Q, gate.ps(A), npad, p);
