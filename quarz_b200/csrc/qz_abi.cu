@@ -1368,13 +1368,27 @@ qz_status run_pipelined(qz_sim* s, int nsteps, double dt, double* mom_host, cuda
         QZ_CUDA(cudaMemsetAsync(s->sw->d_tim, 0, sizeof(unsigned long long) * 16, st));
         A.sw.timing = s->sw->d_tim;
     }
-    int sms = 0;
-    const int grid = qzb::pipeline_max_grid(A, &sms);
-    if (grid < 2) return fail(QZ_ERR_UNSUPPORTED, "qz_sim_run: the pipelined kernel cannot be resident here");
-    const int g1 = std::min(grid, sms);
-    const int wmin = std::max(8, (2 * g1) / 5);             // measured best: ~2/5 of the SMs push
-    int nsweep = P_.sweep_ctas > 0 ? P_.sweep_ctas : std::min(nsteps + 1, g1 - wmin);
-    nsweep = std::max(1, std::min({nsweep, nsteps + 1, g1 - 1}));
+    int sms = 0, g1 = 0, wmin = 0;
+    auto resident = [&](int team) {
+        A.team = team;
+        const int grid = qzb::pipeline_max_grid(A, &sms);
+        g1 = std::min(grid, sms) / team * team;
+        wmin = std::max(8, (2 * g1) / 5);                   // measured best: ~2/5 of the SMs push
+        return grid >= 2 * team;
+    };
+    // modes = 1: a run with fewer steps than sweep CTAs gives each sweep a cluster of 2, 4 or 8 of them (the
+    // plasma particles of a slice are split over it) where every sweep can have one at the same time; with more
+    // steps than that, single CTAs sweep more steps at once
+    int team = 1;
+    if (A.modes == 1 && !A.sw.filter && P_.sweep_ctas <= 0)
+        for (int t = 8; t > 1; t /= 2)
+            if (A.sw.np > (t / 2) * qzb::kSweepThreads && resident(t) && (nsteps + 1) * t <= g1 - wmin) {
+                team = t;
+                break;
+            }
+    if (!resident(team)) return fail(QZ_ERR_UNSUPPORTED, "qz_sim_run: the pipelined kernel cannot be resident here");
+    int nsweep = P_.sweep_ctas > 0 ? P_.sweep_ctas : std::min((nsteps + 1) * team, g1 - wmin);
+    nsweep = std::max(1, std::min({nsweep, (nsteps + 1) * team, g1 - 1}));
     // 3. buffers
     const size_t KM = (size_t)K * M;
     const size_t bslot = sim_bsrc_doubles(s);           // a beam-source slot: two limbs per value for m = 0

@@ -184,15 +184,16 @@ struct PipeArgs {
     SweepArgs sw;                   // bsrc / fld / diag / ps of sw are unused: rings below
     int nsteps;                     // sweeps 0..nsteps, pushes 0..nsteps-1
     int nsweep;                     // CTAs running sweeps
+    int team;                       // modes = 1: CTAs per sweep, a cluster (nsweep and the grid are multiples of it)
     int ring;                       // slots of the field / diagnostics / beam-source rings
     // the push workers gather the fields through L1: set when no field slot is reused within the run
     // (ring > nsteps) and every field row starts on a 128-byte line, so no cached line can hold a row
     // before the sweep published it (rows are only read once published, and kernels start with L1 clean)
     int fld_l1;
     int modes, bnc;                 // azimuthal modes (0 / 1), beam-source components per node
-    size_t fld_slot, diag_slot, bsrc_slot, ps_slot;   // doubles per slot (ps: per sweep CTA)
+    size_t fld_slot, diag_slot, bsrc_slot, ps_slot;   // doubles per slot (ps: per team of sweep CTAs)
     double *fld, *diag, *bsrc, *ps;
-    double* m1s;                    // modes = 1: per sweep CTA, background (3 M) + source buffers (60 M)
+    double* m1s;                    // modes = 1: per team of sweep CTAs, background (3 M) + source buffers (60 M)
     size_t m1s_slot;
     int nbeams;
     BeamArgs beam[kMaxBeams];
@@ -232,7 +233,7 @@ constexpr int kTraceStride = 22;
 constexpr int kWorkerTotals = 6;    // trace totals of the push workers after the steps
 
 size_t pipeline_smem_bytes(int modes, int M, bool dbuf, bool const_smem, bool filter = false, int pcache = 0);
-// resident CTAs of the pipeline kernel on this device (0 if it cannot run); *sms: the SM count
+// resident CTAs of the pipeline kernel on this device, in clusters of P.team (0 if it cannot run); *sms: the SM count
 int pipeline_max_grid(const PipeArgs& P, int* sms);
 // cooperative launch of grid CTAs (fails unless all of them can be resident at once)
 cudaError_t launch_pipeline(const PipeArgs& P, int grid, cudaStream_t stream);

@@ -159,21 +159,22 @@ int pipeline_max_grid(const PipeArgs& P, int* sms) {
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     *sms = nsm;
     const size_t smem = pipeline_smem_bytes(P.modes, P.sw.M, P.sw.dbuf, P.sw.const_smem, P.sw.filter != 0, P.sw.pcache);
-    int per = 0;
+    int per = 0;                     // resident CTAs
     switch (P.sw.ord) {
-        case 1: per = pipeline_occupancy_ord<1>(P, smem); break;
-        case 2: per = pipeline_occupancy_ord<2>(P, smem); break;
-        case 3: per = pipeline_occupancy_ord<3>(P, smem); break;
-        case 4: per = pipeline_occupancy_ord<4>(P, smem); break;
-        case 5: per = pipeline_occupancy_ord<5>(P, smem); break;
+        case 1: per = pipeline_occupancy_ord<1>(P, smem, nsm); break;
+        case 2: per = pipeline_occupancy_ord<2>(P, smem, nsm); break;
+        case 3: per = pipeline_occupancy_ord<3>(P, smem, nsm); break;
+        case 4: per = pipeline_occupancy_ord<4>(P, smem, nsm); break;
+        case 5: per = pipeline_occupancy_ord<5>(P, smem, nsm); break;
         default: return 0;
     }
-    return per * nsm;
+    return per;
 }
 
 cudaError_t launch_pipeline(const PipeArgs& P, int grid, cudaStream_t stream) {
     if (P.sw.rows_per_thread < 1 || P.sw.rows_per_thread > 4) return cudaErrorInvalidValue;
     if (P.nsweep < 1 || grid <= P.nsweep || P.ring < 2 || P.nbeams > kMaxBeams) return cudaErrorInvalidValue;
+    if (P.team < 1 || P.nsweep % P.team || grid % P.team || (P.team > 1 && P.modes != 1)) return cudaErrorInvalidValue;
     const size_t smem = pipeline_smem_bytes(P.modes, P.sw.M, P.sw.dbuf, P.sw.const_smem, P.sw.filter != 0, P.sw.pcache);
     switch (P.sw.ord) {
         case 1: return pipeline_launch_ord<1>(P, grid, smem, stream);

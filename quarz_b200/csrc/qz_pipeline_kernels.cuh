@@ -78,7 +78,8 @@ struct GateState {
     const double* bsrc;   // this step's ring slots
     double* fld;
     double* diag;
-    double* ps;           // this CTA's plasma scratch
+    double* ps;           // this team's plasma scratch
+    double* m1s;          // and its background and source buffers (modes = 1)
     int n;                // time step of this sweep
     int cursor;           // buckets [0, cursor) are known to have pushed step n-1
 };
@@ -93,8 +94,8 @@ struct PipeGate {
     __device__ double* fld(const SweepArgs&) const { return g->fld; }
     __device__ double* diag(const SweepArgs&) const { return g->diag; }
     __device__ double* ps(const SweepArgs&) const { return g->ps; }
-    __device__ double* bgs(const SweepArgs&) const { return P->m1s + blockIdx.x * P->m1s_slot; }
-    __device__ double* srcs(const SweepArgs&) const { return P->m1s + blockIdx.x * P->m1s_slot + 3 * (size_t)P->sw.M; }
+    __device__ double* bgs(const SweepArgs&) const { return g->m1s; }
+    __device__ double* srcs(const SweepArgs&) const { return g->m1s + 3 * (size_t)P->sw.M; }
     __device__ double* traj(const SweepArgs&) const { return P->traj ? P->traj + (size_t)g->n * P->traj_slot : nullptr; }
     __device__ double* wrec(const SweepArgs& A) const {
         return P->wrec ? P->wrec + (size_t)g->n * A.K * A.M : nullptr;
@@ -138,13 +139,13 @@ struct PipeGate {
         return true;
     }
     // every thread, after its stores of slice k: row k-1 of the beam sources is no longer needed
-    __device__ void slice_done_all(int k) {
+    __device__ void slice_done_all(int k, int rank = 0, int size = 1) {
         if (k >= 1) {
             const int nr = P->sw.M * P->bnc;
             double* row = const_cast<double*>(g->bsrc) + (size_t)(k - 1) * nr;
-            for (int i = threadIdx.x; i < nr; i += kT) __stcg(row + i, 0.0);
+            for (int i = rank * kT + threadIdx.x; i < nr; i += size * kT) __stcg(row + i, 0.0);
             if (P->sw.bq)                            // the low limbs of the exact deposits
-                for (int i = threadIdx.x; i < nr; i += kT) __stcg(row + P->sw.bfx_lo + i, 0.0);
+                for (int i = rank * kT + threadIdx.x; i < nr; i += size * kT) __stcg(row + P->sw.bfx_lo + i, 0.0);
         }
     }
     // thread 0, after the barrier that ends slice k: publish it (the fence covers the stores of the
@@ -168,32 +169,41 @@ __device__ __forceinline__ void sweep_role(const PipeArgs& P, double* smem) {
     __shared__ GateState gs;
     const int tid = threadIdx.x;
     const int K = P.sw.K, M = P.sw.M;
-    for (int n = blockIdx.x; n <= P.nsteps; n += P.nsweep) {
+    Team team;                                        // modes = 1: the CTAs of a cluster share a sweep
+    if constexpr (MODES == 1) team = Team::of_cluster();
+    const int ti = blockIdx.x / team.size;
+    for (int n = ti; n <= P.nsteps; n += P.nsweep / team.size) {
         const int slot = n % P.ring;
         if (tid == 0) {
-            s_ok = (n < P.ring) ? 1 : (wait_ge(P, P.pdone + (n - P.ring), P.nbk, W_RING) ? 1 : 0);
+            s_ok = 1;
+            if (team.rank == 0 && n >= P.ring) s_ok = wait_ge(P, P.pdone + (n - P.ring), P.nbk, W_RING) ? 1 : 0;
             gs.bsrc = P.bsrc + slot * P.bsrc_slot;
             gs.fld = P.fld + slot * P.fld_slot;
             gs.diag = P.diag + slot * P.diag_slot;
-            gs.ps = P.ps + blockIdx.x * P.ps_slot;
+            gs.ps = P.ps + ti * P.ps_slot;
+            gs.m1s = MODES == 1 ? P.m1s + ti * P.m1s_slot : nullptr;
             gs.n = n;
             gs.cursor = 0;
         }
-        __syncthreads();
-        if (!s_ok) return;
-        if (P.trace && tid == 0) P.trace[(size_t)kTraceStride * n] = gtimer();
+        team.sync();
+        if (!team.of_first(&s_ok)) {
+            if (team.size > 1) team.sync();           // rank 0's word has been read by all
+            return;
+        }
+        if (P.trace && tid == 0 && team.rank == 0) P.trace[(size_t)kTraceStride * n] = gtimer();
         PipeGate g{&P, &gs};
-        const bool ok = MODES == 1 ? sweep_m1_body<ORD, PipeGate, EXT>(P.sw, smem, g)
-                                   : sweep_body<ORD, REG, kMaxR, PipeGate, EXT>(P.sw, smem, g);
+        bool ok;
+        if constexpr (MODES == 1) ok = sweep_m1_body<ORD, PipeGate, EXT>(P.sw, smem, g, team);
+        else ok = sweep_body<ORD, REG, kMaxR, PipeGate, EXT>(P.sw, smem, g);
         if (!ok) return;
         // the last row (the others were zeroed slice by slice)
         const int nr = M * P.bnc;
         double* row = P.bsrc + slot * P.bsrc_slot + (size_t)(K - 1) * nr;
-        for (int i = tid; i < nr; i += kT) __stcg(row + i, 0.0);
+        for (int i = team.rank * kT + tid; i < nr; i += team.size * kT) __stcg(row + i, 0.0);
         if (P.sw.bq)
             for (int i = tid; i < nr; i += kT) __stcg(row + P.sw.bfx_lo + i, 0.0);
-        __syncthreads();
-        if (tid == 0) {
+        team.sync();
+        if (tid == 0 && team.rank == 0) {
             __threadfence();
             st_release(P.sdone + n, 1);
             if (P.trace) P.trace[(size_t)kTraceStride * n + 1] = gtimer();
@@ -542,22 +552,52 @@ __global__ void moments_reduce_kernel(const __grid_constant__ PipeArgs P, double
     mom[((size_t)n * P.nbeams + q) * 17 + c] = v;
 }
 
+// launch configuration; *at: the cluster dimension for teams of several CTAs
+inline cudaLaunchConfig_t pipe_config(const PipeArgs& P, int grid, size_t smem, cudaLaunchAttribute* at) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = P.team;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.dynamicSmemBytes = smem;
+    return cfg;
+}
+
 template <int MODES, int ORD, bool REG, int RM, bool EXT = false>
 cudaError_t launch_t(const PipeArgs& P, int grid, size_t smem, cudaStream_t stream) {
     auto fn = pipeline_kernel<MODES, ORD, REG, RM, EXT>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    void* args[] = {(void*)&P};
-    return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(kSweepThreads), args, smem, stream);
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = pipe_config(P, grid, smem, at + 1);
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = P.team > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, fn, P);
 }
 
+// CTAs resident at once, nsm SMs
 template <int MODES, int ORD, bool REG, int RM, bool EXT = false>
-int occupancy_t(size_t smem) {
+int occupancy_t(const PipeArgs& P, size_t smem, int nsm) {
     auto fn = pipeline_kernel<MODES, ORD, REG, RM, EXT>;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int nb = 0;
+    if (P.team > 1) {
+        cudaLaunchAttribute at;
+        cudaLaunchConfig_t cfg = pipe_config(P, nsm / P.team * P.team, smem, &at);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&nb, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return nb * P.team;
+    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kSweepThreads, smem) != cudaSuccess) return 0;
-    return nb;
+    return nb * nsm;
 }
 
 // modes = 1 runs one row per thread with the plasma in the scratch (REG and kMaxR unused: false, 1)
@@ -578,18 +618,18 @@ cudaError_t launch_o(const PipeArgs& P, int grid, size_t smem, cudaStream_t s) {
 }
 
 template <int ORD, bool EXT>
-int occupancy_e(const PipeArgs& P, size_t smem) {
+int occupancy_e(const PipeArgs& P, size_t smem, int nsm) {
     const bool reg = P.sw.np <= kSweepThreads;
     if (P.sw.rows_per_thread == 1)
-        return reg ? occupancy_t<0, ORD, true, 1, EXT>(smem) : occupancy_t<0, ORD, false, 1, EXT>(smem);
-    return reg ? occupancy_t<0, ORD, true, 4, EXT>(smem) : occupancy_t<0, ORD, false, 4, EXT>(smem);
+        return reg ? occupancy_t<0, ORD, true, 1, EXT>(P, smem, nsm) : occupancy_t<0, ORD, false, 1, EXT>(P, smem, nsm);
+    return reg ? occupancy_t<0, ORD, true, 4, EXT>(P, smem, nsm) : occupancy_t<0, ORD, false, 4, EXT>(P, smem, nsm);
 }
 
 template <int ORD>
-int occupancy_o(const PipeArgs& P, size_t smem) {
+int occupancy_o(const PipeArgs& P, size_t smem, int nsm) {
     const bool ext = P.sw.filter || P.sw.bstat;
-    if (P.modes == 1) return ext ? occupancy_t<1, ORD, false, 1, true>(smem) : occupancy_t<1, ORD, false, 1, false>(smem);
-    return ext ? occupancy_e<ORD, true>(P, smem) : occupancy_e<ORD, false>(P, smem);
+    if (P.modes == 1) return ext ? occupancy_t<1, ORD, false, 1, true>(P, smem, nsm) : occupancy_t<1, ORD, false, 1, false>(P, smem, nsm);
+    return ext ? occupancy_e<ORD, true>(P, smem, nsm) : occupancy_e<ORD, false>(P, smem, nsm);
 }
 
 }  // namespace
@@ -599,6 +639,6 @@ int occupancy_o(const PipeArgs& P, size_t smem) {
 template <int ORD>
 cudaError_t pipeline_launch_ord(const PipeArgs& P, int grid, size_t smem, cudaStream_t s);
 template <int ORD>
-int pipeline_occupancy_ord(const PipeArgs& P, size_t smem);
+int pipeline_occupancy_ord(const PipeArgs& P, size_t smem, int nsm);
 
 }  // namespace qzb

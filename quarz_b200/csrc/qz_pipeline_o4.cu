@@ -9,8 +9,8 @@ cudaError_t pipeline_launch_ord<4>(const PipeArgs& P, int grid, size_t smem, cud
 }
 
 template <>
-int pipeline_occupancy_ord<4>(const PipeArgs& P, size_t smem) {
-    return occupancy_o<4>(P, smem);
+int pipeline_occupancy_ord<4>(const PipeArgs& P, size_t smem, int nsm) {
+    return occupancy_o<4>(P, smem, nsm);
 }
 
 }  // namespace qzb

@@ -9,8 +9,8 @@ cudaError_t pipeline_launch_ord<5>(const PipeArgs& P, int grid, size_t smem, cud
 }
 
 template <>
-int pipeline_occupancy_ord<5>(const PipeArgs& P, size_t smem) {
-    return occupancy_o<5>(P, smem);
+int pipeline_occupancy_ord<5>(const PipeArgs& P, size_t smem, int nsm) {
+    return occupancy_o<5>(P, smem, nsm);
 }
 
 }  // namespace qzb

@@ -39,7 +39,8 @@ constexpr unsigned FULL = 0xffffffffu;
 struct NoGate {
     static constexpr bool kActive = false;
     __device__ bool before_rows(int) { return true; }       // warp 0: beam-source rows <= row are final
-    __device__ void slice_done_all(int) {}                   // every thread, after its stores of slice k
+    __device__ void slice_done_all(int, int = 0, int = 1) {} // every thread, after its stores of slice k (its CTA's
+                                                             // rank in, and the size of, the team that sweeps)
     __device__ bool slice_done(int) { return true; }         // thread 0, after the barrier: publish slice k
     // this sweep's buffers
     __device__ const double* bsrc(const SweepArgs& A) const { return A.bsrc; }

@@ -14,7 +14,7 @@ template <int ORD, bool EXT>
 __global__ void __launch_bounds__(kSweepThreads, 1) sweep_m1_kernel(const SweepArgs A) {
     extern __shared__ double smem_raw[];
     NoGate g;
-    sweep_m1_body<ORD, NoGate, EXT>(A, smem_raw, g);
+    sweep_m1_body<ORD, NoGate, EXT>(A, smem_raw, g, Team::of_cluster());
 }
 
 template <int ORD, bool EXT>
@@ -22,8 +22,30 @@ cudaError_t launch_e(const SweepArgs& A, size_t smem, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(sweep_m1_kernel<ORD, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    sweep_m1_kernel<ORD, EXT><<<1, kSweepThreads, smem, stream>>>(A);
-    return cudaGetLastError();
+    // the particles of a slice over a cluster of up to 8 CTAs (the smoothing filter works in place on the shared
+    // sources: one CTA); 8 is the largest portable size, and each CTA has at least a particle per thread then
+    int team = 1;
+    if (!A.filter)
+        while (team < 8 && A.np > team * kSweepThreads) team *= 2;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    for (;; team /= 2) {
+        at.val.clusterDim.x = team;
+        cfg.gridDim = dim3(team);
+        int fit = 0;                       // a device (partition) may not hold a cluster of this size
+        if (team > 1 && (cudaOccupancyMaxActiveClusters(&fit, sweep_m1_kernel<ORD, EXT>, &cfg) != cudaSuccess || fit < 1)) {
+            cudaGetLastError();
+            continue;
+        }
+        return cudaLaunchKernelEx(&cfg, sweep_m1_kernel<ORD, EXT>, A);
+    }
 }
 
 template <int ORD>

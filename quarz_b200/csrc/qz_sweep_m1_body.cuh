@@ -30,6 +30,37 @@ namespace m1_detail {
 
 using namespace sweep_detail;
 
+// The CTAs that share one sweep: a thread-block cluster (size > 1, this CTA's rank in it), or this CTA alone. The
+// particles are split over the team (they are 60 to 75 % of a slice); every member solves the slice's fields
+// for itself from the sources in L2, so that only the barriers are shared.
+struct Team {
+    int rank = 0, size = 1;
+    // this CTA's cluster (a kernel launched without cluster dimensions: a team of one)
+    static __device__ __forceinline__ Team of_cluster() {
+        Team t;
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(t.rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(t.size));
+        return t;
+    }
+    __device__ __forceinline__ void sync() const {
+        if (size > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    }
+    // the value of an int in the shared memory of rank 0 (p: this CTA's own copy of it)
+    __device__ __forceinline__ int of_first(const int* p) const {
+        if (size == 1) return *p;
+        unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+        int v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(r) : "memory");
+        return v;
+    }
+};
+
 struct Msc { double *a0, *ar, *ai; };                  // scalar in modes: f0 + 2 Re(f1 e^{i theta})
 struct Mvec { double *r0, *i0, *r1, *i1, *r2, *i2; };  // vector V+ = sum_k v_k e^{i k theta}, k = 0, 1, 2
 
@@ -42,7 +73,7 @@ struct Smem1 {
     double *r, *iv, *ih;
     Msc psi, ez, bz;
     Mvec wp, bp;
-    double* tot;                                       // scan scratch: 2 x 16 x kW
+    double* tot;                                       // scan scratch: 2 x 16 x kW (the groups: 4 x 2 x kTotG)
     int* lost;
     int* flag;
 };
@@ -84,13 +115,11 @@ __device__ __forceinline__ Smem1 carve1(double* base, int M) {
     return S;
 }
 
-// operator constants (global, read-only): stencils, 1/r, L0 Thomas factors, L1D and L1F rows (consts,
-// 13 x M), L1D Thomas factors, L0 rows, L2D rows (consts1, 9 x M)
+// operator constants (global, read-only): stencils, 1/r, L1D and L1F rows (of consts, 13 x M), L0 rows and L2D
+// rows (of consts1, 9 x M); the Thomas factors of L0 and L1D are in them too (solve_fixed)
 struct Consts1 {
     const double *gm, *g0, *gp, *ir;
-    const double *l0r, *l0f, *l0b;
     const double *l1a, *l1b, *l1c, *lfa, *lfb, *lfc;
-    const double *d1r, *d1f, *d1b;
     const double *o0a, *o0b, *o0c, *o2a, *o2b, *o2c;
 };
 
@@ -100,10 +129,8 @@ __device__ __forceinline__ Consts1 consts1(const SweepArgs& A) {
     const double* u = A.consts1;
     Consts1 C;
     C.gm = q; C.g0 = q + M; C.gp = q + 2 * M; C.ir = q + 3 * M;
-    C.l0r = q + 4 * M; C.l0f = q + 5 * M; C.l0b = q + 6 * M;
     C.l1a = q + 7 * M; C.l1b = q + 8 * M; C.l1c = q + 9 * M;
     C.lfa = q + 10 * M; C.lfb = q + 11 * M; C.lfc = q + 12 * M;
-    C.d1r = u; C.d1f = u + M; C.d1b = u + 2 * M;
     C.o0a = u + 3 * M; C.o0b = u + 4 * M; C.o0c = u + 5 * M;
     C.o2a = u + 6 * M; C.o2b = u + 7 * M; C.o2c = u + 8 * M;
     return C;
@@ -255,6 +282,235 @@ __device__ __forceinline__ void scan_bwd_g(const double (&a)[NA], const double (
         const double cw = __shfl_sync(FULL, tb[r], (warp + 1) & 31);
         xa[r] = fma(eA[g[r]], warp < kW - 1 ? cw : 0.0, eB[r]);
     }
+}
+
+// ---------------------------------------------------------------- solves by groups of warps
+// Like the m = 0 sweep's (l0_solve, bplus_solve), a quarter of the warps per operator: P2 L0 with three right-
+// hand sides and L1D with three pairs, P4 the four chi_0-shifted operators with one or two right-hand sides.
+// A thread owns up to 5 rows (M <= 5 x 32 x kG holds for every M the CTA takes); the right-hand sides are read
+// from, and the solutions written to, the same shared arrays, each thread its own rows. With one row per thread
+// and block-wide scans, P2 took 25,100 and P4 89,600 cycles per slice of the hosing grid (shuffles: one per cycle
+// and SM), now 6,800 and 24,000.
+constexpr int kG = kW / 4;                             // warps per group
+constexpr int kR1 = 5;                                 // most rows per thread
+constexpr int kTotG = 16 * kG;                         // doubles of one half of the groups' scan scratch
+
+// exclusive scan of NB affine maps y -> a y + b[n] sharing the slope a, in thread order of the group (kUp) or in
+// reverse; on return b[n] is y before this thread's rows. tot: (1 + NB) doubles per warp
+template <int NB, bool kUp>
+__device__ __forceinline__ void group_affine_n(double a, double (&b)[NB], int wl, double* tot, int id) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+        const double ap = kUp ? __shfl_up_sync(FULL, a, st) : __shfl_down_sync(FULL, a, st);
+        double bp[NB];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) bp[n] = kUp ? __shfl_up_sync(FULL, b[n], st) : __shfl_down_sync(FULL, b[n], st);
+        if (kUp ? lane >= st : lane + st < 32) {
+#pragma unroll
+            for (int n = 0; n < NB; ++n) b[n] = fma(a, bp[n], b[n]);
+            a *= ap;
+        }
+    }
+    if (lane == (kUp ? 31 : 0)) {
+        tot[wl * (1 + NB)] = a;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) tot[wl * (1 + NB) + 1 + n] = b[n];
+    }
+    double ea = kUp ? __shfl_up_sync(FULL, a, 1) : __shfl_down_sync(FULL, a, 1);
+    const bool edge = lane == (kUp ? 0 : 31);
+    if (edge) ea = 1.0;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+        b[n] = kUp ? __shfl_up_sync(FULL, b[n], 1) : __shfl_down_sync(FULL, b[n], 1);
+        if (edge) b[n] = 0.0;
+    }
+    group_sync(id, 32 * kG);
+    double c[NB];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) c[n] = 0.0;
+#pragma unroll
+    for (int w = 0; w < kG; ++w) {
+        const int o = kUp ? w : kG - 1 - w;
+        if (kUp ? o < wl : o > wl)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) c[n] = fma(tot[o * (1 + NB)], c[n], tot[o * (1 + NB) + 1 + n]);
+    }
+#pragma unroll
+    for (int n = 0; n < NB; ++n) b[n] = fma(ea, c[n], b[n]);
+}
+
+// Thomas substitutions of NB systems of one operator on a thread's rows, right-hand sides v on entry, solutions
+// on return: y_i = fa_i y_{i-1} + ri_i v_i, x_i = ba_i x_{i+1} + y_i. Rows past the thread's carry fa = ba = 1, ri = 0.
+template <int NB>
+__device__ __forceinline__ void group_thomas(double (&v)[kR1][NB], const double (&ri)[kR1], const double (&fa)[kR1],
+                                             const double (&ba)[kR1], int wl, double* t0, double* t1, int id) {
+    double a = 1.0, y[NB];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) y[n] = 0.0;
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        a *= fa[u];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            v[u][n] *= ri[u];
+            y[n] = fma(fa[u], y[n], v[u][n]);
+        }
+    }
+    group_affine_n<NB, true>(a, y, wl, t0, id);
+    a = 1.0;
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        a *= ba[u];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            y[n] = fma(fa[u], y[n], v[u][n]);
+            v[u][n] = y[n];
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NB; ++n) y[n] = 0.0;
+    // rows past the thread's own (ri = 0) carry y along in the forward pass; they are not part of the solution
+#pragma unroll
+    for (int u = kR1 - 1; u >= 0; --u)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            if (ri[u] == 0.0) v[u][n] = 0.0;
+            y[n] = fma(ba[u], y[n], v[u][n]);
+        }
+    group_affine_n<NB, false>(a, y, wl, t1, id);
+#pragma unroll
+    for (int u = kR1 - 1; u >= 0; --u)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            y[n] = fma(ba[u], y[n], v[u][n]);
+            v[u][n] = y[n];
+        }
+}
+
+// NB systems of an operator with the host's Thomas factors 1/u, -a/u, -c/u (th, 3 x M), in place
+template <int NB>
+__device__ __forceinline__ void solve_fixed(double* const (&f)[NB], const double* th, int M, int R, int row0, int wl,
+                                            double* t0, double* t1, int id) {
+    double v[kR1][NB], ri[kR1], fa[kR1], ba[kR1];
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const int i = row0 + u;
+        const bool on = u < R && i < M;
+        ri[u] = on ? ldc(th + i) : 0.0;
+        fa[u] = on ? ldc(th + M + i) : 1.0;
+        ba[u] = on ? ldc(th + 2 * (size_t)M + i) : 1.0;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) v[u][n] = on ? f[n][i] : 0.0;
+    }
+    group_thomas<NB>(v, ri, fa, ba, wl, t0, t1, id);
+#pragma unroll
+    for (int u = 0; u < kR1; ++u)
+        if (u < R && row0 + u < M)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) f[n][row0 + u] = v[u][n];
+}
+
+// The factors of one chi_0-shifted operator on a thread's rows (they do not change over the Picard iterations)
+struct Fac1 { double ri[kR1], fa[kR1], ba[kR1], b[kR1]; };
+
+// rows a, b, c (unshifted b) of operator sy (row_bp's order); A.consts1 holds L0 and L2D, A.consts L1D and L1F
+__device__ __forceinline__ void op_rows(const Consts1& C, int sy, const double*& a, const double*& b, const double*& c) {
+    a = sy == 0 ? C.l1a : (sy == 1 ? C.lfa : (sy == 2 ? C.o0a : C.o2a));
+    b = sy == 0 ? C.l1b : (sy == 1 ? C.lfb : (sy == 2 ? C.o0b : C.o2b));
+    c = sy == 0 ? C.l1c : (sy == 1 ? C.lfc : (sy == 2 ? C.o0c : C.o2c));
+}
+// Dirichlet rows: 0 and N (L1D, L2D), 0 (L1F), N (L0)
+__device__ __forceinline__ bool op_dirichlet(int sy, int i, int N) {
+    return (i == 0 && sy != 2) || (i == N && sy != 1);
+}
+
+// sources of a slice's pivots: chi_0 of the slice (global scratch)
+__device__ __forceinline__ void factor_op(const Consts1& C, const double* chi0, int sy, int M, int N, int R, int row0,
+                                          int wl, double* t0, int id, Fac1& F) {
+    const double *pa, *pb, *pc;
+    op_rows(C, sy, pa, pb, pc);
+    double m[4] = {1.0, 0.0, 0.0, 1.0};
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const int i = row0 + u;
+        F.b[u] = 1.0; F.fa[u] = 0.0; F.ba[u] = 0.0;            // fa: a_i, ba: c_{i-1} for now
+        if (u < R && i < M) {
+            F.fa[u] = ldc(pa + i);
+            F.b[u] = ldc(pb + i);
+            F.ba[u] = i > 0 ? ldc(pc + i - 1) : 0.0;
+            if (!op_dirichlet(sy, i, N)) F.b[u] = F.b[u] - lg(chi0 + i);
+            const double t01 = -F.fa[u] * F.ba[u];
+            const double n00 = F.b[u] * m[0] + t01 * m[2], n01 = F.b[u] * m[1] + t01 * m[3];
+            m[2] = m[0]; m[3] = m[1];
+            m[0] = n00; m[1] = n01;
+            if (u == 2) renorm(m[0], m[1], m[2], m[3]);
+        }
+    }
+    renorm(m[0], m[1], m[2], m[3]);
+    double p, q;
+    group_pivots<kG>(m, p, q, wl, t0, id);
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const double pn = F.b[u] * p - F.fa[u] * F.ba[u] * q;
+        q = p;
+        p = pn;
+        pivot_scale(p, q);
+        F.ri[u] = pivot_quot(q, p);                              // 1/u_i = p_{i-1} / p_i
+    }
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const int i = row0 + u;
+        if (u < R && i < M) {
+            F.fa[u] = -F.ri[u] * F.fa[u];
+            F.ba[u] = -(ldc(pc + i) * F.ri[u]);
+        } else {
+            F.ri[u] = 0.0; F.fa[u] = 1.0; F.ba[u] = 1.0;
+        }
+    }
+}
+
+// (op - chi_0) x = d in place for NB systems, with one step of iterative refinement on the same factors: the
+// pivots come from a prefix product, slightly less accurate than Thomas' recurrence on these ill-conditioned
+// rows (L1D on a 100x-stretched grid); r = d - A x with the exact rows, then x += A^-1 r
+template <int NB>
+__device__ __forceinline__ void solve_shifted(double* const (&f)[NB], const Consts1& C, const Fac1& F, int sy, int M,
+                                              int N, int R, int row0, int wl, double* tot, int id) {
+    double d[kR1][NB], v[kR1][NB];
+#pragma unroll
+    for (int u = 0; u < kR1; ++u)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            d[u][n] = u < R && row0 + u < M ? f[n][row0 + u] : 0.0;
+            v[u][n] = d[u][n];
+        }
+    group_thomas<NB>(v, F.ri, F.fa, F.ba, wl, tot, tot + kTotG, id);
+#pragma unroll
+    for (int u = 0; u < kR1; ++u)
+        if (u < R && row0 + u < M)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) f[n][row0 + u] = v[u][n];
+    group_sync(id, 32 * kG);
+    const double *pa, *pb, *pc;
+    op_rows(C, sy, pa, pb, pc);
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const int i = row0 + u;
+        const bool on = u < R && i < M;
+        const double a = on ? ldc(pa + i) : 0.0, c = on ? ldc(pc + i) : 0.0;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            const double xm = on && i > 0 ? f[n][i - 1] : 0.0, xp = on && i < N ? f[n][i + 1] : 0.0;
+            d[u][n] = on ? d[u][n] - (a * xm + F.b[u] * f[n][i] + c * xp) : 0.0;
+        }
+    }
+    group_thomas<NB>(d, F.ri, F.fa, F.ba, wl, tot, tot + kTotG, id);
+    group_sync(id, 32 * kG);                              // the neighbours' rows have been read
+#pragma unroll
+    for (int u = 0; u < kR1; ++u)
+        if (u < R && row0 + u < M)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) f[n][row0 + u] += d[u][n];
 }
 
 // ---------------------------------------------------------------- sources of a slice
@@ -432,8 +688,8 @@ template <int ORD>
 __device__ __forceinline__ Dep1 dep1_basics(const PState<ORD>& P, const PGeo& g, const Smem1& S) {
     Dep1 d;
     const double PX = P.px, PY = P.py, D = P.dl, w = P.w;
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const PKin kin = kin_of(PX, PY, D);
+    const double gam = kin.gam, invd = kin.invd;
     const double pz = gam - D;
     d.ux = PX * invd; d.uy = PY * invd;
     d.c = g.c; d.s = g.s;
@@ -546,8 +802,8 @@ __device__ __forceinline__ void depositS1_values(const PState<ORD>& P, const PGe
     const double qm = P.qm;
     const double PX = P.px, PY = P.py, D = P.dl;
     const PF1 F = gather1(S, g, false);
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const PKin kin = kin_of(PX, PY, D);
+    const double gam = kin.gam, invd = kin.invd;
     const double ux = PX * invd, uy = PY * invd;
     const double ur = g.c * ux + g.s * uy, uth = g.c * uy - g.s * ux;
     const double dD = qm * ((PX * F.Wx + PY * F.Wy) * invd - F.Ez);
@@ -603,8 +859,8 @@ template <int ORD>
 __device__ __forceinline__ bool push1(PState<ORD>& P, const PF1& F, const SweepArgs& A, bool first) {
     const double qm = P.qm;
     const double X = P.x, Y = P.y, PX = P.px, PY = P.py, D = P.dl;
-    const double gam = (1.0 + PX * PX + PY * PY + D * D) / (2.0 * D);
-    const double invd = 1.0 / D;
+    const PKin kin = kin_of(PX, PY, D);
+    const double gam = kin.gam, invd = kin.invd;
     double fv[5];
     fv[0] = PX * invd;
     fv[1] = PY * invd;
@@ -663,10 +919,11 @@ __device__ __forceinline__ bool push1(PState<ORD>& P, const PF1& F, const SweepA
 
 // deposit of all particles of the scratch into the current source arrays (warp by warp)
 template <int ORD, class Gate>
-__device__ __forceinline__ void deposit_all1(const SweepArgs& A, const Smem1& S, const Src1& T, Gate& gate) {
+__device__ __forceinline__ void deposit_all1(const SweepArgs& A, const Smem1& S, const Src1& T, Gate& gate,
+                                             const Team& team) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int np = A.np, npad = A.npad, N = A.N;
-    for (int base = tid - lane; base < np; base += kThreads) {
+    for (int base = team.rank * kThreads + tid - lane; base < np; base += team.size * kThreads) {
         const int p = base + lane;
         bool act = false;
         int j = 0;
@@ -688,29 +945,6 @@ __device__ __forceinline__ void deposit_all1(const SweepArgs& A, const Smem1& S,
     }
 }
 
-// row i of the B+ systems (src/FieldSolver.cpp:172-191 with chi = chi_0):
-//   sys 0: L1D - chi (Dirichlet 0, N)   sys 1: L1F - chi (Dirichlet 0, flux row N)
-//   sys 2: L0 - chi (regular axis, Dirichlet N)   sys 3: L2D - chi (Dirichlet 0, N)
-// a, b, c of the row and c_{i-1}; dir = the row is a Dirichlet row (its right-hand side is 0)
-__device__ __forceinline__ void row_bp(const Consts1& C, const Src1& T, int N, int sys, int i, double& a, double& b,
-                                       double& c, double& cm, bool& dir) {
-    const double chi = lg(T.chi.a0 + i);
-    if (sys == 0) {
-        a = ldc(C.l1a + i); b = ldc(C.l1b + i); c = ldc(C.l1c + i); cm = i > 0 ? ldc(C.l1c + i - 1) : 0.0;
-        dir = (i == 0 || i == N);
-    } else if (sys == 1) {
-        a = ldc(C.lfa + i); b = ldc(C.lfb + i); c = ldc(C.lfc + i); cm = i > 0 ? ldc(C.lfc + i - 1) : 0.0;
-        dir = (i == 0);
-    } else if (sys == 2) {
-        a = ldc(C.o0a + i); b = ldc(C.o0b + i); c = ldc(C.o0c + i); cm = i > 0 ? ldc(C.o0c + i - 1) : 0.0;
-        dir = (i == N);
-    } else {
-        a = ldc(C.o2a + i); b = ldc(C.o2b + i); c = ldc(C.o2c + i); cm = i > 0 ? ldc(C.o2c + i - 1) : 0.0;
-        dir = (i == 0 || i == N);
-    }
-    if (!dir) b = b - chi;
-}
-
 }  // namespace m1_detail
 
 using namespace m1_detail;
@@ -718,20 +952,27 @@ using namespace m1_detail;
 size_t sweep_m1_smem_bytes(int M);
 
 // One m = 1 sweep by the calling CTA (kThreads threads, one radial row per thread: M <= kThreads).
-// EXT: the variant that also handles the smoothing filter (A.filter) and static beam sources (A.bstat)
+// EXT: the variant that also handles the smoothing filter (A.filter; a team of one) and static beam sources
+// (A.bstat). team: every CTA of it calls this, with the same arguments
 template <int ORD, class Gate, bool EXT = false>
-__device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_raw, Gate& gate) {
+__device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_raw, Gate& gate,
+                                              const Team team = Team()) {
     const int M = A.M, N = A.N, K = A.K;
     const int tid = threadIdx.x;
     const int i = tid;                                           // this thread's row
     const bool row = i < M;
+    const bool mine = row && ((i >> 5) % team.size) == team.rank;   // rows whose global arrays this member writes
+    const int first_p = team.rank * kThreads + tid, step_p = team.size * kThreads;   // its particles
     const Smem1 S = carve1(smem_raw, M);
     double* const scr = gate.srcs(A);                            // 2 x 30 x M sources, global
     const Consts1 C = consts1(A);
     const int np = A.np, npad = A.npad, lane = tid & 31;
     const double R = A.R;
     double* bg = gate.bgs(A);                                    // (3, M) background, global scratch
-    unsigned long long* tim = A.timing;                          // optional: clock cycles per phase
+    // the solves: this thread's group of warps and its rows [row0, row0 + Rg) there
+    const int grp = (tid >> 5) / kG, wl = (tid >> 5) % kG;
+    const int Rg = group_rows(M, kG), row0 = (wl * 32 + lane) * Rg;
+    unsigned long long* tim = team.rank == 0 ? A.timing : nullptr;   // optional: clock cycles per phase
     long long t_prev = (tim && tid == 0) ? clock64() : 0;
 #define M1_MARK(ph)                                                           \
     do {                                                                      \
@@ -748,19 +989,21 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         S.iv[i] = A.inv_V[i];
         S.ih[i] = (i < N) ? A.inv_h[i] : 0.0;
         S.bp.r0[i] = S.bp.i0[i] = S.bp.r1[i] = S.bp.i1[i] = S.bp.r2[i] = S.bp.i2[i] = 0.0;
+    }
+    if (mine) {
         const Src1 T = src1_of(scr, M, 0);
         T.rhot.a0[i] = T.rhot.ar[i] = T.rhot.ai[i] = 0.0;             // scratch: immobile rho
         T.drho.a0[i] = T.drho.ar[i] = T.drho.ai[i] = 0.0;             // scratch: mobile rho
     }
     if (tid == 0) *S.lost = 0;
-    for (int p = tid; p < np; p += kThreads) {
+    for (int p = first_p; p < np; p += step_p) {
 #pragma unroll
         for (int v = 0; v < 6; ++v) gate.ps(A)[(size_t)v * npad + p] = A.p_init[(size_t)v * npad + p];
         for (int v = 0; v < 5 * ORD; ++v) gate.ps(A)[(size_t)(6 + v) * npad + p] = 0.0;
     }
-    __syncthreads();
+    team.sync();
     // src/PlasmaSpecies.cpp:480-506 for the immobile species and, when neutralising, the fresh mobile ones
-    for (int p = tid; p < A.nbg; p += kThreads) {
+    for (int p = first_p; p < A.nbg; p += step_p) {
         const double x = A.bg_p[p], y = A.bg_p[A.nbg + p], wq = A.bg_p[2 * A.nbg + p];
         if (wq == 0.0) continue;
         const PGeo g = geometry(S.r, S.ih, N, R, x, y);
@@ -775,7 +1018,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         }
     }
     if (A.neutralize)
-        for (int p = tid; p < np; p += kThreads) {
+        for (int p = first_p; p < np; p += step_p) {
             const double w = A.p_init[5 * (size_t)npad + p];
             if (w == 0.0) continue;
             double q, qm;
@@ -791,19 +1034,22 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                 atomicAdd(T.drho.ai + jj, -a * g.s);
             }
         }
-    __syncthreads();
-    if (row) {
+    team.sync();
+    if (mine) {
         const Src1 T = src1_of(scr, M, 0);
         bg[i] = lg(T.rhot.a0 + i) - lg(T.drho.a0 + i);
         bg[M + i] = lg(T.rhot.ar + i) - lg(T.drho.ar + i);
         bg[2 * M + i] = lg(T.rhot.ai + i) - lg(T.drho.ai + i);
     }
-    if (Gate::kActive && tid < 32) {                     // warp 0 checks the beam-source rows
+    if (Gate::kActive && team.rank == 0 && tid < 32) {   // warp 0 of the team checks the beam-source rows
         const bool ok = gate.before_rows(K - 1 < 2 ? K - 1 : 2);
         if (tid == 0) *S.flag = ok ? 1 : 0;
     }
-    __syncthreads();
-    if (Gate::kActive && !*S.flag) return false;
+    team.sync();
+    if (Gate::kActive && !team.of_first(S.flag)) {
+        team.sync();                                      // rank 0's flag has been read by all
+        return false;
+    }
     const bool filt = EXT && A.filter;
     int scan_par = 0;
     if (filt) {                     // the background is smoothed like the plasma (src/Simulation.cpp:685-690)
@@ -814,12 +1060,12 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         double* t1 = S.tot + (scan_par++ & 1) * 16 * kW;
         filter_rows1<3>(fg, A.fconsts, M, t0, t1);
         if (row) init_sources1_zero(src1_of(scr, M, 0), M, i);
-    } else if (row) {
+    } else if (mine) {
         init_sources1(src1_of(scr, M, 0), bg, M, i, beam_row1<Gate::kActive, EXT>(A, gate.bsrc(A), 0, i));
     }
-    __syncthreads();
-    deposit_all1<ORD>(A, S, src1_of(scr, M, 0), gate);
-    __syncthreads();
+    team.sync();
+    deposit_all1<ORD>(A, S, src1_of(scr, M, 0), gate, team);
+    team.sync();
     M1_MARK(0);
 
     const double fc = A.flux_coef;
@@ -831,7 +1077,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         if (filt) {
             if (k + 1 < K && row) init_sources1_zero(src1_of(scr, M, cb ^ 1), M, i);
             filter_sources1<Gate::kActive>(A, src1_of(scr, M, cb), bg, gate.bsrc(A), k, S.tot, scan_par);
-        } else if (k + 1 < K && row) {
+        } else if (k + 1 < K && mine) {
             init_sources1(src1_of(scr, M, cb ^ 1), bg, M, i, beam_row1<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, i));
         }
         // ---------------- P2: psi, E_z, B_z (9 systems with fixed Thomas factors)
@@ -842,10 +1088,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             double d[9];
 #pragma unroll
             for (int e = 0; e < 9; ++e) d[e] = 0.0;
-            double f0 = 1.0, r0 = 0.0, b0 = 1.0, f1 = 1.0, r1 = 0.0, b1 = 1.0;
             if (row) {
-                f0 = ldc(C.l0f + i); r0 = ldc(C.l0r + i); b0 = ldc(C.l0b + i);
-                f1 = ldc(C.d1f + i); r1 = ldc(C.d1r + i); b1 = ldc(C.d1b + i);
                 if (i < N) {
                     d[0] = -1.0 * lg(T.rhot.a0 + i);
                     d[1] = -1.0 * lg(T.drho.a0 + i);
@@ -864,26 +1107,21 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                     d[8] = 1.0 * (0.5 * (D1r - Dmr));
                 }
             }
-            const int grp[9] = {0, 0, 0, 1, 1, 1, 1, 1, 1};
-            const double fa[2] = {f0, f1};
-            double fb[9], yb[9];
-#pragma unroll
-            for (int e = 0; e < 9; ++e) fb[e] = (e < 3 ? r0 : r1) * d[e];
-            scan_fwd_g<2, 9>(fa, fb, grp, yb, S.tot + (scan_par++ & 1) * 16 * kW);
-            double y[9];                                            // no row: identity (y = 0)
-#pragma unroll
-            for (int e = 0; e < 9; ++e) y[e] = row ? fma(e < 3 ? f0 : f1, yb[e], fb[e]) : 0.0;
-            const double ba[2] = {b0, b1};
-            double xa[9];
-            scan_bwd_g<2, 9>(ba, y, grp, xa, S.tot + (scan_par++ & 1) * 16 * kW);
             if (row) {
-                double x[9];
-#pragma unroll
-                for (int e = 0; e < 9; ++e) x[e] = fma(e < 3 ? b0 : b1, xa[e], y[e]);
-                S.psi.a0[i] = x[0]; S.ez.a0[i] = x[1]; S.bz.a0[i] = x[2];
-                S.psi.ar[i] = x[3]; S.psi.ai[i] = x[4];
-                S.ez.ar[i] = x[5]; S.ez.ai[i] = x[6];
-                S.bz.ar[i] = x[7]; S.bz.ai[i] = x[8];
+                S.psi.a0[i] = d[0]; S.ez.a0[i] = d[1]; S.bz.a0[i] = d[2];
+                S.psi.ar[i] = d[3]; S.psi.ai[i] = d[4];
+                S.ez.ar[i] = d[5]; S.ez.ai[i] = d[6];
+                S.bz.ar[i] = d[7]; S.bz.ai[i] = d[8];
+            }
+            __syncthreads();
+            double* const t0 = S.tot + grp * 2 * kTotG;
+            if (grp == 0) {
+                double* const f[3] = {S.psi.a0, S.ez.a0, S.bz.a0};
+                solve_fixed<3>(f, A.consts + 4 * (size_t)M, M, Rg, row0, wl, t0, t0 + kTotG, 1);
+            } else {
+                const Msc& m = grp == 1 ? S.psi : (grp == 2 ? S.ez : S.bz);
+                double* const f[2] = {m.ar, m.ai};
+                solve_fixed<2>(f, A.consts1, M, Rg, row0, wl, t0, t0 + kTotG, 1 + grp);
             }
         }
         __syncthreads();
@@ -903,7 +1141,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         M1_MARK(1);
 
         // ---------------- P3: S+ (src/PlasmaSpecies.cpp:508-559)
-        for (int base = tid - lane; base < np; base += kThreads) {
+        for (int base = first_p - lane; base < np; base += step_p) {
             const int p = base + lane;
             bool act = false;
             int j = 0;
@@ -921,7 +1159,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             }
             depositS1_warp(act, j, v, src1_of(scr, M, cb));
         }
-        __syncthreads();
+        team.sync();
         M1_MARK(2);
 
         // ---------------- P4: B+ (src/Simulation.cpp:535-591)
@@ -939,14 +1177,6 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             const Src1 T = src1_of(scr, M, cb);
             // fixed part of the right-hand sides: (d/dx + i d/dy) J_z + S
             double gr[6] = {0, 0, 0, 0, 0, 0};                   // g r1 i1 r0 i0 r2 i2
-            double ra[4], rbv[4], rc[4], rcm[4];
-            bool dir[4];
-            double m[4][4];
-#pragma unroll
-            for (int sy = 0; sy < 4; ++sy) {
-                m[sy][0] = 1.0; m[sy][1] = 0.0; m[sy][2] = 0.0; m[sy][3] = 1.0;
-                ra[sy] = 0.0; rbv[sy] = 1.0; rc[sy] = 0.0; rcm[sy] = 0.0; dir[sy] = true;
-            }
             if (row) {
                 const double t1 = grad1g(C, N, T.jz.a0, i, false);
                 const double t2 = grad1g(C, N, T.jz.ar, i, true), t3 = over_r1g(C, T.jz.ar, i);
@@ -957,31 +1187,14 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                 gr[3] = -(t4 + t5) + lg(T.S.i0 + i);
                 gr[4] = (t2 - t3) + lg(T.S.r2 + i);
                 gr[5] = (t4 - t5) + lg(T.S.i2 + i);
-#pragma unroll
-                for (int sy = 0; sy < 4; ++sy) {
-                    row_bp(C, T, N, sy, i, ra[sy], rbv[sy], rc[sy], rcm[sy], dir[sy]);
-                    // T_i = [[b_i, -a_i c_{i-1}], [1, 0]], renormalised as scan_pivots needs
-                    m[sy][0] = rbv[sy]; m[sy][1] = -ra[sy] * rcm[sy]; m[sy][2] = 1.0; m[sy][3] = 0.0;
-                    renorm(m[sy][0], m[sy][1], m[sy][2], m[sy][3]);
-                }
             }
-            double pp[4], qq[4];
-            scan_pivots<4>(m, pp, qq, S.tot + (scan_par++ & 1) * 16 * kW);
-            double rinv[4], fa[4], ba[4];
-#pragma unroll
-            for (int sy = 0; sy < 4; ++sy) {
-                rinv[sy] = 1.0; fa[sy] = 1.0; ba[sy] = 1.0;
-                if (!row) continue;
-                const double pn = rbv[sy] * pp[sy] - ra[sy] * rcm[sy] * qq[sy];
-                rinv[sy] = pp[sy] / pn;                          // 1/u_i = p_{i-1} / p_i
-                fa[sy] = -rinv[sy] * ra[sy];
-                ba[sy] = -(rc[sy] * rinv[sy]);
-            }
-            const int grp[6] = {0, 1, 2, 2, 3, 3};             // r1 (L1D), i1 (L1F), r0 i0 (L0), r2 i2 (L2D)
+            double* const t0 = S.tot + grp * 2 * kTotG;
+            Fac1 F;
+            factor_op(C, T.chi.a0, grp, M, N, Rg, row0, wl, t0, 1 + grp, F);
             const double chr = row ? lg(T.chi.ar + i) : 0.0, chi_i = row ? lg(T.chi.ai + i) : 0.0;
             const double jzN = lg(T.jz.a0 + N);
             for (int it = 0; it < niter; ++it) {
-                double d[6] = {0, 0, 0, 0, 0, 0};
+                // the right-hand sides over the iterate, in place: a row's six need only its own six values
                 if (row) {
                     const double cr = chr, ci = chi_i;
                     const double b0r = S.bp.r0[i], b0i = S.bp.i0[i], b1r = S.bp.r1[i], b1i = S.bp.i1[i];
@@ -992,65 +1205,29 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                     r1v += cr * b0r - ci * b0i + cr * b2r + ci * b2i;
                     i1v += cr * b0i + ci * b0r + cr * b2i - ci * b2r;
                     r2v += cr * b1r - ci * b1i;  i2v += cr * b1i + ci * b1r;
-                    d[0] = dir[0] ? 0.0 : 1.0 * r1v;
-                    d[1] = dir[1] ? 0.0 : 1.0 * i1v;
-                    if (i == N && !dir[1]) d[1] -= fc * jzN;
-                    d[2] = dir[2] ? 0.0 : 1.0 * r0v;
-                    d[3] = dir[2] ? 0.0 : 1.0 * i0v;
-                    d[4] = dir[3] ? 0.0 : 1.0 * r2v;
-                    d[5] = dir[3] ? 0.0 : 1.0 * i2v;
-                }
-                double fb[6], yb[6];
-#pragma unroll
-                for (int e = 0; e < 6; ++e) fb[e] = rinv[grp[e]] * d[e];
-                scan_fwd_g<4, 6>(fa, fb, grp, yb, S.tot + (scan_par++ & 1) * 16 * kW);
-                double y[6];
-#pragma unroll
-                for (int e = 0; e < 6; ++e) y[e] = row ? fma(fa[grp[e]], yb[e], fb[e]) : 0.0;
-                double xa[6];
-                scan_bwd_g<4, 6>(ba, y, grp, xa, S.tot + (scan_par++ & 1) * 16 * kW);
-                double x[6];
-#pragma unroll
-                for (int e = 0; e < 6; ++e) x[e] = fma(ba[grp[e]], xa[e], y[e]);
-                // one step of iterative refinement with the same factors: the pivots come from a prefix
-                // product, slightly less accurate than Thomas' recurrence on these ill-conditioned rows
-                // (L1D on a 100x-stretched grid); r = d - A x with the exact rows, then x += A^-1 r
-                if (row) {                                              // (each thread reads only its own bp row above)
-                    S.bp.r1[i] = x[0]; S.bp.i1[i] = x[1];
-                    S.bp.r0[i] = x[2]; S.bp.i0[i] = x[3];
-                    S.bp.r2[i] = x[4]; S.bp.i2[i] = x[5];
+                    if (i == N) i1v -= fc * jzN;                      // the flux wall of L1F
+                    S.bp.r1[i] = op_dirichlet(0, i, N) ? 0.0 : r1v;
+                    S.bp.i1[i] = op_dirichlet(1, i, N) ? 0.0 : i1v;
+                    S.bp.r0[i] = op_dirichlet(2, i, N) ? 0.0 : r0v;
+                    S.bp.i0[i] = op_dirichlet(2, i, N) ? 0.0 : i0v;
+                    S.bp.r2[i] = op_dirichlet(3, i, N) ? 0.0 : r2v;
+                    S.bp.i2[i] = op_dirichlet(3, i, N) ? 0.0 : i2v;
                 }
                 __syncthreads();
-                double rr[6] = {0, 0, 0, 0, 0, 0};
-                if (row) {
-                    double* const xs[6] = {S.bp.r1, S.bp.i1, S.bp.r0, S.bp.i0, S.bp.r2, S.bp.i2};
-#pragma unroll
-                    for (int e = 0; e < 6; ++e) {
-                        const int sy = grp[e];
-                        const double xm = i > 0 ? xs[e][i - 1] : 0.0, xp = i < N ? xs[e][i + 1] : 0.0;
-                        rr[e] = d[e] - (ra[sy] * xm + rbv[sy] * x[e] + rc[sy] * xp);
-                    }
+                if (grp < 2) {
+                    double* const f[1] = {grp ? S.bp.i1 : S.bp.r1};
+                    solve_shifted<1>(f, C, F, grp, M, N, Rg, row0, wl, t0, 1 + grp);
+                } else {
+                    double* const f[2] = {grp == 2 ? S.bp.r0 : S.bp.r2, grp == 2 ? S.bp.i0 : S.bp.i2};
+                    solve_shifted<2>(f, C, F, grp, M, N, Rg, row0, wl, t0, 1 + grp);
                 }
-#pragma unroll
-                for (int e = 0; e < 6; ++e) fb[e] = rinv[grp[e]] * rr[e];
-                scan_fwd_g<4, 6>(fa, fb, grp, yb, S.tot + (scan_par++ & 1) * 16 * kW);
-#pragma unroll
-                for (int e = 0; e < 6; ++e) y[e] = row ? fma(fa[grp[e]], yb[e], fb[e]) : 0.0;
-                scan_bwd_g<4, 6>(ba, y, grp, xa, S.tot + (scan_par++ & 1) * 16 * kW);
-                if (row) {
-#pragma unroll
-                    for (int e = 0; e < 6; ++e) x[e] += fma(ba[grp[e]], xa[e], y[e]);
-                    S.bp.r1[i] = x[0]; S.bp.i1[i] = x[1];
-                    S.bp.r0[i] = x[2]; S.bp.i0[i] = x[3];
-                    S.bp.r2[i] = x[4]; S.bp.i2[i] = x[5];
-                }
+                __syncthreads();
             }
         }
-        __syncthreads();
         M1_MARK(3);
 
         // ---------------- P5: store slice k (src/Simulation.cpp:594-633)
-        if (row) {
+        if (mine) {
             const Src1 T = src1_of(scr, M, cb);
             const size_t fb = (size_t)k * M;
             double* F = gate.fld(A) + (fb + i) * F_NC1;
@@ -1088,7 +1265,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             // source buffer, initialised at the start of this slice)
             const bool first = (k == 0);
             const Src1 Tn = src1_of(scr, M, cb ^ 1);
-            for (int base = tid - lane; base < np; base += kThreads) {
+            for (int base = first_p - lane; base < np; base += step_p) {
                 const int p = base + lane;
                 bool act = false;
                 int j = 0;
@@ -1115,21 +1292,23 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                 }
                 deposit1_warp(act, j, neg, d, Tn);
             }
-            __syncthreads();
-            M1_MARK(4);
         }
-        if (Gate::kActive) gate.slice_done_all(k);
-        __syncthreads();
+        if (Gate::kActive) gate.slice_done_all(k, team.rank, team.size);
+        team.sync();
+        M1_MARK(4);
         if (Gate::kActive) {
-            if (tid < 32) {                                   // warp 0: publish slice k, check the next rows
+            if (team.rank == 0 && tid < 32) {             // warp 0 of the team: publish slice k, check the next rows
                 bool ok = true;
                 if (tid == 0) ok = gate.slice_done(k);
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (ok && k + 1 < K) ok = gate.before_rows(k + 3 < K ? k + 3 : K - 1);
                 if (tid == 0) *S.flag = ok ? 1 : 0;
             }
-            __syncthreads();
-            if (!*S.flag) return false;
+            team.sync();
+            if (!team.of_first(S.flag)) {
+                team.sync();
+                return false;
+            }
         }
     }
     if (tid == 0 && A.counters) atomicAdd(&A.counters[0], (unsigned long long)*S.lost);
