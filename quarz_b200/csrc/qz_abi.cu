@@ -455,6 +455,8 @@ extern "C" qz_status qz_sweep_create(const qz_grid* g, const qz_sweep_params* p,
     A.r = g->d_r; A.inv_h = g->d_inv_h; A.inv_V = g->d_inv_V;
     A.consts = g->d_consts;
     A.consts0 = g->d_consts0;
+    A.bcs = qzb::B_NC0;
+    A.bjt = qzb::B_JP1I;
     A.lfa_N = g->opa[2][g->N];
     A.lfb_N = g->opb[2][g->N];
     A.flux_coef = g->flux_coef;
@@ -1391,7 +1393,15 @@ qz_status run_pipelined(qz_sim* s, int nsteps, double dt, double* mom_host, cuda
     nsweep = std::max(1, std::min({nsweep, (nsteps + 1) * team, g1 - 1}));
     // 3. buffers
     const size_t KM = (size_t)K * M;
-    const size_t bslot = sim_bsrc_doubles(s);           // a beam-source slot: two limbs per value for m = 0
+    // a beam-source slot; m = 0: the three components the sweep reads, in the exact format two limbs each
+    const bool fxc = s->p.modes == 0 && s->fx.on;
+    A.bnc = s->p.modes ? s->bnc : (fxc ? 6 : 3);
+    const size_t bslot = KM * (s->p.modes ? s->bnc : 6);      // (both formats fit, for rings kept between runs)
+    auto ring_args = [&](const qz_beam_view* v) {
+        qzb::BeamArgs B = sim_beam_args(s, v, &box);
+        B.compact = s->p.modes ? 0 : 1;
+        return B;
+    };
     // ring slots: one per step in flight; one per step of the run when that fits in half the free memory,
     // which lets the push workers read the field rows through L1 (PipeArgs::fld_l1)
     int ring = rec ? std::max(2, nsteps + 1) : std::max(2, std::min(nsteps + 1, nsweep + 2));
@@ -1441,9 +1451,12 @@ qz_status run_pipelined(qz_sim* s, int nsteps, double dt, double* mom_host, cuda
     // 4. beam sources of step 0 into slot 0
     for (auto& b : s->beams) {
         const qz_beam_view v = b.view();
-        QZ_CUDA(qzb::launch_beam_deposit(sim_beam_args(s, &v, &box), P_.bsrc, st));
+        QZ_CUDA(qzb::launch_beam_deposit(ring_args(&v), P_.bsrc, st));
     }
     sim_sweep_fx(s, A.sw);
+    A.sw.bcs = A.bnc;
+    A.sw.bjt = 2;
+    A.sw.bfx_lo = 3;
     // 5. launch
     A.nsteps = nsteps;
     A.nsweep = nsweep;
@@ -1463,7 +1476,7 @@ qz_status run_pipelined(qz_sim* s, int nsteps, double dt, double* mom_host, cuda
     for (int q = 0; q < nb; ++q) {
         const auto& b = s->beams[q];
         const qz_beam_view v = b.view();
-        A.beam[q] = sim_beam_args(s, &v, &box);
+        A.beam[q] = ring_args(&v);
         A.rigid[q] = b.rigid;
         A.startup[q] = b.started ? 0 : 1;
         A.gref[q] = b.gref;

@@ -355,23 +355,23 @@ __global__ void deposit_back_kernel(BeamArgs B, const double* __restrict__ lbsrc
 // ------------------------------------------------------------------ the reverse sweep
 // shared-memory arrays of one slice (M each)
 struct AdjSm {
-    double *r, *iv, *ih, *F1;                       // grid; F1 = r dV (symmetriser of L1D / L1F)
+    double *r, *iv, *ih, *F1, *iF1;                 // grid; F1 = r dV (symmetriser of L1D / L1F), 1 / F1
     double *wpr, *ez, *bz, *bpr, *bpi, *chi;        // forward values of the slice
     double *l_wpr, *l_ez, *l_bz, *l_bpr, *l_bpi;    // adjoints of the fields
     double *l_rhot, *l_drho, *l_jz, *l_chi, *l_jpi, *l_Sr, *l_Si;   // adjoints of the sources
     double *t0, *t1;                                // scratch
-    double* tot;                                    // scan scratch (2 x 8 x kW)
+    double* tot;                                    // scan scratch (2 x 8 x kW = kTot)
     double* lam;                                    // particle adjoints ((5 + 5 ord) x kSweepThreads)
     int* flag;                                      // gate result broadcast
 };
-constexpr int kAdjArrays = 22;
+constexpr int kAdjArrays = 23;
 constexpr int kMaxOrd = 5;                          // the particle adjoints' room: AB order up to 5
 
 __device__ __forceinline__ AdjSm carve_adj(double* p, int M) {
     AdjSm S;
     double** a[kAdjArrays] = {&S.r, &S.iv, &S.ih, &S.F1, &S.wpr, &S.ez, &S.bz, &S.bpr, &S.bpi, &S.chi, &S.l_wpr,
                               &S.l_ez, &S.l_bz, &S.l_bpr, &S.l_bpi, &S.l_rhot, &S.l_drho, &S.l_jz, &S.l_chi, &S.l_jpi,
-                              &S.l_Sr, &S.l_Si};
+                              &S.l_Sr, &S.l_Si, &S.iF1};
     for (int i = 0; i < kAdjArrays; ++i) { *a[i] = p; p += M; }
     S.t0 = p; p += M;
     S.t1 = p; p += M;
@@ -816,11 +816,14 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
     const AdjSm S = carve_adj(smem_raw, M);
     const double* q = A.consts;                     // stencils, 1/r, L0 Thomas, L1D and L1F rows (13 x M)
     const double *gm = q, *g0 = q + M, *gp = q + 2 * M, *ir = q + 3 * M;
-    const double *l0r = q + 4 * M, *l0f = q + 5 * M, *l0b = q + 6 * M;
     const double *l1a = q + 7 * M, *l1b = q + 8 * M, *l1c = q + 9 * M;
     const double *lfa = q + 10 * M, *lfb = q + 11 * M, *lfc = q + 12 * M;
     const int i = tid, lane = tid & 31;              // this thread's row
     const bool row = i < M;
+    // the solves: this thread's group of warps (l0_group, shifted_group; M <= kSweepThreads)
+    constexpr int kR2 = 5, kR4 = 3;
+    constexpr double two_pi = 6.283185307179586;
+    const int warp = tid >> 5, e2 = warp / kG2, wl2 = warp - e2 * kG2, sy4 = warp / kG4, wl4 = warp - sy4 * kG4;
     if (row) {
         S.r[i] = A.r[i];
         S.iv[i] = A.inv_V[i];
@@ -837,6 +840,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
         iVi = A.inv_V[i];
         Vi = 1.0 / iVi;
         S.F1[i] = F1i;
+        S.iF1[i] = iF1i;
     }
     const size_t nv = 6 + 5 * (size_t)ORD;
     const double fcoef = A.flux_coef;
@@ -985,60 +989,42 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
         ADJ_MARK(1);
         // ---- B+ (src/Simulation.cpp:535-591) in reverse: mu = F (L - chi)^-1 (F^-1 lam) per system
         {
-            double m[2][4], ra[2], rbv[2], rc[2], rd[2];
+            // sys 0: L1D - chi (rows 0, N Dirichlet); sys 1: L1F - chi (row 0 Dirichlet); each by its group of warps
+            const int R = group_rows(M, kG4), row0 = (wl4 * 32 + lane) * R;
+            double x[kR4];
+            const double* const lam = sy4 ? S.l_bpi : S.l_bpr;
+            shifted_group<kR4>(
+                S.tot, M, sy4, wl4, R, row0,
+                [&](int r, double& a, double& b, double& cm, double& d) {
+                    a = sy4 ? lfa[r] : l1a[r];
+                    b = sy4 ? lfb[r] : l1b[r];
+                    cm = r > 0 ? l1c[r - 1] : 0.0;
+                    d = 0.0;
+                    if (r >= 1 && (sy4 || r < N)) {
+                        b -= S.chi[r];
+                        d = lam[r] * S.iF1[r];
+                    }
+                },
+                [&](int r) { return sy4 ? lfc[r] : l1c[r]; }, x);
 #pragma unroll
-            for (int sy = 0; sy < 2; ++sy) {
-                m[sy][0] = 1.0; m[sy][1] = 0.0; m[sy][2] = 0.0; m[sy][3] = 1.0;
-                ra[sy] = 0.0; rbv[sy] = 1.0; rc[sy] = 0.0; rd[sy] = 0.0;
-            }
-            if (row) {
-                // sys 0: L1D - chi (rows 0, N Dirichlet); sys 1: L1F - chi (row 0 Dirichlet)
-                ra[0] = l1a[i]; rbv[0] = l1b[i]; rc[0] = i > 0 ? l1c[i - 1] : 0.0;
-                if (i >= 1 && i < N) { rbv[0] -= S.chi[i]; rd[0] = S.l_bpr[i] * iF1i; }
-                ra[1] = lfa[i]; rbv[1] = lfb[i]; rc[1] = i > 0 ? lfc[i - 1] : 0.0;
-                if (i >= 1) { rbv[1] -= S.chi[i]; rd[1] = S.l_bpi[i] * iF1i; }
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy) {
-                    m[sy][0] = rbv[sy]; m[sy][1] = -ra[sy] * rc[sy]; m[sy][2] = 1.0; m[sy][3] = 0.0;
-                    renorm(m[sy][0], m[sy][1], m[sy][2], m[sy][3]);
+            for (int u = 0; u < kR4; ++u) {
+                const int r = row0 + u;
+                if (u >= R || r >= M) continue;
+                const double mu = r >= 1 && (sy4 || r < N) ? x[u] * S.F1[r] : 0.0;
+                if (sy4) {
+                    S.l_Sr[r] = mu;                  // lam of the B_theta right-hand side (J_z' + S_r)
+                    S.t0[r] = mu;
+                } else {
+                    S.l_Si[r] = -mu;
                 }
-            }
-            double pp[2], qq[2];
-            scan_pivots<2>(m, pp, qq, S.tot + (par++ & 1) * 8 * kW);
-            double rinv[2], fA[2], fB[2];
-#pragma unroll
-            for (int sy = 0; sy < 2; ++sy) {
-                rinv[sy] = 0.0; fA[sy] = 1.0; fB[sy] = 0.0;
-                if (!row) continue;
-                const double pn = rbv[sy] * pp[sy] - ra[sy] * rc[sy] * qq[sy];
-                rinv[sy] = pp[sy] / pn;
-                fA[sy] = -rinv[sy] * ra[sy];
-                fB[sy] = rinv[sy] * rd[sy];
-            }
-            double yy[2];
-            scan_fwd_n<2>(fA, fB, yy, S.tot + (par++ & 1) * 8 * kW);
-            double y[2], bA[2], bB[2];
-#pragma unroll
-            for (int sy = 0; sy < 2; ++sy) {
-                y[sy] = row ? fma(fA[sy], yy[sy], fB[sy]) : 0.0;
-                const double c = row ? (sy ? lfc[i] : l1c[i]) : 0.0;
-                bA[sy] = row ? -(c * rinv[sy]) : 1.0;
-                bB[sy] = y[sy];
-            }
-            double xx[2];
-            scan_bwd_n<2>(bA, bB, xx, S.tot + (par++ & 1) * 8 * kW);
-            if (row) {
-                const double mu0 = (i >= 1 && i < N) ? fma(bA[0], xx[0], y[0]) * F1i : 0.0;
-                const double mu1 = (i >= 1) ? fma(bA[1], xx[1], y[1]) * F1i : 0.0;
-                S.l_chi[i] = mu0 * S.bpr[i] + mu1 * S.bpi[i];
-                S.l_Si[i] = -mu0;
-                S.l_Sr[i] = mu1;                     // lam of the B_theta right-hand side (J_z' + S_r)
-                S.t0[i] = mu1;
             }
         }
         __syncthreads();
         ADJ_MARK(2);
-        if (row) S.l_jz[i] = grad_T_at(A, gm, g0, gp, S.t0, i) - (i == N ? fcoef * S.t0[N] : 0.0);
+        if (row) {
+            S.l_chi[i] = S.l_Sr[i] * S.bpi[i] - S.l_Si[i] * S.bpr[i];
+            S.l_jz[i] = grad_T_at(A, gm, g0, gp, S.t0, i) - (i == N ? fcoef * S.t0[N] : 0.0);
+        }
         if constexpr (FILT) {                         // the S+ filter (src/Simulation.cpp:810-812) in reverse
             double* const fa[2] = {S.l_Sr, S.l_Si};
             filter_rows_adj<2>(fa, 1, true, A.fconsts, M, N, Vi, iVi, F1i, iF1i, S.tot + (par++ & 1) * 8 * kW,
@@ -1070,35 +1056,24 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
         if (row) S.t1[i] = -S.l_wpr[i];
         __syncthreads();
         {
-            double d[3] = {0.0, 0.0, 0.0};
-            double af = 1.0, rr = 0.0, ab = 1.0;
-            if (row) {
-                af = l0f[i]; rr = l0r[i]; ab = l0b[i];
-                if (i < N) {
-                    d[0] = S.l_bz[i] * iVi;
-                    d[1] = grad_T_at(A, gm, g0, gp, S.t1, i) * iVi;   // lam of psi
-                    d[2] = S.l_ez[i] * iVi;
+            // mu / V with d = lam / V; the weights w = V / 2 pi and 1 / g of the flux form
+            if (e2 < 3) {
+                const int R = group_rows(M, kG2), row0 = (wl2 * 32 + lane) * R;
+                double x[kR2], z0, xn;
+                l0_group<kR2>(S.tot, A.consts0 + 4 * (size_t)M, A.consts0 + 5 * (size_t)M, N, e2, wl2, R, row0,
+                              [&](int r) {
+                                  const double l = e2 == 0 ? S.l_bz[r]
+                                                           : (e2 == 1 ? grad_T_at(A, gm, g0, gp, S.t1, r) : S.l_ez[r]);
+                                  return l * S.iv[r];                  // (grad_T_at: lam of psi)
+                              },
+                              x, z0, xn);
+                // lam of the B_z right-hand side -(J_th' + J_th / r), of rho - J_z and of its xi-derivative
+                double* const out = e2 == 0 ? S.t0 : (e2 == 1 ? S.l_rhot : S.l_drho);
+#pragma unroll
+                for (int u = 0; u < kR2; ++u) {
+                    const int r = row0 + u;
+                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[4 * (size_t)M + r])) : -0.0;
                 }
-            }
-            double cB[3];
-#pragma unroll
-            for (int e = 0; e < 3; ++e) cB[e] = rr * d[e];
-            double yb[3];
-            scan_fwd<3>(af, cB, yb, S.tot + (par++ & 1) * 8 * kW);
-            double y[3];
-#pragma unroll
-            for (int e = 0; e < 3; ++e) y[e] = row ? fma(af, yb[e], cB[e]) : 0.0;
-            double xa[3];
-            scan_bwd<3>(row ? ab : 1.0, y, xa, S.tot + (par++ & 1) * 8 * kW);
-            if (row) {
-                double mu[3] = {0.0, 0.0, 0.0};
-                if (i < N) {
-#pragma unroll
-                    for (int e = 0; e < 3; ++e) mu[e] = fma(ab, xa[e], y[e]) * Vi;
-                }
-                S.t0[i] = -mu[0];                    // lam of the B_z right-hand side -(J_th' + J_th / r)
-                S.l_rhot[i] = -mu[1];
-                S.l_drho[i] = -mu[2];
             }
         }
         __syncthreads();
@@ -1111,19 +1086,21 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
             S.l_jpi[i] = v;
             // the beam source adjoints of rows k and k +- 1 (combine_sources, src/Simulation.cpp:408-457)
             double* Lk = lbsrc + ((size_t)k * M + i) * B_NC0;
-            Lk[B_RT0] += S.l_rhot[i];
-            Lk[B_JZ0] += S.l_jz[i];
-            Lk[B_JP1I] += v;
+            // (reductions: nothing to wait for; only this thread adds to its node's values, in program order)
             const double ld = S.l_drho[i] * A.idxi;
-            const size_t st = (size_t)M * B_NC0;
+            const ptrdiff_t st = (ptrdiff_t)M * B_NC0;
+            double own = S.l_rhot[i];
             if (A.ngp) {     // the backward difference (the row ahead of the box head is zero)
-                Lk[B_RT0] += ld;
-                if (k > 0) Lk[B_RT0 - (ptrdiff_t)st] -= ld;
+                own += ld;
+                if (k > 0) atomicAdd(Lk + B_RT0 - st, -ld);
             } else if (K > 1) {
-                if (k == 0) { Lk[st + B_RT0] += ld; Lk[B_RT0] -= ld; }
-                else if (k == K - 1) { Lk[B_RT0] += ld; Lk[B_RT0 - (ptrdiff_t)st] -= ld; }
-                else { Lk[st + B_RT0] += 0.5 * ld; Lk[B_RT0 - (ptrdiff_t)st] -= 0.5 * ld; }
+                if (k == 0) { atomicAdd(Lk + st + B_RT0, ld); own -= ld; }
+                else if (k == K - 1) { own += ld; atomicAdd(Lk + B_RT0 - st, -ld); }
+                else { atomicAdd(Lk + st + B_RT0, 0.5 * ld); atomicAdd(Lk + B_RT0 - st, -(0.5 * ld)); }
             }
+            atomicAdd(Lk + B_RT0, own);
+            atomicAdd(Lk + B_JZ0, S.l_jz[i]);
+            atomicAdd(Lk + B_JP1I, v);
         }
         __syncthreads();
         if constexpr (FILT) {   // the filter of the plasma deposit in reverse (the beams came after it)

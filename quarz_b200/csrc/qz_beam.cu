@@ -36,50 +36,6 @@ struct WarpDep {
     int node[32];
 };
 
-// the values of one particle (src/Beam.cpp:725-785): f[c] times the corner's weight
-template <int NC>
-struct DepOne {
-    int k, j;
-    double d0, tk, t, f[NC];
-};
-
-template <int NC>
-__device__ __forceinline__ bool dep_one(const BeamArgs& B, double X, double Y, double PX, double PY, double PZ,
-                                        double XI, double wi, int jguess, DepOne<NC>& D) {
-    const double r = sqrt(X * X + Y * Y);
-    if (r > B.R) return false;
-    double c = 1.0, s = 0.0;
-    if (r > 0.0) {
-        const Recip ir(r);
-        c = ir(X);
-        s = ir(Y);
-    }
-    const double sx = (XI - B.xi_min) * B.idxi;
-    D.k = B.ngp ? (int)floor(sx + 0.5) : (int)floor(sx);
-    if (D.k < -1 || D.k >= B.K) return false;
-    D.tk = B.ngp ? 0.0 : sx - D.k;
-    const double p2 = PX * PX + PY * PY;
-    const double gam = sqrt(1.0 + p2 + PZ * PZ);
-    const double omvz = (1.0 + p2) / (gam * (gam + PZ));
-    const Recip ig(gam);
-    const double vz = ig(PZ), vx = ig(PX), vy = ig(PY);
-    const double vr = c * vx + s * vy, vt = c * vy - s * vx;
-    D.j = locate_near(B.r, B.N, B.R, r, jguess);
-    const double t = (r - B.r[D.j]) * B.inv_h[D.j];
-    D.t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
-    D.d0 = wi * B.q;
-    D.f[B_RT0] = omvz; D.f[B_JZ0] = vz; D.f[B_JP1R] = vr; D.f[B_JP1I] = vt; D.f[B_RHO0] = 1.0;
-    if constexpr (NC == B_NC1) {
-        const double c2 = c * c - s * s, s2 = 2.0 * c * s;
-        D.f[B_RT1R] = omvz * c; D.f[B_RT1I] = -omvz * s;
-        D.f[B_JZ1R] = vz * c; D.f[B_JZ1I] = -vz * s;
-        D.f[B_RHO1R] = c; D.f[B_RHO1I] = -s;
-        D.f[B_JP0R] = vx; D.f[B_JP0I] = vy;
-        D.f[B_JP2R] = vx * c2 + vy * s2; D.f[B_JP2I] = vy * c2 - vx * s2;
-    }
-    return true;
-}
-
 // every lane of the warp calls it; act: the lane has a particle to deposit
 template <int NC>
 __device__ __forceinline__ void warp_deposit(const BeamArgs& B, double* __restrict__ bsrc, bool act,
@@ -170,6 +126,25 @@ __global__ void __launch_bounds__(kDepThreads<NC>) beam_deposit_kernel(const Bea
             if (wi != 0.0) act = dep_one<NC>(B, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi, -1, D);
         }
         warp_deposit<NC>(B, bsrc, act, D, S.w[threadIdx.x >> 5]);
+    }
+}
+
+// the same into compact beam sources (the first step of a pipelined run)
+template <bool kExact>
+__global__ void __launch_bounds__(kBeamThreads) beam_deposit3_kernel(const BeamArgs B, double* __restrict__ bsrc) {
+    __shared__ WarpDep3<kExact> S[kBeamThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const long stride = (long)gridDim.x * blockDim.x;
+    for (long base = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < B.n; base += stride) {
+        const long i = base + lane;
+        DepOne<kDep0> D;
+        D.k = D.j = 0;
+        bool act = false;
+        if (i < B.n) {
+            const double wi = B.w[i];
+            if (wi != 0.0) act = dep_one<kDep0>(B, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi, -1, D);
+        }
+        warp_deposit3<kExact>(B, bsrc, act, D, S[threadIdx.x >> 5]);
     }
 }
 
@@ -445,6 +420,11 @@ int beam_sums_blocks(long n) {
 
 cudaError_t launch_beam_deposit(const BeamArgs& B, double* bsrc, cudaStream_t s) {
     if (B.n <= 0) return cudaSuccess;
+    if (B.compact) {
+        if (B.fx_scale) beam_deposit3_kernel<true><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, bsrc);
+        else beam_deposit3_kernel<false><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, bsrc);
+        return cudaGetLastError();
+    }
     if (B.modes) beam_deposit_kernel<B_NC1><<<grid_dep<B_NC1>(B.n), kDepThreads<B_NC1>, 0, s>>>(B, bsrc);
     else beam_deposit_kernel<B_NC0><<<grid_dep<B_NC0>(B.n), kDepThreads<B_NC0>, 0, s>>>(B, bsrc);
     return cudaGetLastError();

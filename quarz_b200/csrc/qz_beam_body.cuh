@@ -87,73 +87,126 @@ __device__ __forceinline__ void deposit_one(const BeamArgs& B, double* __restric
     }
 }
 
-// The part of the m = 0 deposit that the m = 0 sweep reads, returned instead of applied: rho - J_z,
-// J_z and J_theta (B_RT0, B_JZ0, B_JP1I; the sweep never reads the beam's J_r and rho, and a field file
-// deposits its beam density again) of one particle, v[(2 a + b) * 3 + c] for row k + a, node j + b,
-// rows out of the box carrying zero. Returns false when the particle deposits nothing (outside the wall
-// or box). jguess: a nearby radial cell (the gather's, before the push moved the particle), or < 0
-constexpr int kDep0 = 3;                             // components of deposit_vals0
-__device__ __forceinline__ bool deposit_vals0(const BeamArgs& B, double X, double Y, double PX, double PY, double PZ,
-                                              double XI, double wi, int jguess, int& k, int& j,
-                                              double (&v)[4 * kDep0]) {
-    const double R = B.R;
+// The deposit of one particle (src/Beam.cpp:725-785): its cell, weights, and the values f[c] that every corner
+// multiplies by its weight: B_NC0 or B_NC1 components, or (kDep0) the three the m = 0 sweep reads, rho - J_z, J_z
+// and J_theta (not the beam's J_r and rho; a field file deposits its beam density again). jguess: a nearby
+// radial cell (the gather's, before the push moved the particle), or < 0
+constexpr int kDep0 = 3;
+template <int NC>
+struct DepOne {
+    int k, j;
+    double d0, tk, t, f[NC];
+};
+
+template <int NC>
+__device__ __forceinline__ bool dep_one(const BeamArgs& B, double X, double Y, double PX, double PY, double PZ,
+                                        double XI, double wi, int jguess, DepOne<NC>& D) {
     const double r = sqrt(X * X + Y * Y);
-    if (r > R) return false;
-    const double c = r > 0.0 ? X / r : 1.0, s = r > 0.0 ? Y / r : 0.0;
+    if (r > B.R) return false;
+    double c = 1.0, s = 0.0;
+    if (r > 0.0) {
+        const Recip ir(r);
+        c = ir(X);
+        s = ir(Y);
+    }
     const double sx = (XI - B.xi_min) * B.idxi;
-    k = B.ngp ? (int)floor(sx + 0.5) : (int)floor(sx);
-    const int nloc = B.K;
-    if (k < -1 || k >= nloc) return false;
-    const double tk = B.ngp ? 0.0 : sx - k;
+    D.k = B.ngp ? (int)floor(sx + 0.5) : (int)floor(sx);
+    if (D.k < -1 || D.k >= B.K) return false;
+    D.tk = B.ngp ? 0.0 : sx - D.k;
     const double p2 = PX * PX + PY * PY;
     const double gam = sqrt(1.0 + p2 + PZ * PZ);
     const double omvz = (1.0 + p2) / (gam * (gam + PZ));
-    const double vz = PZ / gam, vx = PX / gam, vy = PY / gam;
-    const double vt = c * vy - s * vx;
-    // the cell of r (src/RadialGrid.hpp:35-50): a short walk from the guess, the search otherwise
-    j = locate_near(B.r, B.N, R, r, jguess);
-    double t = (r - B.r[j]) * B.inv_h[j];
-    t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
-    const double Wr[2] = {1.0 - t, t};
-    const double Wk[2] = {1.0 - tk, tk};
-    const double q = B.q;
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-        const int kk = k + a;
-        const bool row = (a == 0 || !B.ngp) && kk >= 0 && kk < nloc;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const double d = row ? wi * q * Wk[a] * Wr[b] * B.inv_V[j + b] * B.idxi : 0.0;
-            double* o = v + (2 * a + b) * kDep0;
-            o[0] = d * omvz;
-            o[1] = d * vz;
-            o[2] = d * vt;
-        }
+    const Recip ig(gam);
+    const double vz = ig(PZ), vx = ig(PX), vy = ig(PY);
+    const double vr = c * vx + s * vy, vt = c * vy - s * vx;
+    D.j = locate_near(B.r, B.N, B.R, r, jguess);
+    const double t = (r - B.r[D.j]) * B.inv_h[D.j];
+    D.t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
+    D.d0 = wi * B.q;
+    if constexpr (NC == kDep0) {
+        D.f[0] = omvz; D.f[1] = vz; D.f[2] = vt;
+        return true;
+    } else {
+    D.f[B_RT0] = omvz; D.f[B_JZ0] = vz; D.f[B_JP1R] = vr; D.f[B_JP1I] = vt; D.f[B_RHO0] = 1.0;
+    }
+    if constexpr (NC == B_NC1) {
+        const double c2 = c * c - s * s, s2 = 2.0 * c * s;
+        D.f[B_RT1R] = omvz * c; D.f[B_RT1I] = -omvz * s;
+        D.f[B_JZ1R] = vz * c; D.f[B_JZ1I] = -vz * s;
+        D.f[B_RHO1R] = c; D.f[B_RHO1I] = -s;
+        D.f[B_JP0R] = vx; D.f[B_JP0I] = vy;
+        D.f[B_JP2R] = vx * c2 + vy * s2; D.f[B_JP2I] = vy * c2 - vx * s2;
     }
     return true;
 }
 
-// adds the contributions of deposit_vals0 into bsrc (FP64 reductions into L2, or exact)
-__device__ __forceinline__ void deposit_add0(const BeamArgs& B, double* __restrict__ bsrc, int k, int j,
-                                             const double (&v)[4 * kDep0]) {
-    constexpr int comp[kDep0] = {B_RT0, B_JZ0, B_JP1I};
+// The deposit of a warp's particles into compact m = 0 beam sources: kDep0 values per node, or (kExact) their
+// high limbs and then their low limbs, so that a particle's 2 nodes of a row are 6 or 12 contiguous doubles. A
+// reduction instruction of a particle per lane costs its SM one cycle per lane and value; here the values go
+// through shared memory and consecutive lanes add consecutive addresses (0.4 cycles per value). Lanes in the
+// same cell are summed first. The exact limbs are integers, so no order of the adds shows in the sums.
+template <bool kExact>
+struct WarpDep3 {
+    static constexpr int kW = 2 * kDep0 * (kExact ? 2 : 1);      // values of a row
+    double val[32][kW + 1];                                      // odd row length: no bank conflicts
+    long off[32];
+    unsigned mask[32];
+    unsigned char lead[32];
+};
+
+// every lane of the warp calls it; act: the lane has a particle to deposit
+template <bool kExact>
+__device__ __forceinline__ void warp_deposit3(const BeamArgs& B, double* __restrict__ bsrc, bool act,
+                                              const DepOne<kDep0>& D, WarpDep3<kExact>& W) {
+    constexpr int kW = WarpDep3<kExact>::kW;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned key = act ? (unsigned)((D.k + 1) * B.M + D.j) : 0xffffffffu - lane;
+    const unsigned same = __match_any_sync(FULL, key);
+    const bool lead = act && lane == __ffs(same) - 1;
+    const unsigned leads = __ballot_sync(FULL, lead);
+    if (lead) {
+        W.off[lane] = ((long)D.k * B.M + D.j) * (kW / 2);
+        W.mask[lane] = same;
+        W.lead[__popc(leads & ((1u << lane) - 1u))] = (unsigned char)lane;
+    }
+    const int total = __popc(leads) * kW;
+    double w2[2];
+    if (act) {
+        w2[0] = D.d0 * (1.0 - D.t) * B.inv_V[D.j] * B.idxi;
+        w2[1] = D.d0 * D.t * B.inv_V[D.j + 1] * B.idxi;
+    }
+#pragma unroll 1
+    for (int a = 0; a < (B.ngp ? 1 : 2); ++a) {
+        if (act) {
+            const int kk = D.k + a;
+            const double Wk = kk >= 0 && kk < B.K ? (a ? D.tk : 1.0 - D.tk) : 0.0;   // rows out of the box: zeros
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
-        const int kk = k + a;
-        if (kk < 0 || kk >= B.K || (a == 1 && B.ngp)) continue;
+            for (int b = 0; b < 2; ++b) {
+                const double d = w2[b] * Wk;
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            double* o = bsrc + ((size_t)kk * B.M + j + b) * B_NC0;
-            if (B.fx_scale) {
-                const double sc = B.fx_scale[j + b];
-#pragma unroll
-                for (int c = 0; c < kDep0; ++c)
-                    beam_fx_add(o + comp[c], B.fx_lo, v[(2 * a + b) * kDep0 + c], sc, B.fx_inv2s, B.fx_2s);
-            } else {
-#pragma unroll
-                for (int c = 0; c < kDep0; ++c) atomicAdd(o + comp[c], v[(2 * a + b) * kDep0 + c]);
+                for (int c = 0; c < kDep0; ++c) {
+                    const double v = d * D.f[c];
+                    if constexpr (kExact) {
+                        double hi = 0.0, lo = 0.0;
+                        beam_fx_split(v, B.fx_scale[D.j + b], B.fx_inv2s, B.fx_2s, hi, lo);
+                        W.val[lane][b * 2 * kDep0 + c] = hi;
+                        W.val[lane][b * 2 * kDep0 + kDep0 + c] = lo;
+                    } else {
+                        W.val[lane][b * kDep0 + c] = v;
+                    }
+                }
             }
         }
+        __syncwarp();
+        double* const row = bsrc + (size_t)a * B.M * (kW / 2);
+        for (int q = lane; q < total; q += 32) {
+            const int sl = q / kW, w = q - sl * kW, src = W.lead[sl];
+            double v = W.val[src][w];
+            for (unsigned m = W.mask[src] & ~(1u << src); m; m &= m - 1) v += W.val[__ffs(m) - 1][w];
+            if (v != 0.0) atomicAdd(row + W.off[src] + w, v);    // (zero: nothing, or a row out of the box)
+        }
+        __syncwarp();
     }
 }
 
@@ -295,12 +348,12 @@ struct PState7 {
     double x, y, px, py, pz, xi, w;
 };
 
-template <bool kL2>
+template <bool kL2, bool kVec = false>
 __device__ __forceinline__ bool push_one(const BeamArgs& B, const double* __restrict__ fld, PState7& p, double h,
                                          double h_start, double dt, int* jcell = nullptr) {
     double c, sn;
     V3 E, Bf;
-    gather<kL2>(B, fld, p.x, p.y, p.xi, c, sn, E, Bf, jcell);
+    gather<kL2, kVec>(B, fld, p.x, p.y, p.xi, c, sn, E, Bf, jcell);
     V3 u = {p.px, p.py, p.pz};
     if (h_start != 0.0) {
         const double g0 = sqrt(1.0 + dot3(u, u));
@@ -314,7 +367,8 @@ __device__ __forceinline__ bool push_one(const BeamArgs& B, const double* __rest
     const double p2 = u.x * u.x + u.y * u.y;
     const double gam = sqrt(1.0 + p2 + u.z * u.z);
     const double omvz = (1.0 + p2) / (gam * (gam + u.z));
-    const double xn = p.x + u.x / gam * dt, yn = p.y + u.y / gam * dt;
+    const Recip ig(gam);
+    const double xn = p.x + ig(u.x) * dt, yn = p.y + ig(u.y) * dt;
     const double xin = p.xi + omvz * dt;
     const double xmin = B.xi_min, xmax = B.xi_min + (B.K - 1) * B.dxi;
     p.x = xn; p.y = yn; p.px = u.x; p.py = u.y; p.pz = u.z; p.xi = xin;

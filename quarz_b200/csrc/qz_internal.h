@@ -85,6 +85,9 @@ struct SweepArgs {
     const double* bq;
     double bfx_2s;
     long bfx_lo;
+    // m = 0: doubles per node of bsrc and the place of J_theta in a node: B_NC0 and B_JP1I, or in the pipeline's
+    // rings the compact layout rho - J_z, J_z, J_theta (3), in the exact format followed by their low limbs (6)
+    int bcs, bjt;
     // optional, m = 0: one slab of a xi-pipelined run (qz_sweep_run_stage). pin: the plasma entering
     // the slab's first slice ((6 + 5 ord, npad) like ps; null: the fresh plasma of the box head) and
     // pin_pushed: whether it has been pushed before (its AB history is filled); bguard: the beam sources
@@ -134,6 +137,7 @@ struct BeamArgs {
     const double* fx_scale;
     double fx_inv2s, fx_2s;         // 2^-S, 2^S
     long fx_lo;
+    int compact;                    // m = 0, the pipeline's rings: 3 values per node (and their low limbs behind them)
 };
 
 cudaError_t launch_beam_deposit(const BeamArgs& B, double* bsrc, cudaStream_t s);
@@ -190,7 +194,7 @@ struct PipeArgs {
     // (ring > nsteps) and every field row starts on a 128-byte line, so no cached line can hold a row
     // before the sweep published it (rows are only read once published, and kernels start with L1 clean)
     int fld_l1;
-    int modes, bnc;                 // azimuthal modes (0 / 1), beam-source components per node
+    int modes, bnc;                 // azimuthal modes (0 / 1), doubles per node of the beam sources
     size_t fld_slot, diag_slot, bsrc_slot, ps_slot;   // doubles per slot (ps: per team of sweep CTAs)
     double *fld, *diag, *bsrc, *ps;
     double* m1s;                    // modes = 1: per team of sweep CTAs, background (3 M) + source buffers (60 M)

@@ -32,7 +32,6 @@ namespace qzb {
 
 namespace {
 
-using beam_detail::deposit_one;
 using beam_detail::PState7;
 using beam_detail::push_one;
 using beam_detail::sums_add;
@@ -144,8 +143,6 @@ struct PipeGate {
             const int nr = P->sw.M * P->bnc;
             double* row = const_cast<double*>(g->bsrc) + (size_t)(k - 1) * nr;
             for (int i = rank * kT + threadIdx.x; i < nr; i += size * kT) __stcg(row + i, 0.0);
-            if (P->sw.bq)                            // the low limbs of the exact deposits
-                for (int i = rank * kT + threadIdx.x; i < nr; i += size * kT) __stcg(row + P->sw.bfx_lo + i, 0.0);
         }
     }
     // thread 0, after the barrier that ends slice k: publish it (the fence covers the stores of the
@@ -200,8 +197,6 @@ __device__ __forceinline__ void sweep_role(const PipeArgs& P, double* smem) {
         const int nr = M * P.bnc;
         double* row = P.bsrc + slot * P.bsrc_slot + (size_t)(K - 1) * nr;
         for (int i = team.rank * kT + tid; i < nr; i += team.size * kT) __stcg(row + i, 0.0);
-        if (P.sw.bq)
-            for (int i = tid; i < nr; i += kT) __stcg(row + P.sw.bfx_lo + i, 0.0);
         team.sync();
         if (tid == 0 && team.rank == 0) {
             __threadfence();
@@ -286,6 +281,7 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
     double* ih = r + M;
     double* iV = ih + M;
     double* fxs = iV + M + (size_t)(kT / 32) * 17 * 32;        // behind the per-warp moment slots
+    auto* const wdep = reinterpret_cast<beam_detail::WarpDep3<true>*>(fxs + M) + (tid >> 5);   // m = 0
     const double* fx_src = nullptr;
     for (int q = 0; q < P.nbeams && !fx_src; ++q) fx_src = P.beam[q].fx_scale;
     for (int j = tid; j < M; j += kT) {
@@ -327,8 +323,6 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
                 const double* b0 = bnext + (size_t)c0 * M * P.bnc;
                 const long bl = (long)(c1 - c0 + 1) * M * P.bnc;
                 for (long o = (long)lane * 16; o < bl; o += 32 * 16) prefetch_l2(b0 + o);
-                if (Bb.fx_scale)                            // the low limbs of the exact deposits
-                    for (long o = (long)lane * 16; o < bl; o += 32 * 16) prefetch_l2(b0 + Bb.fx_lo + o);
             }
             const long pn = i1 - i0;
             for (long o = (long)lane * 16; o < pn; o += 32 * 16) {
@@ -386,13 +380,11 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
         if (!push) {
             // moments only (the state after the last push)
         } else if (P.modes == 0) {
-            // m = 0: particles are in (xi cell, r cell) order, so neighbouring lanes mostly deposit into
-            // the same 2 x 2 cells: sum runs of equal cells across the warp, one reduction per run
             for (long base = i0; base < i1; base += 32) {
                 const long i = base + lane;
                 bool dep = false;
-                int dk = 0, dj = 0;
-                double v[4 * beam_detail::kDep0];
+                beam_detail::DepOne<beam_detail::kDep0> D;
+                D.k = D.j = 0;
                 if (i < i1) {
                     PState7 p;
                     p.w = __ldcg(Bb.w + i);
@@ -401,35 +393,30 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
                         p.px = __ldcg(Bb.px + i); p.py = __ldcg(Bb.py + i); p.pz = __ldcg(Bb.pz + i);
                         p.xi = __ldcg(Bb.xi + i);
                         if (fuse) beam_detail::sums_add_lane(macc + lane, p, gref, xiref);
-                        if (push) {
-                            bool alive = true;
-                            int jg = 0;
-                            if (!rigid) {
-                                alive = P.fld_l1 ? push_one<false>(Bb, fld, p, h, hs, P.dt_drift, &jg)
-                                                 : push_one<true>(Bb, fld, p, h, hs, P.dt_drift, &jg);
-                                __stcg(Bb.x + i, p.x); __stcg(Bb.y + i, p.y);
-                                __stcg(Bb.px + i, p.px); __stcg(Bb.py + i, p.py); __stcg(Bb.pz + i, p.pz);
-                                __stcg(Bb.xi + i, p.xi);
-                                if (!alive) __stcg(Bb.w + i, 0.0);
-                            } else {
-                                jg = -1;
-                            }
-                            if (alive) {
-                                dep = beam_detail::deposit_vals0(Bb, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w, jg, dk,
-                                                                 dj, v);
-                                cmax = max(cmax, xi_cell(Bb, p.xi));
-                            }
+                        bool alive = true;
+                        int jg = -1;
+                        if (!rigid) {
+                            alive = P.fld_l1 ? push_one<false, true>(Bb, fld, p, h, hs, P.dt_drift, &jg)
+                                             : push_one<true, true>(Bb, fld, p, h, hs, P.dt_drift, &jg);
+                            __stcg(Bb.x + i, p.x); __stcg(Bb.y + i, p.y);
+                            __stcg(Bb.px + i, p.px); __stcg(Bb.py + i, p.py); __stcg(Bb.pz + i, p.pz);
+                            __stcg(Bb.xi + i, p.xi);
+                            if (!alive) __stcg(Bb.w + i, 0.0);
+                        }
+                        if (alive) {
+                            dep = beam_detail::dep_one<beam_detail::kDep0>(Bb, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w, jg,
+                                                                           D);
+                            cmax = max(cmax, xi_cell(Bb, p.xi));
                         }
                     }
                 }
-                if (!dep)
-#pragma unroll
-                    for (int c = 0; c < 4 * beam_detail::kDep0; ++c) v[c] = 0.0;
-                const int key = dep ? (dk + 1) * M + dj : -1 - lane;
-                if (warp_runs_sum<4 * beam_detail::kDep0>(key, v) && dep) beam_detail::deposit_add0(Bb, bnext, dk, dj, v);
+                if (Bb.fx_scale) beam_detail::warp_deposit3<true>(Bb, bnext, dep, D, *wdep);
+                else beam_detail::warp_deposit3<false>(Bb, bnext, dep, D,
+                                                       *reinterpret_cast<beam_detail::WarpDep3<false>*>(wdep));
             }
-        } else if (P.modes == 1) {
-            // m = 1: the same runs of equal cells across the warp, summed per corner (12 components each)
+        } else {
+            // m = 1: particles are in (xi cell, r cell) order, so neighbouring lanes often deposit into the same
+            // 2 x 2 cells: runs of equal cells are summed across the warp, per corner (12 components each)
             for (long base = i0; base < i1; base += 32) {
                 const long i = base + lane;
                 bool dep = false;
@@ -445,8 +432,8 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
                         bool alive = true;
                         int jg = -1;
                         if (!rigid) {
-                            alive = P.fld_l1 ? push_one<false>(Bb, fld, p, h, hs, P.dt_drift, &jg)
-                                             : push_one<true>(Bb, fld, p, h, hs, P.dt_drift, &jg);
+                            alive = P.fld_l1 ? push_one<false, true>(Bb, fld, p, h, hs, P.dt_drift, &jg)
+                                             : push_one<true, true>(Bb, fld, p, h, hs, P.dt_drift, &jg);
                             __stcg(Bb.x + i, p.x); __stcg(Bb.y + i, p.y);
                             __stcg(Bb.px + i, p.px); __stcg(Bb.py + i, p.py); __stcg(Bb.pz + i, p.pz);
                             __stcg(Bb.xi + i, p.xi);
@@ -472,31 +459,6 @@ __device__ __forceinline__ void worker_role(const PipeArgs& P, double* smem) {
                         beam_detail::deposit_add1(Bb, bnext, D.k + a, D.j + b, v);
                 }
             }
-        } else
-        for (long i = i0 + lane; i < i1; i += 32) {
-            PState7 p;
-            p.w = __ldcg(Bb.w + i);
-            if (p.w == 0.0) continue;
-            p.x = __ldcg(Bb.x + i); p.y = __ldcg(Bb.y + i);
-            p.px = __ldcg(Bb.px + i); p.py = __ldcg(Bb.py + i); p.pz = __ldcg(Bb.pz + i);
-            p.xi = __ldcg(Bb.xi + i);
-            if (!push) continue;
-            if (rigid) {
-                deposit_one(Bb, bnext, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
-                cmax = max(cmax, xi_cell(Bb, p.xi));
-                continue;
-            }
-            const bool alive = P.fld_l1 ? push_one<false>(Bb, fld, p, h, hs, P.dt_drift)
-                                        : push_one<true>(Bb, fld, p, h, hs, P.dt_drift);
-            __stcg(Bb.x + i, p.x); __stcg(Bb.y + i, p.y);
-            __stcg(Bb.px + i, p.px); __stcg(Bb.py + i, p.py); __stcg(Bb.pz + i, p.pz);
-            __stcg(Bb.xi + i, p.xi);
-            if (!alive) {
-                __stcg(Bb.w + i, 0.0);
-                continue;
-            }
-            deposit_one(Bb, bnext, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
-            cmax = max(cmax, xi_cell(Bb, p.xi));
         }
         if (fuse) {
             double mine = 0.0;

@@ -259,68 +259,6 @@ __device__ __forceinline__ void scan_bwd_n(const double (&a)[NS], const double (
     }
 }
 
-// Exclusive scan of 2x2 matrix products (later rows on the left) for NS systems: on return
-// (p[s], q[s]) = first column of the product of all matrices before this thread's rows.
-template <int NS>
-__device__ __forceinline__ void scan_pivots(double (&m)[NS][4], double (&p)[NS], double (&q)[NS], double* tot) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // The thread's matrices must come renormalised (largest entry in [1, 2)); a product of at most 32 such
-    // matrices stays below 2^63 and the products of the 16 renormalised warp totals below 2^31, so the
-    // scan renormalises once per lane after the warp stage instead of at every level. Renormalising
-    // scales by powers of two, which is exact, and the pivots use only ratios of p and q: the results
-    // are the same bits either way.
-#pragma unroll
-    for (int st = 1; st < 32; st <<= 1) {
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            const double p00 = __shfl_up_sync(FULL, m[s][0], st), p01 = __shfl_up_sync(FULL, m[s][1], st);
-            const double p10 = __shfl_up_sync(FULL, m[s][2], st), p11 = __shfl_up_sync(FULL, m[s][3], st);
-            if (lane >= st) {
-                const double n00 = m[s][0] * p00 + m[s][1] * p10, n01 = m[s][0] * p01 + m[s][1] * p11;
-                const double n10 = m[s][2] * p00 + m[s][3] * p10, n11 = m[s][2] * p01 + m[s][3] * p11;
-                m[s][0] = n00; m[s][1] = n01; m[s][2] = n10; m[s][3] = n11;
-            }
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < NS; ++s) renorm(m[s][0], m[s][1], m[s][2], m[s][3]);
-    if (lane == 31)
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) tot[kW * (4 * s + e) + warp] = m[s][e];
-    double ex[NS][4];
-#pragma unroll
-    for (int s = 0; s < NS; ++s)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ex[s][e] = __shfl_up_sync(FULL, m[s][e], 1);
-    if (lane == 0)
-#pragma unroll
-        for (int s = 0; s < NS; ++s) { ex[s][0] = 1.0; ex[s][1] = 0.0; ex[s][2] = 0.0; ex[s][3] = 1.0; }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        double t00 = lane < kW ? tot[kW * (4 * s) + lane] : 1.0, t01 = lane < kW ? tot[kW * (4 * s + 1) + lane] : 0.0;
-        double t10 = lane < kW ? tot[kW * (4 * s + 2) + lane] : 0.0, t11 = lane < kW ? tot[kW * (4 * s + 3) + lane] : 1.0;
-#pragma unroll
-        for (int st = 1; st < kW; st <<= 1) {
-            const double p00 = __shfl_up_sync(FULL, t00, st), p01 = __shfl_up_sync(FULL, t01, st);
-            const double p10 = __shfl_up_sync(FULL, t10, st), p11 = __shfl_up_sync(FULL, t11, st);
-            if (lane >= st) {
-                const double n00 = t00 * p00 + t01 * p10, n01 = t00 * p01 + t01 * p11;
-                const double n10 = t10 * p00 + t11 * p10, n11 = t10 * p01 + t11 * p11;
-                t00 = n00; t01 = n01; t10 = n10; t11 = n11;
-            }
-        }
-        const int src = (warp + 31) & 31;
-        double c00 = __shfl_sync(FULL, t00, src), c10 = __shfl_sync(FULL, t10, src);
-        if (warp == 0) { c00 = 1.0; c10 = 0.0; }
-        // column 0 of (within-warp exclusive product) x (carry of the earlier warps)
-        p[s] = ex[s][0] * c00 + ex[s][1] * c10;
-        q[s] = ex[s][2] * c00 + ex[s][3] * c10;
-    }
-}
-
 // ---------------------------------------------------------------- batched shared-memory adds
 // All NA updates of one thread are issued together (independent compare-and-swap rounds) instead
 // of one serialised atomic loop per address. Lock-free: every round at least one contender of
@@ -625,8 +563,8 @@ struct BeamRow { double rt, drt, jz, jt; };
 template <bool kL2>                       // kL2: the rows were written by other SMs, read them from L2
 __device__ __forceinline__ double ldb(const double* p) { return kL2 ? __ldcg(p) : *p; }
 
-// one beam-source value at p (inside bsrc): the pushed beams' deposit plus, in kernels built for it
-// (kStat), the static (analytic) sources when present
+// one beam-source value at p (inside bsrc; NC values per node): the pushed beams' deposit plus, in kernels built
+// for it (kStat), the static (analytic) sources when present
 template <bool kL2, bool kStat>
 __device__ __forceinline__ double ldbs(const SweepArgs& A, const double* bsrc, const double* p) {
     const double v = ldb<kL2>(p);
@@ -644,36 +582,36 @@ __device__ __forceinline__ double guard_at(const SweepArgs& A, int j, int c) {
 
 template <bool kL2, bool kStat = false>
 __device__ __forceinline__ BeamRow beam_row(const SweepArgs& A, const double* bsrc, int k, int j) {
-    const size_t st = (size_t)A.M * B_NC0;
-    const double* bk = bsrc + (size_t)k * st + (size_t)j * B_NC0;
-    // one value of node j: a double, or the exact two-limb accumulator (A.bq) turned into its value
+    const size_t st = (size_t)A.M * A.bcs;
+    const double* const bj = bsrc + (size_t)j * A.bcs;
+    // component c (in place o of a node) of row kk: a double, or the exact two-limb accumulator (A.bq) turned
+    // into its value
     const double qj = A.bq ? A.bq[j] : 0.0;
-    auto ld = [&](const double* p) -> double {
-        if (A.bq) {
-            const double v = beam_fx_value(ldb<kL2>(p), ldb<kL2>(p + A.bfx_lo), qj, A.bfx_2s);
-            if constexpr (kStat) return A.bstat ? v + __ldg(A.bstat + (p - bsrc)) : v;
-            return v;
-        }
-        return ldbs<kL2, kStat>(A, bsrc, p);
+    auto ld = [&](int kk, int o, int c) -> double {
+        const double* p = bj + (size_t)kk * st + o;
+        double v = ldb<kL2>(p);
+        if (A.bq) v = beam_fx_value(v, ldb<kL2>(p + A.bfx_lo), qj, A.bfx_2s);
+        if constexpr (kStat) return A.bstat ? v + __ldg(A.bstat + ((size_t)kk * A.M + j) * B_NC0 + c) : v;
+        return v;
     };
+    auto rt = [&](int kk) { return ld(kk, B_RT0, B_RT0); };
     BeamRow r;
-    r.rt = ld(bk + B_RT0);
-    r.jz = ld(bk + B_JZ0);
-    r.jt = ld(bk + B_JP1I);
+    r.rt = rt(k);
+    r.jz = ld(k, B_JZ0, B_JZ0);
+    r.jt = ld(k, A.bjt, B_JP1I);
     const int K = A.K;
     // the slice ahead of slice 0: none at the box head, the guard row in a later slab of a staged run
     const double guard = guard_at(A, j, B_RT0);
     if (A.ngp) {
-        const double prev = (k > 0) ? ld(bk + B_RT0 - (ptrdiff_t)st) : guard;
-        r.drt = (r.rt - prev) * A.idxi;
+        r.drt = (r.rt - (k > 0 ? rt(k - 1) : guard)) * A.idxi;
     } else if (K == 1) {
         r.drt = 0.0;
     } else if (k == 0) {
-        r.drt = A.bguard ? 0.5 * (ld(bk + st + B_RT0) - guard) * A.idxi : (ld(bk + st + B_RT0) - r.rt) * A.idxi;
+        r.drt = A.bguard ? 0.5 * (rt(1) - guard) * A.idxi : (rt(1) - r.rt) * A.idxi;
     } else if (k == K - 1) {
-        r.drt = (r.rt - ld(bk + B_RT0 - (ptrdiff_t)st)) * A.idxi;
+        r.drt = (r.rt - rt(k - 1)) * A.idxi;
     } else {
-        r.drt = 0.5 * (ld(bk + st + B_RT0) - ld(bk + B_RT0 - (ptrdiff_t)st)) * A.idxi;
+        r.drt = 0.5 * (rt(k + 1) - rt(k - 1)) * A.idxi;
     }
     return r;
 }
@@ -683,9 +621,9 @@ __device__ __forceinline__ BeamRow beam_row(const SweepArgs& A, const double* bs
 struct BeamRaw { double v[5], w[5]; };
 template <bool kL2>
 __device__ __forceinline__ void raw_load(const SweepArgs& A, const double* bsrc, int k, int j, BeamRaw& b) {
-    const size_t st = (size_t)A.M * B_NC0;
-    const double* const bk = bsrc + (size_t)k * st + (size_t)j * B_NC0;
-    const double* const p[5] = {bk + B_RT0, bk + B_JZ0, bk + B_JP1I, k > 0 ? bk + B_RT0 - (ptrdiff_t)st : bk + B_RT0,
+    const size_t st = (size_t)A.M * A.bcs;
+    const double* const bk = bsrc + (size_t)k * st + (size_t)j * A.bcs;
+    const double* const p[5] = {bk + B_RT0, bk + B_JZ0, bk + A.bjt, k > 0 ? bk + B_RT0 - (ptrdiff_t)st : bk + B_RT0,
                                 k + 1 < A.K ? bk + st + B_RT0 : bk + B_RT0};
 #pragma unroll
     for (int c = 0; c < 5; ++c) b.v[c] = ldb<kL2>(p[c]);
@@ -1307,46 +1245,54 @@ __device__ __forceinline__ void row_b(const Smem& S, const Src& s, int N, double
     }
 }
 
-// psi, E_z, B_z and W+ (src/Simulation.cpp:797-807, :501-532, :477-498). L0 is D^-1 times a Laplacian: with
-// w_i = V_i / 2 pi and g_i = r_mid,i / h_i its rows say that the flux g_i (x_{i+1} - x_i) is the sum of w d up
-// to node i. The Thomas pivots of that matrix are -g_i / w_i exactly, so the two substitutions are plain
-// sums: z_i = z_{i-1} + w_i d_i and x_i = x_{i+1} - z_i / g_i.
-template <int kR>
-__device__ __forceinline__ void l0_solve(const Smem& S, const Src& s, int M, int N) {
-    const int warp = threadIdx.x >> 5, e = warp / kG2, wl = warp - e * kG2;
-    if (e >= 3) return;
-    const int R = group_rows(M, kG2), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
-    double* const tz = S.tot + 8 * e;
-    double* const tx = S.tot + 24 + 8 * e;
-    double v[kR], sum = 0.0;
+// One L0 system by a group of kG2 warps (e: 0..2, the group's number), rows [row0, row0 + R) per thread. L0 is
+// D^-1 times a Laplacian: with w_i = V_i / 2 pi and g_i = r_mid,i / h_i its rows say that the flux g_i (x_{i+1} - x_i)
+// is the sum of w d up to node i. The Thomas pivots of that matrix are -g_i / w_i exactly, so the two
+// substitutions are plain sums: z_i = z_{i-1} + w_i d_i and x_i = x_{i+1} - z_i / g_i. rhs(i): d_i for i < N. On return
+// v holds x of the thread's rows, z0 the flux into them and xn the x just after them.
+template <int kR, class Rhs>
+__device__ __forceinline__ void l0_group(double* tot, const double* vw, const double* gw, int N, int e, int wl, int R,
+                                         int row0, Rhs rhs, double (&v)[kR], double& z0, double& xn) {
+    double sum = 0.0;
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
         const int i = row0 + u;
         v[u] = 0.0;
-        if (u < R && i < N) v[u] = S.vw[i] * rhs_l0(S, s, N, e, i);
+        if (u < R && i < N) v[u] = vw[i] * rhs(i);
         sum += v[u];
     }
-    double z = group_sum<true, kG2>(sum, wl, tz, 1 + e);
-    const double z0 = z;
+    double z = group_sum<true, kG2>(sum, wl, tot + 8 * e, 1 + e);
+    z0 = z;
     sum = 0.0;
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
         const int i = row0 + u;
         z += v[u];
-        v[u] = (u < R && i < N) ? -(z * S.gw[i]) : 0.0;
+        v[u] = (u < R && i < N) ? -(z * gw[i]) : 0.0;
     }
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) sum += v[u];
-    double x = group_sum<false, kG2>(sum, wl, tx, 1 + e);
-    double* const out = e == 0 ? S.psi : (e == 1 ? S.ez : S.bz);
-    const double xn = x;                                  // x just after this thread's rows
+    double x = group_sum<false, kG2>(sum, wl, tot + 24 + 8 * e, 1 + e);
+    xn = x;
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) {
-        const int i = row0 + u;
         x += v[u];
         v[u] = x;
-        if (u < R && i < M) out[i] = x;
     }
+}
+
+// psi, E_z, B_z and W+ (src/Simulation.cpp:797-807, :501-532, :477-498)
+template <int kR>
+__device__ __forceinline__ void l0_solve(const Smem& S, const Src& s, int M, int N) {
+    const int warp = threadIdx.x >> 5, e = warp / kG2, wl = warp - e * kG2;
+    if (e >= 3) return;
+    const int R = group_rows(M, kG2), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
+    double v[kR], z0, xn;
+    l0_group<kR>(S.tot, S.vw, S.gw, N, e, wl, R, row0, [&](int i) { return rhs_l0(S, s, N, e, i); }, v, z0, xn);
+    double* const out = e == 0 ? S.psi : (e == 1 ? S.ez : S.bz);
+#pragma unroll
+    for (int u = 0; u < kR; ++u)
+        if (u < R && row0 + u < M) out[row0 + u] = v[u];
     if (e != 0) return;
     // W+ = -psi' on the thread's rows; psi just before them from the flux that enters them
     double xm = (row0 >= 1 && row0 < M) ? v[0] - z0 * S.gw[row0 - 1] : 0.0;
@@ -1362,29 +1308,24 @@ __device__ __forceinline__ void l0_solve(const Smem& S, const Src& s, int M, int
     }
 }
 
-// B_r and B_theta (src/Simulation.cpp:535-591, m = 0: one pass): (L1D - chi) B_r0 = -S_i (rows 0, N Dirichlet)
-// and (L1F - chi) B_theta0 = J_z' + S_r with flux wall J_z(R). 1/u_i = p_{i-1} / p_i, where (p_i, p_{i-1}) is the
-// first column of the product of T_i = [[b_i, -a_i c_{i-1}], [1, 0]] up to row i. Sv: the S+ values of a row
-// (kFinish: turned from the exact accumulators here, each by its only reader)
-template <int kR, bool kFinish>
-__device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, int N, double fc, int bits) {
-    const int warp = threadIdx.x >> 5, sy = warp / kG4, wl = warp - sy * kG4;
-    const int R = group_rows(M, kG4), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
-    double* const tp = S.tot + 64 + 32 * sy;
-    double* const tf = S.tot + 128 + 16 * sy;
-    double* const tb = S.tot + 160 + 16 * sy;
-    double* const sa = sy ? s.S1r : s.S1i;
-    const double qs = kFinish ? fx_quantum(S.fx[sy ? 7 : 8], bits) : 0.0;
-    const int es = kFinish ? S.fx[sy ? 7 : 8] : 0;
-    double ra[kR], rb[kR], rc[kR], rd[kR];
+// One chi-shifted system by a group of kG4 warps (sy: 0 or 1), rows [row0, row0 + R) per thread: 1/u_i = p_{i-1} /
+// p_i, where (p_i, p_{i-1}) is the first column of the product of T_i = [[b_i, -a_i c_{i-1}], [1, 0]] up to row i.
+// row(i, a, b, cm, d): row i with cm = c_{i-1} and its right-hand side; c(i): c_i. On return x holds the solution
+// on the thread's rows.
+template <int kR, class Row, class C>
+__device__ __forceinline__ void shifted_group(double* tot, int M, int sy, int wl, int R, int row0, Row row, C c,
+                                              double (&x)[kR]) {
+    double* const tp = tot + 64 + 32 * sy;
+    double* const tf = tot + 128 + 16 * sy;
+    double* const tb = tot + 160 + 16 * sy;
+    double ra[kR], rb[kR], rc[kR];
     double m[4] = {1.0, 0.0, 0.0, 1.0};
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
         const int i = row0 + u;
-        ra[u] = 0.0; rb[u] = 1.0; rc[u] = 0.0; rd[u] = 0.0;
+        ra[u] = 0.0; rb[u] = 1.0; rc[u] = 0.0; x[u] = 0.0;
         if (u < R && i < M) {
-            const double sv = kFinish ? fx_value(sa + i, es, qs) : sa[i];
-            row_b(S, s, N, fc, sy, i, sv, ra[u], rb[u], rc[u], rd[u]);
+            row(i, ra[u], rb[u], rc[u], x[u]);
             const double t01 = -ra[u] * rc[u];
             const double n00 = rb[u] * m[0] + t01 * m[2], n01 = rb[u] * m[1] + t01 * m[3];
             m[2] = m[0]; m[3] = m[1];
@@ -1407,11 +1348,10 @@ __device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, 
     }
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
-        if (u >= R || i >= M) { rc[u] = 0.0; continue; }
+        if (u >= R || row0 + u >= M) { rc[u] = 0.0; continue; }
         ra[u] = -rc[u] * ra[u];
-        rd[u] = rc[u] * rd[u];
-        fB = fma(ra[u], fB, rd[u]);
+        x[u] = rc[u] * x[u];
+        fB = fma(ra[u], fB, x[u]);
         fA *= ra[u];
     }
     double y = group_affine<true, kG4>(fA, fB, wl, tf, 4 + sy);
@@ -1420,26 +1360,46 @@ __device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, 
     for (int u = 0; u < kR; ++u) {
         const int i = row0 + u;
         if (u >= R || i >= M) continue;
-        y = fma(ra[u], y, rd[u]);
-        rd[u] = y;
-        rc[u] = -((sy && i == N ? 0.0 : S.l1c[i]) * rc[u]);      // x_i = -(c_i / u_i) x_{i+1} + y_i
+        y = fma(ra[u], y, x[u]);
+        x[u] = y;
+        rc[u] = -(c(i) * rc[u]);                              // x_i = -(c_i / u_i) x_{i+1} + y_i
     }
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) {
-        const int i = row0 + u;
-        if (u >= R || i >= M) continue;
-        bB = fma(rc[u], bB, rd[u]);
+        if (u >= R || row0 + u >= M) continue;
+        bB = fma(rc[u], bB, x[u]);
         bA *= rc[u];
     }
-    double x = group_affine<false, kG4>(bA, bB, wl, tb, 4 + sy);
-    double* const out = sy ? S.bpi : S.bpr;
+    double xx = group_affine<false, kG4>(bA, bB, wl, tb, 4 + sy);
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) {
-        const int i = row0 + u;
-        if (u >= R || i >= M) continue;
-        x = fma(rc[u], x, rd[u]);
-        out[i] = x;
+        if (u >= R || row0 + u >= M) continue;
+        xx = fma(rc[u], xx, x[u]);
+        x[u] = xx;
     }
+}
+
+// B_r and B_theta (src/Simulation.cpp:535-591, m = 0: one pass): (L1D - chi) B_r0 = -S_i (rows 0, N Dirichlet)
+// and (L1F - chi) B_theta0 = J_z' + S_r with flux wall J_z(R). kFinish: S_i and S_r are turned from the exact
+// accumulators here, each by its only reader
+template <int kR, bool kFinish>
+__device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, int N, double fc, int bits) {
+    const int warp = threadIdx.x >> 5, sy = warp / kG4, wl = warp - sy * kG4;
+    const int R = group_rows(M, kG4), row0 = (wl * 32 + (threadIdx.x & 31)) * R;
+    double* const sa = sy ? s.S1r : s.S1i;
+    const int es = kFinish ? S.fx[sy ? 7 : 8] : 0;
+    const double qs = kFinish ? fx_quantum(es, bits) : 0.0;
+    double x[kR];
+    shifted_group<kR>(
+        S.tot, M, sy, wl, R, row0,
+        [&](int i, double& a, double& b, double& cm, double& d) {
+            row_b(S, s, N, fc, sy, i, kFinish ? fx_value(sa + i, es, qs) : sa[i], a, b, cm, d);
+        },
+        [&](int i) { return sy && i == N ? 0.0 : S.l1c[i]; }, x);
+    double* const out = sy ? S.bpi : S.bpr;
+#pragma unroll
+    for (int u = 0; u < kR; ++u)
+        if (u < R && row0 + u < M) out[row0 + u] = x[u];
 }
 
 }  // namespace sweep_detail
