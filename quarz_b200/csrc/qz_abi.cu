@@ -186,7 +186,7 @@ extern "C" qz_status qz_grid_create(const double* nodes, int M, qz_grid** out) {
         std::vector<double> cz((size_t)qzb::kConsts0 * M, 0.0);
         for (int k = 0; k < 4; ++k) std::copy(cs.begin() + (size_t)k * M, cs.begin() + (size_t)(k + 1) * M, cz.begin() + (size_t)k * M);
         for (int i = 0; i < M; ++i) {
-            cz[(size_t)4 * M + i] = g->V[i] / (2 * PI);
+            cz[(size_t)4 * M + i] = i < N ? g->V[i] / (2 * PI) : 0.0;        // (row N: Dirichlet)
             cz[(size_t)5 * M + i] = i < N ? g->h[i] / g->rmid[i] : 0.0;
         }
         for (int k = 0; k < 3; ++k) std::copy(cs.begin() + (size_t)(7 + k) * M, cs.begin() + (size_t)(8 + k) * M, cz.begin() + (size_t)(6 + k) * M);
@@ -2480,14 +2480,14 @@ extern "C" qz_status qz_batch_run(qz_batch* b, int nsteps, double dt, double* mo
         Group& G = gr[grp[i]];
         ++G.n;
         G.with_m1 = G.with_m1 || m1;
-        G.with_ext = G.with_ext || A.filter;
+        G.with_ext = G.with_ext || qzb::sweep_ext(A);
         const size_t km = (size_t)A.K * A.M;
         G.fmax = std::max(G.fmax, km * (m1 ? 18 : 6));        // fld (K, M, 18 / 6)
         G.dmax = std::max(G.dmax, km * (m1 ? 9 : 3));         // diag (K, M, 9 / 3)
         G.bmax = std::max(G.bmax, km * (m1 ? 15 : 5));        // bsrc (K, M, 15 / 5)
         G.smem = std::max(G.smem, grp[i] ? qzb::sweep_m1w_smem_bytes(A.M)
                                   : m1 ? qzb::sweep_m1_smem_bytes(A.M)
-                                       : qzb::sweep_m0_smem_bytes(A.M, A.dbuf, A.const_smem, A.filter != 0, A.pcache));
+                                       : std::max(qzb::sweep_m0_smem_bytes(A, false), qzb::sweep_m0_smem_bytes(A, true)));
         mom_off[i] = mom_total;
         mom_total += (size_t)(nsteps + 1) * std::max(1, b->inst[i]->dev.nbeams) * 17;
     }

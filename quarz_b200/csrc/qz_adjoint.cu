@@ -998,7 +998,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
                 [&](int r, double& a, double& b, double& cm, double& d) {
                     a = sy4 ? lfa[r] : l1a[r];
                     b = sy4 ? lfb[r] : l1b[r];
-                    cm = r > 0 ? l1c[r - 1] : 0.0;
+                    cm = l1c[row_lo(r)];                 // (a = 0 at row 0)
                     d = 0.0;
                     if (r >= 1 && (sy4 || r < N)) {
                         b -= S.chi[r];
@@ -1072,7 +1072,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
 #pragma unroll
                 for (int u = 0; u < kR2; ++u) {
                     const int r = row0 + u;
-                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[4 * (size_t)M + r])) : -0.0;
+                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[4 * (size_t)M + r])) : -0.0;   // mu = x V
                 }
             }
         }

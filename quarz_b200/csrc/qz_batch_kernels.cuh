@@ -33,18 +33,18 @@ __device__ __forceinline__ unsigned long long batch_timer() {
 // beam work of one instance by the whole CTA: moments (step n) of every beam, then, when push,
 // the push with the fields of step n and the deposit into bsrc (zeroed first)
 __device__ void beam_phase(const BatchInst& I, const SweepArgs& A, const BatchArgs& B, int n, bool push, bool startup,
-                           double* red) {
+                           double* red, int st) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (push) {
         const size_t nb = (size_t)A.K * A.M * (I.modes ? B_NC1 : B_NC0);
         for (size_t t = tid; t < nb; t += kT) const_cast<double*>(A.bsrc)[t] = 0.0;
         __syncthreads();
     }
-    // the sweep leaves the grid in shared memory (qz_sweep_body.cuh carve: r, 1/V, 1/h first)
+    // the sweep leaves the grid in shared memory (qz_sweep_body.cuh carve: r, 1/V, 1/h first, st doubles apart)
     extern __shared__ double smem_raw[];
     const double* r = smem_raw;
-    const double* iV = smem_raw + A.M;
-    const double* ih = smem_raw + 2 * A.M;
+    const double* iV = smem_raw + st;
+    const double* ih = smem_raw + 2 * st;
     for (int q = 0; q < I.nbeams; ++q) {
         BeamArgs Bb = I.beam[q];
         Bb.r = r;
@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) batch_kernel(const __grid_co
         __syncthreads();
         const SweepArgs& A = I.sw;
         const bool reg = A.np <= kSweepThreads;
-        (void)reg;
+        const bool hist = !I.modes && hist_doubles(ORD, reg, A.rows_per_thread == 1 ? 1 : 4, EXT) > 0;
+        const int st = hist ? kSweepThreads : A.M;       // distance between the sweep's shared arrays
         unsigned long long t_start = 0, t_mark = 0, t_sweep = 0, t_beam = 0;
         if (B.trace && tid == 0) t_start = t_mark = batch_timer();
         beam_deposit0(I, A);
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) batch_kernel(const __grid_co
             }
             __syncthreads();
             if (B.trace && tid == 0) { const unsigned long long t = batch_timer(); t_sweep += t - t_mark; t_mark = t; }
-            beam_phase(I, A, B, n, n < B.nsteps, n == 0, red);
+            beam_phase(I, A, B, n, n < B.nsteps, n == 0, red, st);
         }
         __syncthreads();
         if (B.trace && tid == 0) {

@@ -99,7 +99,16 @@ struct SweepArgs {
     double* pout;
 };
 
+// whether the sweep keeps its per-node constants in shared memory: where A asks for it, and always with one row
+// and one particle per thread (sweep_body)
+inline bool consts_in_smem(const SweepArgs& A) {
+    return A.const_smem || (A.np <= kSweepThreads && A.rows_per_thread == 1);
+}
+// whether A needs the kernel variant with the smoothing filter, static sources and adaptive sub-slicing
+inline bool sweep_ext(const SweepArgs& A) { return A.filter || A.bstat || A.max_cells > 0.0; }
 size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter = false, int pcache = 0);
+// of the kernel variant that runs A; ext: the variant with the smoothing filter and static sources
+size_t sweep_m0_smem_bytes(const SweepArgs& A, bool ext);
 cudaError_t launch_sweep_m0(const SweepArgs& A, cudaStream_t stream);
 // the modes = 1 sweep: one CTA, one radial row per thread (M <= kSweepThreads), plasma in A.ps
 size_t sweep_m1_smem_bytes(int M);
@@ -236,7 +245,7 @@ struct PipeArgs {
 constexpr int kTraceStride = 22;
 constexpr int kWorkerTotals = 6;    // trace totals of the push workers after the steps
 
-size_t pipeline_smem_bytes(int modes, int M, bool dbuf, bool const_smem, bool filter = false, int pcache = 0);
+size_t pipeline_smem_bytes(const PipeArgs& P);
 // resident CTAs of the pipeline kernel on this device, in clusters of P.team (0 if it cannot run); *sms: the SM count
 int pipeline_max_grid(const PipeArgs& P, int* sms);
 // cooperative launch of grid CTAs (fails unless all of them can be resident at once)

@@ -573,7 +573,7 @@ cudaError_t launch_e(const PipeArgs& P, int grid, size_t smem, cudaStream_t s) {
 
 template <int ORD>
 cudaError_t launch_o(const PipeArgs& P, int grid, size_t smem, cudaStream_t s) {
-    const bool ext = P.sw.filter || P.sw.bstat;
+    const bool ext = sweep_ext(P.sw);
     if (P.modes == 1)
         return ext ? launch_t<1, ORD, false, 1, true>(P, grid, smem, s) : launch_t<1, ORD, false, 1, false>(P, grid, smem, s);
     return ext ? launch_e<ORD, true>(P, grid, smem, s) : launch_e<ORD, false>(P, grid, smem, s);
@@ -589,7 +589,7 @@ int occupancy_e(const PipeArgs& P, size_t smem, int nsm) {
 
 template <int ORD>
 int occupancy_o(const PipeArgs& P, size_t smem, int nsm) {
-    const bool ext = P.sw.filter || P.sw.bstat;
+    const bool ext = sweep_ext(P.sw);
     if (P.modes == 1) return ext ? occupancy_t<1, ORD, false, 1, true>(P, smem, nsm) : occupancy_t<1, ORD, false, 1, false>(P, smem, nsm);
     return ext ? occupancy_e<ORD, true>(P, smem, nsm) : occupancy_e<ORD, false>(P, smem, nsm);
 }

@@ -16,10 +16,16 @@ size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter, int p
     size_t d = (size_t)(3 + 2 + 6 + (dbuf ? 18 : 9)) * M + sweep_detail::kTot;
     if (const_smem) d += (size_t)kConsts0 * M;
     if (filter) d += 4 * (size_t)M + 2 * 14 * (kSweepThreads / 32);
-    // + lost, flag, 14 exponent maxima and counters, the cells-crossed word (128 B with the particle copy
-    // behind them: 6 doubles and a cell index per particle)
-    if (pcache > 0) return sizeof(double) * d + 128 + (size_t)pcache * (6 * sizeof(double) + sizeof(int));
-    return sizeof(double) * d + 16 + 4 * 16;
+    // + the words from Smem::lost on, and with the particle copy 6 doubles and a cell index per particle
+    return sizeof(double) * d + sweep_detail::kMiscBytes + (pcache > 0 ? (size_t)pcache * (6 * sizeof(double) + sizeof(int)) : 0);
+}
+
+size_t sweep_m0_smem_bytes(const SweepArgs& A, bool ext) {
+    const bool reg = A.np <= kSweepThreads;
+    const int hist = sweep_detail::hist_doubles(A.ord, reg, A.rows_per_thread == 1 ? 1 : 4, ext);
+    // (the variant with the history lays its arrays out kSweepThreads nodes apart: carve)
+    return sweep_m0_smem_bytes(hist ? kSweepThreads : A.M, hist ? false : A.dbuf != 0, consts_in_smem(A), A.filter != 0, A.pcache) +
+           sizeof(double) * hist * kSweepThreads;
 }
 
 namespace {
@@ -42,13 +48,13 @@ cudaError_t launch_e(const SweepArgs& A, size_t smem, cudaStream_t stream) {
 
 template <int ORD>
 cudaError_t launch_o(const SweepArgs& A, size_t smem, cudaStream_t stream) {
-    return (A.filter || A.bstat) ? launch_e<ORD, true>(A, smem, stream) : launch_e<ORD, false>(A, smem, stream);
+    return sweep_ext(A) ? launch_e<ORD, true>(A, smem, stream) : launch_e<ORD, false>(A, smem, stream);
 }
 }  // namespace
 
 cudaError_t launch_sweep_m0(const SweepArgs& A, cudaStream_t stream) {
     if (A.rows_per_thread < 1 || A.rows_per_thread > 4) return cudaErrorInvalidValue;
-    const size_t smem = sweep_m0_smem_bytes(A.M, A.dbuf, A.const_smem, A.filter != 0, A.pcache);
+    const size_t smem = sweep_m0_smem_bytes(A, sweep_ext(A));
     switch (A.ord) {
         case 1: return launch_o<1>(A, smem, stream);
         case 2: return launch_o<2>(A, smem, stream);

@@ -57,12 +57,11 @@ struct NoGate {
 // Block-wide scans of one row per thread (the smoothing filter and the adjoint's reverse sweep). Shared
 // scratch for the warp totals of one scan: 8 x kW doubles; two of them alternate.
 
-// exact power-of-two rescaling of a 2x2 matrix (its largest entry into [1, 2))
+// exact power-of-two rescaling of a 2x2 matrix (its largest entry into [1, 2)), by the exponent fields
 __device__ __forceinline__ void renorm(double& m00, double& m01, double& m10, double& m11) {
-    const double mx = fmax(fmax(fabs(m00), fabs(m01)), fmax(fabs(m10), fabs(m11)));
-    if (!(mx > 0.0) || !(mx < 1e300)) return;
-    const int e = ((__double2hiint(mx) >> 20) & 0x7ff) - 1023;
-    const double s = __hiloint2double((1023 - e) << 20, 0);
+    const int e = max(max(__double2hiint(m00) & 0x7ff00000, __double2hiint(m01) & 0x7ff00000),
+                      max(__double2hiint(m10) & 0x7ff00000, __double2hiint(m11) & 0x7ff00000));
+    const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
     m00 *= s; m01 *= s; m10 *= s; m11 *= s;
 }
 
@@ -379,6 +378,7 @@ __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1)
 // psi, E_z, B_z together went from 9,800 to 2,900 cycles per slice and B+ from 10,800 to 4,400 (512 nodes).
 // The row count is odd, so that the lanes' rows lie in different shared-memory banks.
 constexpr int kG2 = 5, kG4 = 8;                           // warps per system: 3 x 5 and 2 x 8
+constexpr int kMiscBytes = 256;                           // the words from Smem::lost on
 constexpr int kTot = 256;                                 // S.tot: 24 + 24 (L0), 64 + 32 + 32 (B+)
 __device__ __forceinline__ int group_rows(int M, int warps) { return ((M + 32 * warps - 1) / (32 * warps)) | 1; }
 __device__ __forceinline__ void group_sync(int id, int threads) {
@@ -399,11 +399,13 @@ __device__ __forceinline__ double group_sum(double v, int wl, double* tot, int i
     double e = kUp ? __shfl_up_sync(FULL, s, 1) : __shfl_down_sync(FULL, s, 1);
     if (lane == (kUp ? 0 : 31)) e = 0.0;
     group_sync(id, 32 * kWarps);
-    double c = 0.0;
+    double t[kWarps], c = 0.0;                             // (loads first: one shared-memory latency for all)
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) t[w] = tot[w];
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
         const int o = kUp ? w : kWarps - 1 - w;
-        if (kUp ? o < wl : o > wl) c += tot[o];
+        c += (kUp ? o < wl : o > wl) ? t[o] : 0.0;
     }
     return c + e;
 }
@@ -424,11 +426,17 @@ __device__ __forceinline__ double group_affine(double a, double b, int wl, doubl
     double eb = kUp ? __shfl_up_sync(FULL, b, 1) : __shfl_down_sync(FULL, b, 1);
     if (lane == (kUp ? 0 : 31)) { ea = 1.0; eb = 0.0; }
     group_sync(id, 32 * kWarps);
-    double c = 0.0;
+    double ta[kWarps], tb[kWarps], c = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        ta[w] = tot[2 * w];
+        tb[w] = tot[2 * w + 1];
+    }
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
         const int o = kUp ? w : kWarps - 1 - w;
-        if (kUp ? o < wl : o > wl) c = fma(tot[2 * o], c, tot[2 * o + 1]);
+        const double n = fma(ta[o], c, tb[o]);
+        c = (kUp ? o < wl : o > wl) ? n : c;
     }
     return fma(ea, c, eb);
 }
@@ -460,12 +468,11 @@ __device__ __forceinline__ void group_pivots(double (&m)[4], double& p, double& 
     group_sync(id, 32 * kWarps);
     double c0 = 1.0, c1 = 0.0;
 #pragma unroll
-    for (int w = 0; w < kWarps - 1; ++w)
-        if (w < wl) {
-            const double n0 = tot[4 * w] * c0 + tot[4 * w + 1] * c1;
-            c1 = tot[4 * w + 2] * c0 + tot[4 * w + 3] * c1;
-            c0 = n0;
-        }
+    for (int w = 0; w < kWarps - 1; ++w) {
+        const double n0 = tot[4 * w] * c0 + tot[4 * w + 1] * c1, n1 = tot[4 * w + 2] * c0 + tot[4 * w + 3] * c1;
+        c0 = w < wl ? n0 : c0;
+        c1 = w < wl ? n1 : c1;
+    }
     p = ex[0] * c0 + ex[1] * c1;
     q = ex[2] * c0 + ex[3] * c1;
 }
@@ -489,6 +496,11 @@ __device__ __forceinline__ double pivot_quot(double q, double p) {
     return fma(fma(-p, r, q), y, r);
 }
 
+// doubles per thread of the history kept in shared memory by the sweep variant (0: kept in registers)
+constexpr int hist_doubles(int ord, bool reg, int max_r, bool ext) {
+    return reg && max_r == 1 && !ext && ord <= 3 ? 5 * ord : 0;
+}
+
 // ---------------------------------------------------------------- shared-memory layout
 struct Src {                                              // plasma + beam sources of one slice
     double *rhot, *drho, *jz, *chi, *ne, *ni, *jpi1, *S1r, *S1i;
@@ -504,6 +516,7 @@ struct Smem {
     double *bgt, *bgr;                                    // neutralising background
     double *psi, *ez, *bz, *wr1, *bpr, *bpi;              // fields of the slice (wr1 = -psi')
     double* tot;                                          // scan scratch of the solves, kTot doubles
+    double* hist;                                         // Adams-Bashforth history: slot, component, thread (hist_at)
     double* stage;                                        // A.filter: beam + background part of the next slice (4 x M)
     double* ftot;                                         // A.filter: scan scratch of the filter, 2 x 14 x kW
     int* lost;
@@ -513,6 +526,8 @@ struct Smem {
     // counters: [11] extra sub-slices, [12] particles removed as trapped, [13] non-finite deposits
     int* fx;
     unsigned long long* cmax;                             // most cells crossed (sub-slicing), as double bits
+    long long* tmark;                                     // clock marks of the phase counters: [0] phases, [1] parts
+    double* absl;                                         // sub-slicing: xi of the last pushes, twice 8 (AbState)
     // A.pcache > 0 (plasma in global memory, np = A.pcache): a copy of every particle's x y px py Delta w
     // (pc, 6 x np) and its radial cell (pj), written through with the global state whenever a particle
     // moves; the passes that only read the particles take them from here, without a cell search
@@ -520,30 +535,40 @@ struct Smem {
     int* pj;
 };
 
+// kCS: the constants are in shared memory whatever A says; kHist > 0: sources single-buffered whatever A says, and
+// the kHist doubles per thread of the particles' Adams-Bashforth history
+template <bool kCS, int kHist>
 __device__ __forceinline__ Smem carve(double* base, const SweepArgs& A) {
-    const int M = A.M;
+    // distance between arrays: with the history (M <= kThreads) a constant, so that an element's address is one
+    // register and an immediate, and the 29 array pointers take no registers
+    const int M = kHist ? kThreads : A.M;
     Smem S;
     double* p = base;
     S.r = p; p += M; S.iv = p; p += M; S.ih = p; p += M;
     // the 9 arrays the sweep reads, behind one another as in A.consts0
-    const double* q = A.const_smem ? p : A.consts0;
+    const double* q = p;
+    if constexpr (!kCS)
+        if (!A.const_smem) q = A.consts0;
     S.gm = q; S.g0 = q + M; S.gp = q + 2 * M; S.ir = q + 3 * M;
     S.vw = q + 4 * M; S.gw = q + 5 * M;
     S.l1a = q + 6 * M; S.l1b = q + 7 * M; S.l1c = q + 8 * M;
     S.lfa = A.lfa_N; S.lfb = A.lfb_N;
-    if (A.const_smem) p += (size_t)kConsts0 * M;
+    if (kCS || A.const_smem) p += (size_t)kConsts0 * M;
     S.src0 = p;
-    p += (A.dbuf ? 18 : 9) * (size_t)M;
+    p += (!kHist && A.dbuf ? 18 : 9) * (size_t)M;
     S.bgt = p; p += M; S.bgr = p; p += M;
     S.psi = p; p += M; S.ez = p; p += M; S.bz = p; p += M; S.wr1 = p; p += M; S.bpr = p; p += M; S.bpi = p; p += M;
     S.tot = p; p += kTot;
+    S.hist = p; p += kHist * kThreads;
     S.stage = S.ftot = nullptr;
     if (A.filter) { S.stage = p; p += 4 * (size_t)M; S.ftot = p; p += 2 * 14 * kW; }
     S.lost = reinterpret_cast<int*>(p);
     S.flag = S.lost + 1;
     S.fx = S.lost + 2;
     S.cmax = reinterpret_cast<unsigned long long*>(S.lost + 16);
-    S.pc = A.pcache ? reinterpret_cast<double*>(reinterpret_cast<char*>(S.lost) + 128) : nullptr;
+    S.tmark = reinterpret_cast<long long*>(S.lost + 28);
+    S.absl = reinterpret_cast<double*>(S.lost + 32);
+    S.pc = A.pcache ? reinterpret_cast<double*>(reinterpret_cast<char*>(S.lost) + kMiscBytes) : nullptr;
     S.pj = A.pcache ? reinterpret_cast<int*>(S.pc + 6 * (size_t)A.pcache) : nullptr;
     return S;
 }
@@ -855,6 +880,32 @@ __device__ __forceinline__ void pstore(const PState<ORD>& P, double* __restrict_
         for (int v = 0; v < 5; ++v) ps[(6 + (size_t)m * 5 + v) * npad + p] = P.h[m][v];
 }
 
+// history m pushes ago of thread tid's particle in the shared ring whose newest slot is hs
+template <int ORD>
+__device__ __forceinline__ double* hist_at(const Smem& S, int hs, int m) {
+    const int slot = hs - m < 0 ? hs - m + ORD : hs - m;
+    return S.hist + (size_t)slot * 5 * kThreads + threadIdx.x;
+}
+template <int ORD>
+__device__ __forceinline__ void hist_get(PState<ORD>& P, const Smem& S, int hs) {
+#pragma unroll
+    for (int m = 0; m < ORD; ++m) {
+        const double* h = hist_at<ORD>(S, hs, m);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) P.h[m][v] = h[v * kThreads];
+    }
+}
+template <int ORD>
+__device__ __forceinline__ void hist_put(const PState<ORD>& P, const Smem& S, int hs, bool all) {
+#pragma unroll
+    for (int m = 0; m < ORD; ++m) {
+        if (m > 0 && !all) break;
+        double* h = hist_at<ORD>(S, hs, m);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) h[v * kThreads] = P.h[m][v];
+    }
+}
+
 // x y px py Delta w of particle p: from the shared copy (A.pcache) or from the global state
 template <int ORD>
 __device__ __forceinline__ void pbase(PState<ORD>& P, const Smem& S, const SweepArgs& A, const double* __restrict__ ps,
@@ -1086,7 +1137,7 @@ __device__ __forceinline__ void depositS_finish(const Src& s, int i, const int* 
 }
 
 // src/PlasmaSpecies.cpp:561-668 with uniform steps (the classical AB coefficients); returns 1 when the
-// particle moved, 0 when it was removed beyond the wall, -1 when removed as trapped (Delta <= delta_min
+// particle moved (2 when the wall reflected it, its whole history with it), 0 when it was removed beyond the wall, -1 when removed as trapped (Delta <= delta_min
 // or gamma > max_qsa Delta: no longer quasi-static, src/PlasmaSpecies.cpp:636-650). kin: the particle's
 // kinematics before the push, on return those after it
 template <int ORD>
@@ -1137,7 +1188,9 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin
     }
     const double R = A.R;
     const double rn = sqrt(xn * xn + yn * yn);
+    int moved = 1;
     if (rn > R) {                    // specular reflection at the wall, incl. the history
+        moved = 2;
         const double nx = xn / rn, ny = yn / rn;
         const double rr = 2.0 * R - rn;
         if (rr < 0.0) { P.w = 0.0; return 0; }
@@ -1154,7 +1207,7 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin
         }
     }
     P.x = xn; P.y = yn; P.px = pxn; P.py = pyn; P.dl = dn;
-    return 1;
+    return moved;
 }
 
 // Adams-Bashforth coefficients for history points t[0..ord) (t[0] the newest push) and the step h: the
@@ -1220,55 +1273,69 @@ __device__ __forceinline__ BeamRow beam_row_at(const SweepArgs& A, const double*
     return r;
 }
 
-// right-hand side of system e (psi, E_z, B_z) at row i < N (src/Simulation.cpp:798-799, :517-527)
+// the two neighbours of row i in the 3-point stencils gm f[lo] + g0 f[i] + gp f[hi]: the one-sided wall stencil
+// takes row N - 2 in place of row N + 1; at the axis the stencil is zero (gm = g0 = gp = 0)
+__device__ __forceinline__ int row_lo(int i) { return max(i - 1, 0); }
+__device__ __forceinline__ int row_hi(int i, int N) { return i == N ? N - 2 : i + 1; }
+
+// right-hand side of system e (psi, E_z, B_z) at row i (src/Simulation.cpp:798-799, :517-527)
 __device__ __forceinline__ double rhs_l0(const Smem& S, const Src& s, int N, int e, int i) {
-    if (e == 0) return -1.0 * s.rhot[i];
-    if (e == 1) return -1.0 * s.drho[i];
-    const double t1 = grad_at(S, N, s.jpi1, i, true);
-    const double t2 = (i == 0 ? s.jpi1[1] : s.jpi1[i]) * S.ir[i];
-    return 1.0 * (-(t1 + t2));
+    if (e == 0) return -s.rhot[i];
+    if (e == 1) return -s.drho[i];
+    // the odd gradient (f_1 / r_1 on the axis) plus f / r (f_1 / r_1 on the axis)
+    const double* const f = s.jpi1;
+    const double o = f[max(i, 1)] * S.ir[i];
+    const double g = S.gm[i] * f[row_lo(i)] + S.g0[i] * f[i] + S.gp[i] * f[row_hi(i, N)];
+    return -((i == 0 ? o : g) + o);
 }
 
-// row i of (L1D - chi) (sys 0) or (L1F - chi) (sys 1) with its right-hand side; cm = c_{i-1}
-// (src/FieldSolver.cpp:172-191, src/Simulation.cpp:535-591)
+// row i of (L1D - chi) (sys 0) or (L1F - chi) (sys 1) with its right-hand side; cm = c_{i-1} (any value at row 0,
+// where a = 0); sv: S_i or S_r (src/FieldSolver.cpp:172-191, src/Simulation.cpp:535-591)
 __device__ __forceinline__ void row_b(const Smem& S, const Src& s, int N, double fc, int sys, int i, double sv,
                                       double& a, double& b, double& cm, double& d) {
-    a = S.l1a[i]; b = S.l1b[i]; cm = i > 0 ? S.l1c[i - 1] : 0.0;
-    d = 0.0;
+    a = S.l1a[i];
+    b = S.l1b[i];
+    cm = S.l1c[row_lo(i)];
+    const bool wall = i == N, in = i > 0 && (sys || !wall);      // in: not a Dirichlet row
+    const double chi = s.chi[i];
     if (sys == 0) {
-        if (i >= 1 && i < N) { b = b - s.chi[i]; d = 1.0 * (-sv); }
-    } else if (i >= 1) {
-        if (i == N) { a = S.lfa; b = S.lfb; }
-        b = b - s.chi[i];
-        d = 1.0 * (grad_at(S, N, s.jz, i, false) + sv);
-        if (i == N) d -= fc * s.jz[N];
+        d = -sv;
+    } else {
+        const double* const f = s.jz;
+        const double jn = f[i];
+        d = (S.gm[i] * f[row_lo(i)] + S.g0[i] * jn + S.gp[i] * f[row_hi(i, N)]) + sv;
+        if (wall) { a = S.lfa; b = S.lfb; d -= fc * jn; }
     }
+    b = in ? b - chi : b;
+    d = in ? d : 0.0;
 }
 
 // One L0 system by a group of kG2 warps (e: 0..2, the group's number), rows [row0, row0 + R) per thread. L0 is
 // D^-1 times a Laplacian: with w_i = V_i / 2 pi and g_i = r_mid,i / h_i its rows say that the flux g_i (x_{i+1} - x_i)
 // is the sum of w d up to node i. The Thomas pivots of that matrix are -g_i / w_i exactly, so the two
 // substitutions are plain sums: z_i = z_{i-1} + w_i d_i and x_i = x_{i+1} - z_i / g_i. rhs(i): d_i for i < N. On return
-// v holds x of the thread's rows, z0 the flux into them and xn the x just after them.
+// v holds x of the thread's rows, z0 the flux into them and xn the x just after them. vw and gw are 0 at row N.
 template <int kR, class Rhs>
 __device__ __forceinline__ void l0_group(double* tot, const double* vw, const double* gw, int N, int e, int wl, int R,
                                          int row0, Rhs rhs, double (&v)[kR], double& z0, double& xn) {
-    double sum = 0.0;
+    // rows past the thread's or the grid's end stand at row N, where w = 1 / g = 0: no branch, so that the loads
+    // of all rows are in flight together
+    double g[kR], sum = 0.0;
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
-        v[u] = 0.0;
-        if (u < R && i < N) v[u] = vw[i] * rhs(i);
-        sum += v[u];
+        const int i = u < R ? min(row0 + u, N) : N;
+        v[u] = vw[i] * rhs(i);
+        g[u] = gw[i];
     }
+#pragma unroll
+    for (int u = 0; u < kR; ++u) sum += v[u];
     double z = group_sum<true, kG2>(sum, wl, tot + 8 * e, 1 + e);
     z0 = z;
     sum = 0.0;
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
         z += v[u];
-        v[u] = (u < R && i < N) ? -(z * gw[i]) : 0.0;
+        v[u] = -(z * g[u]);
     }
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) sum += v[u];
@@ -1295,17 +1362,19 @@ __device__ __forceinline__ void l0_solve(const Smem& S, const Src& s, int M, int
         if (u < R && row0 + u < M) out[row0 + u] = v[u];
     if (e != 0) return;
     // W+ = -psi' on the thread's rows; psi just before them from the flux that enters them
-    double xm = (row0 >= 1 && row0 < M) ? v[0] - z0 * S.gw[row0 - 1] : 0.0;
+    const double xm = v[0] - z0 * S.gw[min(row_lo(row0), N)];
+    double w[kR];
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
-        if (u >= R || i >= M) break;
-        const double xc = v[u], xp = (u + 1 < kR && u + 1 < R) ? v[u + 1 < kR ? u + 1 : u] : xn;
-        if (i == 0) S.wr1[0] = -0.0;
-        else if (i < N) S.wr1[i] = -(S.gm[i] * xm + S.g0[i] * xc + S.gp[i] * xp);
-        if (i == N - 1) S.wr1[N] = -(S.g0[N] * xp + S.gm[N] * xc + S.gp[N] * xm);   // one-sided: psi_N, N-1, N-2
-        xm = xc;
+        const int i = u < R ? min(row0 + u, N) : N;
+        const double lo = u ? v[u - 1] : xm, hi = (u + 1 < kR && u + 1 < R) ? v[u + 1 < kR ? u + 1 : u] : xn;
+        w[u] = -(S.gm[i] * lo + S.g0[i] * v[u] + S.gp[i] * hi);          // (row 0: -0)
+        // the row before the wall also gives the wall's one-sided value from psi_N, psi_{N-1}, psi_{N-2}
+        if (u < R && row0 + u == N - 1) S.wr1[N] = -(S.g0[N] * hi + S.gm[N] * v[u] + S.gp[N] * lo);
     }
+#pragma unroll
+    for (int u = 0; u < kR; ++u)
+        if (u < R && row0 + u < N) S.wr1[row0 + u] = w[u];
 }
 
 // One chi-shifted system by a group of kG4 warps (sy: 0 or 1), rows [row0, row0 + R) per thread: 1/u_i = p_{i-1} /
@@ -1320,18 +1389,26 @@ __device__ __forceinline__ void shifted_group(double* tot, int M, int sy, int wl
     double* const tb = tot + 160 + 16 * sy;
     double ra[kR], rb[kR], rc[kR];
     double m[4] = {1.0, 0.0, 0.0, 1.0};
+    // rows past the thread's or the grid's end read row M - 1 and then become x = 0 rows (a = d = 0, b = 1), so that
+    // the loads of all rows are in flight together
+    double cc[kR];
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
-        ra[u] = 0.0; rb[u] = 1.0; rc[u] = 0.0; x[u] = 0.0;
-        if (u < R && i < M) {
-            row(i, ra[u], rb[u], rc[u], x[u]);
-            const double t01 = -ra[u] * rc[u];
-            const double n00 = rb[u] * m[0] + t01 * m[2], n01 = rb[u] * m[1] + t01 * m[3];
-            m[2] = m[0]; m[3] = m[1];
-            m[0] = n00; m[1] = n01;
-            if ((u & 3) == 3) renorm(m[0], m[1], m[2], m[3]);
-        }
+        const int i = u < R ? min(row0 + u, M - 1) : M - 1;
+        row(i, ra[u], rb[u], rc[u], x[u]);
+        cc[u] = c(i);
+    }
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const bool on = u < R && row0 + u < M;
+        ra[u] = on ? ra[u] : 0.0;
+        rb[u] = on ? rb[u] : 1.0;
+        x[u] = on ? x[u] : 0.0;
+        const double t01 = -ra[u] * rc[u];
+        const double n00 = rb[u] * m[0] + t01 * m[2], n01 = rb[u] * m[1] + t01 * m[3];
+        m[2] = on ? m[0] : m[2]; m[3] = on ? m[1] : m[3];
+        m[0] = on ? n00 : m[0]; m[1] = on ? n01 : m[1];
+        if ((u & 3) == 3) renorm(m[0], m[1], m[2], m[3]);
     }
     renorm(m[0], m[1], m[2], m[3]);
     double p, q;
@@ -1346,11 +1423,13 @@ __device__ __forceinline__ void shifted_group(double* tot, int M, int sy, int wl
         pivot_scale(p, q);
         rc[u] = pivot_quot(q, p);
     }
+    // (rows past the end carry y and x along: slope 1, nothing added)
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        if (u >= R || row0 + u >= M) { rc[u] = 0.0; continue; }
-        ra[u] = -rc[u] * ra[u];
+        const bool on = u < R && row0 + u < M;
+        ra[u] = on ? -rc[u] * ra[u] : 1.0;                   // forward: y_i = ra y_{i-1} + x
         x[u] = rc[u] * x[u];
+        rc[u] = on ? -(cc[u] * rc[u]) : 1.0;                 // backward: x_i = rc x_{i+1} + y_i
         fB = fma(ra[u], fB, x[u]);
         fA *= ra[u];
     }
@@ -1358,22 +1437,18 @@ __device__ __forceinline__ void shifted_group(double* tot, int M, int sy, int wl
     double bA = 1.0, bB = 0.0;
 #pragma unroll
     for (int u = 0; u < kR; ++u) {
-        const int i = row0 + u;
-        if (u >= R || i >= M) continue;
+        const bool on = u < R && row0 + u < M;
         y = fma(ra[u], y, x[u]);
-        x[u] = y;
-        rc[u] = -(c(i) * rc[u]);                              // x_i = -(c_i / u_i) x_{i+1} + y_i
+        x[u] = on ? y : 0.0;
     }
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) {
-        if (u >= R || row0 + u >= M) continue;
         bB = fma(rc[u], bB, x[u]);
         bA *= rc[u];
     }
     double xx = group_affine<false, kG4>(bA, bB, wl, tb, 4 + sy);
 #pragma unroll
     for (int u = kR - 1; u >= 0; --u) {
-        if (u >= R || row0 + u >= M) continue;
         xx = fma(rc[u], xx, x[u]);
         x[u] = xx;
     }
@@ -1395,7 +1470,7 @@ __device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, 
         [&](int i, double& a, double& b, double& cm, double& d) {
             row_b(S, s, N, fc, sy, i, kFinish ? fx_value(sa + i, es, qs) : sa[i], a, b, cm, d);
         },
-        [&](int i) { return sy && i == N ? 0.0 : S.l1c[i]; }, x);
+        [&](int i) { return S.l1c[i]; }, x);
     double* const out = sy ? S.bpi : S.bpr;
 #pragma unroll
     for (int u = 0; u < kR; ++u)
@@ -1409,25 +1484,35 @@ using namespace sweep_detail;
 // One sweep by the calling CTA (all kThreads threads). The gate G orders it against other CTAs when
 // several time steps run concurrently (NoGate: a stand-alone sweep). Returns false if a gate wait
 // gave up (the CTA then stops at the next slice boundary). EXT: the kernel also handles the smoothing
-// filter (A.filter) and static beam sources (A.bstat); without it both are ignored, and the kernel of
-// plain decks carries none of their code.
+// filter (A.filter), static beam sources (A.bstat) and adaptive sub-slicing (A.max_cells); without it they are
+// ignored, and the kernel of plain decks carries none of their code (sweep_ext).
 template <int ORD, bool REG, int kMaxR, class Gate, bool EXT = false>
 __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw, Gate& gate) {
     const int M = A.M, N = A.N, K = A.K, Rw = kMaxR == 1 ? 1 : A.rows_per_thread;   // rows per thread
     const int tid = threadIdx.x;
-    const Smem S = carve(smem_raw, A);
+    // with one row and one particle per thread (M <= kSweepThreads) the constants always fit shared memory
+    constexpr bool kCS = REG && kMaxR == 1;
+    // The particles' force history (5 ORD doubles each) is read and written once per slice, by the push: in
+    // registers it takes 30 of a thread's 128 (ORD 3) through all the solves and what they displace goes to local
+    // memory, of which 512 threads have more than the L1 left beside 150 KB of shared memory holds. So it lives in
+    // shared memory (a ring of ORD slots), with single-buffered sources to make room for it and for L1.
+    constexpr int kHist = hist_doubles(ORD, REG, kMaxR, EXT);
+    constexpr bool kHS = kHist > 0;
+    const bool dbuf = !kHS && A.dbuf;
+    const int ST = kHS ? kThreads : M;                          // distance between the shared arrays
+    int hs = 0;                                                 // slot of the newest force
+    const Smem S = carve<kCS, kHist>(smem_raw, A);
     const int np = A.np, npad = A.npad;
     const double R = A.R;
     const int row0 = tid * Rw;                                  // this thread's rows [row0, row0 + Rw)
     unsigned long long* tim = A.timing;
-    long long t_prev = 0, t_sub = 0;
-    if (tim && tid == 0) t_prev = clock64();
+    if (tim && tid == 0) S.tmark[0] = clock64();
 #define PHASE_MARK(ph)                                                        \
     do {                                                                      \
         if (tim && tid == 0) {                                                \
             const long long tn = clock64();                                   \
-            atomicAdd(tim + (ph), (unsigned long long)(tn - t_prev));         \
-            t_prev = tn;                                                      \
+            atomicAdd(tim + (ph), (unsigned long long)(tn - S.tmark[0]));     \
+            S.tmark[0] = tn;                                                  \
         }                                                                     \
     } while (0)
 // parts of the solve phase, by thread 0 (a warp of the psi system): [5] the solves, [6] the next slice's start values
@@ -1435,8 +1520,8 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     do {                                                                      \
         if (tim && tid == 0) {                                                \
             const long long tn = clock64();                                   \
-            atomicAdd(tim + (slot), (unsigned long long)(tn - t_sub));        \
-            t_sub = tn;                                                       \
+            atomicAdd(tim + (slot), (unsigned long long)(tn - S.tmark[1]));   \
+            S.tmark[1] = tn;                                                  \
         }                                                                     \
     } while (0)
 
@@ -1449,10 +1534,13 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         S.bgr[j] = 0.0;
         S.bpr[j] = 0.0;
         S.bpi[j] = 0.0;
-        src_of(S, M, 0).ne[j] = 0.0;
+        src_of(S, ST, 0).ne[j] = 0.0;
     }
-    if (A.const_smem)
-        for (int t = tid; t < kConsts0 * M; t += kThreads) const_cast<double*>(S.gm)[t] = A.consts0[t];
+    if (kCS || A.const_smem)
+        for (int t = tid; t < kConsts0 * M; t += kThreads) {
+            const int c = t / M;
+            const_cast<double*>(S.gm)[c * ST + t - c * M] = A.consts0[t];
+        }
     if (tid == 0) *S.lost = 0;
     if (tid < 14) S.fx[tid] = 0;
     const int bits_p = fx_bits(np), bits_bg = fx_bits(A.nbg);
@@ -1472,6 +1560,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                     for (int v = 0; v < 5; ++v) P.h[m][v] = 0.0;
             }
             species_params(A, tid, P.q, P.qm);
+            if (kHS) hist_put<ORD>(P, S, hs, true);
         } else {
             P.x = P.y = P.px = P.py = 0.0;
             P.dl = 1.0;
@@ -1502,7 +1591,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     // immobile species deposit into the background; mobile ones are subtracted (neutralisation,
     // src/Simulation.cpp:672-684); src[0].ne is the scratch of the mobile deposit. Both exact: a pass
     // for the exponent maxima, a barrier, a pass of quantised adds, a barrier, then the values.
-    double* const ne0 = src_of(S, M, 0).ne;
+    double* const ne0 = src_of(S, ST, 0).ne;
     for (int pass = 0; pass < 2; ++pass) {
         int ebg = 0, ene = 0;
         for (int p = tid; p < A.nbg; p += kThreads) {
@@ -1572,7 +1661,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     // slice 0's arrays accumulate its plasma deposit from zero; its start values (background + beam,
     // init_base) are added when the deposit is finished
     {
-        const Src s0 = src_of(S, M, 0);
+        const Src s0 = src_of(S, ST, 0);
         for (int j = tid; j < M; j += kThreads) {
 #pragma unroll
             for (int c = 0; c < 7; ++c) dep_arr(s0, c)[j] = 0.0;
@@ -1584,7 +1673,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     // deposit of slice 0
     const int lane = tid & 31;
     {
-        const Src s0 = src_of(S, M, 0);
+        const Src s0 = src_of(S, ST, 0);
         if (REG) {
             const bool act = tid < np && P.w != 0.0;
             double v[12];
@@ -1642,34 +1731,45 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     PHASE_MARK(0);
 
     const double fc = A.flux_coef;
-    // The xi positions of the last ORD pushes (tn[0] the newest; the same in every thread) give the
-    // Adams-Bashforth coefficients of the next push: the classical ones for uniform steps, the
-    // variable-step ones after adaptive sub-slicing (src/PlasmaSpecies.cpp:561-580). A slab whose plasma
-    // was pushed before continues uniform steps of dxi.
-    double xcur = 0.0, hlast = A.pin_pushed ? A.dxi : 0.0, tn[ORD], abc[5];
-#pragma unroll
-    for (int m = 0; m < ORD; ++m) tn[m] = -(m + 1) * A.dxi;
-    auto coeffs = [&](double h, bool first) {
-        if (first) {
-#pragma unroll
-            for (int m = 0; m < ORD; ++m) tn[m] = xcur - m * h;
-        } else {
-#pragma unroll
-            for (int m = ORD - 1; m > 0; --m) tn[m] = tn[m - 1];
-            tn[0] = xcur;
-        }
+    // Adaptive sub-slicing only: the xi positions of the last ORD pushes (tn[0] the newest) give the
+    // Adams-Bashforth coefficients of the next push: the classical ones for uniform steps, the variable-step ones
+    // after a change (src/PlasmaSpecies.cpp:561-580). A slab whose plasma was pushed before continues uniform steps
+    // of dxi. The state (tn, then the current xi and the last step) is in shared memory, so that plain sweeps hold no
+    // registers for it: every thread reads one copy, thread 0 writes the other (barriers lie between two pushes).
+    int abp = 0;
+    const bool vsteps = EXT && A.max_cells > 0.0;
+    if (vsteps && tid == 0) {
+        for (int m = 0; m < ORD; ++m) S.absl[m] = -(m + 1) * A.dxi;
+        S.absl[5] = 0.0;
+        S.absl[6] = A.pin_pushed ? A.dxi : 0.0;
+    }
+    auto coeffs = [&](double h, bool first, double (&abc)[5]) {
         bool uniform = true;
+        double tn[ORD];
+        if (vsteps) {
+            const double* const o = S.absl + 8 * abp;
+            const double xcur = o[5];
 #pragma unroll
-        for (int m = 1; m < ORD; ++m) uniform = uniform && fabs((tn[m - 1] - tn[m]) - h) <= 1e-9 * h;
+            for (int m = 0; m < ORD; ++m) tn[m] = first ? xcur - m * h : (m == 0 ? xcur : o[m > 0 ? m - 1 : 0]);
+#pragma unroll
+            for (int m = 1; m < ORD; ++m) uniform = uniform && fabs((tn[m - 1] - tn[m]) - h) <= 1e-9 * h;
+            abp ^= 1;
+            if (tid == 0) {
+                double* const w = S.absl + 8 * abp;
+#pragma unroll
+                for (int m = 0; m < ORD; ++m) w[m] = tn[m];
+                w[5] = xcur + h;
+                w[6] = h;
+            }
+        }
         if (uniform) {
 #pragma unroll
             for (int m = 0; m < 5; ++m) abc[m] = A.ab[m];
         } else {
             ab_variable<ORD>(tn, h, abc);
         }
-        xcur += h;
-        hlast = h;
     };
+    if (vsteps) __syncthreads();
     for (int k = 0; k < K; ++k) {
     // the passes of slice k: its own, then its sub-slices (adaptive sub-slicing, src/Simulation.cpp:755-781):
     // each pushes by dxi / nsub; a sub-slice re-deposits the plasma and re-solves the fields with the beam
@@ -1682,6 +1782,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             double* T = trj + (size_t)(k / tevery) * (6 + 5 * (size_t)ORD) * npad;
             if (REG) {
                 if (tid < np) {
+                    if (kHS) hist_get<ORD>(P, S, hs);
                     T[tid] = P.x; T[npad + tid] = P.y; T[2 * (size_t)npad + tid] = P.px;
                     T[3 * (size_t)npad + tid] = P.py; T[4 * (size_t)npad + tid] = P.dl;
                     T[5 * (size_t)npad + tid] = P.w;
@@ -1695,23 +1796,30 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                     for (int v = 0; v < 6 + 5 * ORD; ++v) T[(size_t)v * npad + p] = gate.ps(A)[(size_t)v * npad + p];
             }
         }
-        const Src s = src_of(S, M, A.dbuf ? (k & 1) : 0);
-        const Src sn = src_of(S, M, A.dbuf ? ((k + 1) & 1) : 0);
+        const Src s = src_of(S, ST, dbuf ? (k & 1) : 0);
+        const Src sn = src_of(S, ST, dbuf ? ((k + 1) & 1) : 0);
         if constexpr (EXT)
             if (A.filter) filter_sources<kMaxR>(s, S, A, Rw);
-        if (tim && tid == 0) t_sub = clock64();
+        if (tim && tid == 0) S.tmark[1] = clock64();
         // beam rows of slice k+1 for this thread's nodes: loaded here without a use, so that the latency
         // (L2 or DRAM) overlaps the solves
         BeamRaw pre[kMaxR];
-        if (A.dbuf && k + 1 < K && ss == 0)
+        if (dbuf && k + 1 < K && ss == 0)
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u)
                 raw_load<Gate::kActive>(A, gate.bsrc(A), k + 1, min(tid + u * kThreads, N), pre[u]);
 
+        // the warp without a system brings the beam row after next towards L2 (a stand-alone sweep streams them
+        // from DRAM; in a pipelined run they are not final yet, and in L2 anyway)
+        if (!Gate::kActive && tid >= 3 * kG2 * 32 && ss == 0 && k + 3 < K) {
+            const double* const nx = gate.bsrc(A) + (size_t)(k + 3) * M * A.bcs;
+            for (int o = lane * 16; o < M * A.bcs; o += 32 * 16)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + o));
+        }
         // ---------------- P2: psi, E_z, B_z with L0, W+
         l0_solve<kMaxR == 1 ? 5 : 11>(S, s, M, N);
         SUB_MARK(5);
-        if (A.dbuf && k + 1 < K && ss == 0)
+        if (dbuf && k + 1 < K && ss == 0)
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u) {
                 const int j = tid + u * kThreads;
@@ -1727,6 +1835,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         if (REG) {
             const bool act = tid < np && P.w != 0.0;
             double v[4];
+            if (act) species_params(A, tid, P.q, P.qm);      // (from the arguments: no register between the phases)
             if (act) depositS_values(P, keep_geo(S, kp, J), kp.k, S, N, v);
             const bool tail = depositS_runs<true>(act, J, v, S.fx + 7);
             __syncthreads();
@@ -1784,7 +1893,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         // adaptive sub-slicing, decided in the slice's own pass from the particles as they stand
         // (src/Simulation.cpp:837-847): nsub = ceil(max cells crossed / max_cells_per_step), at least
         // ceil(dxi / (2 h_last)) (the step at most doubles), at most substep_max
-        if (ss == 0 && A.max_cells > 0.0 && k + 1 < K) {
+        if (EXT && ss == 0 && A.max_cells > 0.0 && k + 1 < K) {
             double c = 0.0;
             if (REG) {
                 if (tid < np && P.w != 0.0) c = cells_crossed(S, N, R, P.x, P.y, P.px, P.py, P.dl, A.dxi);
@@ -1802,6 +1911,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             __syncthreads();
             const double cm = __longlong_as_double((long long)*S.cmax);
             int n = cm <= A.max_cells ? 1 : (int)ceil(cm / A.max_cells);
+            const double hlast = S.absl[8 * abp + 6];
             if (hlast > 0.0) n = max(n, (int)ceil(A.dxi / (2.0 * hlast) - 1e-9));
             nsub = min(n, A.substep_max > 0 ? A.substep_max : 64);
             if (tid == 0 && nsub > 1) S.fx[11] += nsub - 1;
@@ -1839,24 +1949,24 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             }
         }
         if (k + 1 < K) {
-            // the beam part the deposit's values start from, for this thread's rows: slice k+1's (one
-            // buffer), or slice k's extrapolated to the next sub-slice
-            BeamRow nxt[kMaxR];
-            if (!to_next || !A.dbuf)
+            // the beam part the deposit's values start from, for this thread's rows: slice k+1's (one buffer), loaded
+            // here without a use so that the push hides the latency, or slice k's extrapolated to the next sub-slice
+            BeamRaw raw[kMaxR];
+            if (to_next && !dbuf)
 #pragma unroll
-                for (int u = 0; u < kMaxR; ++u) {
-                    const int j = tid + u * kThreads;
-                    if (j < M)
-                        nxt[u] = to_next ? beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j)
-                                         : beam_row_at<Gate::kActive, EXT>(A, gate.bsrc(A), k, j, (ss + 1) * hstep);
-                }
+                for (int u = 0; u < kMaxR; ++u)
+                    raw_load<Gate::kActive>(A, gate.bsrc(A), k + 1, min(tid + u * kThreads, N), raw[u]);
             const bool first = (k == 0) && (ss == 0) && !A.pin_pushed;
-            coeffs(hstep, first);
+            double abc[5];
+            coeffs(hstep, first, abc);
             if (REG) {
                 bool act = tid < np && P.w != 0.0;
                 double v[12];
                 if (act) {
+                    species_params(A, tid, P.q, P.qm);
+                    if (kHS && !first) hist_get<ORD>(P, S, hs);
                     const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, hstep);
+                    if (kHS) hist_put<ORD>(P, S, hs + 1 == ORD ? 0 : hs + 1, first || pr == 2);
                     if (pr > 0) {
                         polar(P.x, P.y, kp.rp, kp.ir, kp.c, kp.s);
                         J = locate_from(S.r, N, R, kp.rp, J);
@@ -1867,6 +1977,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                         if (pr < 0) atomicAdd(S.fx + 12, 1);
                     }
                 }
+                if (kHS) hs = hs + 1 == ORD ? 0 : hs + 1;
                 const bool tail = deposit_runs<true>(act, J, P.q < 0.0, v, S.fx);
                 __syncthreads();
                 deposit_add(tail, J, P.q < 0.0, v, acc, S.fx, bits_p);
@@ -1930,11 +2041,14 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 const int i = tid + u * kThreads;
                 if (i >= M) continue;
                 double b0[7];
-                if (to_next && A.dbuf) {
+                if (to_next && dbuf) {
 #pragma unroll
                     for (int c = 0; c < 7; ++c) b0[c] = dep_arr(sn, c)[i];
                 } else {
-                    init_base<EXT>(S, i, nxt[u], M, b0);
+                    init_base<EXT>(S, i,
+                                   to_next ? raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, i, raw[u])
+                                           : beam_row_at<Gate::kActive, EXT>(A, gate.bsrc(A), k, i, (ss + 1) * hstep),
+                                   M, b0);
                 }
                 deposit_finish(dst, acc, i, b0, S.fx, bits_p);
             }
@@ -1959,11 +2073,18 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         // a slab that hands its plasma on: push the last slice too (src/Simulation.cpp:755, the push of the
         // last local slice produces the state entering the next slab), no deposit
         const bool first = (K == 1) && !A.pin_pushed;
-        coeffs(A.dxi, first);
+        double abc[5];
+        coeffs(A.dxi, first, abc);
         if (REG) {
             if (tid < np && P.w != 0.0) {
+                if (kHS && !first) hist_get<ORD>(P, S, hs);
                 const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, A.dxi);
+                if (kHS) hist_put<ORD>(P, S, hs + 1 == ORD ? 0 : hs + 1, first || pr == 2);
                 if (pr <= 0) { atomicAdd(S.lost, 1); if (pr < 0) atomicAdd(S.fx + 12, 1); }
+            }
+            if (kHS) {                                 // (a particle removed earlier keeps its history)
+                if (tid < np && P.w == 0.0) hist_get<ORD>(P, S, hs);
+                hs = hs + 1 == ORD ? 0 : hs + 1;
             }
             if (tid < np) pstore(P, A.pout, npad, tid);
         } else {
@@ -1982,7 +2103,10 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         }
         __syncthreads();
     }
-    if (REG && tid < np) pstore(P, gate.ps(A), npad, tid);
+    if (REG && tid < np) {
+        if (kHS && !A.pout) hist_get<ORD>(P, S, hs);
+        pstore(P, gate.ps(A), npad, tid);
+    }
     if (tid == 0 && A.counters) {
         atomicAdd(&A.counters[0], (unsigned long long)*S.lost);
         if (S.fx[13]) atomicAdd(&A.counters[1], (unsigned long long)S.fx[13]);
