@@ -56,7 +56,7 @@ struct qz_grid {
     std::vector<double> gm, g0, gp, ir;
     std::vector<double> consts;  // per-node constants of the sweep (13 x M)
     std::vector<double> consts1; // and of the modes = 1 sweep (9 x M)
-    std::vector<double> consts0; // the arrays the modes = 0 sweep reads (9 x M)
+    std::vector<double> consts0; // the arrays the modes = 0 sweep reads
     // device
     double *d_r = nullptr, *d_inv_h = nullptr, *d_inv_V = nullptr, *d_consts = nullptr, *d_consts1 = nullptr, *d_consts0 = nullptr;
     ~qz_grid() {
@@ -183,13 +183,19 @@ extern "C" qz_status qz_grid_create(const double* nodes, int M, qz_grid** out) {
         put(7, g->opa[1]); put(8, g->opb[1]); put(9, g->opc[1]);
         put(10, g->opa[2]); put(11, g->opb[2]); put(12, g->opc[2]);
         g->consts = cs;
-        std::vector<double> cz((size_t)qzb::kConsts0 * M, 0.0);
-        for (int k = 0; k < 4; ++k) std::copy(cs.begin() + (size_t)k * M, cs.begin() + (size_t)(k + 1) * M, cz.begin() + (size_t)k * M);
-        for (int i = 0; i < M; ++i) {
-            cz[(size_t)4 * M + i] = i < N ? g->V[i] / (2 * PI) : 0.0;        // (row N: Dirichlet)
-            cz[(size_t)5 * M + i] = i < N ? g->h[i] / g->rmid[i] : 0.0;
-        }
-        for (int k = 0; k < 3; ++k) std::copy(cs.begin() + (size_t)(7 + k) * M, cs.begin() + (size_t)(8 + k) * M, cz.begin() + (size_t)(6 + k) * M);
+        std::vector<double> cz((size_t)qzb::consts0_arrays(M) * M, 0.0);
+        auto from = [&](int src, int n, int dst) {
+            std::copy(cs.begin() + (size_t)src * M, cs.begin() + (size_t)(src + n) * M, cz.begin() + (size_t)dst * M);
+        };
+        from(0, 4, 0);
+        from(7, 3, 4);
+        if (M <= qzb::kSweepThreads)
+            for (int i = 0; i < N; ++i) {
+                cz[(size_t)7 * M + i] = g->V[i] / (2 * PI);
+                cz[(size_t)8 * M + i] = g->h[i] / g->rmid[i];
+            }
+        else
+            from(4, 3, 7);
         g->consts0 = cz;
         // modes = 1: Thomas factors of L1D (its Dirichlet rows 0 and N are rows b = 1), L0 and L2D rows
         std::vector<double> c1((size_t)9 * M, 0.0);
@@ -375,7 +381,7 @@ extern "C" qz_status qz_sweep_create(const qz_grid* g, const qz_sweep_params* p,
                               (size_t)optin))
         return fail(QZ_ERR_SIZE, "qz_sweep_create: the modes = 1 sweep holds one radial node per thread: M = " +
                                      std::to_string(M) + " > " + std::to_string(2 * qzb::kSweepThreads));
-    if (lay < 0 || rpt > 4)
+    if (lay < 0 || rpt > 3)
         return fail(QZ_ERR_SIZE, "qz_sweep_create: M = " + std::to_string(M) + " is too large for one CTA (" +
                                      std::to_string(qzb::sweep_m0_smem_bytes(M, false, false, filter)) + " B of shared memory, "
                                      "the device allows " + std::to_string(optin) + ")");

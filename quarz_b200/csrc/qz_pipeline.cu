@@ -174,7 +174,7 @@ int pipeline_max_grid(const PipeArgs& P, int* sms) {
 }
 
 cudaError_t launch_pipeline(const PipeArgs& P, int grid, cudaStream_t stream) {
-    if (P.sw.rows_per_thread < 1 || P.sw.rows_per_thread > 4) return cudaErrorInvalidValue;
+    if (P.sw.rows_per_thread < 1 || P.sw.rows_per_thread > 3) return cudaErrorInvalidValue;
     if (P.nsweep < 1 || grid <= P.nsweep || P.ring < 2 || P.nbeams > kMaxBeams) return cudaErrorInvalidValue;
     if (P.team < 1 || P.nsweep % P.team || grid % P.team || (P.team > 1 && P.modes != 1)) return cudaErrorInvalidValue;
     const size_t smem = pipeline_smem_bytes(P);

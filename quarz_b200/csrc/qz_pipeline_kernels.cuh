@@ -568,7 +568,7 @@ cudaError_t launch_e(const PipeArgs& P, int grid, size_t smem, cudaStream_t s) {
     const bool reg = P.sw.np <= kSweepThreads;
     if (P.sw.rows_per_thread == 1)
         return reg ? launch_t<0, ORD, true, 1, EXT>(P, grid, smem, s) : launch_t<0, ORD, false, 1, EXT>(P, grid, smem, s);
-    return reg ? launch_t<0, ORD, true, 4, EXT>(P, grid, smem, s) : launch_t<0, ORD, false, 4, EXT>(P, grid, smem, s);
+    return reg ? launch_t<0, ORD, true, 3, EXT>(P, grid, smem, s) : launch_t<0, ORD, false, 3, EXT>(P, grid, smem, s);
 }
 
 template <int ORD>
@@ -584,7 +584,7 @@ int occupancy_e(const PipeArgs& P, size_t smem, int nsm) {
     const bool reg = P.sw.np <= kSweepThreads;
     if (P.sw.rows_per_thread == 1)
         return reg ? occupancy_t<0, ORD, true, 1, EXT>(P, smem, nsm) : occupancy_t<0, ORD, false, 1, EXT>(P, smem, nsm);
-    return reg ? occupancy_t<0, ORD, true, 4, EXT>(P, smem, nsm) : occupancy_t<0, ORD, false, 4, EXT>(P, smem, nsm);
+    return reg ? occupancy_t<0, ORD, true, 3, EXT>(P, smem, nsm) : occupancy_t<0, ORD, false, 3, EXT>(P, smem, nsm);
 }
 
 template <int ORD>

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_m0_kernel(const SweepA
 
 size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter, int pcache) {
     size_t d = (size_t)(3 + 2 + 6 + (dbuf ? 18 : 9)) * M + sweep_detail::kTot;
-    if (const_smem) d += (size_t)kConsts0 * M;
+    if (const_smem) d += (size_t)consts0_arrays(M) * M;
     if (filter) d += 4 * (size_t)M + 2 * 14 * (kSweepThreads / 32);
     // + the words from Smem::lost on, and with the particle copy 6 doubles and a cell index per particle
     return sizeof(double) * d + sweep_detail::kMiscBytes + (pcache > 0 ? (size_t)pcache * (6 * sizeof(double) + sizeof(int)) : 0);
@@ -22,7 +22,7 @@ size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter, int p
 
 size_t sweep_m0_smem_bytes(const SweepArgs& A, bool ext) {
     const bool reg = A.np <= kSweepThreads;
-    const int hist = sweep_detail::hist_doubles(A.ord, reg, A.rows_per_thread == 1 ? 1 : 4, ext);
+    const int hist = sweep_detail::hist_doubles(A.ord, reg, A.rows_per_thread == 1 ? 1 : 3, ext);
     // (the variant with the history lays its arrays out kSweepThreads nodes apart: carve)
     return sweep_m0_smem_bytes(hist ? kSweepThreads : A.M, hist ? false : A.dbuf != 0, consts_in_smem(A), A.filter != 0, A.pcache) +
            sizeof(double) * hist * kSweepThreads;
@@ -43,7 +43,7 @@ cudaError_t launch_e(const SweepArgs& A, size_t smem, cudaStream_t stream) {
     const bool reg = A.np <= kSweepThreads;
     if (A.rows_per_thread == 1)
         return reg ? launch_t<ORD, true, 1, EXT>(A, smem, stream) : launch_t<ORD, false, 1, EXT>(A, smem, stream);
-    return reg ? launch_t<ORD, true, 4, EXT>(A, smem, stream) : launch_t<ORD, false, 4, EXT>(A, smem, stream);
+    return reg ? launch_t<ORD, true, 3, EXT>(A, smem, stream) : launch_t<ORD, false, 3, EXT>(A, smem, stream);
 }
 
 template <int ORD>
@@ -53,7 +53,7 @@ cudaError_t launch_o(const SweepArgs& A, size_t smem, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_sweep_m0(const SweepArgs& A, cudaStream_t stream) {
-    if (A.rows_per_thread < 1 || A.rows_per_thread > 4) return cudaErrorInvalidValue;
+    if (A.rows_per_thread < 1 || A.rows_per_thread > 3) return cudaErrorInvalidValue;
     const size_t smem = sweep_m0_smem_bytes(A, sweep_ext(A));
     switch (A.ord) {
         case 1: return launch_o<1>(A, smem, stream);

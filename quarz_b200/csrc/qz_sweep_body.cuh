@@ -258,6 +258,68 @@ __device__ __forceinline__ void scan_bwd_n(const double (&a)[NS], const double (
     }
 }
 
+// Exclusive scan of 2x2 matrix products (later rows on the left) for NS systems: on return
+// (p[s], q[s]) = first column of the product of all matrices before this thread's rows.
+template <int NS>
+__device__ __forceinline__ void scan_pivots(double (&m)[NS][4], double (&p)[NS], double (&q)[NS], double* tot) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The thread's matrices must come renormalised (largest entry in [1, 2)); a product of at most 32 such
+    // matrices stays below 2^63 and the products of the 16 renormalised warp totals below 2^31, so the
+    // scan renormalises once per lane after the warp stage instead of at every level. Renormalising
+    // scales by powers of two, which is exact, and the pivots use only ratios of p and q: the results
+    // are the same bits either way.
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double p00 = __shfl_up_sync(FULL, m[s][0], st), p01 = __shfl_up_sync(FULL, m[s][1], st);
+            const double p10 = __shfl_up_sync(FULL, m[s][2], st), p11 = __shfl_up_sync(FULL, m[s][3], st);
+            if (lane >= st) {
+                const double n00 = m[s][0] * p00 + m[s][1] * p10, n01 = m[s][0] * p01 + m[s][1] * p11;
+                const double n10 = m[s][2] * p00 + m[s][3] * p10, n11 = m[s][2] * p01 + m[s][3] * p11;
+                m[s][0] = n00; m[s][1] = n01; m[s][2] = n10; m[s][3] = n11;
+            }
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) renorm(m[s][0], m[s][1], m[s][2], m[s][3]);
+    if (lane == 31)
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tot[kW * (4 * s + e) + warp] = m[s][e];
+    double ex[NS][4];
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ex[s][e] = __shfl_up_sync(FULL, m[s][e], 1);
+    if (lane == 0)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) { ex[s][0] = 1.0; ex[s][1] = 0.0; ex[s][2] = 0.0; ex[s][3] = 1.0; }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        double t00 = lane < kW ? tot[kW * (4 * s) + lane] : 1.0, t01 = lane < kW ? tot[kW * (4 * s + 1) + lane] : 0.0;
+        double t10 = lane < kW ? tot[kW * (4 * s + 2) + lane] : 0.0, t11 = lane < kW ? tot[kW * (4 * s + 3) + lane] : 1.0;
+#pragma unroll
+        for (int st = 1; st < kW; st <<= 1) {
+            const double p00 = __shfl_up_sync(FULL, t00, st), p01 = __shfl_up_sync(FULL, t01, st);
+            const double p10 = __shfl_up_sync(FULL, t10, st), p11 = __shfl_up_sync(FULL, t11, st);
+            if (lane >= st) {
+                const double n00 = t00 * p00 + t01 * p10, n01 = t00 * p01 + t01 * p11;
+                const double n10 = t10 * p00 + t11 * p10, n11 = t10 * p01 + t11 * p11;
+                t00 = n00; t01 = n01; t10 = n10; t11 = n11;
+            }
+        }
+        const int src = (warp + 31) & 31;
+        double c00 = __shfl_sync(FULL, t00, src), c10 = __shfl_sync(FULL, t10, src);
+        if (warp == 0) { c00 = 1.0; c10 = 0.0; }
+        // column 0 of (within-warp exclusive product) x (carry of the earlier warps)
+        p[s] = ex[s][0] * c00 + ex[s][1] * c10;
+        q[s] = ex[s][2] * c00 + ex[s][3] * c10;
+    }
+}
+
 // ---------------------------------------------------------------- batched shared-memory adds
 // All NA updates of one thread are issued together (independent compare-and-swap rounds) instead
 // of one serialised atomic loop per address. Lock-free: every round at least one contender of
@@ -366,6 +428,18 @@ __device__ __forceinline__ void fx_max(const int (&e)[NC], int* E) {
     }
     if (lane < NC && mine) atomicMax(E + lane, (int)mine);
 }
+// Whether a deposit's maxima E differ from those the one before it had (Ep). With the plasma in global memory a deposit
+// adds in the quanta of Ep while it takes its own maxima, which saves a second pass over the particles (1000 cells:
+// S deposit 10,900 -> 8,300 cycles per slice, push and deposit 36,500 -> 27,700; with one particle per thread, whose
+// values are at hand after the barrier, it gains nothing). A maximum's exponent seldom changes from a slice to the next; when one does, the accumulators are
+// cleared and the adds repeated in the quanta of E, so that the quanta always are the slice's own.
+template <int NC>
+__device__ __forceinline__ bool fx_moved(const int* E, const int* Ep) {
+    int d = 0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) d |= E[c] ^ Ep[c];
+    return d != 0;
+}
 // headroom bits for n contributions per node: 2^bits > 2 n
 __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1); }
 
@@ -375,7 +449,7 @@ __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1)
 // all of them, and an SM executes one shuffle per cycle: the five scans took 1,800 to 3,600 cycles each. Here
 // every system has its own warps and a thread owns several of its rows: the recurrences run along
 // a thread's rows in registers (9 cycles per step), and the shuffles per system drop by the number of rows.
-// psi, E_z, B_z together went from 9,800 to 2,900 cycles per slice and B+ from 10,800 to 4,400 (512 nodes).
+// The psi / E_z / B_z phase went from 9,800 to 7,000 cycles per slice and B+ from 10,800 to 6,900 (512 nodes).
 // The row count is odd, so that the lanes' rows lie in different shared-memory banks.
 constexpr int kG2 = 5, kG4 = 8;                           // warps per system: 3 x 5 and 2 x 8
 constexpr int kMiscBytes = 256;                           // the words from Smem::lost on
@@ -510,6 +584,7 @@ struct Smem {
     double *r, *iv, *ih;                                  // grid
     const double *gm, *g0, *gp, *ir;                      // gradient stencils, 1/r
     const double *vw, *gw;                                // L0 in flux form: V / 2 pi, h / r_mid (l0_solve)
+    const double *l0r, *l0f, *l0b;                        // L0 Thomas: 1/u, -a/u, -c/u (l0_block)
     const double *l1a, *l1b, *l1c;                        // L1D rows; L1F's differ in row N only (lfa, lfb, c = 0)
     double lfa, lfb;
     double* src0;                                         // sources: 9 arrays, twice when A.dbuf
@@ -525,6 +600,7 @@ struct Smem {
     // n_e, n_i, J_theta), [7, 9) the S deposit, [9, 11) the background and neutralising deposits; then
     // counters: [11] extra sub-slices, [12] particles removed as trapped, [13] non-finite deposits
     int* fx;
+    int* fxp;                                             // the maxima [0, 9) of the deposits before these
     unsigned long long* cmax;                             // most cells crossed (sub-slicing), as double bits
     long long* tmark;                                     // clock marks of the phase counters: [0] phases, [1] parts
     double* absl;                                         // sub-slicing: xi of the last pushes, twice 8 (AbState)
@@ -545,15 +621,16 @@ __device__ __forceinline__ Smem carve(double* base, const SweepArgs& A) {
     Smem S;
     double* p = base;
     S.r = p; p += M; S.iv = p; p += M; S.ih = p; p += M;
-    // the 9 arrays the sweep reads, behind one another as in A.consts0
+    // the arrays the sweep reads, behind one another as in A.consts0
     const double* q = p;
     if constexpr (!kCS)
         if (!A.const_smem) q = A.consts0;
     S.gm = q; S.g0 = q + M; S.gp = q + 2 * M; S.ir = q + 3 * M;
-    S.vw = q + 4 * M; S.gw = q + 5 * M;
-    S.l1a = q + 6 * M; S.l1b = q + 7 * M; S.l1c = q + 8 * M;
+    S.l1a = q + 4 * M; S.l1b = q + 5 * M; S.l1c = q + 6 * M;
+    S.vw = q + 7 * M; S.gw = q + 8 * M;                   // up to kThreads nodes
+    S.l0r = q + 7 * M; S.l0f = q + 8 * M; S.l0b = q + 9 * M;   // more
     S.lfa = A.lfa_N; S.lfb = A.lfb_N;
-    if (kCS || A.const_smem) p += (size_t)kConsts0 * M;
+    if (kCS || A.const_smem) p += (size_t)consts0_arrays(A.M) * M;
     S.src0 = p;
     p += (!kHist && A.dbuf ? 18 : 9) * (size_t)M;
     S.bgt = p; p += M; S.bgr = p; p += M;
@@ -566,6 +643,7 @@ __device__ __forceinline__ Smem carve(double* base, const SweepArgs& A) {
     S.flag = S.lost + 1;
     S.fx = S.lost + 2;
     S.cmax = reinterpret_cast<unsigned long long*>(S.lost + 16);
+    S.fxp = S.lost + 18;
     S.tmark = reinterpret_cast<long long*>(S.lost + 28);
     S.absl = reinterpret_cast<double*>(S.lost + 32);
     S.pc = A.pcache ? reinterpret_cast<double*>(reinterpret_cast<char*>(S.lost) + kMiscBytes) : nullptr;
@@ -957,6 +1035,21 @@ __device__ __forceinline__ PKin kin_of(double px, double py, double d) {
     k.gam = 0.5 * q(1.0 + px * px + py * py + d * d);
     return k;
 }
+// the same from the particle's state, where nothing is kept from phase to phase (plasma in global memory; with plain
+// divisions: sharing reciprocals gained 2 % there, and the order of roundings is kept for the long chaotic sweeps)
+struct KinNone {};
+__device__ __forceinline__ void kin_get(const PKin& k, double, double, double, double& gam, double& invd) {
+    gam = k.gam;
+    invd = k.invd;
+}
+__device__ __forceinline__ void kin_get(KinNone, double px, double py, double d, double& gam, double& invd) {
+    gam = (1.0 + px * px + py * py + d * d) / (2.0 * d);
+    invd = 1.0 / d;
+}
+__device__ __forceinline__ double kin_next(PKin& k, double px, double py, double d) { return (k = kin_of(px, py, d)).gam; }
+__device__ __forceinline__ double kin_next(KinNone&, double px, double py, double d) {
+    return (1.0 + px * px + py * py + d * d) / (2.0 * d);
+}
 // What the phases of a slice need of a particle whose state is kept in registers, computed once per push: its
 // polar position and kinematics (a square root and two reciprocals)
 struct PKeep {
@@ -973,11 +1066,12 @@ __device__ __forceinline__ double w1_at(const Smem& S, int N, const PGeo& g) { r
 // src/PlasmaSpecies.cpp:409-478, m = 0 (plasma rho and J_r feed nothing on this path: not deposited).
 // Contributions of one particle to nodes j (v[0..5]) and j+1 (v[6..11]): rho - J_z, d/dxi, J_z, chi,
 // density, J_theta.
-template <int ORD>
-__device__ __forceinline__ void deposit_values(const PState<ORD>& P, const PGeo& g, const PKin& kin, const Smem& S,
+template <int ORD, class Kin>
+__device__ __forceinline__ void deposit_values(const PState<ORD>& P, const PGeo& g, const Kin& kin, const Smem& S,
                                                double (&v)[12]) {
     const double PX = P.px, PY = P.py, D = P.dl, w = P.w;
-    const double gam = kin.gam, invd = kin.invd;
+    double gam, invd;
+    kin_get(kin, PX, PY, D, gam, invd);
     const double pz = gam - D;
     const double ux = PX * invd, uy = PY * invd;
     const double ur = g.c * ux + g.s * uy, uth = g.c * uy - g.s * ux;
@@ -1002,9 +1096,9 @@ __device__ __forceinline__ void deposit_values(const PState<ORD>& P, const PGeo&
 }
 
 // The plasma deposit of a slice, exact (see fx_add): phase A sums each warp's runs of equal
-// (cell, species sign) and takes the block maxima of the run sums' exponents; after a barrier phase B
-// adds the quantised run sums into the accumulator arrays; after another barrier deposit_finish turns
-// the accumulators into values. The 7 arrays in this order: rho - J_z, d/dxi, J_z, chi, n_e, n_i,
+// (cell, species sign) and takes the block maxima of the run sums' exponents; phase B adds the quantised run sums
+// into the accumulator arrays (at once in the quanta of the deposit before, again after a barrier when the maxima
+// moved: fx_moved); after another barrier deposit_finish turns the accumulators into values. The 7 arrays in this order: rho - J_z, d/dxi, J_z, chi, n_e, n_i,
 // J_theta (n_e takes the negative species, n_i the positive ones).
 __device__ __forceinline__ double* dep_arr(const Src& s, int c) {
     switch (c) {
@@ -1059,6 +1153,12 @@ __device__ __forceinline__ void deposit_add(bool tail, int j, bool neg, const do
     fx_add<12>(adr, v, sc);
 }
 
+__device__ __forceinline__ void deposit_clear(const Src& acc, int M) {
+    for (int j = threadIdx.x; j < M; j += kThreads)
+#pragma unroll
+        for (int c = 0; c < 7; ++c) dep_arr(acc, c)[j] = 0.0;
+}
+
 // the values of node j: dst = base + accumulated deposit (acc and dst may be the same arrays)
 __device__ __forceinline__ void deposit_finish(const Src& dst, const Src& acc, int j, const double (&base)[7],
                                                const int* E, int bits) {
@@ -1068,15 +1168,16 @@ __device__ __forceinline__ void deposit_finish(const Src& dst, const Src& acc, i
 }
 
 // src/PlasmaSpecies.cpp:508-559, m = 0: S+ contributions to nodes j (v[0..1]) and j+1 (v[2..3])
-template <int ORD>
-__device__ __forceinline__ void depositS_values(const PState<ORD>& P, const PGeo& g, const PKin& kin, const Smem& S,
+template <int ORD, class Kin>
+__device__ __forceinline__ void depositS_values(const PState<ORD>& P, const PGeo& g, const Kin& kin, const Smem& S,
                                                 int N, double (&v)[4]) {
     const double qm = P.qm;
     const double PX = P.px, PY = P.py;
     const double r1 = w1_at(S, N, g);
     const double Wx = r1 * g.c - 0.0 * g.s, Wy = r1 * g.s + 0.0 * g.c;
     const double Ez = lin(S.ez, g), Bz = lin(S.bz, g);
-    const double gam = kin.gam, invd = kin.invd;
+    double gam, invd;
+    kin_get(kin, PX, PY, P.dl, gam, invd);
     const double ux = PX * invd, uy = PY * invd;
     const double ur = g.c * ux + g.s * uy, uth = g.c * uy - g.s * ux;
     const double dD = qm * ((PX * Wx + PY * Wy) * invd - Ez);
@@ -1139,9 +1240,9 @@ __device__ __forceinline__ void depositS_finish(const Src& s, int i, const int* 
 // src/PlasmaSpecies.cpp:561-668 with uniform steps (the classical AB coefficients); returns 1 when the
 // particle moved (2 when the wall reflected it, its whole history with it), 0 when it was removed beyond the wall, -1 when removed as trapped (Delta <= delta_min
 // or gamma > max_qsa Delta: no longer quasi-static, src/PlasmaSpecies.cpp:636-650). kin: the particle's
-// kinematics before the push, on return those after it
-template <int ORD>
-__device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin& kin, const Smem& S,
+// kinematics before the push, on return those after it (or KinNone)
+template <int ORD, class Kin>
+__device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, Kin& kin, const Smem& S,
                                              const SweepArgs& A, bool first, const double (&ab)[5], double h) {
     const double qm = P.qm;
     const double X = P.x, Y = P.y, PX = P.px, PY = P.py, D = P.dl;
@@ -1150,7 +1251,8 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin
     const double Ez = lin(S.ez, g), Bz = lin(S.bz, g);
     const double br = lin(S.bpr, g), bi = lin(S.bpi, g);
     const double Bx = br * g.c - bi * g.s, By = br * g.s + bi * g.c;
-    const double gam = kin.gam, invd = kin.invd;
+    double gam, invd;
+    kin_get(kin, PX, PY, D, gam, invd);
     double fv[5];
     fv[0] = PX * invd;
     fv[1] = PY * invd;
@@ -1181,8 +1283,8 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin
     double xn = X + dxi * sum[0], yn = Y + dxi * sum[1];
     double pxn = PX + dxi * sum[2], pyn = PY + dxi * sum[3];
     const double dn = D + dxi * sum[4];
-    kin = kin_of(pxn, pyn, dn);
-    if (!(dn > A.delta_min) || kin.gam > A.max_qsa * dn) {
+    const double gn = kin_next(kin, pxn, pyn, dn);
+    if (!(dn > A.delta_min) || gn > A.max_qsa * dn) {
         P.w = 0.0;
         return -1;
     }
@@ -1197,7 +1299,7 @@ __device__ __forceinline__ int push_particle(PState<ORD>& P, const PGeo& g, PKin
         xn = nx * rr; yn = ny * rr;
         const double pn = pxn * nx + pyn * ny;
         pxn -= 2.0 * pn * nx; pyn -= 2.0 * pn * ny;
-        kin = kin_of(pxn, pyn, dn);
+        (void)kin_next(kin, pxn, pyn, dn);
 #pragma unroll
         for (int m = 0; m < ORD; ++m) {
             const double a = P.h[m][0] * nx + P.h[m][1] * ny;
@@ -1284,9 +1386,9 @@ __device__ __forceinline__ double rhs_l0(const Smem& S, const Src& s, int N, int
     if (e == 1) return -s.drho[i];
     // the odd gradient (f_1 / r_1 on the axis) plus f / r (f_1 / r_1 on the axis)
     const double* const f = s.jpi1;
-    const double o = f[max(i, 1)] * S.ir[i];
     const double g = S.gm[i] * f[row_lo(i)] + S.g0[i] * f[i] + S.gp[i] * f[row_hi(i, N)];
-    return -((i == 0 ? o : g) + o);
+    const double f1 = f[max(i, 1)], ir = S.ir[i];
+    return -((i == 0 ? f1 * ir : g) + f1 * ir);
 }
 
 // row i of (L1D - chi) (sys 0) or (L1F - chi) (sys 1) with its right-hand side; cm = c_{i-1} (any value at row 0,
@@ -1477,6 +1579,218 @@ __device__ __forceinline__ void bplus_solve(const Smem& S, const Src& s, int M, 
         if (u < R && row0 + u < M) out[row0 + u] = x[u];
 }
 
+// The block-wide solves' own right-hand sides and rows (branches at the ends instead of clamped rows).
+// right-hand sides of the psi, E_z, B_z systems at row i (src/Simulation.cpp:798-799, :517-527)
+__device__ __forceinline__ void block_rhs(const Smem& S, const Src& s, int N, int i, double& d0, double& d1,
+                                       double& d2) {
+    d0 = d1 = d2 = 0.0;
+    if (i < N) {
+        d0 = -1.0 * s.rhot[i];
+        d1 = -1.0 * s.drho[i];
+        const double t1 = grad_at(S, N, s.jpi1, i, true);
+        const double t2 = (i == 0 ? s.jpi1[1] : s.jpi1[i]) * S.ir[i];
+        d2 = 1.0 * (-(t1 + t2));
+    }
+}
+
+// row i of (L1D - chi) (sys 0) and (L1F - chi) (sys 1) with its right-hand side
+// (src/FieldSolver.cpp:172-191, src/Simulation.cpp:535-591)
+__device__ __forceinline__ void block_row(const Smem& S, const Src& s, int N, double fc, int sys, int i, double& a,
+                                      double& b, double& cm, double& d) {
+    if (sys == 0) {
+        a = S.l1a[i]; b = S.l1b[i]; cm = i > 0 ? S.l1c[i - 1] : 0.0;
+        if (i >= 1 && i < N) { b = b - s.chi[i]; d = 1.0 * (-s.S1i[i]); } else { d = 0.0; }
+    } else {
+        a = i == N ? S.lfa : S.l1a[i]; b = i == N ? S.lfb : S.l1b[i]; cm = i > 0 ? S.l1c[i - 1] : 0.0;
+        if (i >= 1) {
+            b = b - s.chi[i];
+            d = 1.0 * (grad_at(S, N, s.jz, i, false) + s.S1r[i]);
+            if (i == N) d -= fc * s.jz[N];
+        } else {
+            d = 0.0;
+        }
+    }
+}
+
+// The solves of grids with more than kThreads nodes: block-wide scans, thread t with the rows [t Rw, t Rw + Rw).
+// (10,700 and 13,600 cycles per slice at 1001 nodes; groups of warps, with 7 rows per L0 thread and 5 per B+ thread
+// in registers, took 17,800 and 18,700.)
+template <int kMaxR>
+__device__ __forceinline__ void l0_block(const Smem& S, const Src& s, int M, int N, int Rw) {
+    const int row0 = threadIdx.x * Rw;
+    // forward: y_i = (-a_i/u_i) y_{i-1} + d_i/u_i
+    double cA = 1.0, cB[3] = {0.0, 0.0, 0.0};
+    double dv[kMaxR][3];
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+        dv[u][0] = dv[u][1] = dv[u][2] = 0.0;
+        if (u >= Rw || i >= M) continue;
+        block_rhs(S, s, N, i, dv[u][0], dv[u][1], dv[u][2]);
+        const double rr = S.l0r[i], af = S.l0f[i];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) cB[e] = fma(af, cB[e], rr * dv[u][e]);
+        cA *= af;
+    }
+                double yb[3];
+    scan_fwd<3>(cA, cB, yb, S.tot);
+                const double ypsi_prev = yb[0];                         // y of psi just before this thread's rows
+    double y[kMaxR][3];
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+        y[u][0] = y[u][1] = y[u][2] = 0.0;
+        if (u >= Rw || i >= M) continue;
+        const double rr = S.l0r[i], af = S.l0f[i];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) { yb[e] = fma(af, yb[e], rr * dv[u][e]); y[u][e] = yb[e]; }
+    }
+    // backward: x_i = (-c_i/u_i) x_{i+1} + y_i
+    double bA = 1.0, bB[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int u = kMaxR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= Rw || i >= M) continue;
+        const double ab = S.l0b[i];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) bB[e] = fma(ab, bB[e], y[u][e]);
+        bA *= ab;
+    }
+    double xa[3];
+    scan_bwd<3>(bA, bB, xa, S.tot + 8 * kW);
+                // psi on the window [row0 - 1, row0 + Rw]: the rows of this thread, x after them (the
+    // backward carry) and x before them, x_{row0-1} = y_{row0-1} - (c/u)_{row0-1} x_{row0}
+    // with y_{row0-1} the forward carry -- so W+ = -psi' needs no further exchange
+    double pw[kMaxR + 2];
+    pw[kMaxR + 1] = 0.0;
+    {
+        double xr = xa[0];
+#pragma unroll
+        for (int u = kMaxR; u >= 1; --u) pw[u] = 0.0;
+        const int last = (row0 + Rw <= M ? Rw : M - row0);
+        if (last >= 0) pw[last + 1 > kMaxR + 1 ? kMaxR + 1 : last + 1] = xr;
+    }
+#pragma unroll
+    for (int u = kMaxR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= Rw || i >= M) continue;
+        const double ab = S.l0b[i];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) xa[e] = fma(ab, xa[e], y[u][e]);
+        S.psi[i] = xa[0];
+        S.ez[i] = xa[1];
+        S.bz[i] = xa[2];
+        pw[u + 1] = xa[0];
+    }
+    pw[0] = (row0 >= 1 && row0 < M) ? fma(S.l0b[row0 - 1], pw[1], ypsi_prev) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+        if (u >= Rw || i >= M) continue;
+        if (i == 0) {
+            S.wr1[0] = -0.0;
+        } else if (i < N) {
+            S.wr1[i] = -(S.gm[i] * pw[u] + S.g0[i] * pw[u + 1] + S.gp[i] * pw[u + 2]);
+        }
+        if (i == N - 1) {                                  // the one-sided wall stencil needs psi_{N-2..N}
+            S.wr1[N] = -(S.g0[N] * pw[u + 2] + S.gm[N] * pw[u + 1] + S.gp[N] * pw[u]);
+        }
+    }
+}
+
+template <int kMaxR>
+__device__ __forceinline__ void bplus_block(const Smem& S, const Src& s, int M, int N, double fc, int Rw) {
+    const int row0 = threadIdx.x * Rw;
+    // pivots: product of T_i = [[b_i, -a_i c_{i-1}], [1, 0]] over the thread's rows
+    double m[2][4];
+#pragma unroll
+    for (int sy = 0; sy < 2; ++sy) { m[sy][0] = 1.0; m[sy][1] = 0.0; m[sy][2] = 0.0; m[sy][3] = 1.0; }
+    double ra[kMaxR][2], rb[kMaxR][2], rc[kMaxR][2], rd[kMaxR][2];
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+#pragma unroll
+        for (int sy = 0; sy < 2; ++sy) {
+            ra[u][sy] = 0.0; rb[u][sy] = 1.0; rc[u][sy] = 0.0; rd[u][sy] = 0.0;
+            if (u >= Rw || i >= M) continue;
+            block_row(S, s, N, fc, sy, i, ra[u][sy], rb[u][sy], rc[u][sy], rd[u][sy]);
+            const double t01 = -ra[u][sy] * rc[u][sy];
+            const double n00 = rb[u][sy] * m[sy][0] + t01 * m[sy][2];
+            const double n01 = rb[u][sy] * m[sy][1] + t01 * m[sy][3];
+            m[sy][2] = m[sy][0]; m[sy][3] = m[sy][1];
+            m[sy][0] = n00; m[sy][1] = n01;
+            renorm(m[sy][0], m[sy][1], m[sy][2], m[sy][3]);
+        }
+    }
+    double pp[2], qq[2];
+    scan_pivots<2>(m, pp, qq, S.tot);
+    // this thread's pivots (rc holds c_{i-1}; rinv = 1/u_i = p_{i-1}/p_i), forward composites
+    double rinv[kMaxR][2];
+    double fA[2] = {1.0, 1.0}, fB[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+#pragma unroll
+        for (int sy = 0; sy < 2; ++sy) {
+            rinv[u][sy] = 0.0;
+            if (u >= Rw || i >= M) continue;
+            const double pn = rb[u][sy] * pp[sy] - ra[u][sy] * rc[u][sy] * qq[sy];
+            qq[sy] = pp[sy];
+            pp[sy] = pn;
+            const double rr = qq[sy] / pp[sy];
+            const double sc = fabs(pp[sy]);
+            if (sc > 1e100 || sc < 1e-100) { pp[sy] /= sc; qq[sy] /= sc; }
+            rinv[u][sy] = rr;
+            const double af = -rr * ra[u][sy];
+            fB[sy] = fma(af, fB[sy], rr * rd[u][sy]);
+            fA[sy] *= af;
+        }
+    }
+    // forward substitution of both systems
+    double yy[2];
+    scan_fwd_n<2>(fA, fB, yy, S.tot + 8 * kW);
+    double y[kMaxR][2];
+#pragma unroll
+    for (int u = 0; u < kMaxR; ++u) {
+        const int i = row0 + u;
+#pragma unroll
+        for (int sy = 0; sy < 2; ++sy) {
+            y[u][sy] = 0.0;
+            if (u >= Rw || i >= M) continue;
+            yy[sy] = fma(-rinv[u][sy] * ra[u][sy], yy[sy], rinv[u][sy] * rd[u][sy]);
+            y[u][sy] = yy[sy];
+        }
+    }
+    // backward substitution: x_i = -(c_i / u_i) x_{i+1} + y_i
+    double bA[2] = {1.0, 1.0}, bB[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = kMaxR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= Rw || i >= M) continue;
+#pragma unroll
+        for (int sy = 0; sy < 2; ++sy) {
+            const double c = S.l1c[i];
+            const double ab = -(c * rinv[u][sy]);
+            bB[sy] = fma(ab, bB[sy], y[u][sy]);
+            bA[sy] *= ab;
+        }
+    }
+    double xx[2];
+    scan_bwd_n<2>(bA, bB, xx, S.tot);
+#pragma unroll
+    for (int u = kMaxR - 1; u >= 0; --u) {
+        const int i = row0 + u;
+        if (u >= Rw || i >= M) continue;
+#pragma unroll
+        for (int sy = 0; sy < 2; ++sy) {
+            const double c = S.l1c[i];
+            xx[sy] = fma(-(c * rinv[u][sy]), xx[sy], y[u][sy]);
+        }
+        S.bpr[i] = xx[0];
+        S.bpi[i] = xx[1];
+    }
+}
+
 }  // namespace sweep_detail
 
 using namespace sweep_detail;
@@ -1495,9 +1809,13 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     // The particles' force history (5 ORD doubles each) is read and written once per slice, by the push: in
     // registers it takes 30 of a thread's 128 (ORD 3) through all the solves and what they displace goes to local
     // memory, of which 512 threads have more than the L1 left beside 150 KB of shared memory holds. So it lives in
-    // shared memory (a ring of ORD slots), with single-buffered sources to make room for it and for L1.
+    // shared memory (a ring of ORD slots), with single-buffered sources to make room for it and for L1: 14.7 -> 12.5 us
+    // per slice at 257 nodes, 17.9 -> 14.9 at 512.
     constexpr int kHist = hist_doubles(ORD, REG, kMaxR, EXT);
     constexpr bool kHS = kHist > 0;
+    // beam rows loaded ahead of their use: one per thread (10 doubles; with more they would displace the rest, and the
+    // prefetched rows come from L2 at their use)
+    constexpr int kPre = 1;
     const bool dbuf = !kHS && A.dbuf;
     const int ST = kHS ? kThreads : M;                          // distance between the shared arrays
     int hs = 0;                                                 // slot of the newest force
@@ -1537,12 +1855,13 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         src_of(S, ST, 0).ne[j] = 0.0;
     }
     if (kCS || A.const_smem)
-        for (int t = tid; t < kConsts0 * M; t += kThreads) {
+        for (int t = tid; t < consts0_arrays(M) * M; t += kThreads) {
             const int c = t / M;
             const_cast<double*>(S.gm)[c * ST + t - c * M] = A.consts0[t];
         }
     if (tid == 0) *S.lost = 0;
     if (tid < 14) S.fx[tid] = 0;
+    if (tid < 9) S.fxp[tid] = 0;
     const int bits_p = fx_bits(np), bits_bg = fx_bits(A.nbg);
     PState<ORD> P;
     int J = 0;                                             // cell of the thread's particle
@@ -1705,7 +2024,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                                      : pgeo(S, A, N, R, p, Q.x, Q.y);
                             if (pass == 0 && A.pcache) S.pj[p] = g.j;
                             j = g.j;
-                            deposit_values(Q, g, kin_of(Q.px, Q.py, Q.dl), S, v);
+                            deposit_values(Q, g, KinNone{}, S, v);
                         }
                     }
                     const bool neg = act && Q.q < 0.0;
@@ -1803,10 +2122,10 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         if (tim && tid == 0) S.tmark[1] = clock64();
         // beam rows of slice k+1 for this thread's nodes: loaded here without a use, so that the latency
         // (L2 or DRAM) overlaps the solves
-        BeamRaw pre[kMaxR];
-        if (dbuf && k + 1 < K && ss == 0)
+        BeamRaw pre[kPre];
+        if (kPre == kMaxR && dbuf && k + 1 < K && ss == 0)
 #pragma unroll
-            for (int u = 0; u < kMaxR; ++u)
+            for (int u = 0; u < kPre; ++u)
                 raw_load<Gate::kActive>(A, gate.bsrc(A), k + 1, min(tid + u * kThreads, N), pre[u]);
 
         // the warp without a system brings the beam row after next towards L2 (a stand-alone sweep streams them
@@ -1817,20 +2136,27 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + o));
         }
         // ---------------- P2: psi, E_z, B_z with L0, W+
-        l0_solve<kMaxR == 1 ? 5 : 11>(S, s, M, N);
+        if constexpr (kMaxR == 1) l0_solve<5>(S, s, M, N);
+        else l0_block<kMaxR>(S, s, M, N, Rw);
         SUB_MARK(5);
         if (dbuf && k + 1 < K && ss == 0)
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u) {
                 const int j = tid + u * kThreads;
-                if (j < M) init_sources<EXT>(sn, S, j, raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j, pre[u]), M);
+                if (j >= M) continue;
+                init_sources<EXT>(sn, S, j,
+                                  kPre == kMaxR ? raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j, pre[u < kPre ? u : 0])
+                                                : beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, j), M);
             }
         SUB_MARK(6);
         __syncthreads();
         PHASE_MARK(1);
 
         // ---------------- P3: S+ (src/PlasmaSpecies.cpp:508-559), exact
-        if (tid < 7) S.fx[tid] = 0;           // the plasma deposit's maxima (read last before P2's barrier)
+        if (tid < 7) {                        // the plasma deposit's maxima (read last before P2's barrier)
+            S.fxp[tid] = S.fx[tid];
+            S.fx[tid] = 0;
+        }
         if (tid == 7) *S.cmax = 0ull;         // the cells-crossed maximum (read last at the last P5)
         if (REG) {
             const bool act = tid < np && P.w != 0.0;
@@ -1840,9 +2166,9 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             const bool tail = depositS_runs<true>(act, J, v, S.fx + 7);
             __syncthreads();
             depositS_add(tail, J, v, s, S.fx + 7, bits_p);
+            __syncthreads();
         } else {
             for (int pass = 0; pass < 2; ++pass) {
-                if (pass == 1) __syncthreads();
                 for (int base = tid - lane; base < np; base += kThreads) {
                     const int p = base + lane;
                     bool act = false;
@@ -1856,40 +2182,48 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                         if (act) {
                             const PGeo g = pgeo(S, A, N, R, p, Q.x, Q.y);
                             j = g.j;
-                            depositS_values(Q, g, kin_of(Q.px, Q.py, Q.dl), S, N, v);
+                            depositS_values(Q, g, KinNone{}, S, N, v);
                         }
                     }
-                    if (pass == 0) {
-                        depositS_runs<true>(act, j, v, S.fx + 7);
-                    } else {
-                        const bool tail = depositS_runs<false>(act, j, v, S.fx + 7);
-                        depositS_add(tail, j, v, s, S.fx + 7, bits_p);
-                    }
+                    const bool tail = pass == 0 ? depositS_runs<true>(act, j, v, S.fx + 7)
+                                                : depositS_runs<false>(act, j, v, S.fx + 7);
+                    depositS_add(tail, j, v, s, pass == 0 ? S.fxp + 7 : S.fx + 7, bits_p);
                 }
+                __syncthreads();
+                if (pass == 1 || !fx_moved<2>(S.fx + 7, S.fxp + 7)) break;
+                for (int j = tid; j < M; j += kThreads) s.S1r[j] = s.S1i[j] = 0.0;
+                __syncthreads();
             }
         }
-        __syncthreads();
         PHASE_MARK(2);
         if (tid == 0) S.fx[13] += (S.fx[7] == 2047) + (S.fx[8] == 2047);
 
         // ---------------- P4: B+
-        if (EXT && A.filter) {              // S+ smoothed with F1 (src/Simulation.cpp:810-812)
+        if (kMaxR > 1 || (EXT && A.filter)) {
 #pragma unroll
             for (int u = 0; u < kMaxR; ++u)
                 if (u < Rw && row0 + u < M) depositS_finish(s, row0 + u, S.fx + 7, bits_p);
-            FilterSet<2> fsS;
-            fsS.f[0] = s.S1r; fsS.f[1] = s.S1i; fsS.op[0] = fsS.op[1] = 1;
-            filter_rows<2, kMaxR>(fsS, A.fconsts, M, Rw, S.ftot);
-            __syncthreads();
-            bplus_solve<kMaxR == 1 ? 3 : 7, false>(S, s, M, N, fc, bits_p);
+            if (EXT && A.filter) {          // S+ smoothed with F1 (src/Simulation.cpp:810-812): a thread's own rows
+                FilterSet<2> fsS;
+                fsS.f[0] = s.S1r; fsS.f[1] = s.S1i; fsS.op[0] = fsS.op[1] = 1;
+                filter_rows<2, kMaxR>(fsS, A.fconsts, M, Rw, S.ftot);
+                if (kMaxR == 1) __syncthreads();
+            }
+        }
+        if constexpr (kMaxR == 1) {
+            if (EXT && A.filter) bplus_solve<3, false>(S, s, M, N, fc, bits_p);
+            else bplus_solve<3, true>(S, s, M, N, fc, bits_p);
         } else {
-            bplus_solve<kMaxR == 1 ? 3 : 7, true>(S, s, M, N, fc, bits_p);
+            bplus_block<kMaxR>(S, s, M, N, fc, Rw);
         }
         __syncthreads();
         PHASE_MARK(3);
 
         // ---------------- P5: store slice k; push k -> k+1 (or to the next sub-slice) and deposit
-        if (tid >= 7 && tid < 9) S.fx[tid] = 0;   // the S deposit's maxima (read last before P4's barrier)
+        if (tid >= 7 && tid < 9) {                // the S deposit's maxima (read last before P4's barrier)
+            S.fxp[tid] = S.fx[tid];
+            S.fx[tid] = 0;
+        }
         // adaptive sub-slicing, decided in the slice's own pass from the particles as they stand
         // (src/Simulation.cpp:837-847): nsub = ceil(max cells crossed / max_cells_per_step), at least
         // ceil(dxi / (2 h_last)) (the step at most doubles), at most substep_max
@@ -1951,10 +2285,10 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
         if (k + 1 < K) {
             // the beam part the deposit's values start from, for this thread's rows: slice k+1's (one buffer), loaded
             // here without a use so that the push hides the latency, or slice k's extrapolated to the next sub-slice
-            BeamRaw raw[kMaxR];
-            if (to_next && !dbuf)
+            BeamRaw raw[kPre];
+            if (kPre == kMaxR && to_next && !dbuf)
 #pragma unroll
-                for (int u = 0; u < kMaxR; ++u)
+                for (int u = 0; u < kPre; ++u)
                     raw_load<Gate::kActive>(A, gate.bsrc(A), k + 1, min(tid + u * kThreads, N), raw[u]);
             const bool first = (k == 0) && (ss == 0) && !A.pin_pushed;
             double abc[5];
@@ -1979,13 +2313,14 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 }
                 if (kHS) hs = hs + 1 == ORD ? 0 : hs + 1;
                 const bool tail = deposit_runs<true>(act, J, P.q < 0.0, v, S.fx);
-                __syncthreads();
+                __syncthreads();                  // (the maxima, and the accumulators cleared after the store above)
                 deposit_add(tail, J, P.q < 0.0, v, acc, S.fx, bits_p);
+                __syncthreads();
             } else {
-                // pass 0 pushes and takes the exponent maxima; pass 1 recomputes the deposit values of
-                // the pushed particles and adds them
+                // pass 0 pushes, takes the exponent maxima and adds in the quanta of the last deposit; pass 1, when
+                // the maxima moved, recomputes the deposit values of the pushed particles and adds them again
+                __syncthreads();                  // the accumulators have been cleared, after the store above
                 for (int pass = 0; pass < 2; ++pass) {
-                    if (pass == 1) __syncthreads();
                     for (int base = tid - lane; base < np; base += kThreads) {
                         const int p = base + lane;
                         bool act = false;
@@ -1999,15 +2334,19 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                 if (pass == 0) {
                                     phist(Q, gate.ps(A), npad, p);
                                     const PGeo g = pgeo(S, A, N, R, p, Q.x, Q.y);
-                                    PKin kin = kin_of(Q.px, Q.py, Q.dl);
+                                    KinNone kin;
                                     const int pr = push_particle(Q, g, kin, S, A, first, abc, hstep);
                                     if (pr > 0) {
-                                        // the new cell by a short walk from the old one
-                                        PKeep q;
-                                        polar(Q.x, Q.y, q.rp, q.ir, q.c, q.s);
-                                        j = locate_from(S.r, N, R, q.rp, g.j);
-                                        if (A.pcache) S.pj[p] = j;
-                                        deposit_values(Q, keep_geo(S, q, j), kin, S, v);
+                                        PGeo g2;
+                                        if (A.pcache) {        // the new cell by a short walk from the old one
+                                            const int jn = locate_from(S.r, N, R, sqrt(Q.x * Q.x + Q.y * Q.y), g.j);
+                                            g2 = geometry_in(S.r, S.ih, Q.x, Q.y, jn);
+                                            S.pj[p] = jn;
+                                        } else {
+                                            g2 = geometry(S.r, S.ih, N, R, Q.x, Q.y);
+                                        }
+                                        j = g2.j;
+                                        deposit_values(Q, g2, kin, S, v);
                                         act = true;
                                     } else {
                                         atomicAdd(S.lost, 1);
@@ -2018,22 +2357,22 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                                 } else {
                                     const PGeo g2 = pgeo(S, A, N, R, p, Q.x, Q.y);
                                     j = g2.j;
-                                    deposit_values(Q, g2, kin_of(Q.px, Q.py, Q.dl), S, v);
+                                    deposit_values(Q, g2, KinNone{}, S, v);
                                     act = true;
                                 }
                             }
                         }
                         const bool neg = act && Q.q < 0.0;
-                        if (pass == 0) {
-                            deposit_runs<true>(act, j, neg, v, S.fx);
-                        } else {
-                            const bool tail = deposit_runs<false>(act, j, neg, v, S.fx);
-                            deposit_add(tail, j, neg, v, acc, S.fx, bits_p);
-                        }
+                        const bool tail = pass == 0 ? deposit_runs<true>(act, j, neg, v, S.fx)
+                                                    : deposit_runs<false>(act, j, neg, v, S.fx);
+                        deposit_add(tail, j, neg, v, acc, pass == 0 ? S.fxp : S.fx, bits_p);
                     }
+                    __syncthreads();
+                    if (pass == 1 || !fx_moved<7>(S.fx, S.fxp)) break;
+                    deposit_clear(acc, M);
+                    __syncthreads();
                 }
             }
-            __syncthreads();
             if (tid == 0)
                 for (int c = 0; c < 7; ++c) S.fx[13] += S.fx[c] == 2047;
 #pragma unroll
@@ -2046,7 +2385,9 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                     for (int c = 0; c < 7; ++c) b0[c] = dep_arr(sn, c)[i];
                 } else {
                     init_base<EXT>(S, i,
-                                   to_next ? raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, i, raw[u])
+                                   to_next ? (kPre == kMaxR ? raw_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, i,
+                                                                                          raw[u < kPre ? u : 0])
+                                                            : beam_row<Gate::kActive, EXT>(A, gate.bsrc(A), k + 1, i))
                                            : beam_row_at<Gate::kActive, EXT>(A, gate.bsrc(A), k, i, (ss + 1) * hstep),
                                    M, b0);
                 }
@@ -2093,7 +2434,7 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                 pload(Q, gate.ps(A), npad, p);
                 species_params(A, p, Q.q, Q.qm);
                 if (Q.w != 0.0) {
-                    PKin kin = kin_of(Q.px, Q.py, Q.dl);
+                    KinNone kin;
                     const int pr = push_particle(Q, geometry(S.r, S.ih, N, R, Q.x, Q.y), kin, S, A, first, abc, A.dxi);
                     if (pr <= 0) { atomicAdd(S.lost, 1); if (pr < 0) atomicAdd(S.fx + 12, 1); }
                 }

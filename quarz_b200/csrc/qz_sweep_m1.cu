@@ -23,7 +23,8 @@ cudaError_t launch_e(const SweepArgs& A, size_t smem, cudaStream_t stream) {
                                          (int)smem);
     if (e != cudaSuccess) return e;
     // the particles of a slice over a cluster of up to 8 CTAs (the smoothing filter works in place on the shared
-    // sources: one CTA); 8 is the largest portable size, and each CTA has at least a particle per thread then
+    // sources: one CTA); 8 is the largest portable size, and each CTA has at least a particle per thread then. 4,088
+    // particles per slice: S deposit 42,700 -> 9,900 cycles, push and deposit 155,000 -> 27,900
     int team = 1;
     if (!A.filter)
         while (team < 8 && A.np > team * kSweepThreads) team *= 2;

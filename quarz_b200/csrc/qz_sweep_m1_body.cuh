@@ -290,7 +290,7 @@ __device__ __forceinline__ void scan_bwd_g(const double (&a)[NA], const double (
 // A thread owns up to 5 rows (M <= 5 x 32 x kG holds for every M the CTA takes); the right-hand sides are read
 // from, and the solutions written to, the same shared arrays, each thread its own rows. With one row per thread
 // and block-wide scans, P2 took 25,100 and P4 89,600 cycles per slice of the hosing grid (shuffles: one per cycle
-// and SM), now 6,800 and 24,000.
+// and SM), now 11,800 and 44,600.
 constexpr int kG = kW / 4;                             // warps per group
 constexpr int kR1 = 5;                                 // most rows per thread
 constexpr int kTotG = 16 * kG;                         // doubles of one half of the groups' scan scratch
@@ -391,19 +391,23 @@ __device__ __forceinline__ void group_thomas(double (&v)[kR1][NB], const double 
 // NB systems of an operator with the host's Thomas factors 1/u, -a/u, -c/u (th, 3 x M), in place
 template <int NB>
 __device__ __forceinline__ void solve_fixed(double* const (&f)[NB], const double* th, int M, int R, int row0, int wl,
-                                            double* t0, double* t1, int id) {
+                                            double* s0, double* s1, int id) {
     double v[kR1][NB], ri[kR1], fa[kR1], ba[kR1];
 #pragma unroll
     for (int u = 0; u < kR1; ++u) {
-        const int i = row0 + u;
-        const bool on = u < R && i < M;
-        ri[u] = on ? ldc(th + i) : 0.0;
-        fa[u] = on ? ldc(th + M + i) : 1.0;
-        ba[u] = on ? ldc(th + 2 * (size_t)M + i) : 1.0;
+        const int i = min(row0 + u, M - 1);
+        const bool on = u < R && row0 + u < M;
+        const double t0 = ldc(th + i), t1 = ldc(th + M + i), t2 = ldc(th + 2 * (size_t)M + i);
+        ri[u] = on ? t0 : 0.0;
+        fa[u] = on ? t1 : 1.0;
+        ba[u] = on ? t2 : 1.0;
 #pragma unroll
-        for (int n = 0; n < NB; ++n) v[u][n] = on ? f[n][i] : 0.0;
+        for (int n = 0; n < NB; ++n) {
+            const double d = f[n][i];
+            v[u][n] = on ? d : 0.0;
+        }
     }
-    group_thomas<NB>(v, ri, fa, ba, wl, t0, t1, id);
+    group_thomas<NB>(v, ri, fa, ba, wl, s0, s1, id);
 #pragma unroll
     for (int u = 0; u < kR1; ++u)
         if (u < R && row0 + u < M)
@@ -431,21 +435,28 @@ __device__ __forceinline__ void factor_op(const Consts1& C, const double* chi0, 
     const double *pa, *pb, *pc;
     op_rows(C, sy, pa, pb, pc);
     double m[4] = {1.0, 0.0, 0.0, 1.0};
+    // rows past the thread's or the grid's end read row N and become x = 0 rows (a = 0, b = 1): no branch, so that the
+    // loads of all rows (chi_0 comes from L2) are in flight together
+    double chi[kR1];
+#pragma unroll
+    for (int u = 0; u < kR1; ++u) {
+        const int i = u < R ? min(row0 + u, N) : N;
+        F.fa[u] = ldc(pa + i);                                  // fa: a_i, ba: c_{i-1} for now
+        F.b[u] = ldc(pb + i);
+        F.ba[u] = ldc(pc + max(i - 1, 0));                      // (a_0 = 0)
+        chi[u] = lg(chi0 + i);
+    }
 #pragma unroll
     for (int u = 0; u < kR1; ++u) {
         const int i = row0 + u;
-        F.b[u] = 1.0; F.fa[u] = 0.0; F.ba[u] = 0.0;            // fa: a_i, ba: c_{i-1} for now
-        if (u < R && i < M) {
-            F.fa[u] = ldc(pa + i);
-            F.b[u] = ldc(pb + i);
-            F.ba[u] = i > 0 ? ldc(pc + i - 1) : 0.0;
-            if (!op_dirichlet(sy, i, N)) F.b[u] = F.b[u] - lg(chi0 + i);
-            const double t01 = -F.fa[u] * F.ba[u];
-            const double n00 = F.b[u] * m[0] + t01 * m[2], n01 = F.b[u] * m[1] + t01 * m[3];
-            m[2] = m[0]; m[3] = m[1];
-            m[0] = n00; m[1] = n01;
-            if (u == 2) renorm(m[0], m[1], m[2], m[3]);
-        }
+        const bool on = u < R && i < M;
+        F.b[u] = on ? (op_dirichlet(sy, i, N) ? F.b[u] : F.b[u] - chi[u]) : 1.0;
+        F.fa[u] = on ? F.fa[u] : 0.0;
+        const double t01 = -F.fa[u] * F.ba[u];
+        const double n00 = F.b[u] * m[0] + t01 * m[2], n01 = F.b[u] * m[1] + t01 * m[3];
+        m[2] = on ? m[0] : m[2]; m[3] = on ? m[1] : m[3];
+        m[0] = on ? n00 : m[0]; m[1] = on ? n01 : m[1];
+        if (u == 2) renorm(m[0], m[1], m[2], m[3]);
     }
     renorm(m[0], m[1], m[2], m[3]);
     double p, q;
@@ -460,13 +471,11 @@ __device__ __forceinline__ void factor_op(const Consts1& C, const double* chi0, 
     }
 #pragma unroll
     for (int u = 0; u < kR1; ++u) {
-        const int i = row0 + u;
-        if (u < R && i < M) {
-            F.fa[u] = -F.ri[u] * F.fa[u];
-            F.ba[u] = -(ldc(pc + i) * F.ri[u]);
-        } else {
-            F.ri[u] = 0.0; F.fa[u] = 1.0; F.ba[u] = 1.0;
-        }
+        const bool on = u < R && row0 + u < M;
+        const double c = ldc(pc + min(row0 + u, N));
+        F.fa[u] = on ? -F.ri[u] * F.fa[u] : 1.0;
+        F.ba[u] = on ? -(c * F.ri[u]) : 1.0;
+        F.ri[u] = on ? F.ri[u] : 0.0;
     }
 }
 
@@ -495,13 +504,14 @@ __device__ __forceinline__ void solve_shifted(double* const (&f)[NB], const Cons
     op_rows(C, sy, pa, pb, pc);
 #pragma unroll
     for (int u = 0; u < kR1; ++u) {
-        const int i = row0 + u;
-        const bool on = u < R && i < M;
-        const double a = on ? ldc(pa + i) : 0.0, c = on ? ldc(pc + i) : 0.0;
+        const int i = min(row0 + u, N);
+        const bool on = u < R && row0 + u < M;
+        const double a = ldc(pa + i), c = ldc(pc + i);          // (a_0 = c_N = 0)
 #pragma unroll
         for (int n = 0; n < NB; ++n) {
-            const double xm = on && i > 0 ? f[n][i - 1] : 0.0, xp = on && i < N ? f[n][i + 1] : 0.0;
-            d[u][n] = on ? d[u][n] - (a * xm + F.b[u] * f[n][i] + c * xp) : 0.0;
+            const double xm = f[n][max(i - 1, 0)], xp = f[n][min(i + 1, N)];
+            const double r = d[u][n] - (a * xm + F.b[u] * f[n][i] + c * xp);
+            d[u][n] = on ? r : 0.0;
         }
     }
     group_thomas<NB>(d, F.ri, F.fa, F.ba, wl, tot, tot + kTotG, id);
@@ -934,7 +944,7 @@ __device__ __forceinline__ void deposit_all1(const SweepArgs& A, const Smem1& S,
             pload(Q, gate.ps(A), npad, p);
             species_params(A, p, Q.q, Q.qm);
             if (Q.w != 0.0) {
-                const PGeo g = geometry(S.r, S.ih, N, A.R, Q.x, Q.y);
+                const PGeo g = geometry_r(S.r, S.ih, N, A.R, Q.x, Q.y);
                 j = g.j;
                 neg = Q.q < 0.0;
                 d = dep1_basics(Q, g, S);
@@ -1006,7 +1016,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
     for (int p = first_p; p < A.nbg; p += step_p) {
         const double x = A.bg_p[p], y = A.bg_p[A.nbg + p], wq = A.bg_p[2 * A.nbg + p];
         if (wq == 0.0) continue;
-        const PGeo g = geometry(S.r, S.ih, N, R, x, y);
+        const PGeo g = geometry_r(S.r, S.ih, N, R, x, y);
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
             const int jj = g.j + cc;
@@ -1023,7 +1033,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             if (w == 0.0) continue;
             double q, qm;
             species_params(A, p, q, qm);
-            const PGeo g = geometry(S.r, S.ih, N, R, A.p_init[p], A.p_init[npad + p]);
+            const PGeo g = geometry_r(S.r, S.ih, N, R, A.p_init[p], A.p_init[npad + p]);
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 const int jj = g.j + cc;
@@ -1151,7 +1161,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                 pload(Q, gate.ps(A), npad, p);
                 species_params(A, p, Q.q, Q.qm);
                 if (Q.w != 0.0) {
-                    const PGeo g = geometry(S.r, S.ih, N, R, Q.x, Q.y);
+                    const PGeo g = geometry_r(S.r, S.ih, N, R, Q.x, Q.y);
                     j = g.j;
                     depositS1_values(Q, g, S, v);
                     act = true;
@@ -1276,10 +1286,10 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
                     pload(Q, gate.ps(A), npad, p);
                     species_params(A, p, Q.q, Q.qm);
                     if (Q.w != 0.0) {
-                        const PGeo g = geometry(S.r, S.ih, N, R, Q.x, Q.y);
+                        const PGeo g = geometry_r(S.r, S.ih, N, R, Q.x, Q.y);
                         const PF1 F = gather1(S, g, true);
                         if (push1(Q, F, A, first)) {
-                            const PGeo g2 = geometry(S.r, S.ih, N, R, Q.x, Q.y);
+                            const PGeo g2 = geometry_r(S.r, S.ih, N, R, Q.x, Q.y);
                             j = g2.j;
                             neg = Q.q < 0.0;
                             d = dep1_basics(Q, g2, S);
