@@ -1,0 +1,134 @@
+"""Sizes where the kernels' splits have their edges, against the CPU oracle on the same inputs:
+
+- the solves by groups of warps (m = 0 up to 512 nodes: 3 x 5 and 2 x 8 warps; m = 1: 4 groups): node counts around
+  whole numbers of rows per thread, and the block-wide solves of more than 512 nodes;
+- every Adams-Bashforth order (the history is kept in shared memory up to order 3);
+- the m = 1 sweep's particles over a cluster: particle counts around multiples of a CTA's threads;
+- the beam kernels' warp-wide adds: counts around a warp, all particles in one cell, a field store off the 16-byte
+  boundary.
+
+Tolerances: fields and diagnostics after one sweep max(1e-10, 4 x the reference algorithm's own round-off floor, the
+difference between its Thomas and partition solvers on the same input), per stored component; beam deposits 1e-12 and
+pushed particles 1e-13, as in test_gpu_parity.py."""
+import numpy as np
+import pytest
+
+import oracle as O
+import quarz_b200 as Q
+from helpers import rel_l2
+from quarz_b200 import deck
+
+pytestmark = pytest.mark.gpu
+
+DECK = """
+xi.convention = z-t
+grid.type = uniform
+grid.rmax = 6
+grid.dr = 1
+xi.min = -1.2
+xi.max = 0
+xi.step = 0.04
+time.dt = 5
+time.steps = 1
+plasma.species = electrons
+beams = driver
+driver.n0 = 3
+driver.sigma_r = 0.5
+driver.sigma_xi = 0.3
+driver.xi0 = -0.5
+driver.gamma = 1000
+driver.espread = 0.001
+driver.emit_n = 0.05
+driver.nparticles = 3000
+"""
+
+
+def _spec(nodes, extra=""):
+    spec = deck.run_spec(deck.parse_deck(DECK + extra))
+    spec.nodes = 6.0 * (np.arange(nodes) / (nodes - 1.0)) ** 1.2      # cells smaller at the axis
+    return spec
+
+
+def _check_sweep(spec):
+    import torch
+
+    beams = [Q.sample_beam(b) for b in spec.beams]
+    a = O.OracleSim(spec, beams=beams, tridiag="thomas")
+    a.step_fields(0.0)
+    b = O.OracleSim(spec, beams=beams, tridiag="partition")
+    b.step_fields(0.0)
+    K, M = spec.K, spec.M
+    nf, nd = (18, 9) if spec.modes else (6, 3)
+    bsrc = torch.from_numpy(np.ascontiguousarray(a.bsrc())).cuda()
+    fld = torch.zeros((K, M, nf), dtype=torch.float64, device="cuda")
+    diag = torch.zeros((K, M, nd), dtype=torch.float64, device="cuda")
+    Q.Sweep(Q.RadialGrid(spec.nodes), Q.sweep_params(spec)).run(bsrc, fld, diag)
+    bad = {}
+    for name, got, ra, rb in (("fld", fld.cpu().numpy(), a.fld(), b.fld()), ("diag", diag.cpu().numpy(), a.diag(), b.diag())):
+        for c in range(got.shape[-1]):
+            if np.any(ra[..., c]):
+                e, floor = rel_l2(got[..., c], ra[..., c]), rel_l2(rb[..., c], ra[..., c])
+                if not e < max(1e-10, 4.0 * floor):
+                    bad[f"{name}{c}"] = (e, floor)
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("nodes", [17, 160, 161, 256, 257, 480, 481, 511, 512, 513, 769, 1025])
+def test_sweep_m0_nodes(nodes):
+    _check_sweep(_spec(nodes, "electrons.ppc = 1\n"))
+
+
+@pytest.mark.parametrize("order", [1, 2, 4, 5])
+@pytest.mark.parametrize("ppc", [1, 3])
+def test_sweep_m0_orders(order, ppc):
+    _check_sweep(_spec(257, f"electrons.ppc = {ppc}\npusher.ab_order = {order}\n"))
+
+
+@pytest.mark.parametrize("nodes,ntheta", [(17, 4), (128, 4), (129, 4), (130, 4), (257, 8), (512, 8), (513, 4), (641, 8)])
+def test_sweep_m1_particles_over_a_cluster(nodes, ntheta):
+    _check_sweep(_spec(nodes, f"modes = 1\nelectrons.ppc = 1\nelectrons.ntheta = {ntheta}\ndriver.x0 = 0.1\n"))
+
+
+@pytest.mark.parametrize("steps", [1, 9])
+def test_run_m1_teams(steps):
+    # two sweeps share clusters of 8 CTAs, ten of 4 (2040 particles per slice)
+    spec = _spec(256, "modes = 1\nelectrons.ppc = 1\nelectrons.ntheta = 8\ndriver.x0 = 0.1\n")
+    beams = [Q.sample_beam(b) for b in spec.beams]
+    mom = Q.Simulation(spec, beams=beams).run(steps, spec.dt)
+    ref = O.OracleSim(spec, beams=beams).run(steps, spec.dt)
+    assert rel_l2(mom, np.asarray(ref).reshape(mom.shape)) < 1e-12
+
+
+@pytest.mark.parametrize("modes", [0, 1])
+@pytest.mark.parametrize("n,one_cell", [(1, False), (31, False), (32, True), (33, True), (257, False), (4000, True)])
+def test_beam_push_deposit(n, one_cell, modes):
+    import torch
+
+    spec = _spec(65, "modes = 1\nelectrons.ntheta = 4\n" if modes else "")
+    spec.beams[0].nparticles = n
+    parts, gref, xiref = Q.sample_beam(spec.beams[0])
+    if one_cell:
+        parts[:, 5] = 0.5 + 0.01 * (parts[:, 5] - 0.5) / 0.9
+        parts[:, :2] *= 0.004
+    K, M = spec.K, spec.M
+    nf, nb = (18, 15) if modes else (6, 5)
+    o = O.OracleSim(spec, beams=[(parts, gref, xiref)])
+    o.step_fields(0.0)
+    F = np.ascontiguousarray(o.fld())
+    o.push_beams(5.0, 5.0)
+    o.deposit_beams()
+    grid = Q.RadialGrid(spec.nodes)
+    box = Q.BeamOps.box(spec.xi_min, spec.dxi, K, spec.ngp, modes)
+    want, wantb = o.beam(0), o.bsrc()
+    for shift in (0, 1):                               # the second field store starts 8 bytes off a 16-byte boundary
+        store = torch.zeros(K * M * nf + 1, dtype=torch.float64, device="cuda")
+        fld = store[shift:shift + K * M * nf]
+        fld.copy_(torch.from_numpy(F.reshape(-1)))
+        cols = torch.from_numpy(np.ascontiguousarray(parts.T)).cuda()
+        bsrc = torch.zeros((K, M, nb), dtype=torch.float64, device="cuda")
+        Q.BeamOps.push_deposit(grid, cols, -1.0, 1.0, box, fld, 5.0, 5.0, 0, bsrc)
+        got = cols.cpu().numpy().T
+        for c in range(7):
+            assert np.max(np.abs(got[:, c] - want[:, c])) <= 1e-13 * max(np.max(np.abs(want[:, c])), 1.0), c
+        B = bsrc.cpu().numpy()
+        assert rel_l2(B, wantb) < 1e-12
