@@ -128,7 +128,11 @@ def test_beam_push_deposit(n, one_cell, modes):
         bsrc = torch.zeros((K, M, nb), dtype=torch.float64, device="cuda")
         Q.BeamOps.push_deposit(grid, cols, -1.0, 1.0, box, fld, 5.0, 5.0, 0, bsrc)
         got = cols.cpu().numpy().T
+        # momenta: the kicks of E and of v x B, each up to 5 max|F| (here up to 2000), nearly cancel; a gather rounds
+        # each of them in about four operations
+        kick = 4 * np.finfo(float).eps * 5.0 * np.max(np.abs(F))
         for c in range(7):
-            assert np.max(np.abs(got[:, c] - want[:, c])) <= 1e-13 * max(np.max(np.abs(want[:, c])), 1.0), c
+            tol = 1e-13 * max(np.max(np.abs(want[:, c])), 1.0) + (kick if 2 <= c <= 4 else 0.0)
+            assert np.max(np.abs(got[:, c] - want[:, c])) <= tol, c
         B = bsrc.cpu().numpy()
         assert rel_l2(B, wantb) < 1e-12
