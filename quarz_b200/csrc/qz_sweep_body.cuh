@@ -1036,7 +1036,7 @@ __device__ __forceinline__ PKin kin_of(double px, double py, double d) {
     return k;
 }
 // the same from the particle's state, where nothing is kept from phase to phase (plasma in global memory; with plain
-// divisions: sharing reciprocals gained 2 % there, and the order of roundings is kept for the long chaotic sweeps)
+// divisions: sharing reciprocals gained 2 % there)
 struct KinNone {};
 __device__ __forceinline__ void kin_get(const PKin& k, double, double, double, double& gam, double& invd) {
     gam = k.gam;
