@@ -164,13 +164,10 @@ __device__ __forceinline__ void warp_deposit3(const BeamArgs& B, double* __restr
     const unsigned key = act ? (unsigned)((D.k + 1) * B.M + D.j) : 0xffffffffu - lane;
     const unsigned same = __match_any_sync(FULL, key);
     const bool lead = act && lane == __ffs(same) - 1;
-    const unsigned leads = __ballot_sync(FULL, lead);
     if (lead) {
         W.off[lane] = ((long)D.k * B.M + D.j) * (kW / 2);
         W.mask[lane] = same;
-        W.lead[__popc(leads & ((1u << lane) - 1u))] = (unsigned char)lane;
     }
-    const int total = __popc(leads) * kW;
     double w2[2];
     if (act) {
         w2[0] = D.d0 * (1.0 - D.t) * B.inv_V[D.j] * B.idxi;
@@ -178,9 +175,15 @@ __device__ __forceinline__ void warp_deposit3(const BeamArgs& B, double* __restr
     }
 #pragma unroll 1
     for (int a = 0; a < (B.ngp ? 1 : 2); ++a) {
-        if (act) {
-            const int kk = D.k + a;
-            const double Wk = kk >= 0 && kk < B.K ? (a ? D.tk : 1.0 - D.tk) : 0.0;   // rows out of the box: zeros
+        // rows ahead of or behind the box are nobody's to add to (kept out by their index: a value that is not finite
+        // times a zero weight is not zero)
+        const int kk = D.k + a;
+        const bool in = kk >= 0 && kk < B.K;
+        const unsigned leads = __ballot_sync(FULL, lead && in);
+        if (lead && in) W.lead[__popc(leads & ((1u << lane) - 1u))] = (unsigned char)lane;
+        const int total = __popc(leads) * kW;
+        if (act && in) {
+            const double Wk = a ? D.tk : 1.0 - D.tk;
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const double d = w2[b] * Wk;
@@ -204,7 +207,7 @@ __device__ __forceinline__ void warp_deposit3(const BeamArgs& B, double* __restr
             const int sl = q / kW, w = q - sl * kW, src = W.lead[sl];
             double v = W.val[src][w];
             for (unsigned m = W.mask[src] & ~(1u << src); m; m &= m - 1) v += W.val[__ffs(m) - 1][w];
-            if (v != 0.0) atomicAdd(row + W.off[src] + w, v);    // (zero: nothing, or a row out of the box)
+            if (v != 0.0) atomicAdd(row + W.off[src] + w, v);
         }
         __syncwarp();
     }

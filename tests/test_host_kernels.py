@@ -1,0 +1,77 @@
+"""Kernels run on the host (host_kernels.py): what must hold whatever the inputs and the order of the warps, and what a
+GPU must not be given to find out."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import host_kernels as H
+import quarz_b200 as Q
+
+if not H.available():
+    pytest.skip("needs g++ on x86-64", allow_module_level=True)
+
+
+def _grid(nodes):
+    g = C.c_void_p()
+    nodes = np.ascontiguousarray(nodes, dtype=np.float64)
+    H.check(H.library().qz_grid_create(nodes.ctypes.data_as(C.POINTER(C.c_double)), len(nodes), C.byref(g)))
+    return g
+
+
+def _view(cols, q=-1.0, m=1.0):
+    from quarz_b200 import _lib as L
+
+    n = cols.shape[1]
+    return L.BeamView(*[cols[c].ctypes.data for c in range(7)], n, q, m, 0)
+
+
+@pytest.mark.parametrize("bad", [None, "momentum", "weight"])
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("ngp", [0, 1])
+def test_compact_deposit_stays_in_its_rows(ngp, exact, bad):
+    # Particles in every xi cell, among them -1 (just ahead of the box: row 0 only) and K - 1 (behind it: row K - 1
+    # only). A row outside the box belongs to another ring slot or to nobody: nothing is added there, not by a particle
+    # whose momentum or weight is not finite either (0 x NaN is not 0).
+    lib = H.library()
+    K, dxi, xi_min = 6, 0.25, -1.5
+    nodes = 3.0 * (np.arange(17) / 16.0) ** 1.2
+    M = len(nodes)
+    rng = np.random.default_rng(5)
+    n = 200
+    cols = np.empty((7, n))
+    r, th = rng.uniform(0.0, 2.9, n), rng.uniform(0.0, 2 * np.pi, n)
+    cols[0], cols[1] = r * np.cos(th), r * np.sin(th)
+    cols[2:4] = rng.normal(size=(2, n))
+    cols[4] = rng.uniform(50.0, 100.0, n)
+    cell = rng.integers(-1, K, n)
+    cell[:40], cell[40:80] = -1, K - 1
+    cols[5] = xi_min + dxi * (cell + rng.uniform(0.1, 0.9, n))
+    cols[6] = rng.uniform(0.5, 1.0, n)
+    finite = cols.copy()
+    if bad:
+        cols[4 if bad == "momentum" else 6, ::7] = np.nan
+    g = _grid(nodes)
+    V = np.empty(M)
+    H.check(lib.qz_grid_volumes(g, V.ctypes.data_as(C.POINTER(C.c_double))))
+    inv_h, inv_V = np.append(1.0 / np.diff(nodes), 0.0), 1.0 / V
+    # exact: quanta of 2^-40, limbs of 20 bits
+    nc, scale = (6, np.full(M, 2.0 ** 40)) if exact else (3, None)
+    store = np.zeros((K + 4, M, nc))                  # two guard rows on either side
+    rc = lib.emu_deposit_compact(M, H.ptr(nodes), H.ptr(inv_h), H.ptr(inv_V), C.c_double(xi_min), C.c_double(dxi), K,
+                                 ngp, H.ptr(cols), C.c_long(n), C.c_double(-1.0), H.ptr(scale) if exact else None, 20,
+                                 H.ptr(store[2:]))
+    assert rc == 0
+    assert not np.any(store[:2]) and not np.any(store[K + 2:])
+    if bad:
+        return
+    want = np.zeros((K, M, 5))
+    box = Q.BeamOps.box(xi_min, dxi, K, ngp, 0)
+    v = _view(finite)
+    H.check(lib.qz_beam_deposit(g, C.byref(v), C.byref(box), H.ptr(want), None))
+    got = store[2:K + 2]
+    if exact:
+        got = (got[..., :3] * 2.0 ** 20 + got[..., 3:]) * 2.0 ** -40
+    # FP64: the same sums in another order; exact: half a quantum per particle and value
+    tol = n * 2.0 ** -41 if exact else 1e-13 * np.max(np.abs(want))
+    assert np.max(np.abs(got - want[..., [0, 1, 3]])) <= tol
