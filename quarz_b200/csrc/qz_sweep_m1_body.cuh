@@ -1173,8 +1173,8 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
         M1_MARK(2);
 
         // ---------------- P4: B+ (src/Simulation.cpp:535-591)
-        if (filt) {                 // S+ smoothed (src/Simulation.cpp:810-816): each thread's own row, the only
-            const Src1 T = src1_of(scr, M, cb);                  // one its B+ right-hand sides read
+        if (filt) {                 // S+ smoothed (src/Simulation.cpp:810-816): each thread's own row, the only one
+            const Src1 T = src1_of(scr, M, cb);                  // its B+ right-hand sides read
             FilterSet<6> fsS;
             fsS.f[0] = T.S.r0; fsS.f[1] = T.S.i0; fsS.f[2] = T.S.r1; fsS.f[3] = T.S.i1; fsS.f[4] = T.S.r2;
             fsS.f[5] = T.S.i2;
@@ -1182,6 +1182,7 @@ __device__ __forceinline__ bool sweep_m1_body(const SweepArgs& A, double* smem_r
             double* t0 = S.tot + (scan_par++ & 1) * 16 * kW;
             double* t1 = S.tot + (scan_par++ & 1) * 16 * kW;
             filter_rows1<6>(fsS, A.fconsts, M, t0, t1);
+            __syncthreads();                // its totals in t1 have been read: the groups' scratch lies over them
         }
         {
             const Src1 T = src1_of(scr, M, cb);

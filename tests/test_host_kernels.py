@@ -75,3 +75,80 @@ def test_compact_deposit_stays_in_its_rows(ngp, exact, bad):
     # FP64: the same sums in another order; exact: half a quantum per particle and value
     tol = n * 2.0 ** -41 if exact else 1e-13 * np.max(np.abs(want))
     assert np.max(np.abs(got - want[..., [0, 1, 3]])) <= tol
+
+
+DECK = """
+xi.convention = z-t
+grid.type = uniform
+grid.rmax = 6
+grid.dr = 1
+xi.min = -0.36
+xi.max = 0
+xi.step = 0.04
+time.dt = 5
+time.steps = 1
+plasma.species = electrons
+electrons.ppc = 1
+beams = driver
+driver.n0 = 3
+driver.sigma_r = 0.5
+driver.sigma_xi = 0.1
+driver.xi0 = -0.2
+driver.gamma = 1000
+driver.espread = 0.001
+driver.emit_n = 0.05
+driver.nparticles = 3000
+"""
+
+
+def _spec(nodes, extra=""):
+    from quarz_b200 import deck
+
+    spec = deck.run_spec(deck.parse_deck(DECK + extra))
+    spec.nodes = 6.0 * (np.arange(nodes) / (nodes - 1.0)) ** 1.2
+    return spec
+
+
+def _sweep(spec):
+    s = C.c_void_p()
+    p = Q.sweep_params(spec)
+    H.check(H.library().qz_sweep_create(_grid(spec.nodes), C.byref(p), C.byref(s)))
+    return s
+
+
+def _fields(spec):
+    nf, nd = (18, 9) if spec.modes else (6, 3)
+    return np.zeros((spec.K, spec.M, nf)), np.zeros((spec.K, spec.M, nd))
+
+
+# the warps that run ahead of the others (each as far as it can): none, all in turn, the last or one half, the first
+ORDERS = [((), False), (range(16), True), (range(15, -1, -1), True), (range(8, 16), True), (range(4), True)]
+
+
+@pytest.mark.parametrize("nodes,extra", [
+    (33, ""), (33, "electrons.ppc = 20\n"), (140, "plasma.smooth_length = 0.05\n"), (550, ""),
+    (550, "plasma.smooth_length = 0.05\n"),
+    (140, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\n"),
+    (140, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\nplasma.smooth_length = 0.05\n"),
+])
+def test_sweep_in_every_order_of_the_warps(nodes, extra):
+    # a barrier too few shows when a warp lags behind; tolerance as on the GPU: max(1e-10, 4 x the reference algorithm's
+    # round-off floor, the difference between its Thomas and partition solvers)
+    import oracle as O
+    from helpers import rel_l2
+
+    spec = _spec(nodes, extra)
+    beams = [Q.sample_beam(b) for b in spec.beams]
+    a, b = (O.OracleSim(spec, beams=beams, tridiag=t) for t in ("thomas", "partition"))
+    a.step_fields(0.0)
+    b.step_fields(0.0)
+    bsrc = np.ascontiguousarray(a.bsrc())
+    s = _sweep(spec)
+    for first, keep in ORDERS:
+        H.schedule(first, keep)
+        fld, diag = _fields(spec)
+        H.check(H.library().qz_sweep_run(s, H.ptr(bsrc), H.ptr(fld), H.ptr(diag), None, None))
+        for got, ra, rb in ((fld, a.fld(), b.fld()), (diag, a.diag(), b.diag())):
+            for c in range(got.shape[-1]):
+                if np.any(ra[..., c]):
+                    assert rel_l2(got[..., c], ra[..., c]) < max(1e-10, 4.0 * rel_l2(rb[..., c], ra[..., c])), (list(first), c)
