@@ -452,8 +452,10 @@ __device__ __forceinline__ int fx_bits(int n) { return 34 - __clz(n > 1 ? n : 1)
 // The psi / E_z / B_z phase went from 9,800 to 7,000 cycles per slice and B+ from 10,800 to 6,900 (512 nodes).
 // The row count is odd, so that the lanes' rows lie in different shared-memory banks.
 constexpr int kG2 = 5, kG4 = 8;                           // warps per system: 3 x 5 and 2 x 8
-constexpr int kMiscBytes = 256;                           // the words from Smem::lost on
-constexpr int kTot = 256;                                 // S.tot: 24 + 24 (L0), 64 + 32 + 32 (B+)
+constexpr int kTot = 192;                                 // S.tot: 24 + 24 (L0), 64 + 64 + 32 + 32 (B+); block scans 128 + 64
+// The words from Smem::lost on; 256 are used. With kTot 2,128 bytes beside the arrays: the largest grid is the
+// 1439 nodes (160 bytes each; 1180 with the smoothing filter) that fill a CTA's 227 KB to the last node
+constexpr int kMiscBytes = 2128 - 8 * kTot;
 __device__ __forceinline__ int group_rows(int M, int warps) { return ((M + 32 * warps - 1) / (32 * warps)) | 1; }
 __device__ __forceinline__ void group_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");

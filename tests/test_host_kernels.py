@@ -152,3 +152,12 @@ def test_sweep_in_every_order_of_the_warps(nodes, extra):
             for c in range(got.shape[-1]):
                 if np.any(ra[..., c]):
                     assert rel_l2(got[..., c], ra[..., c]) < max(1e-10, 4.0 * rel_l2(rb[..., c], ra[..., c])), (list(first), c)
+
+
+@pytest.mark.parametrize("extra,most", [("", 1439), ("plasma.smooth_length = 0.05\n", 1180)])
+def test_largest_grid(extra, most):
+    # the widest grid that a CTA's shared memory holds: 160 bytes per node (192 with the filter) beside 2128 (5712) in
+    # 232448; one node more is refused
+    with pytest.raises(RuntimeError, match=f"M = {most + 1} is too large"):
+        _sweep(_spec(most + 1, extra))
+    test_sweep_in_every_order_of_the_warps(most, extra)
