@@ -62,13 +62,15 @@ __device__ __forceinline__ double beam_fx_value(double hi_sum, double lo_sum, do
 // Quotients of one divisor: the reciprocal once, then a multiplication and one residual correction per
 // quotient (P. Markstein, IBM J. Res. Dev. 34 (1990) 111: q = a y, q + (a - b q) y). The compiler's FP64
 // divide contains a branch, so divides do not overlap: 137 cycles for one, 391 for three independent ones
-// in one warp, against 87 for the reciprocal and 26 for each further quotient here. For finite a and normal b.
+// in one warp, against 87 for the reciprocal and 26 for each further quotient here. Where a, b or q is infinite the
+// correction is not a number and the plain product stands: infinity over a finite b, and 0 over an infinite one, as the
+// division gives (a plasma particle whose gamma overflows must still compare as trapped).
 struct Recip {
     double b, y;
     __device__ __forceinline__ explicit Recip(double d) : b(d), y(1.0 / d) {}
     __device__ __forceinline__ double operator()(double a) const {
-        const double q = a * y;
-        return fma(fma(-b, q, a), y, q);
+        const double q = a * y, r = fma(fma(-b, q, a), y, q);
+        return r == r ? r : q;
     }
 };
 

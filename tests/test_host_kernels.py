@@ -161,3 +161,39 @@ def test_largest_grid(extra, most):
     with pytest.raises(RuntimeError, match=f"M = {most + 1} is too large"):
         _sweep(_spec(most + 1, extra))
     test_sweep_in_every_order_of_the_warps(most, extra)
+
+
+def test_gamma_beyond_the_range():
+    # momenta whose squares overflow: 1 / gamma = 0 and v = 0 in the beam's deposit (m = 0 and 1), as a division gives
+    import oracle as O
+
+    for extra in ("", "modes = 1\nelectrons.ntheta = 4\n"):
+        spec = _spec(17, extra)
+        parts = np.array([[0.3, 0.1, 0.2, 0.1, 1e200, 0.1, 1.0]])
+        o = O.OracleSim(spec, beams=[(parts, 1.0, 0.0)])
+        o.deposit_beams()
+        want = o.bsrc()
+        got = np.zeros_like(want)
+        v, box = _view(np.ascontiguousarray(parts.T)), Q.BeamOps.box(spec.xi_min, spec.dxi, spec.K, spec.ngp, spec.modes)
+        H.check(H.library().qz_beam_deposit(_grid(spec.nodes), C.byref(v), C.byref(box), H.ptr(got), None))
+        assert np.any(want) and np.max(np.abs(got - want)) <= 1e-13 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("ppc", [1, 20])
+@pytest.mark.parametrize("n0", ["3e155", "1e200"])
+def test_plasma_beyond_the_range(n0, ppc):
+    # a driver so strong that the plasma's gamma overflows in its first push: every particle is removed as trapped and
+    # the fields stay the driver's own
+    import oracle as O
+    from quarz_b200 import _lib as L
+
+    spec = _spec(33, f"driver.n0 = {n0}\nelectrons.ppc = {ppc}\n")
+    spec.beams[0].q = 1.0
+    a = O.OracleSim(spec, beams=[Q.sample_beam(b) for b in spec.beams])
+    a.step_fields(0.0)
+    bsrc, want, (fld, diag), cnt = np.ascontiguousarray(a.bsrc()), a.fld(), _fields(spec), L.Counters()
+    H.schedule()
+    H.check(H.library().qz_sweep_run(_sweep(spec), H.ptr(bsrc), H.ptr(fld), H.ptr(diag), C.byref(cnt), None))
+    assert (cnt.lost, cnt.trapped, cnt.nonfinite) == (a.lost(), a.lost(), 0) and cnt.lost > 0
+    top = np.max(np.abs(want))
+    assert np.max(np.abs(fld / top - want / top)) < 1e-12
