@@ -1820,7 +1820,8 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
     constexpr int kPre = 1;
     const bool dbuf = !kHS && A.dbuf;
     const int ST = kHS ? kThreads : M;                          // distance between the shared arrays
-    int hs = 0;                                                 // slot of the newest force
+    int hs = 0;                                                 // slot of the particle's newest force (a removed
+                                                                // particle's history stands still, and its slot)
     const Smem S = carve<kCS, kHist>(smem_raw, A);
     const int np = A.np, npad = A.npad;
     const double R = A.R;
@@ -2302,7 +2303,10 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                     species_params(A, tid, P.q, P.qm);
                     if (kHS && !first) hist_get<ORD>(P, S, hs);
                     const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, hstep);
-                    if (kHS) hist_put<ORD>(P, S, hs + 1 == ORD ? 0 : hs + 1, first || pr == 2);
+                    if (kHS) {
+                        hs = hs + 1 == ORD ? 0 : hs + 1;
+                        hist_put<ORD>(P, S, hs, first || pr == 2);
+                    }
                     if (pr > 0) {
                         polar(P.x, P.y, kp.rp, kp.ir, kp.c, kp.s);
                         J = locate_from(S.r, N, R, kp.rp, J);
@@ -2313,7 +2317,6 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
                         if (pr < 0) atomicAdd(S.fx + 12, 1);
                     }
                 }
-                if (kHS) hs = hs + 1 == ORD ? 0 : hs + 1;
                 const bool tail = deposit_runs<true>(act, J, P.q < 0.0, v, S.fx);
                 __syncthreads();                  // (the maxima, and the accumulators cleared after the store above)
                 deposit_add(tail, J, P.q < 0.0, v, acc, S.fx, bits_p);
@@ -2422,12 +2425,9 @@ __device__ __forceinline__ bool sweep_body(const SweepArgs& A, double* smem_raw,
             if (tid < np && P.w != 0.0) {
                 if (kHS && !first) hist_get<ORD>(P, S, hs);
                 const int pr = push_particle(P, keep_geo(S, kp, J), kp.k, S, A, first, abc, A.dxi);
-                if (kHS) hist_put<ORD>(P, S, hs + 1 == ORD ? 0 : hs + 1, first || pr == 2);
                 if (pr <= 0) { atomicAdd(S.lost, 1); if (pr < 0) atomicAdd(S.fx + 12, 1); }
-            }
-            if (kHS) {                                 // (a particle removed earlier keeps its history)
-                if (tid < np && P.w == 0.0) hist_get<ORD>(P, S, hs);
-                hs = hs + 1 == ORD ? 0 : hs + 1;
+            } else if (kHS && tid < np) {
+                hist_get<ORD>(P, S, hs);               // a particle removed earlier
             }
             if (tid < np) pstore(P, A.pout, npad, tid);
         } else {

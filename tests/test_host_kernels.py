@@ -197,3 +197,37 @@ def test_plasma_beyond_the_range(n0, ppc):
     assert (cnt.lost, cnt.trapped, cnt.nonfinite) == (a.lost(), a.lost(), 0) and cnt.lost > 0
     top = np.max(np.abs(want))
     assert np.max(np.abs(fld / top - want / top)) < 1e-12
+
+
+@pytest.mark.parametrize("ppc", [1, 20])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_removed_particles_keep_their_state(order, ppc):
+    # a slab hands its plasma on with every particle's history; a removed particle's is that of the push that removed it,
+    # however many slices follow (history in shared memory, in registers and in global memory)
+    from quarz_b200 import _lib as L
+
+    lib = H.library()
+    spec = _spec(33, f"beams.xi_shape = ngp\ndriver.n0 = 60\nelectrons.ppc = {ppc}\npusher.ab_order = {order}\n")
+    bsrc = np.zeros((spec.K, spec.M, 5))
+    parts, _, _ = Q.sample_beam(spec.beams[0])
+    v, box = _view(np.ascontiguousarray(parts.T)), Q.BeamOps.box(spec.xi_min, spec.dxi, spec.K, spec.ngp, 0)
+    H.check(lib.qz_beam_deposit(_grid(spec.nodes), C.byref(v), C.byref(box), H.ptr(bsrc), None))
+    H.schedule()
+    states = {}
+    for K in range(3, spec.K + 1):
+        p = Q.sweep_params(spec)
+        p.K, p.max_qsa = K, 1.0 + 1e-3
+        s, n, npad, ord_ = C.c_void_p(), C.c_int(), C.c_int(), C.c_int()
+        H.check(lib.qz_sweep_create(_grid(spec.nodes), C.byref(p), C.byref(s)))
+        H.check(lib.qz_sweep_state_shape(s, C.byref(n), C.byref(npad), C.byref(ord_)))
+        out = np.zeros((6 + 5 * order, npad.value))
+        fld, diag = np.zeros((K, spec.M, 6)), np.zeros((K, spec.M, 3))
+        st = L.PlasmaState(out.ctypes.data, n.value, npad.value, order, 0)
+        H.check(lib.qz_sweep_run_stage(s, H.ptr(bsrc), None, None, H.ptr(fld), H.ptr(diag), C.byref(st), None, None))
+        states[K] = out[:, :n.value]
+    seen = 0
+    for K in range(3, spec.K):
+        gone = states[K][5] == 0.0
+        seen += bool(np.any(gone)) and not np.all(gone)
+        assert np.array_equal(states[K + 1][:, gone], states[K][:, gone]), K
+    assert seen >= 3
