@@ -231,3 +231,12 @@ def test_removed_particles_keep_their_state(order, ppc):
         seen += bool(np.any(gone)) and not np.all(gone)
         assert np.array_equal(states[K + 1][:, gone], states[K][:, gone]), K
     assert seen >= 3
+
+
+def test_grid_set_up_is_one_copy():
+    # a scan makes a grid per instance: its arrays reach the device in one allocation and one blocking copy
+    lib, n = H.library(), [C.c_long() for _ in range(4)]
+    lib.emu_counts(C.byref(n[0]), C.byref(n[1]))
+    _grid(_spec(257).nodes)
+    lib.emu_counts(C.byref(n[2]), C.byref(n[3]))
+    assert (n[2].value - n[0].value, n[3].value - n[1].value) == (1, 1)
