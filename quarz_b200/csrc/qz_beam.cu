@@ -107,6 +107,27 @@ __device__ __forceinline__ void dep_nodes(BeamArgs& B, DepSmem<NC>& S) {
     B.r = S.r;
 }
 
+// The few particles of a small beam: every lane adds its own values, and searches its cell in L1, instead of a copy of the
+// nodes, a barrier and two passes through shared memory before the first value goes out. Calls of up to kFew particles
+// (kFewPush with the push), us per call on 512 nodes, here and with the warp-wide adds: deposit of 100 6.3 and 8.3, of
+// 16000 8.6 and 10.3 (on 33 nodes 10.3 and 9.3), of 32000 12.3 and 10.3; push and deposit of 100 14.4 and 16.5, of 8000 17.0
+// and 17.9, of 16000 17.9 and 18.5 (on 257 nodes 18.5 and 17.5). With mode 1 deposit of 100 8.3 and 14.0, of 300 to 4000
+// the same, of 16000 16.3 and 14.4; push and deposit of 100 16.5 and 22.6, of 300 26.7 and 24.7
+template <int NC>
+constexpr long kFew = NC == B_NC0 ? 16384 : 4096;
+template <int NC>
+constexpr long kFewPush = NC == B_NC0 ? 8192 : 128;
+
+template <int NC>
+__global__ void __launch_bounds__(kBeamThreads) beam_deposit_few_kernel(const BeamArgs B, double* __restrict__ bsrc) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B.n) return;
+    const double wi = B.w[i];
+    DepOne<NC> D;
+    if (wi != 0.0 && dep_one<NC>(B, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi, -1, D))
+        lane_deposit<NC>(B, bsrc, D);
+}
+
 // Bound by the L2 reductions (2 rows x 2 nodes x NC values per particle): 1e6 particles on 512 x 2400 nodes take
 // 104 us, 212 us with an addition per lane and value.
 template <int NC>
@@ -345,6 +366,20 @@ __global__ void __launch_bounds__(kDepThreads<NC>) beam_push_deposit_kernel(cons
     }
 }
 
+template <int NC, bool kVec>
+__global__ void __launch_bounds__(kBeamThreads) beam_push_deposit_few_kernel(const BeamArgs B,
+                                                                             const double* __restrict__ fld,
+                                                                             double dt_kick, double dt,
+                                                                             double* __restrict__ bsrc_next) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B.n) return;
+    const double wi = B.w[i];
+    if (wi == 0.0) return;
+    const Moved m = move_one<kVec>(B, fld, i, 0.5 * (B.q / B.m) * dt_kick, dt);
+    DepOne<NC> D;
+    if (m.live && dep_one<NC>(B, m.x, m.y, m.px, m.py, m.pz, m.xi, wi, m.j, D)) lane_deposit<NC>(B, bsrc_next, D);
+}
+
 // moment sums: fixed grid, fixed per-thread order, fixed tree -> deterministic
 constexpr int kSumThreads = 256;
 
@@ -418,6 +453,14 @@ int beam_sums_blocks(long n) {
     return (int)b;
 }
 
+namespace {
+template <int NC>
+void deposit_full(const BeamArgs& B, double* bsrc, cudaStream_t s) {
+    if (B.n <= kFew<NC>) beam_deposit_few_kernel<NC><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, bsrc);
+    else beam_deposit_kernel<NC><<<grid_dep<NC>(B.n), kDepThreads<NC>, 0, s>>>(B, bsrc);
+}
+}  // namespace
+
 cudaError_t launch_beam_deposit(const BeamArgs& B, double* bsrc, cudaStream_t s) {
     if (B.n <= 0) return cudaSuccess;
     if (B.compact) {
@@ -425,8 +468,8 @@ cudaError_t launch_beam_deposit(const BeamArgs& B, double* bsrc, cudaStream_t s)
         else beam_deposit3_kernel<false><<<grid_for(B.n), kBeamThreads, 0, s>>>(B, bsrc);
         return cudaGetLastError();
     }
-    if (B.modes) beam_deposit_kernel<B_NC1><<<grid_dep<B_NC1>(B.n), kDepThreads<B_NC1>, 0, s>>>(B, bsrc);
-    else beam_deposit_kernel<B_NC0><<<grid_dep<B_NC0>(B.n), kDepThreads<B_NC0>, 0, s>>>(B, bsrc);
+    if (B.modes) deposit_full<B_NC1>(B, bsrc, s);
+    else deposit_full<B_NC0>(B, bsrc, s);
     return cudaGetLastError();
 }
 
@@ -462,11 +505,14 @@ namespace {
 template <int NC>
 cudaError_t push_deposit(const BeamArgs& B, const double* fld, double dt_kick, double dt_drift, double* bsrc_next,
                          cudaStream_t s) {
-    const int grid = grid_dep<NC>(B.n);
-    if (aligned16(fld))
-        beam_push_deposit_kernel<NC, true><<<grid, kDepThreads<NC>, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
-    else
-        beam_push_deposit_kernel<NC, false><<<grid, kDepThreads<NC>, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
+    const bool vec = aligned16(fld);
+    if (B.n <= kFewPush<NC>) {
+        auto* const kernel = vec ? beam_push_deposit_few_kernel<NC, true> : beam_push_deposit_few_kernel<NC, false>;
+        kernel<<<grid_for(B.n), kBeamThreads, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
+    } else {
+        auto* const kernel = vec ? beam_push_deposit_kernel<NC, true> : beam_push_deposit_kernel<NC, false>;
+        kernel<<<grid_dep<NC>(B.n), kDepThreads<NC>, 0, s>>>(B, fld, dt_kick, dt_drift, bsrc_next);
+    }
     return cudaGetLastError();
 }
 }  // namespace

@@ -140,6 +140,35 @@ __device__ __forceinline__ bool dep_one(const BeamArgs& B, double X, double Y, d
     return true;
 }
 
+// adds a particle's deposit to its nodes, each value by the calling lane
+template <int NC>
+__device__ __forceinline__ void lane_deposit(const BeamArgs& B, double* __restrict__ bsrc, const DepOne<NC>& D) {
+#pragma unroll 1
+    for (int a = 0; a < (B.ngp ? 1 : 2); ++a) {
+        const int kk = D.k + a;
+        if (kk < 0 || kk >= B.K) continue;
+        const double Wk = a ? D.tk : 1.0 - D.tk;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            double* const o = bsrc + ((size_t)kk * B.M + D.j + b) * NC;
+            const double d = D.d0 * Wk * (b ? D.t : 1.0 - D.t) * B.inv_V[D.j + b] * B.idxi;
+            if (B.fx_scale) {                                    // exact (m = 0 runs of qz_sim)
+                const double sc = B.fx_scale[D.j + b];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    double hi = 0.0, lo = 0.0;
+                    beam_fx_split(d * D.f[c], sc, B.fx_inv2s, B.fx_2s, hi, lo);
+                    atomicAdd(o + c, hi);
+                    atomicAdd(o + c + B.fx_lo, lo);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) atomicAdd(o + c, d * D.f[c]);
+            }
+        }
+    }
+}
+
 // The deposit of a warp's particles into compact m = 0 beam sources: kDep0 values per node, or (kExact) their
 // high limbs and then their low limbs, so that a particle's 2 nodes of a row are 6 or 12 contiguous doubles. A
 // reduction instruction of a particle per lane costs its SM one cycle per lane and value; here the values go

@@ -4,8 +4,8 @@
   whole numbers of rows per thread, and the block-wide solves of more than 512 nodes;
 - every Adams-Bashforth order (the history is kept in shared memory up to order 3);
 - the m = 1 sweep's particles over a cluster: particle counts around multiples of a CTA's threads;
-- the beam kernels' warp-wide adds: counts around a warp, all particles in one cell, a field store off the 16-byte
-  boundary.
+- the beam kernels: counts around a warp and around the largest call whose lanes add their own values (m = 0: 16384,
+  with the push 8192; m = 1: 4096 and 128), all particles in one cell, a field store off the 16-byte boundary.
 
 Tolerances: fields and diagnostics after one sweep max(1e-10, 4 x the reference algorithm's own round-off floor, the
 difference between its Thomas and partition solvers on the same input), per stored component; beam deposits 1e-12 and
@@ -100,7 +100,9 @@ def test_run_m1_teams(steps):
 
 
 @pytest.mark.parametrize("modes", [0, 1])
-@pytest.mark.parametrize("n,one_cell", [(1, False), (31, False), (32, True), (33, True), (257, False), (4000, True)])
+@pytest.mark.parametrize("n,one_cell", [(1, False), (31, False), (32, True), (33, True), (257, False), (4000, True),
+                                        (128, False), (129, True), (160, False), (4096, False), (4097, True),
+                                        (8192, False), (8193, True), (16384, False), (16417, True)])
 def test_beam_push_deposit(n, one_cell, modes):
     import torch
 
@@ -136,3 +138,6 @@ def test_beam_push_deposit(n, one_cell, modes):
             assert np.max(np.abs(got[:, c] - want[:, c])) <= tol, c
         B = bsrc.cpu().numpy()
         assert rel_l2(B, wantb) < 1e-12
+        bsrc.zero_()                                   # and the deposit by itself, of the pushed particles
+        Q.BeamOps.deposit(grid, cols, -1.0, 1.0, box, bsrc)
+        assert rel_l2(bsrc.cpu().numpy(), wantb) < 1e-12
