@@ -386,7 +386,10 @@ qz_status qz_batch_info(qz_batch* b, double* out4);
    global memory, np > 512), or -1 to keep the current one; and its cost, the key of the largest-first
    queue, or <= 0 to keep it. qz_batch_add picks the fastest layout that fits and the estimate
    K (M + 4 np) + 2 N_beam; the autotuner (quarz_b200.tune) measures both instead. Fails with QZ_ERR_SIZE
-   for a layout that does not fit the device's shared memory. qz_batch_tuning reads them back.
+   for a layout that does not fit the device's shared memory. Instances with at most 512 nodes and 512 particles
+   have the constants in shared memory whatever the layout says, and with an order up to 3, in a batch without
+   smoothing and sub-slicing, single-buffered sources. qz_batch_tuning gives the layout that the kernel of the
+   batch as it stands uses, and the cost.
    No counterpart in the reference. */
 qz_status qz_batch_set_tuning(qz_batch* b, int index, int layout, double cost);
 qz_status qz_batch_tuning(qz_batch* b, int index, int* layout, double* cost);

@@ -610,7 +610,7 @@ class Batch:
         check(lib().qz_batch_set_tuning(self.h, int(index), int(layout), float(cost)))
 
     def tuning(self, index: int) -> Tuple[int, float]:
-        """qz_batch_tuning: (layout bits or -1 for modes = 1, queue cost) of instance `index`."""
+        """qz_batch_tuning: (bits of the layout its kernel uses or -1 for modes = 1, queue cost) of instance `index`."""
         lay, cost = C.c_int(), np.zeros(1)
         check(lib().qz_batch_tuning(self.h, int(index), C.byref(lay), _p(cost)))
         return lay.value, float(cost[0])

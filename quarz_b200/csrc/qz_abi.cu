@@ -2628,21 +2628,23 @@ extern "C" qz_status qz_batch_set_tuning(qz_batch* b, int index, int layout, dou
     auto* I = b->inst[index];
     if (cost > 0.0) I->cost = cost;
     if (layout < 0) return QZ_OK;
-    qzb::SweepArgs& A = I->dev.sw;
+    qzb::SweepArgs A = I->dev.sw;
     if (I->dev.modes != 0 || layout > 7) return fail(QZ_ERR_ARG, "qz_batch_set_tuning: layouts are for modes = 0 (0..7)");
-    const bool dbuf = layout & 1, cs = (layout >> 1) & 1, pc = (layout >> 2) & 1;
+    const bool pc = (layout >> 2) & 1;
     if (pc && A.np <= qzb::kSweepThreads)
         return fail(QZ_ERR_ARG, "qz_batch_set_tuning: the particle copy is for plasma in global memory (np > 512)");
+    A.dbuf = layout & 1;
+    A.const_smem = (layout >> 1) & 1;
+    A.pcache = pc ? A.np : 0;
     int dev = 0, optin = 0;
     QZ_CUDA(cudaGetDevice(&dev));
     QZ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const size_t reserve = sizeof(qzb::BatchInst) + sizeof(double) * 17 * (qzb::kSweepThreads / 32) + 256;
-    if (qzb::sweep_m0_smem_bytes(A.M, dbuf, cs, A.filter != 0, pc ? A.np : 0) + reserve > (size_t)optin)
+    // (of both kernels that may run it: with or without a filtered instance in the batch)
+    if (std::max(qzb::sweep_m0_smem_bytes(A, false), qzb::sweep_m0_smem_bytes(A, true)) + reserve > (size_t)optin)
         return fail(QZ_ERR_SIZE, "qz_batch_set_tuning: layout " + std::to_string(layout) + " does not fit M = " +
                                      std::to_string(A.M));
-    A.dbuf = dbuf;
-    A.const_smem = cs;
-    A.pcache = pc ? A.np : 0;
+    I->dev.sw = A;
     return QZ_OK;
 }
 
@@ -2651,7 +2653,9 @@ extern "C" qz_status qz_batch_tuning(qz_batch* b, int index, int* layout, double
         return fail(QZ_ERR_ARG, "qz_batch_tuning: bad argument");
     const auto* I = b->inst[index];
     const qzb::SweepArgs& A = I->dev.sw;
-    *layout = I->dev.modes ? -1 : (A.dbuf ? 1 : 0) | (A.const_smem ? 2 : 0) | (A.pcache ? 4 : 0);
+    bool ext = false;                    // the kernel of the batch as it stands
+    for (const auto* J : b->inst) ext = ext || qzb::sweep_ext(J->dev.sw);
+    *layout = I->dev.modes ? -1 : (qzb::sweep_m0_dbuf(A, ext) ? 1 : 0) | (qzb::consts_in_smem(A) ? 2 : 0) | (A.pcache ? 4 : 0);
     *cost = I->cost;
     return QZ_OK;
 }

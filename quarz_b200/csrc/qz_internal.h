@@ -108,6 +108,9 @@ inline bool consts_in_smem(const SweepArgs& A) {
 }
 // whether A needs the kernel variant with the smoothing filter, static sources and adaptive sub-slicing
 inline bool sweep_ext(const SweepArgs& A) { return A.filter || A.bstat || A.max_cells > 0.0; }
+// whether the kernel variant that runs A double-buffers the slice's sources: where A asks for it, and not where it keeps
+// the particles' history in shared memory
+bool sweep_m0_dbuf(const SweepArgs& A, bool ext);
 size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter = false, int pcache = 0);
 // of the kernel variant that runs A; ext: the variant with the smoothing filter and static sources
 size_t sweep_m0_smem_bytes(const SweepArgs& A, bool ext);

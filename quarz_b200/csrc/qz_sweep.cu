@@ -20,11 +20,16 @@ size_t sweep_m0_smem_bytes(int M, bool dbuf, bool const_smem, bool filter, int p
     return sizeof(double) * d + sweep_detail::kMiscBytes + (pcache > 0 ? (size_t)pcache * (6 * sizeof(double) + sizeof(int)) : 0);
 }
 
+static int hist_of(const SweepArgs& A, bool ext) {
+    return sweep_detail::hist_doubles(A.ord, A.np <= kSweepThreads, A.rows_per_thread == 1 ? 1 : 3, ext);
+}
+
+bool sweep_m0_dbuf(const SweepArgs& A, bool ext) { return A.dbuf && !hist_of(A, ext); }
+
 size_t sweep_m0_smem_bytes(const SweepArgs& A, bool ext) {
-    const bool reg = A.np <= kSweepThreads;
-    const int hist = sweep_detail::hist_doubles(A.ord, reg, A.rows_per_thread == 1 ? 1 : 3, ext);
+    const int hist = hist_of(A, ext);
     // (the variant with the history lays its arrays out kSweepThreads nodes apart: carve)
-    return sweep_m0_smem_bytes(hist ? kSweepThreads : A.M, hist ? false : A.dbuf != 0, consts_in_smem(A), A.filter != 0, A.pcache) +
+    return sweep_m0_smem_bytes(hist ? kSweepThreads : A.M, sweep_m0_dbuf(A, ext), consts_in_smem(A), A.filter != 0, A.pcache) +
            sizeof(double) * hist * kSweepThreads;
 }
 

@@ -7,7 +7,9 @@ queue hands instances to CTAs:
 - the layout, a bit set: 1 double-buffered slice sources (the next slice's deposit lands in the free half
   while the current one is stored), 2 the per-node operator constants in shared memory (instead of L1-cached
   global loads), 4 a shared-memory copy of the plasma particles when they live in global memory (np > 512
-  particles per slice). Which of them fit depends on M; which is fastest is measured;
+  particles per slice). Which of them fit depends on M; which is fastest is measured. With at most 512 nodes
+  and 512 particles the constants are in shared memory always, and the sources single-buffered in the kernel
+  that keeps the particles' history in shared memory (orders up to 3, no filter or sub-slicing in the batch);
 - the queue cost: the largest-first queue wants each instance's run time. The built-in estimate
   K (M + 4 np) + 2 N_beam misses that plasma in global memory costs about twice as much per particle as
   plasma in registers, so those instances start late and leave a tail.
@@ -43,13 +45,26 @@ def size_class(spec) -> Tuple[int, int, int, int]:
             int(plasma_per_slice(spec) > REG_PARTICLES), int(spec.M) // 128)
 
 
-def candidate_layouts(spec) -> List[int]:
+def needs_ext(spec) -> bool:
+    """Whether an instance makes its batch run the kernel with the smoothing filter and sub-slicing."""
+    return getattr(spec, "smooth_length", 0.0) > 0.0 or getattr(spec, "max_cells", 0.0) > 0.0
+
+
+def used_layout(spec, layout: int, ext: bool = False) -> int:
+    """The layout that an m = 0 instance given `layout` runs with, in a batch that runs the kernel with the
+    filter and sub-slicing (ext) or not."""
+    if layout < 0 or spec.M > REG_PARTICLES or plasma_per_slice(spec) > REG_PARTICLES:
+        return layout
+    return (layout | 2) & ~(1 if spec.ab_order <= 3 and not (ext or needs_ext(spec)) else 0)
+
+
+def candidate_layouts(spec, ext: bool = False) -> List[int]:
     """The layouts to try (the library rejects those that do not fit): none for modes = 1, the particle
-    copy only with plasma in global memory."""
+    copy only with plasma in global memory, and of those that run the same kernel one."""
     if spec.modes != 0:
         return [-1]
     glob = plasma_per_slice(spec) > REG_PARTICLES
-    return [l for l in LAYOUTS if glob or not (l & 4)]
+    return sorted({used_layout(spec, l, ext) for l in LAYOUTS if glob or not (l & 4)})
 
 
 @dataclass
@@ -61,8 +76,8 @@ class Tuning:
     beam_us: float = 0.0
     device: str = ""
 
-    def layout(self, spec) -> int:
-        return self.layouts.get(size_class(spec), -1)
+    def layout(self, spec, ext: bool = False) -> int:
+        return used_layout(spec, self.layouts.get(size_class(spec), -1), ext)
 
     def cost(self, spec, beam_particles: int, nsteps: int) -> float:
         """Predicted run time (us) of nsteps (nsteps + 1 sweeps): the class's measured slice time, or that
@@ -126,9 +141,10 @@ def calibrate(specs: Sequence, beams: Sequence, dt: float, steps: int = 2, per_c
     from .api import Batch, QZError
 
     b = Batch()
+    ext = any(needs_ext(s) for s in specs)
     entries = []                      # (batch index, class, layout, spec index)
     for i in representatives(specs, per_class):
-        for lay in candidate_layouts(specs[i]):
+        for lay in candidate_layouts(specs[i], ext):
             j = b.add(specs[i], beams[i])
             ok = True
             if lay >= 0:
@@ -160,11 +176,12 @@ def apply(batch, specs: Sequence, beams: Sequence, nsteps: int, tuning: Tuning) 
     A layout that does not fit an instance (a tuning loaded for other shapes) leaves its layout as it is."""
     from .api import QZError
 
+    ext = any(needs_ext(s) for s in specs)
     for i, s in enumerate(specs):
         nb = sum(len(p) for p, _, _ in beams[i])
         cost = tuning.cost(s, nb, nsteps)
         try:
-            batch.set_tuning(i, tuning.layout(s), cost)
+            batch.set_tuning(i, tuning.layout(s, ext), cost)
         except QZError:
             batch.set_tuning(i, -1, cost)
 

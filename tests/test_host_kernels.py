@@ -240,3 +240,44 @@ def test_grid_set_up_is_one_copy():
     _grid(_spec(257).nodes)
     lib.emu_counts(C.byref(n[2]), C.byref(n[3]))
     assert (n[2].value - n[0].value, n[3].value - n[1].value) == (1, 1)
+
+
+@pytest.mark.parametrize("with_filter", [False, True])
+@pytest.mark.parametrize("nodes,ppc,order", [(65, 1, 3), (512, 1, 1), (512, 1, 4), (513, 1, 3), (257, 4, 3), (600, 1, 3)])
+def test_batch_layouts_are_the_kernels(nodes, ppc, order, with_filter):
+    # qz_batch_tuning gives the layout the kernel uses, and the autotuner's candidates are different kernels: each reads
+    # back as it was set, and every layout as one of them
+    from quarz_b200 import tune
+
+    lib, b, n = H.library(), C.c_void_p(), C.c_int()
+    H.check(lib.qz_batch_create(C.byref(b)))
+
+    def add(spec):
+        p = Q.sweep_params(spec)
+        a = np.ascontiguousarray(spec.nodes)
+        H.check(lib.qz_batch_add(b, a.ctypes.data_as(C.POINTER(C.c_double)), len(a), C.byref(p), 0, None, None, None,
+                                 None, None, None, None, C.byref(n)))
+        return n.value
+
+    def read(i):
+        lay, cost = C.c_int(), C.c_double()
+        H.check(lib.qz_batch_tuning(b, i, C.byref(lay), C.byref(cost)))
+        return lay.value
+
+    extra = f"pusher.ab_order = {order}\n"
+    spec = _spec(nodes, f"electrons.ppc = {ppc}\n" + extra)
+    i = add(spec)
+    if with_filter:
+        add(_spec(33, "plasma.smooth_length = 0.05\n" + extra))
+    cands = tune.candidate_layouts(spec, with_filter)
+    assert read(i) in cands
+    glob = tune.plasma_per_slice(spec) > tune.REG_PARTICLES
+    for lay in range(8):
+        rc = lib.qz_batch_set_tuning(b, i, lay, 0.0)
+        if lay & 4 and not glob:
+            assert rc != 0
+        elif rc == 0:
+            assert read(i) == tune.used_layout(spec, lay, with_filter) and read(i) in cands
+        else:
+            assert glob or nodes > 512               # does not fit
+    H.check(lib.qz_batch_destroy(b))
