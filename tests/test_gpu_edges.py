@@ -7,9 +7,12 @@
 - the beam kernels: counts around a warp and around the largest call whose lanes add their own values (m = 0: 16384,
   with the push 8192; m = 1: 4096 and 128), all particles in one cell, a field store off the 16-byte boundary.
 
+- batches of every order.
+
 Tolerances: fields and diagnostics after one sweep max(1e-10, 4 x the reference algorithm's own round-off floor, the
-difference between its Thomas and partition solvers on the same input), per stored component; beam deposits 1e-12 and
-pushed particles 1e-13, as in test_gpu_parity.py."""
+difference between its Thomas and partition solvers on the same input), per stored component; components that vanish in
+the reference 1e-10 of the largest one; beam deposits 1e-12 and pushed particles 1e-13 as in test_gpu_parity.py, the
+momenta plus the rounding of the kicks."""
 import numpy as np
 import pytest
 
@@ -65,7 +68,10 @@ def _check_sweep(spec):
     Q.Sweep(Q.RadialGrid(spec.nodes), Q.sweep_params(spec)).run(bsrc, fld, diag)
     bad = {}
     for name, got, ra, rb in (("fld", fld.cpu().numpy(), a.fld(), b.fld()), ("diag", diag.cpu().numpy(), a.diag(), b.diag())):
+        top = np.max(np.abs(ra))
         for c in range(got.shape[-1]):
+            if not np.any(ra[..., c]) and not np.max(np.abs(got[..., c])) <= 1e-10 * top:
+                bad[f"{name}{c}"] = (np.max(np.abs(got[..., c])), top)
             if np.any(ra[..., c]):
                 e, floor = rel_l2(got[..., c], ra[..., c]), rel_l2(rb[..., c], ra[..., c])
                 if not e < max(1e-10, 4.0 * floor):
@@ -89,14 +95,46 @@ def test_sweep_m1_particles_over_a_cluster(nodes, ntheta):
     _check_sweep(_spec(nodes, f"modes = 1\nelectrons.ppc = 1\nelectrons.ntheta = {ntheta}\ndriver.x0 = 0.1\n"))
 
 
-@pytest.mark.parametrize("steps", [1, 9])
-def test_run_m1_teams(steps):
-    # two sweeps share clusters of 8 CTAs, ten of 4 (2040 particles per slice)
-    spec = _spec(256, "modes = 1\nelectrons.ppc = 1\nelectrons.ntheta = 8\ndriver.x0 = 0.1\n")
-    beams = [Q.sample_beam(b) for b in spec.beams]
-    mom = Q.Simulation(spec, beams=beams).run(steps, spec.dt)
+def _teams(steps):
+    # 2056 particles per slice: as many CTAs per sweep (8, 4, 2) as let every sweep have them at once, else one
+    spec = _spec(258, "modes = 1\nelectrons.ppc = 1\nelectrons.ntheta = 8\ndriver.x0 = 0.1\n")
+    return spec, [Q.sample_beam(b) for b in spec.beams]
+
+
+@pytest.mark.parametrize("steps,team", [(1, 8), (12, 4), (25, 2), (46, 1)])
+def test_run_m1_teams(steps, team):
+    spec, beams = _teams(steps)
+    sim = Q.Simulation(spec, beams=beams)
+    mom = sim.run(steps, spec.dt)
+    assert sim.schedule()["sweep_ctas"] == (steps + 1) * team
     ref = O.OracleSim(spec, beams=beams).run(steps, spec.dt)
     assert rel_l2(mom, np.asarray(ref).reshape(mom.shape)) < 1e-12
+
+
+def test_run_m1_team_gives_up_together():
+    # a wait of the team's first CTA that runs out (its limit is 100 ns) ends every CTA of the cluster, and the run with
+    # an error; the device is as usable as before
+    spec, beams = _teams(1)
+    sim = Q.Simulation(spec, beams=beams)
+    sim.set_schedule(True, timeout_s=1e-7)
+    with pytest.raises(Q.QZError, match="timed out"):
+        sim.run(1, spec.dt)
+    test_run_m1_teams(1, 8)
+
+
+@pytest.mark.parametrize("order", [1, 2, 4, 5])
+def test_batch_orders(order):
+    # plasma in registers and in global memory, up to and beyond 512 nodes, both modes
+    extra = f"pusher.ab_order = {order}\n"
+    specs = [_spec(65, extra), _spec(257, "electrons.ppc = 3\n" + extra), _spec(600, extra),
+             _spec(65, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\n" + extra)]
+    beams = [[Q.sample_beam(b) for b in s.beams] for s in specs]
+    batch = Q.Batch()
+    for s, bm in zip(specs, beams):
+        batch.add(s, bm)
+    for s, bm, mom in zip(specs, beams, batch.run(2, specs[0].dt)):
+        ref = O.OracleSim(s, beams=bm).run(2, s.dt)
+        assert rel_l2(mom, np.asarray(ref).reshape(mom.shape)) < 1e-12
 
 
 @pytest.mark.parametrize("modes", [0, 1])

@@ -126,8 +126,12 @@ ORDERS = [((), False), (range(16), True), (range(15, -1, -1), True), (range(8, 1
 
 
 @pytest.mark.parametrize("nodes,extra", [
-    (33, ""), (33, "electrons.ppc = 20\n"), (140, "plasma.smooth_length = 0.05\n"), (550, ""),
-    (550, "plasma.smooth_length = 0.05\n"),
+    (3, ""), (33, "beams.xi_shape = ngp\n"), (33, "electrons.ppc = 20\n"), (513, ""), (550, "electrons.ppc = 2\n"),
+    (300, "electrons.ppc = 3\npusher.ab_order = 5\n"),
+    (140, "plasma.smooth_length = 0.05\n"), (550, "plasma.smooth_length = 0.05\n"),
+    (65, "pusher.max_cells_per_step = 0.3\n"), (65, "pusher.max_cells_per_step = 0.3\nelectrons.ppc = 12\n"),
+    (9, "modes = 1\nelectrons.ntheta = 4\n"),
+    (130, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\nbeams.xi_shape = ngp\n"),
     (140, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\n"),
     (140, "modes = 1\nelectrons.ntheta = 4\ndriver.x0 = 0.1\nplasma.smooth_length = 0.05\n"),
 ])
