@@ -1102,7 +1102,7 @@ namespace {
 // 2 (sum over beams of max |w q|) / V_j / dxi (the weights of the particles do not change during a run;
 // |1 - v_z| <= 2 and every other factor is at most 1), so the quantum of node j is that bound / 2^B.
 // With at most n contributions per value (n = all beam particles, 2^nbits > n) the limbs split at
-// S = 53 - nbits and B = 2 S keep both limb sums integers below 2^53 (exact in FP64, beam_fx_add).
+// S = 53 - nbits and B = 2 S keep both limb sums integers below 2^53 (exact in FP64, beam_fx_split).
 // The run deposits exactly for m = 0 up to 2^25 particles (B >= 56: the quantum is at most 2^-56 of
 // the bound); m = 1 runs and larger beams keep FP64 reductions.
 // the node quanta for n contributions bounded by wq (sum over beams of max |w q|): every contribution to

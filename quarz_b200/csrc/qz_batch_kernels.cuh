@@ -17,7 +17,6 @@ namespace qzb {
 
 namespace {
 
-using beam_detail::deposit_one;
 using beam_detail::PState7;
 using beam_detail::push_one;
 using beam_detail::sums_add;
@@ -28,6 +27,14 @@ __device__ __forceinline__ unsigned long long batch_timer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
+}
+
+// one particle's deposit into the slot's beam sources
+__device__ __forceinline__ void batch_deposit(const BatchInst& I, const SweepArgs& A, const BeamArgs& B, double x, double y,
+                                              double px, double py, double pz, double xi, double w) {
+    double* const bsrc = const_cast<double*>(A.bsrc);
+    if (I.modes) beam_detail::deposit_one<B_NC1>(B, bsrc, x, y, px, py, pz, xi, w);
+    else beam_detail::deposit_one<B_NC0>(B, bsrc, x, y, px, py, pz, xi, w);
 }
 
 // beam work of one instance by the whole CTA: moments (step n) of every beam, then, when push,
@@ -64,7 +71,7 @@ __device__ void beam_phase(const BatchInst& I, const SweepArgs& A, const BatchAr
             sums_add(acc, p, I.gref[q], I.xiref[q]);
             if (!push) continue;
             if (I.rigid[q]) {
-                deposit_one(Bb, const_cast<double*>(A.bsrc), p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
+                batch_deposit(I, A, Bb, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
                 continue;
             }
             const bool alive = push_one<false>(Bb, A.fld, p, h, hs, B.dt);
@@ -73,7 +80,7 @@ __device__ void beam_phase(const BatchInst& I, const SweepArgs& A, const BatchAr
                 Bb.w[i] = 0.0;
                 continue;
             }
-            deposit_one(Bb, const_cast<double*>(A.bsrc), p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
+            batch_deposit(I, A, Bb, p.x, p.y, p.px, p.py, p.pz, p.xi, p.w);
         }
         // deterministic block reduction of the 17 sums
 #pragma unroll
@@ -104,7 +111,7 @@ __device__ void beam_deposit0(const BatchInst& I, const SweepArgs& A) {
         for (long i = tid; i < Bb.n; i += kT) {
             const double w = Bb.w[i];
             if (w == 0.0) continue;
-            deposit_one(Bb, const_cast<double*>(A.bsrc), Bb.x[i], Bb.y[i], Bb.px[i], Bb.py[i], Bb.pz[i], Bb.xi[i], w);
+            batch_deposit(I, A, Bb, Bb.x[i], Bb.y[i], Bb.px[i], Bb.py[i], Bb.pz[i], Bb.xi[i], w);
         }
     }
     __syncthreads();

@@ -123,9 +123,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_deposit_few_kernel(const Be
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B.n) return;
     const double wi = B.w[i];
-    DepOne<NC> D;
-    if (wi != 0.0 && dep_one<NC>(B, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi, -1, D))
-        lane_deposit<NC>(B, bsrc, D);
+    if (wi != 0.0) deposit_one<NC>(B, bsrc, B.x[i], B.y[i], B.px[i], B.py[i], B.pz[i], B.xi[i], wi);
 }
 
 // Bound by the L2 reductions (2 rows x 2 nodes x NC values per particle): 1e6 particles on 512 x 2400 nodes take
@@ -376,8 +374,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_push_deposit_few_kernel(con
     const double wi = B.w[i];
     if (wi == 0.0) return;
     const Moved m = move_one<kVec>(B, fld, i, 0.5 * (B.q / B.m) * dt_kick, dt);
-    DepOne<NC> D;
-    if (m.live && dep_one<NC>(B, m.x, m.y, m.px, m.py, m.pz, m.xi, wi, m.j, D)) lane_deposit<NC>(B, bsrc_next, D);
+    if (m.live) deposit_one<NC>(B, bsrc_next, m.x, m.y, m.px, m.py, m.pz, m.xi, wi, m.j);
 }
 
 // moment sums: fixed grid, fixed per-thread order, fixed tree -> deterministic
@@ -435,7 +432,8 @@ int grid_for(long n) {
     return (int)b;
 }
 
-// CTAs of a depositing kernel: as many as fit (at most 8 of 256 threads per SM)
+// CTAs of a depositing kernel: one pass for up to 8 x 256 particles per SM, more in further passes of the same CTAs (of
+// which an SM holds 6 of 256 threads, or 5 of 128 with mode 1: their shared scratch)
 template <int NC>
 int grid_dep(long n) {
     const long b = (n + kDepThreads<NC> - 1) / kDepThreads<NC>, cap = 148L * 8 * 256 / kDepThreads<NC>;

@@ -24,69 +24,6 @@ __device__ __forceinline__ double2 fload2(const double* p) {
     }
 }
 
-__device__ __forceinline__ void deposit_one(const BeamArgs& B, double* __restrict__ bsrc, double X, double Y,
-                                            double PX, double PY, double PZ, double XI, double wi) {
-    const double R = B.R;
-    const double r = sqrt(X * X + Y * Y);
-    if (r > R) return;
-    const double c = r > 0.0 ? X / r : 1.0, s = r > 0.0 ? Y / r : 0.0;
-    const double sx = (XI - B.xi_min) * B.idxi;
-    const int k = B.ngp ? (int)floor(sx + 0.5) : (int)floor(sx);
-    const int nloc = B.K;
-    if (k < -1 || k >= nloc) return;
-    const double tk = B.ngp ? 0.0 : sx - k;
-    const double p2 = PX * PX + PY * PY;
-    const double gam = sqrt(1.0 + p2 + PZ * PZ);
-    const double omvz = (1.0 + p2) / (gam * (gam + PZ));
-    const double vz = PZ / gam, vx = PX / gam, vy = PY / gam;
-    const double vr = c * vx + s * vy, vt = c * vy - s * vx;
-    int j;
-    double t;
-    weights(B.r, B.inv_h, B.N, R, r, j, t);
-    const double Wr[2] = {1.0 - t, t};
-    const double Wk[2] = {1.0 - tk, tk};
-    const double q = B.q;
-    const int nc = B.modes ? B_NC1 : B_NC0;
-    const int na = B.ngp ? 1 : 2;
-    for (int a = 0; a < na; ++a) {
-        const int kk = k + a;
-        if (kk < 0 || kk >= nloc) continue;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const int jj = j + b;
-            double* o = bsrc + ((size_t)kk * B.M + jj) * nc;
-            const double d = wi * q * Wk[a] * Wr[b] * B.inv_V[jj] * B.idxi;
-            if (B.fx_scale) {                       // exact (m = 0 runs of qz_sim)
-                const double sc = B.fx_scale[jj];
-                beam_fx_add(o + B_RT0, B.fx_lo, d * omvz, sc, B.fx_inv2s, B.fx_2s);
-                beam_fx_add(o + B_JZ0, B.fx_lo, d * vz, sc, B.fx_inv2s, B.fx_2s);
-                beam_fx_add(o + B_JP1R, B.fx_lo, d * vr, sc, B.fx_inv2s, B.fx_2s);
-                beam_fx_add(o + B_JP1I, B.fx_lo, d * vt, sc, B.fx_inv2s, B.fx_2s);
-                beam_fx_add(o + B_RHO0, B.fx_lo, d, sc, B.fx_inv2s, B.fx_2s);
-                continue;
-            }
-            atomicAdd(o + B_RT0, d * omvz);
-            atomicAdd(o + B_JZ0, d * vz);
-            atomicAdd(o + B_JP1R, d * vr);
-            atomicAdd(o + B_JP1I, d * vt);
-            atomicAdd(o + B_RHO0, d);
-            if (B.modes) {
-                atomicAdd(o + B_RT1R, d * omvz * c);
-                atomicAdd(o + B_RT1I, -d * omvz * s);
-                atomicAdd(o + B_JZ1R, d * vz * c);
-                atomicAdd(o + B_JZ1I, -d * vz * s);
-                atomicAdd(o + B_RHO1R, d * c);
-                atomicAdd(o + B_RHO1I, -d * s);
-                atomicAdd(o + B_JP0R, d * vx);
-                atomicAdd(o + B_JP0I, d * vy);
-                const double c2 = c * c - s * s, s2 = 2.0 * c * s;
-                atomicAdd(o + B_JP2R, d * (vx * c2 + vy * s2));
-                atomicAdd(o + B_JP2I, d * (vy * c2 - vx * s2));
-            }
-        }
-    }
-}
-
 // The deposit of one particle (src/Beam.cpp:725-785): its cell, weights, and the values f[c] that every corner
 // multiplies by its weight: B_NC0 or B_NC1 components, or (kDep0) the three the m = 0 sweep reads, rho - J_z, J_z
 // and J_theta (not the beam's J_r and rho; a field file deposits its beam density again). jguess: a nearby
@@ -125,9 +62,8 @@ __device__ __forceinline__ bool dep_one(const BeamArgs& B, double X, double Y, d
     D.d0 = wi * B.q;
     if constexpr (NC == kDep0) {
         D.f[0] = omvz; D.f[1] = vz; D.f[2] = vt;
-        return true;
     } else {
-    D.f[B_RT0] = omvz; D.f[B_JZ0] = vz; D.f[B_JP1R] = vr; D.f[B_JP1I] = vt; D.f[B_RHO0] = 1.0;
+        D.f[B_RT0] = omvz; D.f[B_JZ0] = vz; D.f[B_JP1R] = vr; D.f[B_JP1I] = vt; D.f[B_RHO0] = 1.0;
     }
     if constexpr (NC == B_NC1) {
         const double c2 = c * c - s * s, s2 = 2.0 * c * s;
@@ -167,6 +103,13 @@ __device__ __forceinline__ void lane_deposit(const BeamArgs& B, double* __restri
             }
         }
     }
+}
+
+template <int NC>
+__device__ __forceinline__ void deposit_one(const BeamArgs& B, double* __restrict__ bsrc, double X, double Y,
+                                            double PX, double PY, double PZ, double XI, double wi, int jguess = -1) {
+    DepOne<NC> D;
+    if (dep_one<NC>(B, X, Y, PX, PY, PZ, XI, wi, jguess, D)) lane_deposit<NC>(B, bsrc, D);
 }
 
 // The deposit of a warp's particles into compact m = 0 beam sources: kDep0 values per node, or (kExact) their
@@ -244,7 +187,7 @@ __device__ __forceinline__ void warp_deposit3(const BeamArgs& B, double* __restr
 
 // The part of the m = 1 deposit that the m = 1 sweep reads (rho - J_z, J_z and J_perp in modes 0 and 1,
 // J_perp also in mode 2; not the beam densities), per corner: deposit_setup1 takes the particle's cell,
-// weights and velocities once (deposit_one's m = 1 branch, src/Beam.cpp:725-785), deposit_corner1 the 12
+// weights and velocities once (as dep_one with mode 1, src/Beam.cpp:725-785), deposit_corner1 the 12
 // values of corner (row k + a, node j + b), deposit_add1 adds them with FP64 reductions.
 constexpr int kDep1 = 12;
 struct Dep1 {

@@ -38,16 +38,8 @@ enum DiagComp : int { D_PSI0 = 0, D_NE0, D_NI0, D_PSI1R, D_PSI1I, D_NE1R, D_NE1I
 // path here: with one reduction per value, a push task of the pipelined pinched-witness run took 251 us
 // with 64-bit integer reductions and 175 us with FP64 ones.)
 // The value is (2^S sum_hi + sum_lo) 2^qe_j.
-__device__ __forceinline__ void beam_fx_add(double* hi_p, long lo_off, double v, double scale, double inv2s,
-                                            double two_s) {
-    if (v == 0.0) return;
-    const double t = v * scale;
-    const double hi = floor(t * inv2s);
-    const double lo = rint(fma(-hi, two_s, t));           // fma exact: t - hi 2^S in [0, 2^S)
-    atomicAdd(hi_p, hi);
-    atomicAdd(hi_p + lo_off, lo);
-}
-// the two limbs of a contribution, added to the limbs of others
+//
+// beam_fx_split: the two limbs of a contribution, added to the limbs of others
 __device__ __forceinline__ void beam_fx_split(double v, double scale, double inv2s, double two_s, double& hi_sum,
                                               double& lo_sum) {
     const double t = v * scale;
