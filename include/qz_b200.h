@@ -132,8 +132,9 @@ qz_status qz_sweep_run_stage(qz_sweep* s, const double* bsrc_dev, const double* 
                              double* fld_dev, double* diag_dev, qz_plasma_state* out, qz_counters* counters_host,
                              void* stream);
 /* per-phase clock cycles of the last run, 16 counters: [0] prologue, [1] psi/E_z/B_z phase, [2] S+ deposit,
-   [3] B+ phase, [4] store + push + deposit, [5..8] parts of phase 1; enable = 1 turns the counters on for
-   later runs */
+   [3] B+ phase, [4] store + push + deposit; m = 0 also parts of phase 1, [5] the solves and [6] the next slice's
+   start values; [9..15] the phases of a reverse sweep (qz_sim_adjoint); enable = 1 turns the counters on for later
+   runs */
 qz_status qz_sweep_timing(qz_sweep* s, int enable, unsigned long long* cycles16_host);
 
 /* ------------------------------------------------------------------ beams

@@ -4,7 +4,7 @@
 
 namespace qzb {
 
-// EXT: the variant for decks with the smoothing filter or static (analytic) beam sources
+// EXT: the variant for decks with the smoothing filter, static (analytic) beam sources or adaptive sub-slicing (sweep_ext)
 template <int ORD, bool REG, int kMaxR, bool EXT>
 __global__ void __launch_bounds__(kSweepThreads, 1) sweep_m0_kernel(const SweepArgs A) {
     extern __shared__ double smem_raw[];

@@ -1634,9 +1634,9 @@ __device__ __forceinline__ void l0_block(const Smem& S, const Src& s, int M, int
         for (int e = 0; e < 3; ++e) cB[e] = fma(af, cB[e], rr * dv[u][e]);
         cA *= af;
     }
-                double yb[3];
+    double yb[3];
     scan_fwd<3>(cA, cB, yb, S.tot);
-                const double ypsi_prev = yb[0];                         // y of psi just before this thread's rows
+    const double ypsi_prev = yb[0];                        // y of psi just before this thread's rows
     double y[kMaxR][3];
 #pragma unroll
     for (int u = 0; u < kMaxR; ++u) {
@@ -1660,7 +1660,7 @@ __device__ __forceinline__ void l0_block(const Smem& S, const Src& s, int M, int
     }
     double xa[3];
     scan_bwd<3>(bA, bB, xa, S.tot + 8 * kW);
-                // psi on the window [row0 - 1, row0 + Rw]: the rows of this thread, x after them (the
+    // psi on the window [row0 - 1, row0 + Rw]: the rows of this thread, x after them (the
     // backward carry) and x before them, x_{row0-1} = y_{row0-1} - (c/u)_{row0-1} x_{row0}
     // with y_{row0-1} the forward carry -- so W+ = -psi' needs no further exchange
     double pw[kMaxR + 2];

@@ -27,40 +27,10 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_m1w_kernel(const Sweep
     sweep_m1_body<ORD, NoGate, EXT>(A, smem_raw, g, Team::of_cluster());
 }
 
-template <int ORD, bool EXT>
-cudaError_t launch_e(const SweepArgs& A, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(sweep_m1w_kernel<ORD, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    // the particles of a slice over a cluster of up to 8 CTAs (the smoothing filter works in place on the shared
-    // sources: one CTA); 8 is the largest portable size, and each CTA has at least a particle per thread then
-    int team = 1;
-    if (!A.filter)
-        while (team < 8 && A.np > team * kSweepThreads) team *= 2;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.blockDim = dim3(kSweepThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    for (;; team /= 2) {
-        at.val.clusterDim.x = team;
-        cfg.gridDim = dim3(team);
-        int fit = 0;                       // a device (partition) may not hold a cluster of this size
-        if (team > 1 && (cudaOccupancyMaxActiveClusters(&fit, sweep_m1w_kernel<ORD, EXT>, &cfg) != cudaSuccess || fit < 1)) {
-            cudaGetLastError();
-            continue;
-        }
-        return cudaLaunchKernelEx(&cfg, sweep_m1w_kernel<ORD, EXT>, A);
-    }
-}
-
 template <int ORD>
 cudaError_t launch_t(const SweepArgs& A, size_t smem, cudaStream_t stream) {
-    return (A.filter || A.bstat) ? launch_e<ORD, true>(A, smem, stream) : launch_e<ORD, false>(A, smem, stream);
+    return (A.filter || A.bstat) ? launch_team(sweep_m1w_kernel<ORD, true>, A, smem, stream)
+                                 : launch_team(sweep_m1w_kernel<ORD, false>, A, smem, stream);
 }
 }  // namespace
 
