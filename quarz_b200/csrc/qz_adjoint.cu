@@ -817,14 +817,14 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
     const AdjSm S = carve_adj(smem_raw, M, ORD);
     const double* q = A.consts;                     // stencils, 1/r, L0 Thomas, L1D and L1F rows (13 x M)
     const double *gm = q, *g0 = q + M, *gp = q + 2 * M, *ir = q + 3 * M;
+    const double *l0r = q + 4 * M, *l0f = q + 5 * M, *l0b = q + 6 * M;
     const double *l1a = q + 7 * M, *l1b = q + 8 * M, *l1c = q + 9 * M;
     const double *lfa = q + 10 * M, *lfb = q + 11 * M, *lfc = q + 12 * M;
     const int i = tid, lane = tid & 31;              // this thread's row
     const bool row = i < M;
-    // the solves: this thread's group of warps (l0_group, shifted_group; M <= kSweepThreads)
-    constexpr int kR2 = 5, kR4 = 3;
-    constexpr double two_pi = 6.283185307179586;
-    const int warp = tid >> 5, e2 = warp / kG2, wl2 = warp - e2 * kG2, sy4 = warp / kG4, wl4 = warp - sy4 * kG4;
+    // the B+ solves: this thread's group of warps (shifted_group; M <= kSweepThreads)
+    constexpr int kR4 = 3;
+    const int warp = tid >> 5, sy4 = warp / kG4, wl4 = warp - sy4 * kG4;
     if (row) {
         S.r[i] = A.r[i];
         S.iv[i] = A.inv_V[i];
@@ -1057,24 +1057,35 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
         if (row) S.t1[i] = -S.l_wpr[i];
         __syncthreads();
         {
-            // mu / V with d = lam / V; the weights w = V / 2 pi and 1 / g of the flux form
-            if (e2 < 3) {
-                const int R = group_rows(M, kG2), row0 = (wl2 * 32 + lane) * R;
-                double x[kR2], z0, xn;
-                l0_group<kR2>(S.tot, A.consts0 + 7 * (size_t)M, A.consts0 + 8 * (size_t)M, N, e2, wl2, R, row0,
-                              [&](int r) {
-                                  const double l = e2 == 0 ? S.l_bz[r]
-                                                           : (e2 == 1 ? grad_T_at(A, gm, g0, gp, S.t1, r) : S.l_ez[r]);
-                                  return l * S.iv[r];                  // (grad_T_at: lam of psi)
-                              },
-                              x, z0, xn);
-                // lam of the B_z right-hand side -(J_th' + J_th / r), of rho - J_z and of its xi-derivative
-                double* const out = e2 == 0 ? S.t0 : (e2 == 1 ? S.l_rhot : S.l_drho);
-#pragma unroll
-                for (int u = 0; u < kR2; ++u) {
-                    const int r = row0 + u;
-                    if (u < R && r < M) out[r] = r < N ? -(x[u] * (two_pi * A.consts0[7 * (size_t)M + r])) : -0.0;   // mu = x V
+            double d[3] = {0.0, 0.0, 0.0};
+            double af = 1.0, rr = 0.0, ab = 1.0;
+            if (row) {
+                af = l0f[i]; rr = l0r[i]; ab = l0b[i];
+                if (i < N) {
+                    d[0] = S.l_bz[i] * iVi;
+                    d[1] = grad_T_at(A, gm, g0, gp, S.t1, i) * iVi;   // lam of psi
+                    d[2] = S.l_ez[i] * iVi;
                 }
+            }
+            double cB[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) cB[e] = rr * d[e];
+            double yb[3];
+            scan_fwd<3>(af, cB, yb, S.tot + (par++ & 1) * 8 * kW);
+            double y[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) y[e] = row ? fma(af, yb[e], cB[e]) : 0.0;
+            double xa[3];
+            scan_bwd<3>(row ? ab : 1.0, y, xa, S.tot + (par++ & 1) * 8 * kW);
+            if (row) {
+                double mu[3] = {0.0, 0.0, 0.0};
+                if (i < N) {
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) mu[e] = fma(ab, xa[e], y[e]) * Vi;
+                }
+                S.t0[i] = -mu[0];                    // lam of the B_z right-hand side -(J_th' + J_th / r)
+                S.l_rhot[i] = -mu[1];
+                S.l_drho[i] = -mu[2];
             }
         }
         __syncthreads();
