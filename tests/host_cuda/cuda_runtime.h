@@ -2,8 +2,8 @@
 // and inline PTX) compile with g++ against this header, and a launch runs its blocks here. Every thread of a block
 // is a fiber that runs until a barrier, a warp vote or a shuffle and is resumed when the others have arrived. Which
 // warp goes first is chosen by emu::order: a missing barrier shows as a wrong result for an order that keeps a warp
-// back, an access out of range as a changed guard word or a fault of this process, a barrier that not all reach as
-// an abort. One launch after the other; a cluster's blocks run together, other blocks one after the other.
+// back, a write out of range as a changed guard word behind shared or allocated memory, a barrier that not all reach
+// as an abort. One launch after the other; a cluster's blocks run together, other blocks one after the other.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -171,8 +171,37 @@ inline cudaError_t cudaDeviceGetAttribute(int* v, int a, int) {
     return cudaSuccess;
 }
 extern long emu_mallocs, emu_copies;
-inline cudaError_t cudaMalloc(void** p, size_t n) { ++emu_mallocs; *p = std::calloc(1, n + 64); return cudaSuccess; }
-inline cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
+namespace emu {
+constexpr size_t kGuard = 4096;               // bytes on either side of an allocation, and behind shared memory
+constexpr unsigned char kGuardByte = 0xfd;    // (0xfdfd...: as a double a large negative number)
+inline void check_guard(const unsigned char* p, const char* what) {
+    for (size_t i = 0; i < kGuard; ++i)
+        if (p[i] != kGuardByte) {
+            std::fprintf(stderr, "emu: a write out of range, %s\n", what);
+            std::abort();
+        }
+}
+}  // namespace emu
+inline cudaError_t cudaMalloc(void** p, size_t n) {
+    ++emu_mallocs;
+    unsigned char* q = (unsigned char*)std::malloc(n + 2 * emu::kGuard + 64);
+    std::memcpy(q, &n, sizeof n);
+    std::memset(q + 64, emu::kGuardByte, emu::kGuard);
+    std::memset(q + 64 + emu::kGuard, 0, n);
+    std::memset(q + 64 + emu::kGuard + n, emu::kGuardByte, emu::kGuard);
+    *p = q + 64 + emu::kGuard;
+    return cudaSuccess;
+}
+inline cudaError_t cudaFree(void* p) {
+    if (!p) return cudaSuccess;
+    unsigned char* q = (unsigned char*)p - emu::kGuard - 64;
+    size_t n;
+    std::memcpy(&n, q, sizeof n);
+    emu::check_guard(q + 64, "before an allocation");
+    emu::check_guard((unsigned char*)p + n, "behind an allocation");
+    std::free(q);
+    return cudaSuccess;
+}
 inline cudaError_t cudaMemcpy(void* d, const void* s, size_t n, int) { ++emu_copies; std::memmove(d, s, n); return cudaSuccess; }
 inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, int k, cudaStream_t) { return cudaMemcpy(d, s, n, k); }
 inline cudaError_t cudaMemset(void* d, int v, size_t n) { std::memset(d, v, n); return cudaSuccess; }

@@ -82,7 +82,8 @@ void launch(dim3 grid, dim3 block, size_t smem, const std::function<void()>& fn,
             B.index = (int)b0 + c;
             B.warps.resize(nw);
             for (Warp& w : B.warps) std::memset(w.gen, 0, sizeof w.gen);
-            B.smem.assign(smem / sizeof(double) + 1, std::nan(""));     // shared memory starts undefined
+            B.smem.assign((smem + kGuard) / sizeof(double) + 1, std::nan(""));      // shared memory starts undefined
+            std::memset((char*)B.smem.data() + smem, kGuardByte, kGuard);
         }
         for (size_t i = 0; i < fibers.size(); ++i) {
             if (stacks.size() <= i) stacks.push_back((char*)std::aligned_alloc(64, kStack));
@@ -116,6 +117,7 @@ void launch(dim3 grid, dim3 block, size_t smem, const std::function<void()>& fn,
             }
             if (!any) break;
         }
+        for (const Block& B : blocks) check_guard((const unsigned char*)B.smem.data() + smem, "behind shared memory");
         for (const Fiber& f : fibers)
             if (!f.done) {
                 std::fprintf(stderr, "emu: thread %d of block %d waits for ever\n", f.tid, (int)b0 + f.block);

@@ -1,5 +1,6 @@
 """Kernels run on the host (host_kernels.py): what must hold whatever the inputs and the order of the warps, and what a
 GPU must not be given to find out."""
+import contextlib
 import ctypes as C
 
 import numpy as np
@@ -109,11 +110,18 @@ def _spec(nodes, extra=""):
     return spec
 
 
-def _sweep(spec):
-    s = C.c_void_p()
+@contextlib.contextmanager
+def _sweep(spec, change=lambda p: None):
+    lib, s, g = H.library(), C.c_void_p(), _grid(spec.nodes)
     p = Q.sweep_params(spec)
-    H.check(H.library().qz_sweep_create(_grid(spec.nodes), C.byref(p), C.byref(s)))
-    return s
+    change(p)
+    try:
+        H.check(lib.qz_sweep_create(g, C.byref(p), C.byref(s)))
+        yield s
+    finally:                                          # (freeing looks at the words around every allocation)
+        if s:
+            lib.qz_sweep_destroy(s)
+        lib.qz_grid_destroy(g)
 
 
 def _fields(spec):
@@ -147,11 +155,11 @@ def test_sweep_in_every_order_of_the_warps(nodes, extra):
     a.step_fields(0.0)
     b.step_fields(0.0)
     bsrc = np.ascontiguousarray(a.bsrc())
-    s = _sweep(spec)
     for first, keep in ORDERS:
         H.schedule(first, keep)
         fld, diag = _fields(spec)
-        H.check(H.library().qz_sweep_run(s, H.ptr(bsrc), H.ptr(fld), H.ptr(diag), None, None))
+        with _sweep(spec) as s:
+            H.check(H.library().qz_sweep_run(s, H.ptr(bsrc), H.ptr(fld), H.ptr(diag), None, None))
         for got, ra, rb in ((fld, a.fld(), b.fld()), (diag, a.diag(), b.diag())):
             for c in range(got.shape[-1]):
                 if np.any(ra[..., c]):
@@ -162,8 +170,8 @@ def test_sweep_in_every_order_of_the_warps(nodes, extra):
 def test_largest_grid(extra, most):
     # the widest grid that a CTA's shared memory holds: 160 bytes per node (192 with the filter) beside 2128 (5712) in
     # 232448; one node more is refused
-    with pytest.raises(RuntimeError, match=f"M = {most + 1} is too large"):
-        _sweep(_spec(most + 1, extra))
+    with pytest.raises(RuntimeError, match=f"M = {most + 1} is too large"), _sweep(_spec(most + 1, extra)):
+        pass
     test_sweep_in_every_order_of_the_warps(most, extra)
 
 
@@ -197,7 +205,8 @@ def test_plasma_beyond_the_range(n0, ppc):
     a.step_fields(0.0)
     bsrc, want, (fld, diag), cnt = np.ascontiguousarray(a.bsrc()), a.fld(), _fields(spec), L.Counters()
     H.schedule()
-    H.check(H.library().qz_sweep_run(_sweep(spec), H.ptr(bsrc), H.ptr(fld), H.ptr(diag), C.byref(cnt), None))
+    with _sweep(spec) as s:
+        H.check(H.library().qz_sweep_run(s, H.ptr(bsrc), H.ptr(fld), H.ptr(diag), C.byref(cnt), None))
     assert (cnt.lost, cnt.trapped, cnt.nonfinite) == (a.lost(), a.lost(), 0) and cnt.lost > 0
     top = np.max(np.abs(want))
     assert np.max(np.abs(fld / top - want / top)) < 1e-12
@@ -219,15 +228,16 @@ def test_removed_particles_keep_their_state(order, ppc):
     H.schedule()
     states = {}
     for K in range(3, spec.K + 1):
-        p = Q.sweep_params(spec)
-        p.K, p.max_qsa = K, 1.0 + 1e-3
-        s, n, npad, ord_ = C.c_void_p(), C.c_int(), C.c_int(), C.c_int()
-        H.check(lib.qz_sweep_create(_grid(spec.nodes), C.byref(p), C.byref(s)))
-        H.check(lib.qz_sweep_state_shape(s, C.byref(n), C.byref(npad), C.byref(ord_)))
-        out = np.zeros((6 + 5 * order, npad.value))
-        fld, diag = np.zeros((K, spec.M, 6)), np.zeros((K, spec.M, 3))
-        st = L.PlasmaState(out.ctypes.data, n.value, npad.value, order, 0)
-        H.check(lib.qz_sweep_run_stage(s, H.ptr(bsrc), None, None, H.ptr(fld), H.ptr(diag), C.byref(st), None, None))
+        def change(p):
+            p.K, p.max_qsa = K, 1.0 + 1e-3
+
+        n, npad, ord_ = C.c_int(), C.c_int(), C.c_int()
+        with _sweep(spec, change) as s:
+            H.check(lib.qz_sweep_state_shape(s, C.byref(n), C.byref(npad), C.byref(ord_)))
+            out = np.zeros((6 + 5 * order, npad.value))
+            fld, diag = np.zeros((K, spec.M, 6)), np.zeros((K, spec.M, 3))
+            st = L.PlasmaState(out.ctypes.data, n.value, npad.value, order, 0)
+            H.check(lib.qz_sweep_run_stage(s, H.ptr(bsrc), None, None, H.ptr(fld), H.ptr(diag), C.byref(st), None, None))
         states[K] = out[:, :n.value]
     seen = 0
     for K in range(3, spec.K):
