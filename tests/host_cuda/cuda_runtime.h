@@ -222,6 +222,8 @@ inline cudaError_t cudaGetDriverEntryPointByVersion(const char*, void**, unsigne
     return cudaErrorInvalidValue;
 }
 template <class F> cudaError_t cudaFuncSetAttribute(F, int, int) { return cudaSuccess; }
+template <class F> cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int*, F, int, size_t) { return cudaErrorInvalidValue; }
+inline cudaError_t cudaLaunchCooperativeKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaErrorInvalidValue; }
 template <class F> cudaError_t cudaOccupancyMaxActiveClusters(int* n, F, const cudaLaunchConfig_t*) { *n = 1; return cudaSuccess; }
 template <class K, class... A> cudaError_t cudaLaunchKernelEx(const cudaLaunchConfig_t* c, K k, const A&... a) {
     emu::launch(c->gridDim, c->blockDim, c->dynamicSmemBytes, [&] { k(a...); },

@@ -1,8 +1,8 @@
 """The CUDA kernels of quarz_b200/csrc compiled for the host, for tests of what a GPU must not be given to find out:
-accesses out of range and missing barriers. `library()` compiles the C ABI, the sweeps and the beam kernels with g++
+accesses out of range and missing barriers. `library()` compiles the C ABI, the sweeps, the beam and the adjoint kernels with g++
 against host_cuda/cuda_runtime.h (which runs a block's threads as fibers) and returns the ctypes library: the entry
 points of include/qz_b200.h on host memory (numpy arrays where a GPU caller passes device pointers), and
-`schedule()`, which warps run first. Adams-Bashforth orders 2 and 3 only; no pipelined, batched or adjoint runs.
+`schedule()`, which warps run first. Runs and adjoints go step by step: no pipelined or batched ones.
 """
 import ctypes as C
 import hashlib
@@ -17,7 +17,7 @@ import numpy as np
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "quarz_b200", "csrc")
 EMU = os.path.join(ROOT, "tests", "host_cuda")
-UNITS = ["qz_abi.cu", "qz_beam.cu", "qz_sweep.cu", "qz_sweep_m1.cu"]
+UNITS = ["qz_abi.cu", "qz_beam.cu", "qz_sweep.cu", "qz_sweep_m1.cu", "qz_adjoint.cu"]
 HEADERS = ["qz_device.cuh", "qz_internal.h", "qz_beam_body.cuh", "qz_sweep_body.cuh", "qz_sweep_m1_body.cuh"]
 # (PTX of the kernels, what the host does instead)
 PTX = [
@@ -32,6 +32,11 @@ PTX = [
     (r'asm volatile\("ld\.shared::cluster.*?\);\n',
      "v = *(const int*)((const char*)emu::dyn_smem_of(0) + ((const char*)p - (const char*)emu::dyn_smem()));\n"),
     (r"__cvta_generic_to_shared\(p\)", "0"),
+    # (the pipelined reverse pass is not run: a launch of it is an error)
+    (r'asm volatile\("ld\.acquire.*?\);\n', "v = *p;\n"),
+    (r'asm volatile\("st\.release.*?\);\n', "*p = v;\n"),
+    (r'asm volatile\("mov\.u64 %0, %%globaltimer;".*?\);\n', "t = 0;\n"),
+    (r"\b__noinline__\b", ""),
 ]
 
 

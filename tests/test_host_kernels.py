@@ -295,3 +295,40 @@ def test_batch_layouts_are_the_kernels(nodes, ppc, order, with_filter):
         else:
             assert glob or nodes > 512               # does not fit
     H.check(lib.qz_batch_destroy(b))
+
+
+def _sim(spec, beams):
+    lib, sim = H.library(), C.c_void_p()
+    p = Q.sweep_params(spec)
+    H.check(lib.qz_sim_create(_grid(spec.nodes), C.byref(p), C.byref(sim)))
+    for b, (parts, gref, xiref) in zip(spec.beams, beams):
+        a = np.ascontiguousarray(parts)
+        H.check(lib.qz_sim_add_beam(sim, a.ctypes.data_as(C.POINTER(C.c_double)), len(a), b.q, b.m, 0, gref, xiref))
+    H.check(lib.qz_sim_set_schedule(sim, 0, 0, 0, 0, 0.0))
+    return sim
+
+
+@pytest.mark.parametrize("nodes,extra", [(33, ""), (200, "pusher.ab_order = 2\n"), (65, "plasma.smooth_length = 0.05\n"),
+                                         (65, "beams.xi_shape = ngp\n"), (512, "pusher.ab_order = 5\n")])
+def test_adjoint_in_every_order_of_the_warps(nodes, extra):
+    # the reverse sweep like the forward, against the oracle's adjoint: 1e-8 per component as on the GPU
+    import oracle as O
+
+    lib, dp = H.library(), C.POINTER(C.c_double)
+    spec = _spec(nodes, "driver.nparticles = 300\n" + extra)
+    beams, T, dt = [Q.sample_beam(b) for b in spec.beams], 2, 5.0
+    mom0 = O.OracleSim(spec, beams=beams).run(T, dt)
+    seeds = np.random.default_rng(5).normal(size=(1, 17)) / (np.abs(mom0[-1]) + 1e-30)
+    seeds[:, 16] = 0.0
+    ref, _ = O.OracleSim(spec, beams=beams).adjoint(T, dt, seeds)
+    for first, keep in ORDERS:
+        H.schedule(first, keep)
+        sim = _sim(spec, beams)
+        lam, mom, ms = np.zeros((7, len(beams[0][0]))), np.zeros((T + 1, 1, 17)), np.zeros(2)
+        out = (C.c_void_p * 1)(lam.ctypes.data)
+        H.check(lib.qz_sim_adjoint(sim, T, dt, seeds.ctypes.data_as(dp), out, mom.ctypes.data_as(dp),
+                                   ms.ctypes.data_as(dp), None))
+        H.check(lib.qz_sim_destroy(sim))
+        for c in range(7):
+            want = ref[0][:, c]
+            assert np.linalg.norm(lam[c] - want) <= 1e-8 * np.linalg.norm(want), (list(first), c)
