@@ -88,8 +88,9 @@ def _config(spec, nb_total, steps, extra=None, workload=WORKLOAD):
     c = {"workload": workload, "modes": spec.modes, "radial_nodes": spec.M, "xi_slices": spec.K,
          "dxi": spec.dxi, "plasma_ppc": spec.species[0].ppc, "plasma_particles_per_slice": spec.M - 1,
          "beam_particles": nb_total, "ab_order": spec.ab_order, "dt": spec.dt, "time_steps_per_run": steps,
-         "l2": "inputs larger than L2: beams 112 MB + a field store of 59 MB and beam sources of 49 MB per step "
-               "in flight (rings of one slot per step)",
+         "l2": f"inputs larger than L2: beams {56e-6 * nb_total:.0f} MB + a field store of "
+               f"{8e-6 * spec.K * spec.M * (18 if spec.modes else 6):.0f} MB and beam sources of "
+               f"{8e-6 * spec.K * spec.M * (15 if spec.modes else 6):.0f} MB per step in flight (rings of one slot per step)",
          "parallelism": "replicas"}
     if getattr(spec, "smooth_length", 0.0):
         c["smooth_length"] = spec.smooth_length
