@@ -9,8 +9,8 @@
 //
 // The reverse sweep runs the slices from the tail to the head in one CTA, one radial row and one
 // plasma particle per thread, with the plasma state of every slice recorded by the forward sweep of
-// the same step (SweepArgs::traj). Its transposed tridiagonal solves reuse the forward's factorised
-// scans: each operator L (L0, L1D - chi, L1F - chi) becomes symmetric when its interior rows are
+// the same step (SweepArgs::traj). Its transposed tridiagonal solves reuse the forward's factors and
+// solves: each operator L (L0, L1D - chi, L1F - chi) becomes symmetric when its interior rows are
 // scaled by a diagonal F (L0 = D^-1 S with D = V / 2pi; F = r dV for the fv_rows operators), so
 // L^-T lam = F L^-1 (F^-1 lam) on the non-Dirichlet rows, and the Dirichlet rows carry no adjoint.
 // Particle removal, cell changes and clamps are piecewise constant: their derivative is zero.
@@ -360,7 +360,7 @@ struct AdjSm {
     double *l_wpr, *l_ez, *l_bz, *l_bpr, *l_bpi;    // adjoints of the fields
     double *l_rhot, *l_drho, *l_jz, *l_chi, *l_jpi, *l_Sr, *l_Si;   // adjoints of the sources
     double *t0, *t1;                                // scratch
-    double* tot;                                    // scan scratch (2 x 8 x kW = kTot)
+    double* tot;                                    // scratch of the block scans (2 x 8 x kW); the B+ groups use kTot of it
     // particle adjoints ((5 + 5 ord) x kSweepThreads), no more than the order needs: what shared memory leaves is
     // the L1 that holds this large body's spilled registers
     double* lam;
@@ -1053,7 +1053,9 @@ __device__ bool sweep_back_body(const SweepArgs& A, const double* __restrict__ t
         }
         __syncthreads();
         ADJ_MARK(3);
-        // ---- psi (W+ = -psi'), E_z, B_z: three L0 systems, mu = V L0^-1 (lam / V) on rows < N
+        // ---- psi (W+ = -psi'), E_z, B_z: three L0 systems, mu = V L0^-1 (lam / V) on rows < N. Block scans, one row per
+        // thread: the operator comes from global memory here (the particle adjoints have the shared memory), and a
+        // group's threads with several consecutive rows each read it uncoalesced: 7,200 cycles, 15,800 by groups of warps
         if (row) S.t1[i] = -S.l_wpr[i];
         __syncthreads();
         {
